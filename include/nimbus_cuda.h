@@ -1041,20 +1041,18 @@ int nimbus_cuda_engine_lanes(const nimbus_engine* e);
  * step.
  *   NIMBUS_ACOUSTIC_TABLE  one thread per cell, each member's parameters and
  *                          buffers read from the member table in HBM;
- *   NIMBUS_ACOUSTIC_CONST  one thread per cell, each lane's members' constants
- *                          passed as one kernel parameter (the constant bank),
- *                          only the rotating buffers read from the table
- *                          (the continuity pass's default; lanes of more than
- *                          64 members fall back to the table form);
+ *   NIMBUS_ACOUSTIC_CONST  four vertically adjacent cells per thread, each
+ *                          lane's members' constants passed as one kernel
+ *                          parameter (the constant bank), only the rotating
+ *                          buffers read from the table (both passes' default;
+ *                          lanes of more than 64 members fall back to the
+ *                          table form);
  *   NIMBUS_ACOUSTIC_MARCH  one thread advances nimbus_cuda_engine_set_march
  *                          consecutive cells of a row along x (default 16),
  *                          neighbour data of the previous cell carried over in
- *                          registers (the momentum pass's default);
- *   NIMBUS_ACOUSTIC_PAIR   the constant-bank form with two vertically
- *                          adjacent cells per thread (in members with an even
- *                          nz the pair's values are one 8-byte load per field
- *                          and neighbour; both cells' loads are issued before
- *                          either's arithmetic);
+ *                          registers;
+ *   NIMBUS_ACOUSTIC_PAIR   accepted and run as NIMBUS_ACOUSTIC_CONST, whose
+ *                          four cells per thread replaced the two of this form;
  *   NIMBUS_ACOUSTIC_BULK   the constant-bank form with each 256-cell tile's
  *                          stencil data staged in shared memory by bulk
  *                          copies (cp.async.bulk on an mbarrier, four tiles in

@@ -320,7 +320,7 @@ __device__ __forceinline__ void bc_vertical_column(const BoundaryParams& B, floa
 {
     const Dims d = B.d;
     {
-        const int base = col * d.nz;
+        const int base = col * d.pz;
         if (B.bottom == kBottomNoSlip)
         {
             u[base] = 0.0f;

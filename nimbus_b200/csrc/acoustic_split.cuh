@@ -17,36 +17,23 @@
 namespace nimbus
 {
 
-// Retained-flux update from an already loaded slot value.  Reference policy:
-// the FP64 weighted sum rounded once to the FP32 slot (fused_accumulate);
-// FP32 policy: one FMA (retain_flux_f32).  With store the slot starts from
-// zero -- the first substep of a large step writes instead of accumulating,
-// bit-identical to accumulating into a zeroed slot (the 0.0 + product turns a
-// -0.0 into +0.0 exactly as the add would).
+// Retained-flux update from an already loaded slot value; returns the slot's
+// new value.  Reference policy: the FP64 weighted sum rounded once to the FP32
+// slot (fused_accumulate); FP32 policy: one FMA (retain_flux_f32).  With store
+// the slot starts from zero -- the first substep of a large step writes
+// instead of accumulating, bit-identical to accumulating into a zeroed slot
+// (the 0.0 + product turns a -0.0 into +0.0 exactly as the add would).  A
+// non-finite sum keeps the old value (zero with store) and raises the flag.
 template <class Policy>
-__device__ __forceinline__ void retain_flux_from(float* slot, float old, const FusedParams& P, double flux64,
-                                                 float flux32, unsigned& flags, bool store)
+__device__ __forceinline__ float retained_flux(float old, const FusedParams& P, double flux64, float flux32,
+                                               unsigned& flags, bool store)
 {
-    if constexpr (Policy::exact_pow)
-    {
-        const float st = (float)((store ? 0.0 : (double)old) + P.weight * flux64);
-        if (isfinite(st)) *slot = st;
-        else
-        {
-            if (store) *slot = 0.0f;
-            flags |= kStatusNonfiniteMassFlux;
-        }
-    }
-    else
-    {
-        const float st = __fmaf_rn(P.weight_f, flux32, store ? 0.0f : old);
-        if (isfinite(st)) *slot = st;
-        else
-        {
-            if (store) *slot = 0.0f;
-            flags |= kStatusNonfiniteMassFlux;
-        }
-    }
+    float st;
+    if constexpr (Policy::exact_pow) st = (float)((store ? 0.0 : (double)old) + P.weight * flux64);
+    else st = __fmaf_rn(P.weight_f, flux32, store ? 0.0f : old);
+    if (isfinite(st)) return st;
+    flags |= kStatusNonfiniteMassFlux;
+    return store ? 0.0f : old;
 }
 
 // The old-state neighbourhood one cell's continuity reads: density at the
@@ -61,11 +48,119 @@ struct ContinuityStencil
     float mx, my, mz;
 };
 
-// Continuity, rho forward Euler and EOS of cell c = (i, j, k) from its loaded
-// stencil: the retained fluxes of its three upper faces (written when
-// store_flux, else accumulated), the new density into rho_out[c] and the
-// pressure into p_out[c].  Every way of loading the stencil (one thread per
-// cell, or marching along i) ends here, so the arithmetic is one sequence.
+// The parts of one cell's continuity.  Every way of loading the stencil (one
+// thread per cell, four cells per thread, or marching along i) goes through
+// these, so the arithmetic is one sequence.
+
+// Retained flux of the upper x- or y-face: density at the cell and beyond the
+// face, the face's velocity, the frame's.
+template <class Policy>
+__device__ __forceinline__ float retained_lateral(const FusedParams& P, float old, float rc, float rp, float vel,
+                                                  double frame, float frame_f, unsigned& flags, bool store)
+{
+    if constexpr (Policy::exact_pow)
+        return retained_flux<Policy>(old, P, 0.5 * ((double)rc + (double)rp) * ((double)vel - frame), 0.0f, flags,
+                                     store);
+    else
+        return retained_flux<Policy>(old, P, 0.0, 0.5f * (rc + rp) * (vel - frame_f), flags, store);
+}
+
+// Retained flux of the upper z-face (the lid's own under an open top, else 0).
+template <class Policy>
+__device__ __forceinline__ float retained_vertical(const FusedParams& P, float old, float rc, float rp, float wc,
+                                                   bool zhi, unsigned& flags, bool store)
+{
+    if constexpr (Policy::exact_pow)
+    {
+        const double r = (double)rc;
+        const double zf = !zhi ? (P.top_open ? r * (double)wc : 0.0) : 0.5 * (r + (double)rp) * (double)wc;
+        return retained_flux<Policy>(old, P, zf, 0.0f, flags, store);
+    }
+    else
+    {
+        const float zf = !zhi ? (P.top_open ? rc * wc : 0.0f) : 0.5f * (rc + rp) * wc;
+        return retained_flux<Policy>(old, P, 0.0, zf, flags, store);
+    }
+}
+
+// Mass leaving through the upper face less mass entering through the lower.
+template <class real>
+__device__ __forceinline__ real flux_difference(float rc, float rp, float rm, float vp, float vm)
+{
+    const real half = (real)0.5;
+    const real r = (real)rc;
+    const real pos = half * (r + (real)rp) * (real)vp;
+    const real neg = half * ((real)rm + r) * (real)vm;
+    return pos - neg;
+}
+
+template <class real>
+__device__ __forceinline__ real flux_difference_z(float rc, float rp, float rm, float wp, float wm, bool zlo, bool zhi)
+{
+    const real half = (real)0.5;
+    const real r = (real)rc;
+    const real pos = zhi ? half * (r + (real)rp) * (real)wp : r * (real)wp;
+    const real neg = zlo ? half * ((real)rm + r) * (real)wm : (real)0;
+    return pos - neg;
+}
+
+// The stored continuity tendency from the three differences.
+template <class Policy>
+__device__ __forceinline__ float continuity_tendency(const FusedParams& P, typename Policy::real dx,
+                                                     typename Policy::real dy, typename Policy::real dz)
+{
+    if constexpr (Policy::exact_pow) return (float)finite_or_zero(-(dx * P.inv_dx + dy * P.inv_dy + dz * P.inv_dz));
+    else
+    {
+        const float drho = -(dx * P.inv_dx_f + dy * P.inv_dy_f + dz * P.inv_dz_f);
+        return isfinite(drho) ? drho : 0.0f;
+    }
+}
+
+// What one cell's continuity forms: the stored tendency, the new density and
+// pressure and the retained fluxes of its three upper faces (meaningful where
+// the face exists: i < nx-1, j < ny-1, every k).
+struct ContinuityResult
+{
+    float drho, rho, p;
+    float mx, my, mz;
+};
+
+// Continuity, rho forward Euler and EOS of cell (i, j, k) from its loaded
+// stencil; with flux the retained fluxes are written (store_flux) or
+// accumulated.
+template <class Policy>
+__device__ __forceinline__ ContinuityResult continuity_eos_point(const FusedParams& P, const ContinuityStencil& s,
+                                                                 bool xlo, bool xhi, bool ylo, bool yhi, int k,
+                                                                 const double* __restrict__ rho0,
+                                                                 const float4* __restrict__ eos0, bool flux,
+                                                                 unsigned& flags, bool store_flux)
+{
+    using real = typename Policy::real;
+    const bool zlo = k > 0, zhi = k + 1 < P.d.nz;
+    ContinuityResult o;
+    o.mx = s.mx;
+    o.my = s.my;
+    o.mz = s.mz;
+    if (flux)
+    {
+        if (xhi)
+            o.mx = retained_lateral<Policy>(P, s.mx, s.rho_c, s.rxp, s.uc, P.frame_u, P.frame_u_f, flags, store_flux);
+        if (yhi)
+            o.my = retained_lateral<Policy>(P, s.my, s.rho_c, s.ryp, s.vc, P.frame_v, P.frame_v_f, flags, store_flux);
+        o.mz = retained_vertical<Policy>(P, s.mz, s.rho_c, s.rzp, s.wc, zhi, flags, store_flux);
+    }
+    o.drho = 0.0f;
+    if (xlo && xhi && ylo && yhi)
+        o.drho = continuity_tendency<Policy>(P, flux_difference<real>(s.rho_c, s.rxp, s.rxm, s.uc, s.uxm),
+                                             flux_difference<real>(s.rho_c, s.ryp, s.rym, s.vc, s.vym),
+                                             flux_difference_z<real>(s.rho_c, s.rzp, s.rzm, s.wc, s.wzm, zlo, zhi));
+    o.rho = substep_density<Policy>(P, s.rho_c, o.drho, rho0, k);
+    o.p = substep_pressure<Policy>(P, eos0, k, o.rho, s.th);
+    return o;
+}
+
+// continuity_eos_point of cell c = (i, j, k), stored.
 template <class Policy>
 __device__ __forceinline__ void continuity_eos_values(const FusedParams& P, const ContinuityStencil& s, int i, int j,
                                                       int k, int c, const double* __restrict__ rho0,
@@ -75,64 +170,21 @@ __device__ __forceinline__ void continuity_eos_values(const FusedParams& P, cons
                                                       float* __restrict__ mfz, unsigned& flags, bool store_flux,
                                                       float* __restrict__ rho_copy)
 {
-    using real = typename Policy::real;
     const Dims d = P.d;
-    const bool xlo = i >= 1, xhi = i < d.nx - 1, ylo = j >= 1, yhi = j < d.ny - 1;
-    const bool zlo = k > 0, zhi = k + 1 < d.nz;
-    const float rho_c = s.rho_c;
+    const bool xhi = i < d.nx - 1, yhi = j < d.ny - 1;
     const bool flux = mfx != nullptr;
-
-    if (rho_copy != nullptr) rho_copy[c] = rho_c;
+    if (rho_copy != nullptr) rho_copy[c] = s.rho_c;
+    const ContinuityResult o =
+        continuity_eos_point<Policy>(P, s, i >= 1, xhi, j >= 1, yhi, k, rho0, eos0, flux, flags, store_flux);
     if (flux)
     {
-        if constexpr (sizeof(real) == 8)
-        {
-            const double rc = (double)rho_c;
-            if (xhi)
-                retain_flux_from<Policy>(mfx + c, s.mx, P, 0.5 * (rc + (double)s.rxp) * ((double)s.uc - P.frame_u),
-                                         0.0f, flags, store_flux);
-            if (yhi)
-                retain_flux_from<Policy>(mfy + c, s.my, P, 0.5 * (rc + (double)s.ryp) * ((double)s.vc - P.frame_v),
-                                         0.0f, flags, store_flux);
-            const double zf =
-                !zhi ? (P.top_open ? rc * (double)s.wc : 0.0) : 0.5 * (rc + (double)s.rzp) * (double)s.wc;
-            retain_flux_from<Policy>(mfz + c, s.mz, P, zf, 0.0f, flags, store_flux);
-        }
-        else
-        {
-            if (xhi)
-                retain_flux_from<Policy>(mfx + c, s.mx, P, 0.0, 0.5f * (rho_c + s.rxp) * (s.uc - P.frame_u_f), flags,
-                                         store_flux);
-            if (yhi)
-                retain_flux_from<Policy>(mfy + c, s.my, P, 0.0, 0.5f * (rho_c + s.ryp) * (s.vc - P.frame_v_f), flags,
-                                         store_flux);
-            const float zf = !zhi ? (P.top_open ? rho_c * s.wc : 0.0f) : 0.5f * (rho_c + s.rzp) * s.wc;
-            retain_flux_from<Policy>(mfz + c, s.mz, P, 0.0, zf, flags, store_flux);
-        }
+        if (xhi) mfx[c] = o.mx;
+        if (yhi) mfy[c] = o.my;
+        mfz[c] = o.mz;
     }
-    real drho = (real)0;
-    if (xlo && xhi && ylo && yhi)
-    {
-        const real rc = (real)rho_c;
-        const real half = (real)0.5;
-        const real fx_pos = half * (rc + (real)s.rxp) * (real)s.uc;
-        const real fx_neg = half * ((real)s.rxm + rc) * (real)s.uxm;
-        const real fy_pos = half * (rc + (real)s.ryp) * (real)s.vc;
-        const real fy_neg = half * ((real)s.rym + rc) * (real)s.vym;
-        const real fz_pos = zhi ? half * (rc + (real)s.rzp) * (real)s.wc : rc * (real)s.wc;
-        const real fz_neg = zlo ? half * ((real)s.rzm + rc) * (real)s.wzm : (real)0;
-        if constexpr (sizeof(real) == 8)
-            drho = -((fx_pos - fx_neg) * P.inv_dx + (fy_pos - fy_neg) * P.inv_dy + (fz_pos - fz_neg) * P.inv_dz);
-        else
-            drho = -((fx_pos - fx_neg) * P.inv_dx_f + (fy_pos - fy_neg) * P.inv_dy_f + (fz_pos - fz_neg) * P.inv_dz_f);
-    }
-    float drho_stored;
-    if constexpr (sizeof(real) == 8) drho_stored = (float)finite_or_zero(drho);
-    else drho_stored = isfinite(drho) ? drho : 0.0f;
-    if (drho_out != nullptr) drho_out[c] = drho_stored;
-    const float rho_stored = substep_density<Policy>(P, rho_c, drho_stored, rho0, k);
-    rho_out[c] = rho_stored;
-    p_out[c] = substep_pressure<Policy>(P, eos0, k, rho_stored, s.th);
+    if (drho_out != nullptr) drho_out[c] = o.drho;
+    rho_out[c] = o.rho;
+    p_out[c] = o.p;
 }
 
 // Loads cell c = (i, j, k)'s continuity stencil (acc: the stored retained-flux
@@ -188,6 +240,7 @@ __device__ __forceinline__ void continuity_eos_cell(const FusedParams& P, const 
 {
     int i, j, k;
     decompose(P.d, c, i, j, k);
+    if (k >= P.d.nz) return;
     const ContinuityStencil s =
         continuity_load(P.d, rho, u, v, w, theta, mfx, mfy, mfz, mfx != nullptr && !store_flux, c, i, j, k);
     continuity_eos_values<Policy>(P, s, i, j, k, c, rho0, eos0, rho_out, p_out, drho_out, mfx, mfy, mfz, flags,
@@ -198,7 +251,7 @@ __device__ __forceinline__ void continuity_eos_cell(const FusedParams& P, const 
 // x, marching in i: the density of planes i-1, i and the x-velocity of plane
 // i-1 carry over in registers from the previous cell, so a cell loads one new
 // x-neighbour instead of three, and its neighbour offsets and boundary flags
-// in j and k are formed once per row.  q = j nz + k.
+// in j and k are formed once per row.  q = j pz + k.
 template <class Policy>
 __device__ __forceinline__ void continuity_eos_march(const FusedParams& P, const float* __restrict__ rho,
                                                      const float* __restrict__ u, const float* __restrict__ v,
@@ -212,7 +265,7 @@ __device__ __forceinline__ void continuity_eos_march(const FusedParams& P, const
 {
     const Dims d = P.d;
     const int sx = d.sx();
-    const int oyp = j < d.ny - 1 ? d.nz : 0, oym = j >= 1 ? -d.nz : 0;
+    const int oyp = j < d.ny - 1 ? d.sy() : 0, oym = j >= 1 ? -d.sy() : 0;
     const int ozp = k + 1 < d.nz ? 1 : 0, ozm = k > 0 ? -1 : 0;
     const bool acc = mfx != nullptr && !store_flux;
     int c = i0 * sx + q;
@@ -317,17 +370,14 @@ struct MomentumStencil
     float uc, vc, wc;
 };
 
-// Momentum forward Euler of the faces of cell c = (i, j, k) from its loaded
-// stencil (see momentum_cell).
+// The new face velocities of cell (i, j, k) from its loaded stencil (interior:
+// 1 <= i < nx-1, 1 <= j < ny-1, k < nz-1; elsewhere only the clamp acts).
 template <class Policy>
-__device__ __forceinline__ void momentum_values(const FusedParams& P, const MomentumStencil& s, int i, int j, int k,
-                                                int c, const double* __restrict__ p0,
-                                                const float2* __restrict__ dp0_split, float* u_out, float* v_out,
-                                                float* w_out, int fuse_vertical)
+__device__ __forceinline__ float3 momentum_point(const FusedParams& P, const MomentumStencil& s, bool interior, int k,
+                                                 const double* __restrict__ p0,
+                                                 const float2* __restrict__ dp0_split)
 {
     using real = typename Policy::real;
-    const Dims d = P.d;
-    const bool interior = i >= 1 && i < d.nx - 1 && j >= 1 && j < d.ny - 1 && k < d.nz - 1;
     float du = 0.0f, dv = 0.0f, dw = 0.0f;
     if constexpr (sizeof(real) == 8)
     {
@@ -343,17 +393,15 @@ __device__ __forceinline__ void momentum_values(const FusedParams& P, const Mome
             dv = (float)finite_or_zero(-((double)s.py - pcd) * P.inv_dy / safe_rho(rho_y));
             dw = (float)finite_or_zero(-((((double)s.pz - pcd) * P.inv_dz) - dp0_dz) / safe_rho(rho_z));
         }
-        momentum_store(d, i, j, k, c, fuse_vertical,
-                       clamp_value((float)((double)s.uc + (double)du * P.dt_small), 0.0f, -P.wind_h, P.wind_h),
-                       clamp_value((float)((double)s.vc + (double)dv * P.dt_small), 0.0f, -P.wind_h, P.wind_h),
-                       clamp_value((float)((double)s.wc + (double)dw * P.dt_small), 0.0f, -P.wind_v, P.wind_v),
-                       u_out, v_out, w_out);
+        return make_float3(clamp_value((float)((double)s.uc + (double)du * P.dt_small), 0.0f, -P.wind_h, P.wind_h),
+                           clamp_value((float)((double)s.vc + (double)dv * P.dt_small), 0.0f, -P.wind_h, P.wind_h),
+                           clamp_value((float)((double)s.wc + (double)dw * P.dt_small), 0.0f, -P.wind_v, P.wind_v));
     }
     else
     {
-        const float2 dp0 = dp0_split[k];
         if (interior)
         {
+            const float2 dp0 = dp0_split[k];
             const float rho_x = 0.5f * (s.rc + s.rx);
             const float rho_y = 0.5f * (s.rc + s.ry);
             const float rho_z = 0.5f * (s.rc + s.rz);
@@ -369,10 +417,23 @@ __device__ __forceinline__ void momentum_values(const FusedParams& P, const Mome
             dw = isfinite(cz) ? cz : 0.0f;
         }
         const float dt = P.dt_f;
-        momentum_store(d, i, j, k, c, fuse_vertical, clamp_value(__fmaf_rn(du, dt, s.uc), 0.0f, -P.wind_h, P.wind_h),
-                       clamp_value(__fmaf_rn(dv, dt, s.vc), 0.0f, -P.wind_h, P.wind_h),
-                       clamp_value(__fmaf_rn(dw, dt, s.wc), 0.0f, -P.wind_v, P.wind_v), u_out, v_out, w_out);
+        return make_float3(clamp_value(__fmaf_rn(du, dt, s.uc), 0.0f, -P.wind_h, P.wind_h),
+                           clamp_value(__fmaf_rn(dv, dt, s.vc), 0.0f, -P.wind_h, P.wind_h),
+                           clamp_value(__fmaf_rn(dw, dt, s.wc), 0.0f, -P.wind_v, P.wind_v));
     }
+}
+
+// momentum_point of cell c = (i, j, k), stored (see momentum_store).
+template <class Policy>
+__device__ __forceinline__ void momentum_values(const FusedParams& P, const MomentumStencil& s, int i, int j, int k,
+                                                int c, const double* __restrict__ p0,
+                                                const float2* __restrict__ dp0_split, float* u_out, float* v_out,
+                                                float* w_out, int fuse_vertical)
+{
+    const Dims d = P.d;
+    const bool interior = i >= 1 && i < d.nx - 1 && j >= 1 && j < d.ny - 1 && k < d.nz - 1;
+    const float3 n = momentum_point<Policy>(P, s, interior, k, p0, dp0_split);
+    momentum_store(d, i, j, k, c, fuse_vertical, n.x, n.y, n.z, u_out, v_out, w_out);
 }
 
 // Loads cell c = (i, j, k)'s momentum stencil; outside the interior the
@@ -407,13 +468,14 @@ __device__ __forceinline__ void momentum_cell(const FusedParams& P, const float*
 {
     int i, j, k;
     decompose(P.d, c, i, j, k);
+    if (k >= P.d.nz) return;
     const MomentumStencil s = momentum_load(P.d, rho, p, u, v, w, c, i, j, k);
     momentum_values<Policy>(P, s, i, j, k, c, p0, dp0_split, u_out, v_out, w_out, fuse_vertical);
 }
 
 // The same momentum for the cells (i0 .. i1-1, j, k) of one row along x,
 // marching in i: the new density and pressure of plane i+1 loaded for cell i
-// are those of cell i+1, so they carry over in registers.  q = j nz + k.
+// are those of cell i+1, so they carry over in registers.  q = j pz + k.
 template <class Policy>
 __device__ __forceinline__ void momentum_march(const FusedParams& P, const float* __restrict__ rho,
                                                const float* __restrict__ p, const double* __restrict__ p0,
@@ -422,7 +484,7 @@ __device__ __forceinline__ void momentum_march(const FusedParams& P, const float
 {
     const Dims d = P.d;
     const int sx = d.sx();
-    const int oy = j < d.ny - 1 ? d.nz : 0, oz = k < d.nz - 1 ? 1 : 0;
+    const int oy = j < d.ny - 1 ? d.sy() : 0, oz = k < d.nz - 1 ? 1 : 0;
     int c = i0 * sx + q;
     float rc = rho[c], pc = p[c];
     for (int i = i0; i < i1; ++i, c += sx)
@@ -446,94 +508,213 @@ __device__ __forceinline__ void momentum_march(const FusedParams& P, const float
     }
 }
 
-// ---- Two vertically adjacent cells per thread ------------------------------
-// Cells c and c + 1 with c even, of a grid whose nz is even: both lie in one
-// column (k even, k + 1 <= nz - 1), share i and j, and every field's values at
-// the pair and at the pair shifted by +-sx or +-sy are one aligned 8-byte load
-// (member fields start on 256-byte boundaries; sx and sy are even).  Each
-// cell's stencil holds the values the one-cell loads give wherever its
-// arithmetic reads them (a neighbour outside the grid or the interior may
-// hold another in-range value), and its arithmetic is the one-cell form's.
-__device__ __forceinline__ float2 load_pair(const float* __restrict__ f, int c)
+// ---- Four vertically adjacent cells per thread -----------------------------
+// Cells c .. c + 3 with k a multiple of 4, of a grid whose columns start on
+// 16-byte boundaries: they lie in one column, share i and j, and each field's
+// values at the four cells and at the four shifted by +-sx or +-sy are one
+// aligned 16-byte load.  The cell passes' limit is the issue of instructions
+// (291 and 144 a cell in the one-cell and marching forms, two thirds of the
+// slots used), most of them loads, addresses, index arithmetic and range
+// tests, which the four cells share here.  Each cell's arithmetic is the
+// one-cell form's.
+struct Quad
 {
-    return *reinterpret_cast<const float2*>(f + c);
+    float v[4];
+};
+
+// Keeps the compiler from moving loads across it (no instruction).
+__device__ __forceinline__ void load_stage() { asm volatile("" ::: "memory"); }
+
+__device__ __forceinline__ Quad load_quad(const float* __restrict__ f, int c)
+{
+    const float4 t = *reinterpret_cast<const float4*>(f + c);
+    return Quad{{t.x, t.y, t.z, t.w}};
+}
+
+__device__ __forceinline__ void store_quad(float* f, int c, const Quad& q)
+{
+    *reinterpret_cast<float4*>(f + c) = make_float4(q.v[0], q.v[1], q.v[2], q.v[3]);
 }
 
 template <class Policy>
-__device__ __forceinline__ void continuity_eos_kpair(const FusedParams& P, const float* __restrict__ rho,
-                                                     const float* __restrict__ u, const float* __restrict__ v,
-                                                     const float* __restrict__ w, const float* __restrict__ theta,
-                                                     const double* __restrict__ rho0,
-                                                     const float4* __restrict__ eos0, float* __restrict__ rho_out,
-                                                     float* __restrict__ p_out, float* __restrict__ mfx,
-                                                     float* __restrict__ mfy, float* __restrict__ mfz, int c,
-                                                     unsigned& flags, bool store_flux, float* __restrict__ rho_copy)
+__device__ __forceinline__ void continuity_eos_quad(const FusedParams& P, const float* __restrict__ rho,
+                                                    const float* __restrict__ u, const float* __restrict__ v,
+                                                    const float* __restrict__ w, const float* __restrict__ theta,
+                                                    const double* __restrict__ rho0,
+                                                    const float4* __restrict__ eos0, float* __restrict__ rho_out,
+                                                    float* __restrict__ p_out, float* __restrict__ mfx,
+                                                    float* __restrict__ mfy, float* __restrict__ mfz, int c,
+                                                    unsigned& flags, bool store_flux, float* __restrict__ rho_copy)
 {
     const Dims d = P.d;
     int i, j, k;
     decompose(d, c, i, j, k);
     const int sx = d.sx(), sy = d.sy();
     const bool xlo = i >= 1, xhi = i < d.nx - 1, ylo = j >= 1, yhi = j < d.ny - 1;
-    const bool acc = mfx != nullptr && !store_flux;
-    const float2 r = load_pair(rho, c);
-    const float2 rxp = load_pair(rho, xhi ? c + sx : c), rxm = load_pair(rho, xlo ? c - sx : c);
-    const float2 ryp = load_pair(rho, yhi ? c + sy : c), rym = load_pair(rho, ylo ? c - sy : c);
-    const float rzm = rho[k > 0 ? c - 1 : c];
-    const float rzp = rho[k + 2 < d.nz ? c + 2 : c + 1];
-    const float2 uc = load_pair(u, c), uxm = load_pair(u, xlo ? c - sx : c);
-    const float2 vc = load_pair(v, c), vym = load_pair(v, ylo ? c - sy : c);
-    const float2 wc = load_pair(w, c);
-    const float wzm = w[k > 0 ? c - 1 : c];
-    const float2 th = load_pair(theta, c);
-    float2 mx = make_float2(0.0f, 0.0f), my = mx, mz = mx;
-    if (acc)
+    using real = typename Policy::real;
+    const bool flux = mfx != nullptr, acc = flux && !store_flux;
+    const bool interior = xlo && xhi && ylo && yhi;
+    // Axis by axis: each axis' loads end at a barrier to the compiler's
+    // reordering, so that the registers of one serve the next and the kernel
+    // runs at eight CTAs of 128 threads an SM instead of four or five.
+    unsigned bad[4] = {0, 0, 0, 0};
+    const Quad r = load_quad(rho, c);
+    if (rho_copy != nullptr) store_quad(rho_copy, c, r);
+    real dx[4], dy[4], dz[4];
     {
-        mx = load_pair(mfx, c);
-        my = load_pair(mfy, c);
-        mz = load_pair(mfz, c);
+        const Quad rp = load_quad(rho, xhi ? c + sx : c), rm = load_quad(rho, xlo ? c - sx : c);
+        const Quad vp = load_quad(u, c), vm = load_quad(u, xlo ? c - sx : c);
+        Quad m{};
+        if (acc) m = load_quad(mfx, c);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            if (flux && xhi)
+                m.v[q] = retained_lateral<Policy>(P, m.v[q], r.v[q], rp.v[q], vp.v[q], P.frame_u, P.frame_u_f, bad[q],
+                                                  store_flux);
+            dx[q] = flux_difference<real>(r.v[q], rp.v[q], rm.v[q], vp.v[q], vm.v[q]);
+        }
+        if (flux && xhi) store_quad(mfx, c, m);
     }
-    ContinuityStencil a, b;
-    a.rho_c = r.x; a.rxp = rxp.x; a.rxm = rxm.x; a.ryp = ryp.x; a.rym = rym.x; a.rzp = r.y; a.rzm = rzm;
-    a.uc = uc.x; a.uxm = uxm.x; a.vc = vc.x; a.vym = vym.x; a.wc = wc.x; a.wzm = wzm; a.th = th.x;
-    a.mx = mx.x; a.my = my.x; a.mz = mz.x;
-    b.rho_c = r.y; b.rxp = rxp.y; b.rxm = rxm.y; b.ryp = ryp.y; b.rym = rym.y; b.rzp = rzp; b.rzm = r.x;
-    b.uc = uc.y; b.uxm = uxm.y; b.vc = vc.y; b.vym = vym.y; b.wc = wc.y; b.wzm = wc.x; b.th = th.y;
-    b.mx = mx.y; b.my = my.y; b.mz = mz.y;
-    continuity_eos_values<Policy>(P, a, i, j, k, c, rho0, eos0, rho_out, p_out, nullptr, mfx, mfy, mfz, flags,
-                                  store_flux, rho_copy);
-    continuity_eos_values<Policy>(P, b, i, j, k + 1, c + 1, rho0, eos0, rho_out, p_out, nullptr, mfx, mfy, mfz, flags,
-                                  store_flux, rho_copy);
+    load_stage();
+    {
+        const Quad rp = load_quad(rho, yhi ? c + sy : c), rm = load_quad(rho, ylo ? c - sy : c);
+        const Quad vp = load_quad(v, c), vm = load_quad(v, ylo ? c - sy : c);
+        Quad m{};
+        if (acc) m = load_quad(mfy, c);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            if (flux && yhi)
+                m.v[q] = retained_lateral<Policy>(P, m.v[q], r.v[q], rp.v[q], vp.v[q], P.frame_v, P.frame_v_f, bad[q],
+                                                  store_flux);
+            dy[q] = flux_difference<real>(r.v[q], rp.v[q], rm.v[q], vp.v[q], vm.v[q]);
+        }
+        if (flux && yhi) store_quad(mfy, c, m);
+    }
+    load_stage();
+    const Quad th = load_quad(theta, c);
+    {
+        const float rzm = rho[k > 0 ? c - 1 : c], rzp = rho[k + 4 < d.nz ? c + 4 : c + 3];
+        const Quad wc = load_quad(w, c);
+        const float wzm = w[k > 0 ? c - 1 : c];
+        Quad m{};
+        if (acc) m = load_quad(mfz, c);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            const float rp = q < 3 ? r.v[q < 3 ? q + 1 : 3] : rzp, rm = q > 0 ? r.v[q > 0 ? q - 1 : 0] : rzm;
+            const float wm = q > 0 ? wc.v[q > 0 ? q - 1 : 0] : wzm;
+            const bool zlo = k + q > 0, zhi = k + q + 1 < d.nz;
+            if (flux)
+                m.v[q] = retained_vertical<Policy>(P, m.v[q], r.v[q], rp, wc.v[q], zhi, bad[q], store_flux);
+            dz[q] = flux_difference_z<real>(r.v[q], rp, rm, wc.v[q], wm, zlo, zhi);
+        }
+        if (flux) store_quad(mfz, c, m);
+    }
+    Quad rn, pn;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+    {
+        const float drho = interior ? continuity_tendency<Policy>(P, dx[q], dy[q], dz[q]) : 0.0f;
+        rn.v[q] = substep_density<Policy>(P, r.v[q], drho, rho0, k + q);
+        pn.v[q] = substep_pressure<Policy>(P, eos0, k + q, rn.v[q], th.v[q]);
+        if (k + q < d.nz) flags |= bad[q];  // a padded cell's values are not state
+    }
+    store_quad(rho_out, c, rn);
+    store_quad(p_out, c, pn);
 }
 
-// Momentum of the pair (c, c + 1), in place.  Both stencils are loaded before
-// either cell stores: under the vertical closure the cell at nz - 2 writes
-// level nz - 1, which is the pair's second cell when nz - 2 is even, and that
-// cell stores nothing.
 template <class Policy>
-__device__ __forceinline__ void momentum_kpair(const FusedParams& P, const float* __restrict__ rho,
-                                               const float* __restrict__ p, const double* __restrict__ p0,
-                                               const float2* __restrict__ dp0_split, float* u, float* v, float* w,
-                                               int c, int fuse_vertical)
+__device__ __forceinline__ void momentum_quad(const FusedParams& P, const float* __restrict__ rho,
+                                              const float* __restrict__ p, const double* __restrict__ p0,
+                                              const float2* __restrict__ dp0_split, const float* u, const float* v,
+                                              const float* w, float* u_out, float* v_out, float* w_out, int c,
+                                              int fuse_vertical)
 {
     const Dims d = P.d;
     int i, j, k;
     decompose(d, c, i, j, k);
     const bool ij = i >= 1 && i < d.nx - 1 && j >= 1 && j < d.ny - 1;
-    const int cx = ij ? c + d.sx() : c, cy = ij ? c + d.sy() : c;
-    const float2 r = load_pair(rho, c), rx = load_pair(rho, cx), ry = load_pair(rho, cy);
-    const float2 pc = load_pair(p, c), px = load_pair(p, cx), py = load_pair(p, cy);
-    const int cz2 = ij && k + 2 < d.nz ? c + 2 : c + 1;
-    const float rz2 = rho[cz2], pz2 = p[cz2];
-    const float2 uc = load_pair(u, c), vc = load_pair(v, c), wc = load_pair(w, c);
-    MomentumStencil a, b;
-    a.rc = r.x; a.rx = rx.x; a.ry = ry.x; a.rz = r.y;
-    a.pc = pc.x; a.px = px.x; a.py = py.x; a.pz = pc.y;
-    a.uc = uc.x; a.vc = vc.x; a.wc = wc.x;
-    b.rc = r.y; b.rx = rx.y; b.ry = ry.y; b.rz = rz2;
-    b.pc = pc.y; b.px = px.y; b.py = py.y; b.pz = pz2;
-    b.uc = uc.y; b.vc = vc.y; b.wc = wc.y;
-    momentum_values<Policy>(P, a, i, j, k, c, p0, dp0_split, u, v, w, fuse_vertical);
-    momentum_values<Policy>(P, b, i, j, k + 1, c + 1, p0, dp0_split, u, v, w, fuse_vertical);
+    const int cx = ij ? c + d.sx() : c, cy = ij ? c + d.sy() : c, cz = k + 4 < d.nz ? c + 4 : c + 3;
+    const Quad r = load_quad(rho, c), rx = load_quad(rho, cx), ry = load_quad(rho, cy);
+    const Quad pc = load_quad(p, c), px = load_quad(p, cx), py = load_quad(p, cy);
+    const float rz = rho[cz], pz = p[cz];
+    Quad un = load_quad(u, c), vn = load_quad(v, c), wn = load_quad(w, c);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+    {
+        MomentumStencil s;
+        s.rc = r.v[q];
+        s.rx = rx.v[q];
+        s.ry = ry.v[q];
+        s.rz = q < 3 ? r.v[q < 3 ? q + 1 : 3] : rz;
+        s.pc = pc.v[q];
+        s.px = px.v[q];
+        s.py = py.v[q];
+        s.pz = q < 3 ? pc.v[q < 3 ? q + 1 : 3] : pz;
+        s.uc = un.v[q];
+        s.vc = vn.v[q];
+        s.wc = wn.v[q];
+        const float3 n = momentum_point<Policy>(P, s, ij && k + q < d.nz - 1, k + q, p0, dp0_split);
+        un.v[q] = n.x;
+        vn.v[q] = n.y;
+        wn.v[q] = n.z;
+    }
+    if ((fuse_vertical & kFuseVertical) && i >= 1 && i <= d.nx - 3 && j >= 1 && j <= d.ny - 3)
+    {
+        // momentum_store's vertical closure on the four cells; the top level
+        // is cell kt of them.
+        if (k == 0 && (fuse_vertical & kFuseNoSlipBottom)) un.v[0] = vn.v[0] = 0.0f;
+        const int kt = d.nz - 1 - k;
+        const bool open = (fuse_vertical & kFuseOpenTop) != 0;
+        if (kt == 0) return;  // the level below writes it, and the rest is padding
+#pragma unroll
+        for (int q = 1; q < 4; ++q)
+            if (q == kt)
+            {
+                un.v[q] = un.v[q - 1];
+                vn.v[q] = vn.v[q - 1];
+                wn.v[q] = open ? wn.v[q - 1] : 0.0f;
+            }
+        if (kt == 4)
+        {
+            u_out[c + 4] = un.v[3];
+            v_out[c + 4] = vn.v[3];
+            w_out[c + 4] = open ? wn.v[3] : 0.0f;
+        }
+    }
+    store_quad(u_out, c, un);
+    store_quad(v_out, c, vn);
+    store_quad(w_out, c, wn);
+}
+
+constexpr int kQuadBlock = 128;  // threads of a quad kernel
+
+template <class Policy>
+static __global__ void __launch_bounds__(kQuadBlock, 8) split_continuity_quad_kernel(
+    FusedParams P, const float* __restrict__ rho, const float* __restrict__ u, const float* __restrict__ v,
+    const float* __restrict__ w, const float* __restrict__ theta, const double* __restrict__ rho0,
+    const float4* __restrict__ eos0, float* __restrict__ rho_out, float* __restrict__ p_out,
+    float* __restrict__ mfx, float* __restrict__ mfy, float* __restrict__ mfz, unsigned* __restrict__ status)
+{
+    const int n = P.d.cells();
+    unsigned flags = 0;
+    for (int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x); c < n; c += 4 * gridDim.x * blockDim.x)
+        continuity_eos_quad<Policy>(P, rho, u, v, w, theta, rho0, eos0, rho_out, p_out, mfx, mfy, mfz, c, flags, false,
+                                    nullptr);
+    if (flags) atomicOr(status, flags);
+}
+
+template <class Policy>
+static __global__ void __launch_bounds__(kQuadBlock, 8) split_momentum_quad_kernel(
+    FusedParams P, const float* __restrict__ rho, const float* __restrict__ p, const double* __restrict__ p0,
+    const float2* __restrict__ dp0_split, const float* __restrict__ u, const float* __restrict__ v,
+    const float* __restrict__ w, float* __restrict__ u_out, float* __restrict__ v_out, float* __restrict__ w_out)
+{
+    const int n = P.d.cells();
+    for (int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x); c < n; c += 4 * gridDim.x * blockDim.x)
+        momentum_quad<Policy>(P, rho, p, p0, dp0_split, u, v, w, u_out, v_out, w_out, c, 0);
 }
 
 template <class Policy>

@@ -30,7 +30,18 @@ constexpr size_t kAlign = 256;
 using nimbus_engine_detail::Lane;
 using nimbus_engine_detail::MemberSlot;
 
+// Cells of a member's state as its owner sees it (no padding).
+size_t state_cells(const MemberSlot& s)
+{
+    return static_cast<size_t>(s.desc.nx) * s.desc.ny * static_cast<size_t>(s.desc.nz);
+}
+
 size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
+
+// Column pitch of a member's fields: whole 16-byte groups of cells, so that a
+// column starts on a 16-byte boundary whatever nz is (at most three cells of
+// 40 to 64 levels) and the cell passes read and write four cells at once.
+int column_pitch(int nz) { return (nz + 3) & ~3; }
 
 // Byte layout of one member's arena.
 struct ArenaLayout
@@ -43,7 +54,8 @@ struct ArenaLayout
 ArenaLayout arena_layout(const nimbus_member_desc* d)
 {
     ArenaLayout L{};
-    L.cells = static_cast<size_t>(d->nx) * d->ny * d->nz;
+    const int pz = column_pitch(d->nz);
+    L.cells = static_cast<size_t>(d->nx) * d->ny * pz;
     L.history = 2 * (static_cast<size_t>(d->nx) + d->ny) * d->nz;
     const size_t field = align_up(L.cells * sizeof(float));
     size_t off = 0;
@@ -57,9 +69,10 @@ ArenaLayout arena_layout(const nimbus_member_desc* d)
     L.off_xs = off;     off += align_up(4 * L.cells * sizeof(float));
     L.off_eos = off;    off += field;
     L.off_status = off; off += kAlign;
-    L.off_prof = off;   off += align_up(5 * static_cast<size_t>(d->nz) * sizeof(double));
-    L.off_dp0 = off;    off += align_up(static_cast<size_t>(d->nz) * sizeof(float2));
-    L.off_eos0 = off;   off += align_up(static_cast<size_t>(d->nz) * sizeof(float4));
+    // Per-level tables, one entry a stored level.
+    L.off_prof = off;   off += align_up(5 * static_cast<size_t>(pz) * sizeof(double));
+    L.off_dp0 = off;    off += align_up(static_cast<size_t>(pz) * sizeof(float2));
+    L.off_eos0 = off;   off += align_up(static_cast<size_t>(pz) * sizeof(float4));
     L.off_sponge = off;
     if (const nimbus_sponge_desc* sp = d->sponge)
     {
@@ -118,7 +131,7 @@ void fill_params(EngineMember& M, const nimbus_member_desc* a)
     const double dt_small = a->dt / a->n_substeps;
     FusedParams& F = M.F;
     F = FusedParams{};
-    F.d = make_dims(a->nx, a->ny, a->nz);
+    F.d = make_dims(a->nx, a->ny, a->nz, column_pitch(a->nz));
     F.inv_dx = 1.0 / a->dx;
     F.inv_dy = 1.0 / a->dy;
     F.inv_dz = 1.0 / a->dz;
@@ -198,13 +211,13 @@ void fill_params(EngineMember& M, const nimbus_member_desc* a)
     M.eos_series = eos_series(gamma);
     M.n_substeps = a->n_substeps;
     M.microphysics = a->microphysics;
-    M.items[kItemCells] = a->nx * a->ny * a->nz;
+    M.items[kItemCells] = F.d.cells();
     M.items[kItemRowsWE] = a->ny * a->nz;
     M.items[kItemRowsSN] = a->nx * a->nz;
     M.items[kItemColumns] = a->nx * a->ny;
     M.items[kItemHistory] = (a->ny + a->nx) * a->nz;
     M.items[kItemPerimeter] = 3 * a->nx + 3 * (a->ny - 3);
-    M.items[kItemScan] = (M.items[kItemCells] + kScanCells - 1) / kScanCells;
+    M.items[kItemQuads] = M.items[kItemCells] / 4;
 }
 
 }  // namespace
@@ -438,10 +451,10 @@ nimbus_status rebuild_table(nimbus_engine* e)
     for (auto& slot : e->slots)
     {
         slot.m.image_offset = image;
-        image += 9LL * slot.m.items[kItemCells];
+        image += 9LL * state_cells(slot);
         // Marching tiles: (j, k) blocks of one CTA times i-chunks of march_len planes.
         EngineMember& M = slot.m;
-        const int blocks = (M.F.d.ny * M.F.d.nz + kEngineBlock - 1) / kEngineBlock;
+        const int blocks = (M.F.d.sx() + kEngineBlock - 1) / kEngineBlock;
         const int chunks = (M.F.d.nx + e->march_len - 1) / e->march_len;
         M.march_len = e->march_len;
         M.march_blocks = blocks;
@@ -450,7 +463,6 @@ nimbus_status rebuild_table(nimbus_engine* e)
     std::vector<EngineMember> host(n);
     for (size_t r = 0; r < n; ++r) host[r] = e->slots[e->order[r]].m;
     e->prefix.assign(pre, 0);
-    const int tile = kEngineBlock * kItemsPerThread;
     for (Lane& L : e->lanes)
     {
         const EngineMember* rows = host.data() + L.first;
@@ -460,6 +472,7 @@ nimbus_status rebuild_table(nimbus_engine* e)
         {
             long long* p = e->prefix.data() + L.prefix_first + static_cast<size_t>(k) * (L.members + 1);
             p[0] = 0;
+            const int tile = k == kItemQuads ? kQuadTile : kEngineBlock * kItemsPerThread;
             for (int r = 0; r < L.members; ++r) p[r + 1] = p[r] + (rows[r].items[k] + tile - 1) / tile;
         }
         L.closing = false;
@@ -517,11 +530,12 @@ nimbus_status enqueue_scan(nimbus_engine* e)
     NB_CUDA(ctx, cudaMemsetAsync(e->d_c2, 0, n * sizeof(unsigned long long), e->stream));
     for (const Lane& L : e->lanes)
     {
-        const long long tiles = tiles_of(e, L, kItemScan, L.members);
+        const long long tiles = tiles_of(e, L, kItemQuads, L.members);
         if (tiles <= 0) continue;
-        engine_sound_speed_kernel<<<engine_grid(e, reinterpret_cast<const void*>(engine_sound_speed_kernel), tiles),
-                                    kEngineBlock, 0, e->stream>>>(e->d_table + L.first, prefix_of(e, L, kItemScan),
-                                                                  tiles, e->d_c2 + L.first);
+        engine_sound_speed_kernel<<<engine_grid(e, reinterpret_cast<const void*>(engine_sound_speed_kernel), tiles,
+                                                kQuadTile),
+                                    kQuadTile, 0, e->stream>>>(e->d_table + L.first, prefix_of(e, L, kItemQuads),
+                                                               tiles, e->d_c2 + L.first);
         ctx->launches += 1;
     }
     NB_CUDA(ctx, cudaGetLastError());
@@ -686,7 +700,7 @@ MemberSlot* find_slot(nimbus_engine* e, int id, size_t* index = nullptr)
 size_t image_bytes_of(const nimbus_engine* e)
 {
     size_t floats = 0;
-    for (const auto& slot : e->slots) floats += 9ull * static_cast<size_t>(slot.m.items[kItemCells]);
+    for (const auto& slot : e->slots) floats += 9ull * state_cells(slot);
     return floats * sizeof(float);
 }
 
@@ -721,6 +735,38 @@ void launch_image(nimbus_engine* e, int gather, float* image = nullptr)
         e->ctx->launches += 1;
     }
 }
+
+// A stream-ordered device block holding one member's unpadded state, for
+// members whose columns are padded (nz not a multiple of four): the host's
+// nine fields move to and from it in plain copies and member_image_kernel
+// spreads it into the member's buffers or collects it from them.
+struct StateStage
+{
+    nimbus_engine* e;
+    float* block = nullptr;
+    ~StateStage()
+    {
+        if (block) cudaFreeAsync(block, e->stream);  // after what is enqueued on it
+    }
+    nimbus_status open(size_t cells)
+    {
+        const cudaError_t err =
+            cudaMallocAsync(reinterpret_cast<void**>(&block), 9 * cells * sizeof(float), e->stream);
+        if (err != cudaSuccess)
+        {
+            block = nullptr;
+            return cuda_fail(e->ctx, err, "member staging");
+        }
+        return NIMBUS_OK;
+    }
+    void move(const EngineMember& M, int gather)
+    {
+        member_image_kernel<<<grid_for(e->ctx, M.items[kItemCells]), kThreads, 0, e->stream>>>(M, block, gather);
+        e->ctx->launches += 1;
+    }
+};
+
+bool padded(const EngineMember& M) { return M.F.d.pz != M.F.d.nz; }
 
 const char* check_state(const nimbus_member_state* s)
 {
@@ -882,12 +928,12 @@ nimbus_status nimbus_cuda_engine_admit(nimbus_engine* e, const nimbus_member_des
     M.eos = reinterpret_cast<float*>(base + L.off_eos);
     M.status = reinterpret_cast<unsigned*>(base + L.off_status);
     double* prof = reinterpret_cast<double*>(base + L.off_prof);
-    const size_t nz = static_cast<size_t>(desc->nz);
+    const size_t nz = static_cast<size_t>(desc->nz), pz = static_cast<size_t>(column_pitch(desc->nz));
     M.rho0 = prof;
-    M.p0 = prof + nz;
-    M.qv0 = prof + 2 * nz;
-    M.u0 = prof + 3 * nz;
-    M.v0 = prof + 4 * nz;
+    M.p0 = prof + pz;
+    M.qv0 = prof + 2 * pz;
+    M.u0 = prof + 3 * pz;
+    M.v0 = prof + 4 * pz;
     float2* dp0 = reinterpret_cast<float2*>(base + L.off_dp0);
     float4* eos0 = reinterpret_cast<float4*>(base + L.off_eos0);
     M.dp0 = dp0;
@@ -895,21 +941,36 @@ nimbus_status nimbus_cuda_engine_admit(nimbus_engine* e, const nimbus_member_des
     fill_params(M, &first);
 
     // Profiles, the split hydrostatic difference and the initial state.
-    std::vector<double> hp(5 * nz, 0.0);
-    std::memcpy(hp.data(), desc->rho0_base, nz * sizeof(double));
-    std::memcpy(hp.data() + nz, desc->p0_base, nz * sizeof(double));
-    std::memcpy(hp.data() + 2 * nz, desc->qv0_base, nz * sizeof(double));
-    if (desc->u0_base) std::memcpy(hp.data() + 3 * nz, desc->u0_base, nz * sizeof(double));
-    if (desc->v0_base) std::memcpy(hp.data() + 4 * nz, desc->v0_base, nz * sizeof(double));
-    const size_t bytes = L.cells * sizeof(float);
+    std::vector<double> hp(5 * pz, 0.0);
+    const double* profiles[5] = {desc->rho0_base, desc->p0_base, desc->qv0_base, desc->u0_base, desc->v0_base};
+    for (size_t f = 0; f < 5; ++f)
+    {
+        if (!profiles[f]) continue;
+        std::memcpy(hp.data() + f * pz, profiles[f], nz * sizeof(double));
+        std::fill(hp.begin() + static_cast<long>(f * pz + nz), hp.begin() + static_cast<long>((f + 1) * pz),
+                  profiles[f][nz - 1]);  // padded levels repeat the top
+    }
+    const size_t cells = static_cast<size_t>(desc->nx) * desc->ny * nz;
+    const size_t bytes = cells * sizeof(float);
     cudaError_t err = cudaSuccess;
     const float* src[9] = {initial->u, initial->v, initial->w, initial->rho, initial->p, initial->theta,
                            initial->qv, initial->qc, initial->qr};
     float* dst[9] = {M.u, M.v, M.w, M.rho, M.p, M.theta, M.qv, M.qc, M.qr};
+    StateStage stage{e};
+    if (padded(M))
+    {
+        if (const nimbus_status rc = stage.open(cells); rc != NIMBUS_OK)
+        {
+            cudaFreeAsync(slot.arena, e->stream);
+            return rc;
+        }
+        for (int f = 0; f < 9; ++f) dst[f] = stage.block + static_cast<size_t>(f) * cells;
+    }
     // Pageable sources are staged before each call returns (the caller's
     // arrays and the local vectors may go); pinned ones are read by the copy.
     for (int f = 0; f < 9 && err == cudaSuccess; ++f)
         err = cudaMemcpyAsync(dst[f], src[f], bytes, cudaMemcpyHostToDevice, e->stream);
+    if (err == cudaSuccess && padded(M)) stage.move(M, 0);
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(prof, hp.data(), hp.size() * sizeof(double), cudaMemcpyHostToDevice, e->stream);
     M.R = RelaxTables{};
@@ -932,7 +993,8 @@ nimbus_status nimbus_cuda_engine_admit(nimbus_engine* e, const nimbus_member_des
     {
         // The same per-level kernel the per-operation path runs, so both forms
         // see identical base data.
-        level_base_kernel<<<(desc->nz + 127) / 128, 128, 0, e->stream>>>(M.p0, desc->nz, M.gamma, dp0, eos0);
+        level_base_kernel<<<(static_cast<int>(pz) + 127) / 128, 128, 0, e->stream>>>(M.p0, static_cast<int>(pz),
+                                                                                     M.gamma, dp0, eos0);
         err = cudaGetLastError();
     }
     if (err == cudaSuccess) err = cudaMemsetAsync(M.status, 0, sizeof(unsigned), e->stream);
@@ -972,9 +1034,16 @@ nimbus_status nimbus_cuda_engine_read_async(nimbus_engine* e, int member_id, con
     if (!s) return fail(ctx, NIMBUS_ERR_INVALID_ARGUMENT, "unknown member id");
     if (!e->mirror_exact) NB_TRY(sync_table_to_host(e));
     const EngineMember& M = s->m;
-    const size_t bytes = static_cast<size_t>(M.items[kItemCells]) * sizeof(float);
+    const size_t cells = state_cells(*s), bytes = cells * sizeof(float);
     const float* src[9] = {M.u, M.v, M.w, M.rho, M.p, M.theta, M.qv, M.qc, M.qr};
     float* dst[9] = {out->u, out->v, out->w, out->rho, out->p, out->theta, out->qv, out->qc, out->qr};
+    StateStage stage{e};
+    if (padded(M))
+    {
+        NB_TRY(stage.open(cells));
+        stage.move(M, 1);
+        for (int f = 0; f < 9; ++f) src[f] = stage.block + static_cast<size_t>(f) * cells;
+    }
     for (int f = 0; f < 9; ++f)
         NB_CUDA(ctx, cudaMemcpyAsync(dst[f], src[f], bytes, cudaMemcpyDeviceToHost, e->stream));
     return NIMBUS_OK;
@@ -990,11 +1059,19 @@ nimbus_status nimbus_cuda_engine_write_async(nimbus_engine* e, int member_id, co
     if (!s) return fail(ctx, NIMBUS_ERR_INVALID_ARGUMENT, "unknown member id");
     if (!e->mirror_exact) NB_TRY(sync_table_to_host(e));
     const EngineMember& M = s->m;
-    const size_t bytes = static_cast<size_t>(M.items[kItemCells]) * sizeof(float);
+    const size_t cells = state_cells(*s), bytes = cells * sizeof(float);
     const float* src[9] = {in->u, in->v, in->w, in->rho, in->p, in->theta, in->qv, in->qc, in->qr};
     float* dst[9] = {M.u, M.v, M.w, M.rho, M.p, M.theta, M.qv, M.qc, M.qr};
+    StateStage stage{e};
+    if (padded(M))
+    {
+        NB_TRY(stage.open(cells));
+        for (int f = 0; f < 9; ++f) dst[f] = stage.block + static_cast<size_t>(f) * cells;
+    }
     for (int f = 0; f < 9; ++f)
         NB_CUDA(ctx, cudaMemcpyAsync(dst[f], src[f], bytes, cudaMemcpyHostToDevice, e->stream));
+    if (padded(M)) stage.move(M, 0);
+    NB_CUDA(ctx, cudaGetLastError());
     return NIMBUS_OK;
 }
 
@@ -1011,7 +1088,8 @@ nimbus_status nimbus_cuda_engine_history_async(nimbus_engine* e, int member_id, 
     NB_CUDA(ctx, cudaSetDevice(ctx->device));
     if (!e->mirror_exact) NB_TRY(sync_table_to_host(e));
     const EngineMember& M = s->m;
-    const size_t need = 3 * static_cast<size_t>(M.items[kItemCells]) * sizeof(float);
+    const size_t cells = state_cells(*s);
+    const size_t need = 3 * cells * sizeof(float);
     if (need > e->centre_cap)
     {
         NB_CUDA(ctx, cudaStreamSynchronize(e->stream));
@@ -1022,6 +1100,13 @@ nimbus_status nimbus_cuda_engine_history_async(nimbus_engine* e, int member_id, 
         e->centre_cap = need;
     }
     const float* src[kHistoryFields] = {M.u, M.v, M.w, M.rho, M.p, M.theta, M.qv, M.qc, M.qr};
+    StateStage stage{e};
+    if (padded(M))
+    {
+        NB_TRY(stage.open(cells));
+        stage.move(M, 1);
+        for (int f = 0; f < kHistoryFields; ++f) src[f] = stage.block + static_cast<size_t>(f) * cells;
+    }
     return enqueue_history(ctx, e->stream, src, fields, nullptr, s->desc.nx, s->desc.ny, s->desc.nz, e->d_centre,
                            static_cast<float*>(host_image));
 }
@@ -1055,7 +1140,7 @@ size_t nimbus_cuda_engine_image_offset(const nimbus_engine* e, int member_id)
     for (const auto& slot : e->slots)
     {
         if (slot.id == member_id) return floats * sizeof(float);
-        floats += 9ull * static_cast<size_t>(slot.m.items[kItemCells]);
+        floats += 9ull * state_cells(slot);
     }
     return static_cast<size_t>(-1);
 }
@@ -1229,8 +1314,8 @@ nimbus_status nimbus_cuda_engine_autotune(nimbus_engine* e, int steps, nimbus_en
         if (lanes > members && lanes != 1) continue;
         if (!(ok = trial({lanes, NIMBUS_ACOUSTIC_CONST, NIMBUS_ACOUSTIC_CONST, saved.march}))) break;
     }
-    const int forms[] = {NIMBUS_ACOUSTIC_CONST, NIMBUS_ACOUSTIC_PAIR, NIMBUS_ACOUSTIC_TABLE, NIMBUS_ACOUSTIC_MARCH,
-                         NIMBUS_ACOUSTIC_BULK, NIMBUS_ACOUSTIC_CMARCH};
+    const int forms[] = {NIMBUS_ACOUSTIC_CONST, NIMBUS_ACOUSTIC_TABLE, NIMBUS_ACOUSTIC_MARCH, NIMBUS_ACOUSTIC_BULK,
+                         NIMBUS_ACOUSTIC_CMARCH};
     const int lanes = chosen.lanes;
     for (int cf : forms)
     {

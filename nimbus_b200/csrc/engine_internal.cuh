@@ -65,7 +65,7 @@ struct nimbus_engine
     int lane_target = 4;            // lanes when there are at least that many members
     int march_len = 16;             // i-planes per thread of the marching acoustic kernels
     int acoustic_form = NIMBUS_ACOUSTIC_CONST;  // nimbus_acoustic_form of the continuity pass
-    int momentum_form = NIMBUS_ACOUSTIC_MARCH;  // and of the momentum pass (marching measured fastest)
+    int momentum_form = NIMBUS_ACOUSTIC_CONST;  // and of the momentum pass
     std::vector<cudaStream_t> lane_streams;  // lanes 1.. (lane 0 runs on the engine stream)
     std::vector<cudaEvent_t> lane_done;
     cudaEvent_t fork = nullptr;
@@ -286,8 +286,7 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
     // parameter (lanes of at most kConstMembers members; larger ones take the
     // member-table form).
     auto in_bank = [](int f) {
-        return f == NIMBUS_ACOUSTIC_CONST || f == NIMBUS_ACOUSTIC_PAIR || f == NIMBUS_ACOUSTIC_BULK ||
-               f == NIMBUS_ACOUSTIC_CMARCH;
+        return f == NIMBUS_ACOUSTIC_CONST || f == NIMBUS_ACOUSTIC_BULK || f == NIMBUS_ACOUSTIC_CMARCH;
     };
     // Bulk copies move 16-byte units between 16-byte-aligned addresses: every
     // member field starts on a 256-byte boundary of its arena, so the arenas
@@ -304,6 +303,7 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
     const size_t smem_cont = bulk_smem_bytes(continuity_stage_floats(sy4));
     const size_t smem_mom = bulk_smem_bytes(momentum_stage_floats(sy4));
     auto resolve_form = [&](int f) {
+        if (f == NIMBUS_ACOUSTIC_PAIR) f = NIMBUS_ACOUSTIC_CONST;  // four cells a thread where two were asked for
         if (in_bank(f) && n > kConstMembers) return static_cast<int>(NIMBUS_ACOUSTIC_TABLE);
         if (f == NIMBUS_ACOUSTIC_BULK && (smem_cont > kBulkSmemLimit || !arenas_aligned))
             return static_cast<int>(NIMBUS_ACOUSTIC_CONST);
@@ -319,10 +319,11 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
     {
         al.reset(new AcousticLaunch());
         const long long* p = e->prefix.data() + L.prefix_first + static_cast<size_t>(kItemCells) * (n + 1);
+        const long long* pq = e->prefix.data() + L.prefix_first + static_cast<size_t>(kItemQuads) * (n + 1);
         for (int r = 0; r <= n; ++r)
         {
             al->prefix[r] = p[r];
-            al->prefix32[r] = static_cast<int>(p[r]);
+            al->quad_prefix[r] = static_cast<int>(pq[r]);
         }
         const long long* pmr = e->prefix.data() + L.prefix_first + static_cast<size_t>(kItemMarch) * (n + 1);
         for (int r = 0; r <= n; ++r) al->march_prefix[r] = pmr[r];
@@ -364,39 +365,26 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
         const int si = static_cast<int>(s);
         const long long tiles = tiles_of(e, L, kItemCells, a);
         const long long march_tiles = tiles_of(e, L, kItemMarch, a);
+        const long long quad_tiles = tiles_of(e, L, kItemQuads, a);
         switch (cform)
         {
         case NIMBUS_ACOUSTIC_CONST:
             if (s == 0 && shared)
-                ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, (engine_continuity_const_kernel<Policy, true, true>),
-                              tiles, 1, *al, T, tiles, si);
-            else if (s == 0)
-                ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, (engine_continuity_const_kernel<Policy, true, false>),
-                              tiles, 1, *al, T, tiles, si);
-            else if (shared)
-                ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, (engine_continuity_const_kernel<Policy, false, true>),
-                              tiles, 1, *al, T, tiles, si);
-            else
-                ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, (engine_continuity_const_kernel<Policy, false, false>),
-                              tiles, 1, *al, T, tiles, si);
-            break;
-        case NIMBUS_ACOUSTIC_PAIR:
-            if (s == 0 && shared)
                 ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP,
-                                    (engine_continuity_pair_kernel<Policy, true, true>), tiles, kEngineBlock / 2, *al,
-                                    T, tiles, si);
+                                    (engine_continuity_const_kernel<Policy, true, true>), quad_tiles, kQuadTile, *al,
+                                    T, quad_tiles, si);
             else if (s == 0)
                 ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP,
-                                    (engine_continuity_pair_kernel<Policy, true, false>), tiles, kEngineBlock / 2, *al,
-                                    T, tiles, si);
+                                    (engine_continuity_const_kernel<Policy, true, false>), quad_tiles, kQuadTile, *al,
+                                    T, quad_tiles, si);
             else if (shared)
                 ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP,
-                                    (engine_continuity_pair_kernel<Policy, false, true>), tiles, kEngineBlock / 2, *al,
-                                    T, tiles, si);
+                                    (engine_continuity_const_kernel<Policy, false, true>), quad_tiles, kQuadTile, *al,
+                                    T, quad_tiles, si);
             else
                 ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP,
-                                    (engine_continuity_pair_kernel<Policy, false, false>), tiles, kEngineBlock / 2,
-                                    *al, T, tiles, si);
+                                    (engine_continuity_const_kernel<Policy, false, false>), quad_tiles, kQuadTile, *al,
+                                    T, quad_tiles, si);
             break;
         case NIMBUS_ACOUSTIC_MARCH:
             ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, engine_continuity_march_kernel<Policy>, march_tiles, 1, T,
@@ -425,12 +413,8 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
         switch (mform)
         {
         case NIMBUS_ACOUSTIC_CONST:
-            ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, engine_momentum_const_kernel<Policy>, tiles, 1, *al, T,
-                          tiles, si);
-            break;
-        case NIMBUS_ACOUSTIC_PAIR:
-            ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, engine_momentum_pair_kernel<Policy>, tiles,
-                                kEngineBlock / 2, *al, T, tiles, si);
+            ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, engine_momentum_const_kernel<Policy>, quad_tiles,
+                                kQuadTile, *al, T, quad_tiles, si);
             break;
         case NIMBUS_ACOUSTIC_MARCH:
             ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, engine_momentum_march_kernel<Policy>, march_tiles, 1, T,
@@ -528,8 +512,8 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
     }
     // The acoustic speed scan of the state the next step starts from.
     if (e->resolving)
-        ENGINE_LAUNCH(NIMBUS_KERNEL_MICROPHYSICS, engine_sound_speed_kernel, tiles_of(e, L, kItemScan, n), 1, T,
-                      prefix_of(e, L, kItemScan), tiles_of(e, L, kItemScan, n), e->d_c2 + L.first);
+        ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_MICROPHYSICS, engine_sound_speed_kernel, tiles_of(e, L, kItemQuads, n),
+                            kQuadTile, T, prefix_of(e, L, kItemQuads), tiles_of(e, L, kItemQuads, n), e->d_c2 + L.first);
     return count;
 }
 

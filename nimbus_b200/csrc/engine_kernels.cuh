@@ -37,11 +37,11 @@ enum ItemKind
     kItemHistory,    // (ny + nx)*nz KW78 history slots
     kItemPerimeter,  // 3 nx + 3 (ny - 3) columns the lateral closures write
     kItemMarch,      // rows along x: (j, k) positions in blocks times i-chunks (for_member_rows)
-    kItemScan,       // cells in groups of kScanCells (engine_sound_speed_kernel)
+    kItemQuads,      // cells in groups of four (the constant-bank acoustic passes and the speed scan)
     kItemKinds
 };
 
-constexpr int kScanCells = 8;  // cells one thread of the acoustic speed scan reads
+constexpr int kQuadTile = kQuadBlock;  // groups of four cells in a kItemQuads tile (one a thread)
 
 constexpr int kEngineScalars = 4;  // theta, qv, qc, qr
 
@@ -117,7 +117,7 @@ __device__ __forceinline__ void for_member_items(const EngineMember* __restrict_
 }
 
 // Calls fn(member, i0, i1, j, k, q) for the rows of the first tiles of
-// kItemMarch: a member's (j, k) positions q = j nz + k are cut into blocks of
+// kItemMarch: a member's (j, k) positions q = j pz + k are cut into blocks of
 // blockDim.x (a warp reads 32 consecutive floats of a plane) and its x range
 // into chunks of march_len planes; tile = chunk * march_blocks + block.  The
 // thread of position q advances the cells (i0 .. i1-1, j, k) of its row.
@@ -134,9 +134,10 @@ __device__ __forceinline__ void for_member_rows(const EngineMember* __restrict__
         const int chunk = local / M.march_blocks;
         const int q = (local - chunk * M.march_blocks) * (int)blockDim.x + (int)threadIdx.x;
         const Dims d = M.F.d;
-        if (q >= d.ny * d.nz) continue;
+        if (q >= d.sx()) continue;
         int i, j, k;
         decompose(d, q, i, j, k);
+        if (k >= d.nz) continue;
         const int i0 = chunk * M.march_len;
         fn(M, i0, min(d.nx, i0 + M.march_len), j, k, q);
     }
@@ -468,21 +469,22 @@ __device__ __forceinline__ FusedParams with_shared(const FusedParams& F, const A
     return P;
 }
 
-// Resident CTAs per SM the launch bounds ask for (continuity, momentum):
-// measured on the 64-member ensemble, FP32, ms per step: natural register
-// counts (48 / 36 registers) 14.41, 6 / 7 CTAs (40 / 36) 13.49, 8 / 8 (32
-// registers, spilling) 14.49.
+// Resident CTAs (of kQuadTile threads) per SM the launch bounds ask for
+// (continuity, momentum): at 8 the FP32 form keeps to 64 registers without
+// spills.  FP32, 512x512x128, ps per cell: 8 / 8 8.98 / 4.70, 7 / 7
+// 9.72 / 4.81, 6 / 8 10.27 / 4.71 (one cell per thread 11.1 / 6.8); reference
+// precision, 256x256x80: 17.1 / 9.5 (one cell 19.3 / 10.2).
 #ifndef NIMBUS_CONST_MINB
-#define NIMBUS_CONST_MINB 6
+#define NIMBUS_CONST_MINB 8
 #endif
 #ifndef NIMBUS_CONST_MINB_MOM
-#define NIMBUS_CONST_MINB_MOM 7
+#define NIMBUS_CONST_MINB_MOM 8
 #endif
 
 struct AcousticLaunch
 {
     long long prefix[kConstMembers + 1];        // first cell tile of each member
-    int prefix32[kConstMembers + 1];            // the same as 32-bit values (a lane's tiles fit)
+    int quad_prefix[kConstMembers + 1];         // first quad tile of each member (a lane's tiles fit 32 bits)
     long long march_prefix[kConstMembers + 1];  // first row tile of each member (marching forms)
     AcousticConst m[kConstMembers];
     int bulk_sy4;                               // the members' largest nz rounded up to 4 (bulk-staged forms)
@@ -490,49 +492,36 @@ struct AcousticLaunch
 };
 static_assert(sizeof(AcousticLaunch) <= 32000, "a kernel parameter block holds at most 32764 bytes");
 
+// Four cells per thread (continuity_eos_quad, momentum_quad).
 // kFirst: the first substep of the step (the retained fluxes are written, not
 // accumulated, and the beginning density is kept).
 // kShared: every member's shared values equal L.shared (acoustic_shared_of).
-// Measured on the 64-member ensemble, FP32: continuity 3.58 -> 3.49 ms per
-// step.  (Deriving the member's buffers from one pointer and the arena's field
-// stride as well, two indexed loads instead of eight, spilled at the launch
-// bound and took 3.78 ms; an inner loop over one member's tiles, so that its
-// values could be loaded once per member, kept the loads per cell and took
-// 3.58 ms.)
 template <class Policy, bool kFirst, bool kShared>
-static __global__ void __launch_bounds__(256, NIMBUS_CONST_MINB) engine_continuity_const_kernel(const __grid_constant__ AcousticLaunch L,
+static __global__ void __launch_bounds__(kQuadTile, NIMBUS_CONST_MINB) engine_continuity_const_kernel(const __grid_constant__ AcousticLaunch L,
                                                                       const EngineMember* __restrict__ table,
                                                                       long long tiles, int s)
 {
-    constexpr bool first = kFirst;
     const bool even = (s & 1) == 0;
     int m = 0;
     const int ntiles = (int)tiles;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
     {
-        while (t >= L.prefix32[m + 1]) ++m;
+        while (t >= L.quad_prefix[m + 1]) ++m;
         const AcousticConst& A = L.m[m];
-        const int c = (t - L.prefix32[m]) * (int)blockDim.x + (int)threadIdx.x;
+        const int c = 4 * ((t - L.quad_prefix[m]) * kQuadTile + (int)threadIdx.x);
         if (c >= A.F.d.cells()) continue;
         const EngineMember& M = table[m];
         unsigned flags = 0;
-        if constexpr (kShared)
-        {
-            const FusedParams F = with_shared(A.F, L.shared);
-            continuity_eos_cell<Policy>(F, even ? M.rho : M.rho_alt, A.u, A.v, A.w, A.theta, A.rho0, A.eos0,
-                                        even ? M.rho_alt : M.rho, M.p, nullptr, A.mfx, A.mfy, A.mfz, c, flags, first,
-                                        first ? A.rho_begin : nullptr);
-        }
-        else
-            continuity_eos_cell<Policy>(A.F, even ? M.rho : M.rho_alt, A.u, A.v, A.w, A.theta, A.rho0, A.eos0,
-                                        even ? M.rho_alt : M.rho, M.p, nullptr, A.mfx, A.mfy, A.mfz, c, flags, first,
-                                        first ? A.rho_begin : nullptr);
+        const FusedParams F = kShared ? with_shared(A.F, L.shared) : A.F;
+        continuity_eos_quad<Policy>(F, even ? M.rho : M.rho_alt, A.u, A.v, A.w, A.theta, A.rho0, A.eos0,
+                                    even ? M.rho_alt : M.rho, M.p, A.mfx, A.mfy, A.mfz, c, flags, kFirst,
+                                    kFirst ? A.rho_begin : nullptr);
         if (flags) atomicOr(A.status, flags);
     }
 }
 
 template <class Policy>
-static __global__ void __launch_bounds__(256, NIMBUS_CONST_MINB_MOM) engine_momentum_const_kernel(const __grid_constant__ AcousticLaunch L,
+static __global__ void __launch_bounds__(kQuadTile, NIMBUS_CONST_MINB_MOM) engine_momentum_const_kernel(const __grid_constant__ AcousticLaunch L,
                                                                     const EngineMember* __restrict__ table,
                                                                     long long tiles, int s)
 {
@@ -541,12 +530,12 @@ static __global__ void __launch_bounds__(256, NIMBUS_CONST_MINB_MOM) engine_mome
     const int ntiles = (int)tiles;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
     {
-        while (t >= L.prefix32[m + 1]) ++m;
+        while (t >= L.quad_prefix[m + 1]) ++m;
         const AcousticConst& A = L.m[m];
-        const int c = (t - L.prefix32[m]) * (int)blockDim.x + (int)threadIdx.x;
+        const int c = 4 * ((t - L.quad_prefix[m]) * kQuadTile + (int)threadIdx.x);
         if (c >= A.F.d.cells()) continue;
         const EngineMember& M = table[m];
-        momentum_cell<Policy>(A.F, even ? M.rho_alt : M.rho, M.p, A.p0, A.dp0, A.u, A.v, A.w, A.u, A.v, A.w, c,
+        momentum_quad<Policy>(A.F, even ? M.rho_alt : M.rho, M.p, A.p0, A.dp0, A.u, A.v, A.w, A.u, A.v, A.w, c,
                               A.vertical);
     }
 }
@@ -568,9 +557,10 @@ __device__ __forceinline__ void for_const_rows(const AcousticLaunch& L, const En
         const int chunk = local / A.march_blocks;
         const int q = (local - chunk * A.march_blocks) * (int)blockDim.x + (int)threadIdx.x;
         const Dims d = A.F.d;
-        if (q >= d.ny * d.nz) continue;
+        if (q >= d.sx()) continue;
         int i, j, k;
         decompose(d, q, i, j, k);
+        if (k >= d.nz) continue;
         const int i0 = chunk * A.march_len;
         fn(A, table[m], i0, min(d.nx, i0 + A.march_len), j, k, q);
     }
@@ -601,90 +591,6 @@ static __global__ void __launch_bounds__(256, NIMBUS_CMARCH_MINB) engine_momentu
         momentum_march<Policy>(A.F, even ? M.rho_alt : M.rho, M.p, A.p0, A.dp0, A.u, A.v, A.w, i0, i1, j, k, q,
                                A.vertical);
     });
-}
-
-// The same two passes with two vertically adjacent cells per thread: a CTA
-// of half a tile's threads takes cells c and c + 1 (c even) of each tile.  In
-// a member whose nz is even the pair lies in one column, so the pair's index,
-// neighbour offsets and member constants are formed once and every field's
-// values at the pair (and at the pair shifted by +-sx or +-sy) are one 8-byte
-// load (continuity_eos_kpair, momentum_kpair); in a member with an odd nz the
-// thread advances its two cells one after the other.  Each cell's arithmetic
-// is the one-cell form's.  ensemble_64, FP32, one lane: continuity
-// 3.49 -> 3.30 ms per step against the one-cell constant-bank form (cells c
-// and c + 128 per thread instead: 3.97), momentum 2.38 against 2.33 marching.
-#ifndef NIMBUS_PAIR_MINB
-#define NIMBUS_PAIR_MINB 8
-#endif
-#ifndef NIMBUS_PAIR_MINB_MOM
-#define NIMBUS_PAIR_MINB_MOM 8
-#endif
-
-template <class Policy, bool kFirst, bool kShared>
-static __global__ void __launch_bounds__(128, NIMBUS_PAIR_MINB) engine_continuity_pair_kernel(const __grid_constant__ AcousticLaunch L,
-                                                                     const EngineMember* __restrict__ table,
-                                                                     long long tiles, int s)
-{
-    const bool even = (s & 1) == 0;
-    const int half = (int)blockDim.x;
-    int m = 0;
-    const int ntiles = (int)tiles;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
-    {
-        while (t >= L.prefix32[m + 1]) ++m;
-        const AcousticConst& A = L.m[m];
-        const FusedParams F = kShared ? with_shared(A.F, L.shared) : A.F;
-        const int n = F.d.cells();
-        const int c0 = (t - L.prefix32[m]) * (2 * half) + 2 * (int)threadIdx.x;
-        if (c0 >= n) continue;
-        const EngineMember& M = table[m];
-        const float* rho = even ? M.rho : M.rho_alt;
-        float* rho_out = even ? M.rho_alt : M.rho;
-        unsigned flags = 0;
-        if ((F.d.nz & 1) == 0)
-            continuity_eos_kpair<Policy>(F, rho, A.u, A.v, A.w, A.theta, A.rho0, A.eos0, rho_out, M.p, A.mfx, A.mfy,
-                                         A.mfz, c0, flags, kFirst, kFirst ? A.rho_begin : nullptr);
-        else
-        {
-            continuity_eos_cell<Policy>(F, rho, A.u, A.v, A.w, A.theta, A.rho0, A.eos0, rho_out, M.p, nullptr, A.mfx,
-                                        A.mfy, A.mfz, c0, flags, kFirst, kFirst ? A.rho_begin : nullptr);
-            if (c0 + 1 < n)
-                continuity_eos_cell<Policy>(F, rho, A.u, A.v, A.w, A.theta, A.rho0, A.eos0, rho_out, M.p, nullptr,
-                                            A.mfx, A.mfy, A.mfz, c0 + 1, flags, kFirst,
-                                            kFirst ? A.rho_begin : nullptr);
-        }
-        if (flags) atomicOr(A.status, flags);
-    }
-}
-
-template <class Policy>
-static __global__ void __launch_bounds__(128, NIMBUS_PAIR_MINB_MOM) engine_momentum_pair_kernel(const __grid_constant__ AcousticLaunch L,
-                                                                       const EngineMember* __restrict__ table,
-                                                                       long long tiles, int s)
-{
-    const bool even = (s & 1) == 0;
-    const int half = (int)blockDim.x;
-    int m = 0;
-    const int ntiles = (int)tiles;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
-    {
-        while (t >= L.prefix32[m + 1]) ++m;
-        const AcousticConst& A = L.m[m];
-        const Dims d = A.F.d;
-        const int n = d.cells();
-        const int c0 = (t - L.prefix32[m]) * (2 * half) + 2 * (int)threadIdx.x;
-        if (c0 >= n) continue;
-        const EngineMember& M = table[m];
-        const float* rho = even ? M.rho_alt : M.rho;
-        if ((d.nz & 1) == 0)
-            momentum_kpair<Policy>(A.F, rho, M.p, A.p0, A.dp0, A.u, A.v, A.w, c0, A.vertical);
-        else
-        {
-            momentum_cell<Policy>(A.F, rho, M.p, A.p0, A.dp0, A.u, A.v, A.w, A.u, A.v, A.w, c0, A.vertical);
-            if (c0 + 1 < n)
-                momentum_cell<Policy>(A.F, rho, M.p, A.p0, A.dp0, A.u, A.v, A.w, A.u, A.v, A.w, c0 + 1, A.vertical);
-        }
-    }
 }
 
 // The same two passes with each tile's stencil data staged in shared memory
@@ -861,6 +767,8 @@ static __global__ void __launch_bounds__(256, NIMBUS_BULK_MINB) engine_continuit
                 const float* S = stages + q * stage_floats;
                 int i, j, k;
                 decompose(d, c, i, j, k);
+                if (k < d.nz)
+                {
                 const bool xlo = i >= 1, xhi = i < d.nx - 1, ylo = j >= 1, yhi = j < d.ny - 1;
                 const bool zlo = k > 0, zhi = k + 1 < d.nz;
                 const float* r1 = S + o_r1 + (c - R.r1.lo);  // rho at the cell
@@ -889,6 +797,7 @@ static __global__ void __launch_bounds__(256, NIMBUS_BULK_MINB) engine_continuit
                                               nullptr, A.mfx, A.mfy, A.mfz, flags, kFirst,
                                               kFirst ? A.rho_begin : nullptr);
                 if (flags) atomicOr(A.status, flags);
+                }
             }
         }
         // Every thread is done with stage q (and agrees whether its wait
@@ -996,7 +905,7 @@ static __global__ void __launch_bounds__(256, NIMBUS_BULK_MINB) engine_momentum_
                 st.uc = S[o_u + ct];
                 st.vc = S[o_v + ct];
                 st.wc = S[o_w + ct];
-                momentum_values<Policy>(A.F, st, i, j, k, c, A.p0, A.dp0, A.u, A.v, A.w, A.vertical);
+                if (k < d.nz) momentum_values<Policy>(A.F, st, i, j, k, c, A.p0, A.dp0, A.u, A.v, A.w, A.vertical);
             }
         }
         if (!__syncthreads_and(ok))
@@ -1015,36 +924,53 @@ static __global__ void __launch_bounds__(256, NIMBUS_BULK_MINB) engine_momentum_
 }
 
 // ---- state image ----------------------------------------------------------
-// The engine's state image holds every member's nine prognostic fields back to
-// back (u, v, w, rho, p, theta, qv, qc, qr, each items[kItemCells] floats) from
-// image + image_offset.  gather = 0 scatters the image into the members'
-// current buffers, gather = 1 collects them into it; one coalesced pass over
-// all cells of all members either way.
+// A member's nine prognostic fields back to back (u, v, w, rho, p, theta, qv,
+// qc, qr, each nx ny nz floats without padding), the host's form of a state.
+// gather = 0 scatters an image into the member's current buffers, gather = 1
+// collects them into it.
+__device__ __forceinline__ void image_cell(const EngineMember& M, float* __restrict__ image, int c, int gather)
+{
+    int i, j, k;
+    const Dims d = M.F.d;
+    decompose(d, c, i, j, k);
+    if (k >= d.nz) return;
+    const long long n = (long long)d.nx * d.ny * d.nz;
+    float* blk = image + (long long)(i * d.ny + j) * d.nz + k;
+    float* const field[9] = {M.u, M.v, M.w, M.rho, M.p, M.theta, M.qv, M.qc, M.qr};
+    float x[9];
+    if (gather)
+    {
+#pragma unroll
+        for (int f = 0; f < 9; ++f) x[f] = field[f][c];
+#pragma unroll
+        for (int f = 0; f < 9; ++f) blk[f * n] = x[f];
+    }
+    else
+    {
+#pragma unroll
+        for (int f = 0; f < 9; ++f) x[f] = blk[f * n];
+#pragma unroll
+        for (int f = 0; f < 9; ++f) field[f][c] = x[f];
+    }
+}
+
+// The engine's state image: every member's from image + image_offset; one
+// coalesced pass over all cells of all members.
 static __global__ void __launch_bounds__(256) engine_image_kernel(const EngineMember* __restrict__ table,
                                                                   const long long* __restrict__ prefix,
                                                                   long long tiles, float* __restrict__ image,
                                                                   int gather)
 {
-    for_member_items(table, prefix, tiles, kItemCells, [&](const EngineMember& M, int c) {
-        const long long n = M.items[kItemCells];
-        float* blk = image + M.image_offset + c;
-        float* const field[9] = {M.u, M.v, M.w, M.rho, M.p, M.theta, M.qv, M.qc, M.qr};
-        float x[9];
-        if (gather)
-        {
-#pragma unroll
-            for (int f = 0; f < 9; ++f) x[f] = field[f][c];
-#pragma unroll
-            for (int f = 0; f < 9; ++f) blk[f * n] = x[f];
-        }
-        else
-        {
-#pragma unroll
-            for (int f = 0; f < 9; ++f) x[f] = blk[f * n];
-#pragma unroll
-            for (int f = 0; f < 9; ++f) field[f][c] = x[f];
-        }
-    });
+    for_member_items(table, prefix, tiles, kItemCells,
+                     [&](const EngineMember& M, int c) { image_cell(M, image + M.image_offset, c, gather); });
+}
+
+// One member's image (its table entry by value, before or beside the table).
+static __global__ void __launch_bounds__(256) member_image_kernel(const __grid_constant__ EngineMember M,
+                                                                  float* __restrict__ image, int gather)
+{
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < M.items[kItemCells]; c += gridDim.x * blockDim.x)
+        image_cell(M, image, c, gather);
 }
 
 // Pointer rotation after the acoustic loop (rho: with an odd substep count
@@ -1215,11 +1141,10 @@ static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_UPDATE_MINB_F32 : 3
 // (src/numerics/runtime.cpp:346-401,854-880).  The member of a tile is
 // block-uniform, so a block keeps a running maximum while it walks one
 // member's tiles and publishes it with one atomicMax when it moves on.
-// One thread reads kScanCells cells (kItemScan tiles), which keeps the
-// per-tile member lookup off the scan's critical path.
-static __global__ void __launch_bounds__(256) engine_sound_speed_kernel(const EngineMember* __restrict__ table,
-                                                                        const long long* __restrict__ prefix,
-                                                                        long long tiles, unsigned long long* c2)
+// One thread reads a group of four cells (one 16-byte load of each field).
+static __global__ void __launch_bounds__(kQuadTile) engine_sound_speed_kernel(const EngineMember* __restrict__ table,
+                                                                              const long long* __restrict__ prefix,
+                                                                              long long tiles, unsigned long long* c2)
 {
     int m = 0, held = -1;
     unsigned long long best = 0;
@@ -1237,14 +1162,15 @@ static __global__ void __launch_bounds__(256) engine_sound_speed_kernel(const En
             best = 0;
         }
         const EngineMember& M = table[m];
-        const int c0 = (int)((t - prefix[m]) * blockDim.x * kScanCells) + (int)threadIdx.x;
+        const int c = 4 * ((int)(t - prefix[m]) * kQuadTile + (int)threadIdx.x);
+        if (c >= M.items[kItemCells]) continue;
         unsigned flags = 0;
+        int i, j, k;
+        decompose(M.F.d, c, i, j, k);
+        const Quad p = load_quad(M.p, c), r = load_quad(M.rho, c);
 #pragma unroll
-        for (int q = 0; q < kScanCells; ++q)
-        {
-            const int c = c0 + q * (int)blockDim.x;
-            if (c < M.items[kItemCells]) best = max(best, sound_speed_sq_bits(M.gamma, M.p[c], M.rho[c], flags));
-        }
+        for (int q = 0; q < 4; ++q)
+            if (k + q < M.F.d.nz) best = max(best, sound_speed_sq_bits(M.gamma, p.v[q], r.v[q], flags));
         if (flags) atomicOr(M.status, flags);
     }
     if (held >= 0)
@@ -1273,6 +1199,9 @@ static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_MICRO_MINB_F32 : 4)
 {
     for_member_items(table, prefix, tiles, kItemCells, [&](const EngineMember& M, int c) {
         unsigned flags = 0;
+        int i, j, k;
+        decompose(M.K.d, c, i, j, k);
+        if (k >= M.K.d.nz) return;
         float4 s;
         const float po = M.p[c];
         if (M.microphysics)
@@ -1289,7 +1218,7 @@ static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_MICRO_MINB_F32 : 4)
         float p_new;
         bool ok;
         if constexpr (kFp32)
-            ok = eos_candidate_value_f32(M.K.d, c, c % M.K.d.nz, M.rho[c], s.x, M.eos0, M.eos_series, M.gamma, true,
+            ok = eos_candidate_value_f32(M.K.d, c, k, M.rho[c], s.x, M.eos0, M.eos_series, M.gamma, true,
                                          po, s.y, s.z, s.w, p_new, flags);
         else
             ok = eos_candidate_value(M.K.d, c, M.rho[c], s.x, M.gamma, true, po, s.y, s.z, s.w, p_new, flags);
@@ -1298,8 +1227,6 @@ static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_MICRO_MINB_F32 : 4)
         // The end-of-step sponge after the EOS projection (dynamics.cpp:7323-7340).
         if (M.R.do_upper | M.R.do_w_only | M.R.do_lateral)
         {
-            int i, j, k;
-            decompose(M.K.d, c, i, j, k);
             float uu = M.u[c], vv = M.v[c], ww = M.w[c], th = s.x;
             if (relax_cell(M.R, M.K.d.nx, M.K.d.ny, i, j, k, uu, vv, ww, th))
             {

@@ -429,6 +429,7 @@ __device__ __forceinline__ void slow_predict_packed(
 {
     int i, j, k;
     decompose(S.d, c, i, j, k);
+    if (k >= S.d.nz) return;
     float tu, tv, tw, tp;
     slow_tendencies_at<Policy>(S, c, i, j, k, PlanarState{u + c, v + c, w + c, p + c}, rho, qv, qc, qr, rho0, qv0, u0,
                                v0, tu, tv, tw, tp);
@@ -447,6 +448,7 @@ __device__ __forceinline__ void slow_correct_packed(
 {
     int i, j, k;
     decompose(S.d, c, i, j, k);
+    if (k >= S.d.nz) return;
     float tu, tv, tw, tp;
     slow_tendencies_at<Policy>(S, c, i, j, k, PackedState{xs + c}, rho, qv, qc, qr, rho0, qv0, u0, v0, tu, tv, tw, tp);
     const float4 a = k1[c];

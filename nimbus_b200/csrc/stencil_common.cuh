@@ -1,6 +1,9 @@
 // Shared device helpers for the C-grid hot-path kernels (sm_100a).
 //
-// Layout: [nx][ny][nz] float, k fastest; cell (i,j,k) at (i*ny + j)*nz + k.
+// Layout: [nx][ny][nz] float, k fastest; cell (i,j,k) at (i*ny + j)*pz + k
+// with the column pitch pz = nz in caller-owned fields.  The member engine
+// pads its columns to a multiple of four cells (pz >= nz), so that every
+// column starts on a 16-byte boundary; cells k >= nz hold no state.
 // Every kernel here is a bandwidth-bound stencil (no tensor-core work), so
 // the design points are coalesced k-contiguous access, grids sized in
 // multiples of the SM count, and as few passes over HBM as the method's
@@ -56,16 +59,17 @@ enum : unsigned
 struct Dims
 {
     int nx, ny, nz;
-    // Division by nz and ny as (x * magic) >> 32 with magic = ceil(2^32 / d)
+    int pz;  // column pitch (cells)
+    // Division by pz and ny as (x * magic) >> 32 with magic = ceil(2^32 / d)
     // = (2^32 + e) / d: floor(x*magic / 2^32) = floor(x / d) whenever
     // x * e < 2^32, since the excess x*e/(d*2^32) then stays below 1/d.
     // make_dims() checks that bound for the largest dividend and leaves the
     // magic at 0 (plain division) when it does not hold.
     unsigned nz_magic = 0, ny_magic = 0;
-    __host__ __device__ __forceinline__ int cells() const { return nx * ny * nz; }
-    __host__ __device__ __forceinline__ int at(int i, int j, int k) const { return (i * ny + j) * nz + k; }
-    __host__ __device__ __forceinline__ int sx() const { return ny * nz; }  // stride of i
-    __host__ __device__ __forceinline__ int sy() const { return nz; }       // stride of j
+    __host__ __device__ __forceinline__ int cells() const { return nx * ny * pz; }  // stored cells
+    __host__ __device__ __forceinline__ int at(int i, int j, int k) const { return (i * ny + j) * pz + k; }
+    __host__ __device__ __forceinline__ int sx() const { return ny * pz; }  // stride of i
+    __host__ __device__ __forceinline__ int sy() const { return pz; }       // stride of j
 };
 
 __host__ __device__ __forceinline__ unsigned div_magic(unsigned d)
@@ -82,14 +86,15 @@ __host__ __device__ __forceinline__ unsigned checked_magic(unsigned d, unsigned 
     return (x_max * e < 0x100000000ull) ? m : 0u;
 }
 
-__host__ __device__ __forceinline__ Dims make_dims(int nx, int ny, int nz)
+__host__ __device__ __forceinline__ Dims make_dims(int nx, int ny, int nz, int pitch = 0)
 {
     Dims d;
     d.nx = nx;
     d.ny = ny;
     d.nz = nz;
-    const unsigned long long cells = (unsigned long long)nx * ny * nz;
-    d.nz_magic = checked_magic((unsigned)nz, cells);
+    d.pz = pitch > nz ? pitch : nz;
+    const unsigned long long cells = (unsigned long long)nx * ny * d.pz;
+    d.nz_magic = checked_magic((unsigned)d.pz, cells);
     d.ny_magic = checked_magic((unsigned)ny, (unsigned long long)nx * ny);
     if (d.nz_magic == 0 || d.ny_magic == 0) d.nz_magic = d.ny_magic = 0;
     return d;
@@ -100,13 +105,13 @@ __device__ __forceinline__ void decompose(const Dims& d, int c, int& i, int& j, 
     if (d.nz_magic != 0)
     {
         const int t = (int)__umulhi((unsigned)c, d.nz_magic);
-        k = c - t * d.nz;
+        k = c - t * d.pz;
         i = (int)__umulhi((unsigned)t, d.ny_magic);
         j = t - i * d.ny;
         return;
     }
-    k = c % d.nz;
-    const int t = c / d.nz;
+    k = c % d.pz;
+    const int t = c / d.pz;
     j = t % d.ny;
     i = t / d.ny;
 }

@@ -689,6 +689,7 @@ __device__ __forceinline__ void transport_faces_cell4(const TP& T, const float4*
     const int kz_end = T.top_open ? d.nz : d.nz - 1;
     int i, j, k;
     decompose(d, c, i, j, k);
+    if (k >= d.nz) return;
     const bool hx = i <= d.nx - 2, hy = j <= d.ny - 2, hz = k < kz_end, top = k == d.nz - 1;
     const float fx = hx ? mfx[c] : 0.0f, fy = hy ? mfy[c] : 0.0f, fz = hz ? mfz[c] : 0.0f;
     const FaceStencil sx = face_stencil(c - i * d.sx(), d.sx(), i, d.nx, fx >= 0.0f, T.weno);
@@ -727,6 +728,7 @@ __device__ __forceinline__ void transport_limiter_cell4(const TP& T, const float
     const size_t n = (size_t)d.cells();
     int i, j, k;
     decompose(d, c, i, j, k);
+    if (k >= d.nz) return;
     const bool xm = i >= 1, xp = i <= d.nx - 2, ym = j >= 1, yp = j <= d.ny - 2, zm = k >= 1;
     const bool zp = k <= d.nz - 2 || (T.top_open && k == d.nz - 1);
     const int cxm = xm ? c - d.sx() : c, cym = ym ? c - d.sy() : c, czm = zm ? c - 1 : c;
@@ -756,6 +758,7 @@ __device__ __forceinline__ void transport_update_cell4(const TP& T, const float4
     const size_t n = (size_t)d.cells();
     int i, j, k;
     decompose(d, c, i, j, k);
+    if (k >= d.nz) return;
     if (!(i >= 1 && i < d.nx - 1 && j >= 1 && j < d.ny - 1))
     {
 #pragma unroll

@@ -240,7 +240,8 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
     if (NIMBUS_SLOW_CONST && n <= kSlowConstMembers)
     {
         std::unique_ptr<SlowLaunch> sl(new SlowLaunch());
-        const long long* p = e->prefix.data() + L.prefix_first + static_cast<size_t>(kItemCells) * (n + 1);
+        const int kind = kFp32 ? kItemQuads : kItemCells;
+        const long long* p = e->prefix.data() + L.prefix_first + static_cast<size_t>(kind) * (n + 1);
         for (int r = 0; r <= n; ++r) sl->prefix[r] = p[r];
         for (int r = 0; r < n; ++r)
         {
@@ -261,8 +262,17 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
             A.u0 = H.u0;
             A.v0 = H.v0;
         }
-        ENGINE_LAUNCH(NIMBUS_KERNEL_SLOW, engine_slow_predict_const_kernel<Policy>, cells, 1, *sl, T, cells);
-        ENGINE_LAUNCH(NIMBUS_KERNEL_SLOW, engine_slow_correct_const_kernel<Policy>, cells, 1, *sl, T, cells);
+        if constexpr (kFp32)
+        {
+            const long long quads = tiles_of(e, L, kItemQuads, n);
+            ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_SLOW, engine_slow_predict_quad_kernel<Policy>, quads, kQuadTile, *sl, T, quads);
+            ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_SLOW, engine_slow_correct_quad_kernel<Policy>, quads, kQuadTile, *sl, T, quads);
+        }
+        else
+        {
+            ENGINE_LAUNCH(NIMBUS_KERNEL_SLOW, engine_slow_predict_const_kernel<Policy>, cells, 1, *sl, T, cells);
+            ENGINE_LAUNCH(NIMBUS_KERNEL_SLOW, engine_slow_correct_const_kernel<Policy>, cells, 1, *sl, T, cells);
+        }
     }
     else
     {

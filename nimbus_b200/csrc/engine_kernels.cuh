@@ -156,11 +156,6 @@ __device__ __forceinline__ void for_member_rows(const EngineMember* __restrict__
 #define NIMBUS_SLOW_MINB_F32 5
 #endif
 template <class Policy>
-constexpr int slow_min_blocks()
-{
-    return sizeof(typename Policy::real) == 4 ? NIMBUS_SLOW_MINB_F32 : NIMBUS_SLOW_MINB;
-}
-template <class Policy>
 static __global__ void __launch_bounds__(256, NIMBUS_SLOW_MINB) engine_slow_predict_kernel(const EngineMember* __restrict__ table,
                                                                   const long long* __restrict__ prefix,
                                                                   long long tiles)
@@ -209,7 +204,7 @@ struct SlowLaunch
 static_assert(sizeof(SlowLaunch) <= 32000, "a kernel parameter block holds at most 32764 bytes");
 
 template <class Policy>
-static __global__ void __launch_bounds__(256, slow_min_blocks<Policy>()) engine_slow_predict_const_kernel(
+static __global__ void __launch_bounds__(256, NIMBUS_SLOW_MINB) engine_slow_predict_const_kernel(
     const __grid_constant__ SlowLaunch L, const EngineMember* __restrict__ table, long long tiles)
 {
     int m = 0;
@@ -227,7 +222,7 @@ static __global__ void __launch_bounds__(256, slow_min_blocks<Policy>()) engine_
 }
 
 template <class Policy>
-static __global__ void __launch_bounds__(256, slow_min_blocks<Policy>()) engine_slow_correct_const_kernel(
+static __global__ void __launch_bounds__(256, NIMBUS_SLOW_MINB) engine_slow_correct_const_kernel(
     const __grid_constant__ SlowLaunch L, const EngineMember* __restrict__ table, long long tiles)
 {
     int m = 0;
@@ -240,6 +235,45 @@ static __global__ void __launch_bounds__(256, slow_min_blocks<Policy>()) engine_
         const EngineMember& M = table[m];
         slow_correct_packed<Policy>(A.S, A.xs, M.rho, A.qv, A.qc, M.qr, A.rho0, A.qv0, A.u0, A.v0, A.k1, A.u, A.v,
                                     A.w, M.p, c);
+    }
+}
+
+// The FP32 form, four cells per thread (slow_tendencies_quad): tiles of
+// kItemQuads, k1 and the predictor as four planes each.
+template <class Policy>
+static __global__ void __launch_bounds__(kQuadTile, NIMBUS_SLOW_MINB_F32) engine_slow_predict_quad_kernel(
+    const __grid_constant__ SlowLaunch L, const EngineMember* __restrict__ table, long long tiles)
+{
+    int m = 0;
+    for (long long t = blockIdx.x; t < tiles; t += gridDim.x)
+    {
+        while (t >= L.prefix[m + 1]) ++m;
+        const SlowConst& A = L.m[m];
+        const int n = A.S.d.cells(), c = 4 * ((int)(t - L.prefix[m]) * kQuadTile + (int)threadIdx.x);
+        if (c >= n) continue;
+        const EngineMember& M = table[m];
+        slow_predict_quad(A.S, A.u, A.v, A.w, M.rho, M.p, A.qv, A.qc, M.qr, A.rho0, A.qv0, A.u0, A.v0,
+                          reinterpret_cast<float*>(A.k1), reinterpret_cast<float*>(A.xs), (size_t)n, c);
+        const Quad th = load_quad(A.theta, c), qv = load_quad(A.qv, c), qc = load_quad(A.qc, c), qr = load_quad(M.qr, c);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) A.q4[c + q] = make_float4(th.v[q], qv.v[q], qc.v[q], qr.v[q]);
+    }
+}
+
+template <class Policy>
+static __global__ void __launch_bounds__(kQuadTile, NIMBUS_SLOW_MINB_F32) engine_slow_correct_quad_kernel(
+    const __grid_constant__ SlowLaunch L, const EngineMember* __restrict__ table, long long tiles)
+{
+    int m = 0;
+    for (long long t = blockIdx.x; t < tiles; t += gridDim.x)
+    {
+        while (t >= L.prefix[m + 1]) ++m;
+        const SlowConst& A = L.m[m];
+        const int n = A.S.d.cells(), c = 4 * ((int)(t - L.prefix[m]) * kQuadTile + (int)threadIdx.x);
+        if (c >= n) continue;
+        const EngineMember& M = table[m];
+        slow_correct_quad(A.S, reinterpret_cast<const float*>(A.xs), M.rho, A.qv, A.qc, M.qr, A.rho0, A.qv0, A.u0,
+                          A.v0, reinterpret_cast<const float*>(A.k1), (size_t)n, A.u, A.v, A.w, M.p, c);
     }
 }
 

@@ -14,6 +14,7 @@
 #pragma once
 
 #include "acoustic_fused.cuh"
+#include "acoustic_split.cuh"
 
 namespace nimbus
 {
@@ -460,6 +461,325 @@ __device__ __forceinline__ void slow_correct_packed(
     v[c] = slow_apply_one<Policy>(S, v[c], tv);
     w[c] = slow_apply_one<Policy>(S, w[c], tw);
     p[c] = slow_apply_one<Policy>(S, p[c], tp);
+}
+
+// ---- Four vertically adjacent cells per thread (FP32 form) ------------------
+// The slow tendencies of cells c .. c + 3 (k a multiple of 4, columns on
+// 16-byte boundaries; acoustic_split.cuh has the reasons for the quad).  A
+// stencil point of the four cells along x or y is one 16-byte load, the ten
+// points along z three; one axis and field at a time, each block of loads
+// ending at a barrier to the compiler's reordering, so that one block's
+// registers serve the next.  The arithmetic of each cell is
+// slow_tendencies_at's.  (FP64 arithmetic needs twice the registers and keeps
+// the one-cell form.)
+struct QuadStencil
+{
+    Quad m3, m2, m1, c, p1, p2, p3;
+};
+
+// The points of f along one axis (stride) around cells c .. c + 3, as far as
+// the half-width allows; the centre is given.
+__device__ __forceinline__ QuadStencil load_stencil(const float* __restrict__ f, int c, int stride, int half,
+                                                    const Quad& centre)
+{
+    QuadStencil t;
+    t.c = centre;
+    t.m1 = load_quad(f, c - stride);
+    t.p1 = load_quad(f, c + stride);
+    t.m2 = t.p2 = t.m3 = t.p3 = centre;
+    if (half >= 2)
+    {
+        t.m2 = load_quad(f, c - 2 * stride);
+        t.p2 = load_quad(f, c + 2 * stride);
+    }
+    if (half >= 3)
+    {
+        t.m3 = load_quad(f, c - 3 * stride);
+        t.p3 = load_quad(f, c + 3 * stride);
+    }
+    return t;
+}
+
+// Upwind derivative of the four cells along x or y (one half-width for all).
+__device__ __forceinline__ Quad upwind_quad(const QuadStencil& t, int half, const Quad& a, float inv_d, float d6,
+                                            float d60)
+{
+    Quad o;
+    if (half >= 3)
+    {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            o.v[q] = upwind_from<float>(3, t.c.v[q], t.m1.v[q], t.p1.v[q], t.m2.v[q], t.p2.v[q], t.m3.v[q], t.p3.v[q],
+                                        a.v[q], inv_d, d6, d60);
+    }
+    else
+    {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            o.v[q] = upwind_from<float>(half, t.c.v[q], t.m1.v[q], t.p1.v[q], t.m2.v[q], t.p2.v[q], 0.0f, 0.0f,
+                                        a.v[q], inv_d, d6, d60);
+    }
+    return o;
+}
+
+// Upwind derivative along z: lo, c, hi are the groups of four around the
+// cells (values past the column's ends are not used).  Every cell is formed
+// as an inner one; the groups at the column's ends redo the cells whose
+// half-width is smaller.  vertical_w: f is w, whose ground face is 0.
+__device__ __forceinline__ Quad upwind_quad_z(const Quad& lo, const Quad& cc, const Quad& hi, int k, int nz,
+                                              const Quad& a, float inv_d, float d6, float d60, bool vertical_w)
+{
+    const float t[10] = {lo.v[1], lo.v[2], lo.v[3], cc.v[0], cc.v[1], cc.v[2], cc.v[3], hi.v[0], hi.v[1], hi.v[2]};
+    Quad o;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        o.v[q] = upwind_from<float>(3, t[q + 3], t[q + 2], t[q + 4], t[q + 1], t[q + 5], t[q], t[q + 6], a.v[q], inv_d,
+                                    d6, d60);
+    if (k < 3 || k + 3 > nz - 4)
+    {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            const int kq = k + q, half = min(kq, nz - 1 - kq);
+            if (kq == 0)
+                o.v[q] = (a.v[q] >= 0.0f) ? (vertical_w ? (t[q + 3] - 0.0f) * inv_d : 0.0f)
+                                          : (t[q + 4] - t[q + 3]) * inv_d;
+            else if (half < 3)
+                o.v[q] = upwind_from<float>(half, t[q + 3], t[q + 2], t[q + 4], t[q + 1], t[q + 5], 0.0f, 0.0f, a.v[q],
+                                            inv_d, d6, d60);
+        }
+    }
+    return o;
+}
+
+// f at the four cells one level up (next: the value at c + 4).
+__device__ __forceinline__ Quad level_up(const Quad& f, float next)
+{
+    return Quad{{f.v[1], f.v[2], f.v[3], next}};
+}
+
+__device__ __forceinline__ void slow_tendencies_quad(const SlowParams& S, int c, int i, int j, int k,
+                                                     const float* __restrict__ u, const float* __restrict__ v,
+                                                     const float* __restrict__ w, const float* __restrict__ p,
+                                                     const float* __restrict__ rho, const float* __restrict__ qv,
+                                                     const float* __restrict__ qc, const float* __restrict__ qr,
+                                                     const double* __restrict__ rho0, const double* __restrict__ qv0,
+                                                     const double* __restrict__ u0, const double* __restrict__ v0,
+                                                     Quad& out_u, Quad& out_v, Quad& out_w, Quad& out_p)
+{
+    const Dims d = S.d;
+    out_u = out_v = out_w = out_p = Quad{{0.0f, 0.0f, 0.0f, 0.0f}};
+    if (!(i >= 1 && i < d.nx - 1 && j >= 1 && j < d.ny - 1)) return;
+    const int sx = d.sx(), sy = d.sy();
+    const int hx = min(i, d.nx - 1 - i), hy = min(j, d.ny - 1 - j);
+    const float fu = S.frame_u_f, fv = S.frame_v_f, cf = S.coriolis_f_f;
+    const float inv_dx = S.inv_dx_f, inv_dy = S.inv_dy_f, inv_dz = S.inv_dz_f;
+    const float x6 = S.d6_f[0], y6 = S.d6_f[1], z6 = S.d6_f[2];
+    const float x60 = S.d60_f[0], y60 = S.d60_f[1], z60 = S.d60_f[2];
+    const float h = 0.5f, qt = 0.25f;
+    // Every product wind * derivative of a cell enters its sum in the order x, y, z.
+    Quad tx_u, tx_v, tx_w, dxu, dxv, dxw;  // advecting winds and derivatives along x
+    Quad tuc, tvc, wc;                     // centre winds of the pressure
+    const Quad uc = load_quad(u, c), vc = load_quad(v, c), wz = load_quad(w, c);
+    {
+        const QuadStencil t = load_stencil(u, c, sx, hx, uc);
+        const Quad n = load_quad(u, c + sy), nw = load_quad(u, c + sy - sx);
+        const float up = u[c + 4], upw = u[c + 4 - sx];
+        const Quad a = level_up(uc, up), b = level_up(t.m1, upw);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            tx_u.v[q] = uc.v[q] - fu;
+            const float ux_v = qt * (t.m1.v[q] + uc.v[q] + nw.v[q] + n.v[q]);
+            tx_v.v[q] = ux_v - fu;
+            out_v.v[q] = ux_v;  // kept for the Coriolis term
+            const float ux_w = qt * (t.m1.v[q] + uc.v[q] + b.v[q] + a.v[q]);
+            tx_w.v[q] = ux_w - fu;
+            tuc.v[q] = h * (uc.v[q] + t.m1.v[q]) - fu;
+        }
+        dxu = upwind_quad(t, hx, tx_u, inv_dx, x6, x60);
+    }
+    load_stage();
+    dxv = upwind_quad(load_stencil(v, c, sx, hx, vc), hx, tx_v, inv_dx, x6, x60);
+    load_stage();
+    dxw = upwind_quad(load_stencil(w, c, sx, hx, wz), hx, tx_w, inv_dx, x6, x60);
+    load_stage();
+    Quad ty_u, ty_w, dyu, dyv, dyw;
+    Quad sum_u, sum_v, sum_w;
+    {
+        const QuadStencil t = load_stencil(v, c, sy, hy, vc);
+        const Quad e = load_quad(v, c + sx), es = load_quad(v, c + sx - sy);
+        const float up = v[c + 4], ups = v[c + 4 - sy];
+        const Quad a = level_up(vc, up), b = level_up(t.m1, ups);
+        Quad tvy;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            tvy.v[q] = vc.v[q] - fv;
+            const float uy_u = qt * (t.m1.v[q] + vc.v[q] + es.v[q] + e.v[q]);
+            ty_u.v[q] = uy_u - fv;
+            out_u.v[q] = uy_u;  // kept for the Coriolis term
+            const float uy_w = qt * (t.m1.v[q] + vc.v[q] + b.v[q] + a.v[q]);
+            ty_w.v[q] = uy_w - fv;
+            tvc.v[q] = h * (vc.v[q] + t.m1.v[q]) - fv;
+        }
+        dyv = upwind_quad(t, hy, tvy, inv_dy, y6, y60);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sum_v.v[q] = -tx_v.v[q] * dxv.v[q] - tvy.v[q] * dyv.v[q];
+    }
+    load_stage();
+    dyu = upwind_quad(load_stencil(u, c, sy, hy, uc), hy, ty_u, inv_dy, y6, y60);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sum_u.v[q] = -tx_u.v[q] * dxu.v[q] - ty_u.v[q] * dyu.v[q];
+    load_stage();
+    dyw = upwind_quad(load_stencil(w, c, sy, hy, wz), hy, ty_w, inv_dy, y6, y60);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sum_w.v[q] = -tx_w.v[q] * dxw.v[q] - ty_w.v[q] * dyw.v[q];
+    load_stage();
+    // Along z: the group below and above in the column (c - 4 and c + 4 are
+    // cells of the member for every interior column).
+    {
+        const Quad lo = load_quad(w, c - 4), hi = load_quad(w, c + 4);
+        const Quad wxe = load_quad(w, c + sx), wyn = load_quad(w, c + sy);
+        const float wxb = w[c + sx - 1], wyb = w[c + sy - 1];
+        Quad wx, wy;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            const float below = q > 0 ? wz.v[q > 0 ? q - 1 : 0] : lo.v[3];
+            const float xb = q > 0 ? wxe.v[q > 0 ? q - 1 : 0] : wxb, yb = q > 0 ? wyn.v[q > 0 ? q - 1 : 0] : wyb;
+            const bool ground = k + q == 0;
+            wx.v[q] = ground ? qt * (wz.v[q] + wxe.v[q]) : qt * (below + wz.v[q] + xb + wxe.v[q]);
+            wy.v[q] = ground ? qt * (wz.v[q] + wyn.v[q]) : qt * (below + wz.v[q] + yb + wyn.v[q]);
+            wc.v[q] = h * (wz.v[q] + below);
+        }
+        const Quad dzw = upwind_quad_z(lo, wz, hi, k, d.nz, wz, inv_dz, z6, z60, true);
+        const Quad ul = load_quad(u, c - 4), uh = load_quad(u, c + 4);
+        const Quad dzu = upwind_quad_z(ul, uc, uh, k, d.nz, wx, inv_dz, z6, z60, false);
+        const Quad vl = load_quad(v, c - 4), vh = load_quad(v, c + 4);
+        const Quad dzv = upwind_quad_z(vl, vc, vh, k, d.nz, wy, inv_dz, z6, z60, false);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            const bool on = k + q < d.nz - 1;
+            const float v0k = v0 && on ? (float)v0[k + q] : 0.0f, u0k = u0 && on ? (float)u0[k + q] : 0.0f;
+            const float du = sum_u.v[q] - wx.v[q] * dzu.v[q] + cf * (out_u.v[q] - v0k);
+            const float dv = sum_v.v[q] - wy.v[q] * dzv.v[q] - cf * (out_v.v[q] - u0k);
+            out_u.v[q] = on && isfinite(du) ? du : 0.0f;
+            out_v.v[q] = on && isfinite(dv) ? dv : 0.0f;
+            sum_w.v[q] = sum_w.v[q] - wz.v[q] * dzw.v[q];
+        }
+    }
+    load_stage();
+    // Buoyancy, vapour and loading on w.
+    {
+        const float g = S.gravity_f;
+        const Quad r = load_quad(rho, c);
+        const Quad r1 = level_up(r, rho[c + 4]);
+        Quad a{}, a1{}, b{}, b1{}, e{}, e1{};
+        if (S.moist)
+        {
+            a = load_quad(qv, c);
+            a1 = level_up(a, qv[c + 4]);
+        }
+        if (S.loading)
+        {
+            b = load_quad(qc, c);
+            b1 = level_up(b, qc[c + 4]);
+            e = load_quad(qr, c);
+            e1 = level_up(e, qr[c + 4]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            const int kq = k + q;
+            if (kq >= d.nz - 1) continue;
+            const float rho_face = 0.5f * (r.v[q] + r1.v[q]);
+            const float rho_s = (isfinite(rho_face) && rho_face > 1.0e-6f) ? rho_face : 1.0f;
+            const float rho0_face = (float)(0.5 * (rho0[kq] + rho0[kq + 1]));
+            float forcing = -g * (rho_face - rho0_face) / rho_s;
+            if (S.moist)
+            {
+                const float qf = 0.5f * (a.v[q] + a1.v[q]);
+                const float q0f = (float)(0.5 * ((double)(float)qv0[kq] + (double)(float)qv0[kq + 1]));
+                forcing += g * 0.608f * (qf - q0f);
+            }
+            if (S.loading) forcing += -g * (0.5f * ((b.v[q] + e.v[q]) + (b1.v[q] + e1.v[q])));
+            const float dw = sum_w.v[q] + forcing;
+            out_w.v[q] = isfinite(dw) ? dw : 0.0f;
+        }
+    }
+    load_stage();
+    // Pressure at the centres.
+    {
+        const float hx2 = S.half_inv_dx_f, hy2 = S.half_inv_dy_f, hz2 = S.half_inv_dz_f;
+        const Quad pc = load_quad(p, c);
+        const Quad pe = load_quad(p, c + sx), pw = load_quad(p, c - sx);
+        const Quad pn = load_quad(p, c + sy), ps = load_quad(p, c - sy);
+        const float pb = p[c - 1], pt = p[c + 4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            const float up = q < 3 ? pc.v[q < 3 ? q + 1 : 3] : pt, dn = q > 0 ? pc.v[q > 0 ? q - 1 : 0] : pb;
+            const float dpdx = (pe.v[q] - pw.v[q]) * hx2;
+            const float dpdy = (pn.v[q] - ps.v[q]) * hy2;
+            const float dpdz = (up - dn) * hz2;
+            const float dp = -tuc.v[q] * dpdx - tvc.v[q] * dpdy - wc.v[q] * dpdz;
+            out_p.v[q] = k + q >= 1 && k + q < d.nz - 1 && isfinite(dp) ? dp : 0.0f;
+        }
+    }
+}
+
+// k1 and the predictor of four cells, each as four planes {u, v, w, p} of
+// `plane` cells.
+__device__ __forceinline__ void slow_predict_quad(
+    const SlowParams& S, const float* __restrict__ u, const float* __restrict__ v, const float* __restrict__ w,
+    const float* __restrict__ rho, const float* __restrict__ p, const float* __restrict__ qv,
+    const float* __restrict__ qc, const float* __restrict__ qr, const double* __restrict__ rho0,
+    const double* __restrict__ qv0, const double* __restrict__ u0, const double* __restrict__ v0,
+    float* __restrict__ k1, float* __restrict__ xs, size_t plane, int c)
+{
+    int i, j, k;
+    decompose(S.d, c, i, j, k);
+    Quad t[4];
+    slow_tendencies_quad(S, c, i, j, k, u, v, w, p, rho, qv, qc, qr, rho0, qv0, u0, v0, t[0], t[1], t[2], t[3]);
+    const float* const x[4] = {u, v, w, p};
+#pragma unroll
+    for (int f = 0; f < 4; ++f)
+    {
+        store_quad(k1 + f * plane, c, t[f]);
+        Quad y = load_quad(x[f], c);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) y.v[q] = slow_apply_one<Fp32Policy>(S, y.v[q], t[f].v[q]);
+        store_quad(xs + f * plane, c, y);
+    }
+}
+
+// k2 at the predictor, the Heun average and its application; the averaged
+// tendencies to `out` (four planes) when given.
+__device__ __forceinline__ void slow_correct_quad(
+    const SlowParams& S, const float* __restrict__ xs, const float* __restrict__ rho, const float* __restrict__ qv,
+    const float* __restrict__ qc, const float* __restrict__ qr, const double* __restrict__ rho0,
+    const double* __restrict__ qv0, const double* __restrict__ u0, const double* __restrict__ v0,
+    const float* __restrict__ k1, size_t plane, float* __restrict__ u, float* __restrict__ v, float* __restrict__ w,
+    float* __restrict__ p, int c)
+{
+    int i, j, k;
+    decompose(S.d, c, i, j, k);
+    Quad t[4];
+    slow_tendencies_quad(S, c, i, j, k, xs, xs + plane, xs + 2 * plane, xs + 3 * plane, rho, qv, qc, qr, rho0, qv0, u0,
+                         v0, t[0], t[1], t[2], t[3]);
+    float* const x[4] = {u, v, w, p};
+#pragma unroll
+    for (int f = 0; f < 4; ++f)
+    {
+        const Quad a = load_quad(k1 + f * plane, c);
+        Quad y = load_quad(x[f], c);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            y.v[q] = slow_apply_one<Fp32Policy>(S, y.v[q], __fmul_rn(0.5f, __fadd_rn(t[f].v[q], a.v[q])));
+        store_quad(x[f], c, y);
+    }
 }
 
 template <class Policy>

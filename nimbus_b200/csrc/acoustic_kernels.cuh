@@ -11,10 +11,8 @@
 //                    of a ping-pong pair (neighbours still need the old rho);
 //                    p is written in place (the old p is never read).
 //   momentum       : u,v,w forward Euler from the new pressure gradient.
-//   bc_we, bc_sn, bc_vertical : the boundary closure in the reference's
-//                    face order W,E -> S,N -> vertical.  Each thread owns one
-//                    boundary row, so within a kernel W precedes E (and S
-//                    precedes N) exactly as in the reference's sequential loops.
+//   bc_ring        : the boundary closure in the reference's face order
+//                    W,E -> S,N -> vertical, one launch (bc_ring_levels).
 #pragma once
 
 #include "stencil_common.cuh"
@@ -166,152 +164,146 @@ __device__ __forceinline__ float kw78_updated_face(float previous, float phase, 
     return __fsub_rn(previous, increment);
 }
 
-// West then east faces for one (j,k) row r: boundary_conditions_cartesian_cgrid.cpp:927-1032.
-__device__ __forceinline__ void bc_we_row(const BoundaryParams& B, float* __restrict__ u, float* __restrict__ v,
-                                          float* __restrict__ w, float* __restrict__ rho, float* __restrict__ p,
-                                          float* __restrict__ u_west, float* __restrict__ u_east, int r)
+// V consecutive levels of a field (V = 4: one 16-byte access, where columns and
+// field bases allow it; else V = 1).
+template <int V>
+struct Levels
 {
-    const Dims d = B.d;
-    const bool radiate = B.dt_rad > 0.0f;
+    float v[V];
+};
+
+template <int V>
+__device__ __forceinline__ Levels<V> load_levels(const float* f)
+{
+    Levels<V> o;
+    if constexpr (V == 4)
     {
-        const int j = r / d.nz, k = r % d.nz;
-        // ---- West: ghost i=0, wall face u[0] ----
+        const float4 t = *reinterpret_cast<const float4*>(f);
+        o.v[0] = t.x;
+        o.v[1] = t.y;
+        o.v[2] = t.z;
+        o.v[3] = t.w;
+    }
+    else o.v[0] = *f;
+    return o;
+}
+
+template <int V>
+__device__ __forceinline__ void store_levels(float* f, const Levels<V>& x)
+{
+    if constexpr (V == 4) *reinterpret_cast<float4*>(f) = make_float4(x.v[0], x.v[1], x.v[2], x.v[3]);
+    else *f = x.v[0];
+}
+
+// One lateral axis of the closure: its cells and their stride, the codes of its
+// low (west / south) and high (east / north) face, 1 / spacing and the frame's
+// velocity along the axis and across it.
+struct BoundaryAxis
+{
+    int n, stride, lo, hi;
+    float inv, frame_n, frame_c;
+};
+
+// The low then the high face of one row along an axis, for V levels from
+// `base` (the row's cell 0): boundary_conditions_cartesian_cgrid.cpp:927-1121.
+// normal and cross are the velocities along and across the axis; hist_lo and
+// hist_hi the rows' KW78 memory.  The faces share no cell (n >= 4; the low one
+// writes cell 0, the high one reads cells 1 and up), so every value is loaded
+// before any is stored.
+template <int V>
+__device__ __forceinline__ void bc_axis_row(const BoundaryAxis& A, float dt_rad, float* normal, float* cross, float* w,
+                                            float* rho, float* p, float* hist_lo, float* hist_hi, int base)
+{
+    const bool radiate = dt_rad > 0.0f;
+    const bool rad_lo = A.lo == kBcRadiative && radiate, rad_hi = A.hi == kBcRadiative && radiate;
+    const int in = base + A.stride, a = base + (A.n - 2) * A.stride;
+    const int g0 = base, g1 = base + (A.n - 1) * A.stride, am = base + (A.n - 3) * A.stride;
+    const int sl = A.lo == kBcPeriodic ? a : in, sh = A.hi == kBcPeriodic ? in : a;
+    Levels<V> nl = load_levels<V>(normal + sl), cl = load_levels<V>(cross + sl), wl = load_levels<V>(w + sl);
+    const Levels<V> rl = load_levels<V>(rho + sl), pl = load_levels<V>(p + sl);
+    Levels<V> nh = load_levels<V>(normal + sh), ch = load_levels<V>(cross + sh), wh = load_levels<V>(w + sh);
+    const Levels<V> rh = load_levels<V>(rho + sh), ph = load_levels<V>(p + sh);
+    const Levels<V> nm = load_levels<V>(normal + am);
+    Levels<V> fl = nl, fh = nh;  // the faces' memory
+    if (rad_lo) fl = load_levels<V>(hist_lo);
+    if (rad_hi) fh = load_levels<V>(hist_hi);
+    // ---- low: ghost 0, wall face normal[0] ----
+    bool store_n = true;
+    if (A.lo != kBcPeriodic)
+    {
+        if (A.lo == kBcRadiative)
         {
-            const int g = d.at(0, j, k), in = d.at(1, j, k);
-            if (B.west == kBcPeriodic)
+            store_n = rad_lo;
+            if (rad_lo)
             {
-                const int s = d.at(d.nx - 2, j, k);
-                u[g] = u[s]; v[g] = v[s]; w[g] = w[s]; rho[g] = rho[s]; p[g] = p[s];
-            }
-            else
-            {
-                if (B.west == kBcRadiative)
+#pragma unroll
+                for (int q = 0; q < V; ++q)
                 {
-                    if (radiate)
-                    {
-                        const float up = u_west[r];
-                        const float phase = __fsub_rn(__fsub_rn(up, B.frame_u), kCStar);
-                        const float un = kw78_updated_face(up, phase, __fsub_rn(u[in], up), B.dt_rad, B.inv_dx, true);
-                        u[g] = un;
-                        u_west[r] = un;
-                    }
+                    const float up = fl.v[q];
+                    const float phase = __fsub_rn(__fsub_rn(up, A.frame_n), kCStar);
+                    nl.v[q] = kw78_updated_face(up, phase, __fsub_rn(nl.v[q], up), dt_rad, A.inv, true);
                 }
-                else if (B.west == kBcZeroGradient) u[g] = u[in];
-                else u[g] = B.frame_u;
-                if (B.west == kBcRigid) { v[g] = B.frame_v; w[g] = 0.0f; }
-                else { v[g] = v[in]; w[g] = w[in]; }
-                rho[g] = rho[in]; p[g] = p[in];
+                store_levels<V>(hist_lo, nl);
             }
         }
-        // ---- East: ghost i=nx-1, wall face u[nx-2] ----
+        else if (A.lo != kBcZeroGradient)
         {
-            const int g = d.at(d.nx - 1, j, k), a = d.at(d.nx - 2, j, k), am = d.at(d.nx - 3, j, k);
-            if (B.east == kBcPeriodic)
+#pragma unroll
+            for (int q = 0; q < V; ++q) nl.v[q] = A.frame_n;
+        }
+        if (A.lo == kBcRigid)
+        {
+#pragma unroll
+            for (int q = 0; q < V; ++q)
             {
-                const int s = d.at(1, j, k);
-                u[g] = u[s]; v[g] = v[s]; w[g] = w[s]; rho[g] = rho[s]; p[g] = p[s];
-            }
-            else
-            {
-                if (B.east == kBcRigid || B.east == kBcRigidSlip) u[a] = B.frame_u;
-                if (B.east == kBcRadiative && radiate)
-                {
-                    const float up = u_east[r];
-                    const float phase = __fadd_rn(__fsub_rn(up, B.frame_u), kCStar);
-                    const float un = kw78_updated_face(up, phase, __fsub_rn(up, u[am]), B.dt_rad, B.inv_dx, false);
-                    u[a] = un;
-                    u_east[r] = un;
-                }
-                else if (B.east == kBcZeroGradient) u[a] = u[am];
-                u[g] = (B.east == kBcRadiative || B.east == kBcZeroGradient) ? u[a] : B.frame_u;
-                if (B.east == kBcRigid) { v[g] = B.frame_v; w[g] = 0.0f; }
-                else { v[g] = v[a]; w[g] = w[a]; }
-                rho[g] = rho[a]; p[g] = p[a];
+                cl.v[q] = A.frame_c;
+                wl.v[q] = 0.0f;
             }
         }
     }
-}
-
-static __global__ void acoustic_bc_we_kernel(BoundaryParams B, float* __restrict__ u, float* __restrict__ v,
-                                      float* __restrict__ w, float* __restrict__ rho, float* __restrict__ p,
-                                      float* __restrict__ u_west, float* __restrict__ u_east)
-{
-    const int rows = B.d.ny * B.d.nz;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x)
-        bc_we_row(B, u, v, w, rho, p, u_west, u_east, r);
-}
-
-// South then north faces for one (i,k) row r: boundary_conditions_cartesian_cgrid.cpp:1034-1121.
-__device__ __forceinline__ void bc_sn_row(const BoundaryParams& B, float* __restrict__ u, float* __restrict__ v,
-                                          float* __restrict__ w, float* __restrict__ rho, float* __restrict__ p,
-                                          float* __restrict__ v_south, float* __restrict__ v_north, int r)
-{
-    const Dims d = B.d;
-    const bool radiate = B.dt_rad > 0.0f;
+    if (store_n) store_levels<V>(normal + g0, nl);
+    store_levels<V>(cross + g0, cl);
+    store_levels<V>(w + g0, wl);
+    store_levels<V>(rho + g0, rl);
+    store_levels<V>(p + g0, pl);
+    // ---- high: ghost n-1, wall face normal[n-2] ----
+    if (A.hi != kBcPeriodic)
     {
-        const int i = r / d.nz, k = r % d.nz;
+        bool store_a = true;
+        if (A.hi == kBcRigid || A.hi == kBcRigidSlip)
         {
-            const int g = d.at(i, 0, k), in = d.at(i, 1, k);
-            if (B.south == kBcPeriodic)
-            {
-                const int s = d.at(i, d.ny - 2, k);
-                v[g] = v[s]; u[g] = u[s]; w[g] = w[s]; rho[g] = rho[s]; p[g] = p[s];
-            }
-            else
-            {
-                if (B.south == kBcRadiative)
-                {
-                    if (radiate)
-                    {
-                        const float vp = v_south[r];
-                        const float phase = __fsub_rn(__fsub_rn(vp, B.frame_v), kCStar);
-                        const float vn = kw78_updated_face(vp, phase, __fsub_rn(v[in], vp), B.dt_rad, B.inv_dy, true);
-                        v[g] = vn;
-                        v_south[r] = vn;
-                    }
-                }
-                else if (B.south == kBcZeroGradient) v[g] = v[in];
-                else v[g] = B.frame_v;
-                if (B.south == kBcRigid) { u[g] = B.frame_u; w[g] = 0.0f; }
-                else { u[g] = u[in]; w[g] = w[in]; }
-                rho[g] = rho[in]; p[g] = p[in];
-            }
+#pragma unroll
+            for (int q = 0; q < V; ++q) nh.v[q] = A.frame_n;
         }
+        else if (rad_hi)
         {
-            const int g = d.at(i, d.ny - 1, k), a = d.at(i, d.ny - 2, k), am = d.at(i, d.ny - 3, k);
-            if (B.north == kBcPeriodic)
+#pragma unroll
+            for (int q = 0; q < V; ++q)
             {
-                const int s = d.at(i, 1, k);
-                v[g] = v[s]; u[g] = u[s]; w[g] = w[s]; rho[g] = rho[s]; p[g] = p[s];
+                const float up = fh.v[q];
+                const float phase = __fadd_rn(__fsub_rn(up, A.frame_n), kCStar);
+                nh.v[q] = kw78_updated_face(up, phase, __fsub_rn(up, nm.v[q]), dt_rad, A.inv, false);
             }
-            else
+            store_levels<V>(hist_hi, nh);
+        }
+        else if (A.hi == kBcZeroGradient) nh = nm;
+        else store_a = false;  // radiative without radiation keeps its face
+        if (store_a) store_levels<V>(normal + a, nh);
+        if (A.hi == kBcRigid)
+        {
+#pragma unroll
+            for (int q = 0; q < V; ++q)
             {
-                if (B.north == kBcRigid || B.north == kBcRigidSlip) v[a] = B.frame_v;
-                if (B.north == kBcRadiative && radiate)
-                {
-                    const float vp = v_north[r];
-                    const float phase = __fadd_rn(__fsub_rn(vp, B.frame_v), kCStar);
-                    const float vn = kw78_updated_face(vp, phase, __fsub_rn(vp, v[am]), B.dt_rad, B.inv_dy, false);
-                    v[a] = vn;
-                    v_north[r] = vn;
-                }
-                else if (B.north == kBcZeroGradient) v[a] = v[am];
-                v[g] = (B.north == kBcRadiative || B.north == kBcZeroGradient) ? v[a] : B.frame_v;
-                if (B.north == kBcRigid) { u[g] = B.frame_u; w[g] = 0.0f; }
-                else { u[g] = u[a]; w[g] = w[a]; }
-                rho[g] = rho[a]; p[g] = p[a];
+                ch.v[q] = A.frame_c;
+                wh.v[q] = 0.0f;
             }
         }
     }
-}
-
-static __global__ void acoustic_bc_sn_kernel(BoundaryParams B, float* __restrict__ u, float* __restrict__ v,
-                                      float* __restrict__ w, float* __restrict__ rho, float* __restrict__ p,
-                                      float* __restrict__ v_south, float* __restrict__ v_north)
-{
-    const int rows = B.d.nx * B.d.nz;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x)
-        bc_sn_row(B, u, v, w, rho, p, v_south, v_north, r);
+    store_levels<V>(normal + g1, nh);
+    store_levels<V>(cross + g1, ch);
+    store_levels<V>(w + g1, wh);
+    store_levels<V>(rho + g1, rh);
+    store_levels<V>(p + g1, ph);
 }
 
 // Vertical closure for one (i,j) column: boundary_conditions_cartesian_cgrid.cpp:1124-1175.
@@ -339,6 +331,125 @@ static __global__ void acoustic_bc_vertical_kernel(BoundaryParams B, float* __re
     const int cols = B.d.nx * B.d.ny;
     for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < cols; col += gridDim.x * blockDim.x)
         bc_vertical_column(B, u, v, w, col);
+}
+
+// Columns whose vertical closure the momentum pass may apply itself: those no
+// lateral closure writes or reads.  The others are the perimeter.
+__device__ __forceinline__ bool bc_inner_column(const Dims& d, int i, int j)
+{
+    return i >= 2 && i <= d.nx - 4 && j >= 2 && j <= d.ny - 4;
+}
+
+// The closure is independent from level to level except for the top level,
+// which takes the one below: a CTA closes a band of four levels (the last one
+// up to seven) all around the member, with a block barrier between the
+// reference's steps W,E -> S,N -> vertical instead of a launch.  A ring is a
+// few thousand values, so its time is the latency of its chain of loads and
+// stores: three launches took 19 us between events at every size up to
+// 160x160x56, one takes a third of that.
+constexpr int kRingLevels = 4;
+constexpr int kRingBlock = 512;
+
+__host__ __device__ __forceinline__ int ring_bands(int nz)
+{
+    const int bands = (nz + kRingLevels - 1) / kRingLevels;
+    return nz % kRingLevels == 1 && bands > 1 ? bands - 1 : bands;  // the top two levels in one band
+}
+
+// One band.  vertical: also close the perimeter's columns (their bottom and
+// top levels, in the bands that hold them); seed: then fill the KW78 memory
+// from the closed faces (seed_radiative_state).  Every thread of the block
+// calls it.
+template <int V>
+__device__ __forceinline__ void bc_ring_levels(const BoundaryParams& B, float* u, float* v, float* w, float* rho,
+                                               float* p, float* wave, int band, bool vertical, bool seed)
+{
+    const Dims d = B.d;
+    const int last = ring_bands(d.nz) - 1;
+    const int k0 = band * kRingLevels, k1 = band == last ? d.nz : k0 + kRingLevels;
+    const int runs = (k1 - k0 + V - 1) / V;
+    const int yz = d.ny * d.pz, xz = d.nx * d.pz;
+    {
+        const BoundaryAxis A{d.nx, d.sx(), B.west, B.east, B.inv_dx, B.frame_u, B.frame_v};
+        for (int t = threadIdx.x; t < d.ny * runs; t += blockDim.x)
+        {
+            const int j = t / runs, k = k0 + V * (t - j * runs), r = j * d.pz + k;
+            bc_axis_row<V>(A, B.dt_rad, u, v, w, rho, p, wave + r, wave + yz + r, d.at(0, j, k));
+        }
+    }
+    __syncthreads();
+    {
+        const BoundaryAxis A{d.ny, d.sy(), B.south, B.north, B.inv_dy, B.frame_v, B.frame_u};
+        float* south = wave + 2 * yz;
+        for (int t = threadIdx.x; t < d.nx * runs; t += blockDim.x)
+        {
+            const int i = t / runs, k = k0 + V * (t - i * runs), r = i * d.pz + k;
+            bc_axis_row<V>(A, B.dt_rad, v, u, w, rho, p, south + r, south + xz + r, d.at(i, 0, k));
+        }
+    }
+    if (vertical && (k0 == 0 || k1 == d.nz))
+    {
+        __syncthreads();
+        // Rows j < lo and j > ny-4 for every i, then i < lo and i > nx-4 between them.
+        const int loj = min(2, d.ny - 3), loi = min(2, d.nx - 3);
+        const int rows = (loj + 3) * d.nx, sides = loi + 3, mid = d.ny - 3 - loj;
+        for (int q = threadIdx.x; q < rows + sides * mid; q += blockDim.x)
+        {
+            int i, j;
+            if (q < rows)
+            {
+                j = q / d.nx;
+                i = q - j * d.nx;
+                if (j >= loj) j += mid;
+            }
+            else
+            {
+                const int r = q - rows;
+                j = r / sides;
+                i = r - j * sides;
+                j += loj;
+                if (i >= loi) i += d.nx - 3 - loi;
+            }
+            const int c = d.at(i, j, 0);
+            if (k0 == 0 && B.bottom == kBottomNoSlip)
+            {
+                u[c] = 0.0f;
+                v[c] = 0.0f;
+            }
+            if (k1 == d.nz)
+            {
+                const int kt = c + d.nz - 1, km = kt - 1;
+                // With two levels the level below is the zeroed bottom.
+                w[kt] = (B.top == kTopOpen) ? w[km] : 0.0f;
+                u[kt] = u[km];
+                v[kt] = v[km];
+            }
+        }
+    }
+    if (seed)
+    {
+        __syncthreads();
+        for (int t = threadIdx.x; t < d.ny * (k1 - k0); t += blockDim.x)
+        {
+            const int j = t / (k1 - k0), k = k0 + (t - j * (k1 - k0)), r = j * d.pz + k;
+            wave[r] = u[d.at(0, j, k)];
+            wave[yz + r] = u[d.at(d.nx - 2, j, k)];
+        }
+        for (int t = threadIdx.x; t < d.nx * (k1 - k0); t += blockDim.x)
+        {
+            const int i = t / (k1 - k0), k = k0 + (t - i * (k1 - k0)), r = i * d.pz + k;
+            wave[2 * yz + r] = v[d.at(i, 0, k)];
+            wave[2 * yz + xz + r] = v[d.at(i, d.ny - 2, k)];
+        }
+    }
+}
+
+template <int V>
+static __global__ void __launch_bounds__(kRingBlock) acoustic_bc_ring_kernel(BoundaryParams B, float* u, float* v,
+                                                                             float* w, float* rho, float* p,
+                                                                             float* wave, int vertical)
+{
+    bc_ring_levels<V>(B, u, v, w, rho, p, wave, (int)blockIdx.x, vertical != 0, false);
 }
 
 // seed_radiative_state (boundary_conditions_cartesian_cgrid.cpp:798-822) for

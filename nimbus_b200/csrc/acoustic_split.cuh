@@ -13,6 +13,7 @@
 #pragma once
 
 #include "acoustic_fused.cuh"
+#include "acoustic_kernels.cuh"
 
 namespace nimbus
 {
@@ -325,7 +326,7 @@ static __global__ void __launch_bounds__(256) split_continuity_eos_kernel(
 __device__ __forceinline__ void momentum_store(const Dims& d, int i, int j, int k, int c, int fuse_vertical, float un,
                                                float vn, float wn, float* u_out, float* v_out, float* w_out)
 {
-    if ((fuse_vertical & 1) && i >= 1 && i <= d.nx - 3 && j >= 1 && j <= d.ny - 3)
+    if ((fuse_vertical & 1) && bc_inner_column(d, i, j))
     {
         if (k == d.nz - 1) return;  // written by the cell below
         if (k == 0 && (fuse_vertical & 2))
@@ -346,13 +347,10 @@ __device__ __forceinline__ void momentum_store(const Dims& d, int i, int j, int 
 }
 
 // fuse_vertical (kFuse* bits): the momentum pass also applies the vertical
-// closure (bc_vertical_column) to the columns no lateral closure writes
-// (1 <= i <= nx-3, 1 <= j <= ny-3): the no-slip bottom zeros u and v at k = 0,
-// the cell at k = nz-2 writes its new u, v and w (or 0 under a rigid top)
-// into level nz-1 as well, and the cell at nz-1 does not store.  The lateral
-// closures that run in between neither write nor depend on those columns'
-// levels 0 and nz-1 for any value that survives the closure of their own
-// columns, so the state is the one the separate closure pass gives.
+// closure (bc_vertical_column) to the columns no lateral closure writes or
+// reads (bc_inner_column): the no-slip bottom zeros u and v at k = 0, the cell
+// at k = nz-2 writes its new u, v and w (or 0 under a rigid top) into level
+// nz-1 as well, and the cell at nz-1 does not store.
 enum : int
 {
     kFuseVertical = 1,
@@ -661,7 +659,7 @@ __device__ __forceinline__ void momentum_quad(const FusedParams& P, const float*
         vn.v[q] = n.y;
         wn.v[q] = n.z;
     }
-    if ((fuse_vertical & kFuseVertical) && i >= 1 && i <= d.nx - 3 && j >= 1 && j <= d.ny - 3)
+    if ((fuse_vertical & kFuseVertical) && bc_inner_column(d, i, j))
     {
         // momentum_store's vertical closure on the four cells; the top level
         // is cell kt of them.
@@ -710,22 +708,24 @@ template <class Policy>
 static __global__ void __launch_bounds__(kQuadBlock, 8) split_momentum_quad_kernel(
     FusedParams P, const float* __restrict__ rho, const float* __restrict__ p, const double* __restrict__ p0,
     const float2* __restrict__ dp0_split, const float* __restrict__ u, const float* __restrict__ v,
-    const float* __restrict__ w, float* __restrict__ u_out, float* __restrict__ v_out, float* __restrict__ w_out)
+    const float* __restrict__ w, float* __restrict__ u_out, float* __restrict__ v_out, float* __restrict__ w_out,
+    int fuse_vertical)
 {
     const int n = P.d.cells();
     for (int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x); c < n; c += 4 * gridDim.x * blockDim.x)
-        momentum_quad<Policy>(P, rho, p, p0, dp0_split, u, v, w, u_out, v_out, w_out, c, 0);
+        momentum_quad<Policy>(P, rho, p, p0, dp0_split, u, v, w, u_out, v_out, w_out, c, fuse_vertical);
 }
 
 template <class Policy>
 static __global__ void __launch_bounds__(256) split_momentum_kernel(
     FusedParams P, const float* __restrict__ rho, const float* __restrict__ p, const double* __restrict__ p0,
     const float2* __restrict__ dp0_split, const float* __restrict__ u, const float* __restrict__ v,
-    const float* __restrict__ w, float* __restrict__ u_out, float* __restrict__ v_out, float* __restrict__ w_out)
+    const float* __restrict__ w, float* __restrict__ u_out, float* __restrict__ v_out, float* __restrict__ w_out,
+    int fuse_vertical)
 {
     const int n = P.d.cells();
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
-        momentum_cell<Policy>(P, rho, p, p0, dp0_split, u, v, w, u_out, v_out, w_out, c);
+        momentum_cell<Policy>(P, rho, p, p0, dp0_split, u, v, w, u_out, v_out, w_out, c, fuse_vertical);
 }
 
 }  // namespace nimbus

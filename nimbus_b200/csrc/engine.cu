@@ -56,7 +56,7 @@ ArenaLayout arena_layout(const nimbus_member_desc* d)
     ArenaLayout L{};
     const int pz = column_pitch(d->nz);
     L.cells = static_cast<size_t>(d->nx) * d->ny * pz;
-    L.history = 2 * (static_cast<size_t>(d->nx) + d->ny) * d->nz;
+    L.history = 2 * (static_cast<size_t>(d->nx) + d->ny) * pz;
     const size_t field = align_up(L.cells * sizeof(float));
     size_t off = 0;
     L.off_state = off;  off += 11 * field;                  // u v w rho rho_alt p theta qv qc qr qr_alt
@@ -212,11 +212,8 @@ void fill_params(EngineMember& M, const nimbus_member_desc* a)
     M.n_substeps = a->n_substeps;
     M.microphysics = a->microphysics;
     M.items[kItemCells] = F.d.cells();
-    M.items[kItemRowsWE] = a->ny * a->nz;
-    M.items[kItemRowsSN] = a->nx * a->nz;
     M.items[kItemColumns] = a->nx * a->ny;
-    M.items[kItemHistory] = (a->ny + a->nx) * a->nz;
-    M.items[kItemPerimeter] = 3 * a->nx + 3 * (a->ny - 3);
+    M.items[kItemRing] = ring_bands(a->nz);
     M.items[kItemQuads] = M.items[kItemCells] / 4;
 }
 
@@ -472,7 +469,7 @@ nimbus_status rebuild_table(nimbus_engine* e)
         {
             long long* p = e->prefix.data() + L.prefix_first + static_cast<size_t>(k) * (L.members + 1);
             p[0] = 0;
-            const int tile = k == kItemQuads ? kQuadTile : kEngineBlock * kItemsPerThread;
+            const int tile = k == kItemRing ? 1 : k == kItemQuads ? kQuadTile : kEngineBlock * kItemsPerThread;
             for (int r = 0; r < L.members; ++r) p[r + 1] = p[r] + (rows[r].items[k] + tile - 1) / tile;
         }
         L.closing = false;

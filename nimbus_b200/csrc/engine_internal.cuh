@@ -226,11 +226,8 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
     int count = 0;
     EngineMember* T = e->d_table + L.first;
     const long long* pc = prefix_of(e, L, kItemCells);
-    const long long* pwe = prefix_of(e, L, kItemRowsWE);
-    const long long* psn = prefix_of(e, L, kItemRowsSN);
+    const long long* pring = prefix_of(e, L, kItemRing);
     const long long* pcol = prefix_of(e, L, kItemColumns);
-    const long long* phist = prefix_of(e, L, kItemHistory);
-    const long long* pper = prefix_of(e, L, kItemPerimeter);
     const long long cells = tiles_of(e, L, kItemCells, n);
 
     if (part == 0)
@@ -279,15 +276,12 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
         ENGINE_LAUNCH(NIMBUS_KERNEL_SLOW, engine_slow_predict_kernel<Policy>, cells, 1, T, pc, cells);
         ENGINE_LAUNCH(NIMBUS_KERNEL_SLOW, engine_slow_correct_kernel<Policy>, cells, 1, T, pc, cells);
     }
-    // seed_acoustic_radiation: apply_acoustic(0) then the KW78 seed.
-    ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_we_kernel, tiles_of(e, L, kItemRowsWE, n), 1, T, pwe,
-                  tiles_of(e, L, kItemRowsWE, n), 0, 1);
-    ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_sn_kernel, tiles_of(e, L, kItemRowsSN, n), 1, T, psn,
-                  tiles_of(e, L, kItemRowsSN, n), 0, 1);
+    // seed_acoustic_radiation: apply_acoustic(0) then the KW78 seed (its rows
+    // lie in perimeter columns, which the ring closes before it seeds).
+    ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_ring_kernel, tiles_of(e, L, kItemRing, n),
+                        kRingBlock, T, pring, tiles_of(e, L, kItemRing, n), 0, 1);
     ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_vertical_kernel, tiles_of(e, L, kItemColumns, n), 1, T,
                   pcol, tiles_of(e, L, kItemColumns, n), 1);
-    ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_seed_kernel, tiles_of(e, L, kItemHistory, n), 1, T, phist,
-                  tiles_of(e, L, kItemHistory, n));
     return count;
     }
     // The acoustic loop: members still inside it are a prefix of the lane.
@@ -442,12 +436,8 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
             ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, engine_momentum_kernel<Policy>, tiles, 1, T, pc, tiles,
                           si);
         }
-        ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_we_kernel, tiles_of(e, L, kItemRowsWE, a), 1, T, pwe,
-                      tiles_of(e, L, kItemRowsWE, a), si, 0);
-        ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_sn_kernel, tiles_of(e, L, kItemRowsSN, a), 1, T, psn,
-                      tiles_of(e, L, kItemRowsSN, a), si, 0);
-        ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_vertical_perimeter_kernel,
-                      tiles_of(e, L, kItemPerimeter, a), 1, T, pper, tiles_of(e, L, kItemPerimeter, a));
+        ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_ring_kernel, tiles_of(e, L, kItemRing, a),
+                            kRingBlock, T, pring, tiles_of(e, L, kItemRing, a), si, 0);
     }
     engine_swap_kernel<<<(n + 127) / 128, 128, 0, st>>>(T, n, 0);
     ++count;
@@ -513,10 +503,8 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
     // for the members that ask for it, on the published density and pressure.
     if (L.closing)
     {
-        ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_we_kernel, tiles_of(e, L, kItemRowsWE, n), 1, T, pwe,
-                      tiles_of(e, L, kItemRowsWE, n), 0, 2);
-        ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_sn_kernel, tiles_of(e, L, kItemRowsSN, n), 1, T, psn,
-                      tiles_of(e, L, kItemRowsSN, n), 0, 2);
+        ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_ring_kernel, tiles_of(e, L, kItemRing, n),
+                            kRingBlock, T, pring, tiles_of(e, L, kItemRing, n), 0, 2);
         ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_vertical_kernel, tiles_of(e, L, kItemColumns, n), 1,
                       T, pcol, tiles_of(e, L, kItemColumns, n), 2);
     }

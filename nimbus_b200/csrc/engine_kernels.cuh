@@ -31,11 +31,8 @@ namespace nimbus
 enum ItemKind
 {
     kItemCells = 0,
-    kItemRowsWE,     // ny*nz west/east boundary rows
-    kItemRowsSN,     // nx*nz south/north boundary rows
     kItemColumns,    // nx*ny columns
-    kItemHistory,    // (ny + nx)*nz KW78 history slots
-    kItemPerimeter,  // 3 nx + 3 (ny - 3) columns the lateral closures write
+    kItemRing,       // bands of levels of the lateral closures (ring_bands), one a CTA
     kItemMarch,      // rows along x: (j, k) positions in blocks times i-chunks (for_member_rows)
     kItemQuads,      // cells in groups of four (the constant-bank acoustic passes and the speed scan)
     kItemKinds
@@ -290,32 +287,26 @@ __device__ __forceinline__ float* engine_density(const EngineMember& M, int s, b
     return written ? (even ? M.rho_alt : M.rho) : (even ? M.rho : M.rho_alt);
 }
 
-static __global__ void __launch_bounds__(256) engine_bc_we_kernel(const EngineMember* __restrict__ table,
-                                                           const long long* __restrict__ prefix, long long tiles,
-                                                           int s, int refresh)
+// The closure of a band of levels per CTA (bc_ring_levels).  refresh 0: inside
+// the acoustic loop, after substep s, with the perimeter's vertical closure
+// (the momentum pass closes the inner columns itself, fuse_vertical); 1 before
+// the loop, seeding the KW78 memory as well; 2 the closing refresh, of the
+// members that ask for it.
+static __global__ void __launch_bounds__(kRingBlock) engine_bc_ring_kernel(const EngineMember* __restrict__ table,
+                                                                           const long long* __restrict__ prefix,
+                                                                           long long tiles, int s, int refresh)
 {
-    for_member_items(table, prefix, tiles, kItemRowsWE, [&](const EngineMember& M, int r) {
-        if (refresh == 2 && !M.close_step) return;  // the closing refresh only where asked
+    int m = 0;
+    for (long long t = blockIdx.x; t < tiles; t += gridDim.x)
+    {
+        while (t >= prefix[m + 1]) ++m;
+        const EngineMember& M = table[m];
+        if (refresh == 2 && !M.close_step) continue;
         BoundaryParams B = M.B;
         if (refresh) B.dt_rad = 0.0f;
-        float* rho = refresh ? M.rho : engine_density(M, s, true);
-        const int yz = B.d.ny * B.d.nz;
-        bc_we_row(B, M.u, M.v, M.w, rho, M.p, M.wave, M.wave + yz, r);
-    });
-}
-
-static __global__ void __launch_bounds__(256) engine_bc_sn_kernel(const EngineMember* __restrict__ table,
-                                                           const long long* __restrict__ prefix, long long tiles,
-                                                           int s, int refresh)
-{
-    for_member_items(table, prefix, tiles, kItemRowsSN, [&](const EngineMember& M, int r) {
-        if (refresh == 2 && !M.close_step) return;
-        BoundaryParams B = M.B;
-        if (refresh) B.dt_rad = 0.0f;
-        float* rho = refresh ? M.rho : engine_density(M, s, true);
-        const int yz = B.d.ny * B.d.nz, xz = B.d.nx * B.d.nz;
-        bc_sn_row(B, M.u, M.v, M.w, rho, M.p, M.wave + 2 * yz, M.wave + 2 * yz + xz, r);
-    });
+        bc_ring_levels<4>(B, M.u, M.v, M.w, refresh ? M.rho : engine_density(M, s, true), M.p, M.wave,
+                          (int)(t - prefix[m]), true, refresh == 1);
+    }
 }
 
 // refresh: 1 before the acoustic loop, 2 the closing refresh at the end of the
@@ -327,41 +318,6 @@ static __global__ void __launch_bounds__(256) engine_bc_vertical_kernel(const En
     for_member_items(table, prefix, tiles, kItemColumns, [&](const EngineMember& M, int col) {
         if (refresh == 2 && !M.close_step) return;
         bc_vertical_column(M.B, M.u, M.v, M.w, col);
-    });
-}
-
-// The vertical closure inside the acoustic loop, for the columns the lateral
-// closures write (i in {0, nx-2, nx-1} or j in {0, ny-2, ny-1}); the momentum
-// kernel closes every other column itself (momentum_cell, fuse_vertical).
-// Item q: rows j = 0, ny-2, ny-1 for every i first, then i = 0, nx-2, nx-1
-// for j = 1 .. ny-3.
-static __global__ void __launch_bounds__(256) engine_bc_vertical_perimeter_kernel(
-    const EngineMember* __restrict__ table, const long long* __restrict__ prefix, long long tiles)
-{
-    for_member_items(table, prefix, tiles, kItemPerimeter, [&](const EngineMember& M, int q) {
-        const int nx = M.B.d.nx, ny = M.B.d.ny;
-        int i, j;
-        if (q < 3 * nx)
-        {
-            const int row = q / nx;
-            i = q - row * nx;
-            j = row == 0 ? 0 : ny - 3 + row;
-        }
-        else
-        {
-            const int r = q - 3 * nx, side = r % 3;
-            j = 1 + r / 3;
-            i = side == 0 ? 0 : nx - 3 + side;
-        }
-        bc_vertical_column(M.B, M.u, M.v, M.w, i * ny + j);
-    });
-}
-
-static __global__ void __launch_bounds__(256) engine_seed_kernel(const EngineMember* __restrict__ table,
-                                                          const long long* __restrict__ prefix, long long tiles)
-{
-    for_member_items(table, prefix, tiles, kItemHistory, [&](const EngineMember& M, int r) {
-        seed_radiation_row(M.B.d, M.u, M.v, M.wave, r);
     });
 }
 

@@ -21,10 +21,10 @@ nimbus_status launch_fused(nimbus_cuda_context* ctx, cudaStream_t st, const nimb
 nimbus_status launch_split(nimbus_cuda_context* ctx, cudaStream_t st, const nimbus::FusedParams& F,
                            const nimbus_host::Prognostic& in, const nimbus_host::Prognostic& out, float* p,
                            const float* theta, const double* rho0, const double* p0, const float2* dp0,
-                           const float4* eos0, float* drho, float* mfx, float* mfy, float* mfz)
+                           const float4* eos0, float* drho, float* mfx, float* mfy, float* mfz, int vertical)
 {
     return launch_split_impl<nimbus::Fp32Policy>(ctx, st, F, in, out, p, theta, rho0, p0, dp0, eos0, drho, mfx, mfy,
-                                                 mfz);
+                                                 mfz, vertical);
 }
 
 nimbus_status run_slow(nimbus_cuda_context* ctx, cudaStream_t st, const nimbus::SlowParams& S,

@@ -93,7 +93,7 @@ template <class Policy>
 nimbus_status launch_split_impl(nimbus_cuda_context* ctx, cudaStream_t st, FusedParams F, const Prognostic& in,
                                 const Prognostic& out, float* p, const float* theta, const double* rho0,
                                 const double* p0, const float2* dp0, const float4* eos0, float* drho, float* mfx,
-                                float* mfy, float* mfz)
+                                float* mfy, float* mfz, int vertical)
 {
     const long long n = F.d.cells();
     if (F.d.nz % 4 == 0 && drho == nullptr && aligned16(in.rho) && aligned16(in.u) && aligned16(in.v) &&
@@ -110,7 +110,7 @@ nimbus_status launch_split_impl(nimbus_cuda_context* ctx, cudaStream_t st, Fused
         {
             LaunchTimer t(ctx, st, NIMBUS_KERNEL_ACOUSTIC_MOMENTUM);
             split_momentum_quad_kernel<Policy><<<static_cast<int>(qblocks), kQuadBlock, 0, st>>>(
-                F, out.rho, p, p0, dp0, in.u, in.v, in.w, out.u, out.v, out.w);
+                F, out.rho, p, p0, dp0, in.u, in.v, in.w, out.u, out.v, out.w, vertical);
         }
         ctx->launches += 2;
         return NIMBUS_OK;
@@ -126,7 +126,7 @@ nimbus_status launch_split_impl(nimbus_cuda_context* ctx, cudaStream_t st, Fused
     {
         LaunchTimer t(ctx, st, NIMBUS_KERNEL_ACOUSTIC_MOMENTUM);
         split_momentum_kernel<Policy><<<static_cast<int>(blocks), kThreads, 0, st>>>(F, out.rho, p, p0, dp0, in.u,
-                                                                                      in.v, in.w, out.u, out.v, out.w);
+                                                                                      in.v, in.w, out.u, out.v, out.w, vertical);
     }
     ctx->launches += 2;
     return NIMBUS_OK;
@@ -202,7 +202,7 @@ nimbus_status launch_split(nimbus_cuda_context* ctx, cudaStream_t st, const nimb
                            const nimbus_host::Prognostic& in, const nimbus_host::Prognostic& out, float* p,
                            const float* theta,
                            const double* rho0, const double* p0, const float2* dp0, const float4* eos0, float* drho,
-                           float* mfx, float* mfy, float* mfz);
+                           float* mfx, float* mfy, float* mfz, int vertical);
 nimbus_status run_slow(nimbus_cuda_context* ctx, cudaStream_t st, const nimbus::SlowParams& S,
                        const nimbus_host::SlowDevice& D, bool step);
 nimbus_status launch_transport(nimbus_cuda_context* ctx, cudaStream_t st, const nimbus::TransportParams& T,

@@ -112,15 +112,24 @@ int resolve_form(const nimbus_cuda_context* ctx, const Dims& d)
     return NIMBUS_SUBSTEP_SPLIT;
 }
 
+// One substep without its boundary closure.  vertical: kFuse* bits of the
+// vertical closure the caller wants of the momentum pass; returns in *closed
+// whether the form launched applies them (the split form does).
 nimbus_status launch_fused(nimbus_cuda_context* ctx, cudaStream_t st, const FusedParams& F, const Prognostic& in,
                            const Prognostic& out, float* p, const float* theta, const double* rho0, const double* p0,
-                           const float2* dp0, const float4* eos0, float* drho, float* mfx, float* mfy, float* mfz)
+                           const float2* dp0, const float4* eos0, float* drho, float* mfx, float* mfy, float* mfz,
+                           int vertical = 0, bool* closed = nullptr)
 {
     const bool fp32 = ctx->precision == NIMBUS_PRECISION_FP32;
-    if (resolve_form(ctx, F.d) == NIMBUS_SUBSTEP_SPLIT)
+    const bool split = resolve_form(ctx, F.d) == NIMBUS_SUBSTEP_SPLIT;
+    if (closed) *closed = split && vertical != 0;
+    if (split)
     {
-        if (fp32) return nimbus_fp32::launch_split(ctx, st, F, in, out, p, theta, rho0, p0, dp0, eos0, drho, mfx, mfy, mfz);
-        return launch_split_impl<RefPolicy>(ctx, st, F, in, out, p, theta, rho0, p0, dp0, eos0, drho, mfx, mfy, mfz);
+        if (fp32)
+            return nimbus_fp32::launch_split(ctx, st, F, in, out, p, theta, rho0, p0, dp0, eos0, drho, mfx, mfy, mfz,
+                                             vertical);
+        return launch_split_impl<RefPolicy>(ctx, st, F, in, out, p, theta, rho0, p0, dp0, eos0, drho, mfx, mfy, mfz,
+                                            vertical);
     }
     if (fp32) return nimbus_fp32::launch_fused(ctx, st, F, in, out, p, theta, rho0, p0, dp0, eos0, drho, mfx, mfy, mfz);
     return launch_fused_impl<RefPolicy>(ctx, st, F, in, out, p, theta, rho0, p0, dp0, eos0, drho, mfx, mfy, mfz);
@@ -178,17 +187,23 @@ FusedParams fused_params(const nimbus_cuda_context* ctx, int nx, int ny, int nz,
     return F;
 }
 
+// The boundary closure; inner_closed: the momentum pass closed the inner
+// columns (bc_inner_column) vertically, and the ring closes the rest.
 void launch_boundaries(nimbus_cuda_context* ctx, cudaStream_t st, const BoundaryParams& B, const AcousticDevice& D,
-                       float* rho, float* wave)
+                       float* rho, float* wave, bool inner_closed)
 {
     const Dims d = B.d;
-    const int yz = d.ny * d.nz, xz = d.nx * d.nz;
     LaunchTimer t(ctx, st, NIMBUS_KERNEL_ACOUSTIC_BOUNDARY);
-    acoustic_bc_we_kernel<<<grid_for(ctx, yz), kThreads, 0, st>>>(B, D.u, D.v, D.w, rho, D.p, wave, wave + yz);
-    acoustic_bc_sn_kernel<<<grid_for(ctx, xz), kThreads, 0, st>>>(B, D.u, D.v, D.w, rho, D.p, wave + 2 * yz,
-                                                                  wave + 2 * yz + xz);
+    const int bands = ring_bands(d.nz);
+    if (d.nz % 4 == 0 && aligned16(D.u) && aligned16(D.v) && aligned16(D.w) && aligned16(rho) && aligned16(D.p) &&
+        aligned16(wave))
+        acoustic_bc_ring_kernel<4><<<bands, kRingBlock, 0, st>>>(B, D.u, D.v, D.w, rho, D.p, wave, inner_closed);
+    else
+        acoustic_bc_ring_kernel<1><<<bands, kRingBlock, 0, st>>>(B, D.u, D.v, D.w, rho, D.p, wave, inner_closed);
+    ctx->launches += 1;
+    if (inner_closed) return;
     acoustic_bc_vertical_kernel<<<grid_for(ctx, d.nx * d.ny), kThreads, 0, st>>>(B, D.u, D.v, D.w);
-    ctx->launches += 3;
+    ctx->launches += 1;
 }
 
 nimbus_status run_batched_device(nimbus_cuda_context* ctx, cudaStream_t st, const nimbus_acoustic_batched_args* a,
@@ -236,13 +251,16 @@ nimbus_status run_batched_device(nimbus_cuda_context* ctx, cudaStream_t st, cons
     Prognostic user{D.u, D.v, D.w, D.rho};
     Prognostic work{D.u_alt, D.v_alt, D.w_alt, D.rho_alt};
     Prognostic cur = user, alt = work;
+    const int vertical = kFuseVertical | (B.bottom == kBottomNoSlip ? kFuseNoSlipBottom : 0) |
+                         (B.top == kTopOpen ? kFuseOpenTop : 0);
     for (int s = 0; s < a->n_substeps; ++s)
     {
+        bool closed = false;
         NB_TRY(launch_fused(ctx, st, F, cur, alt, D.p, D.theta, D.rho0, D.p0, dp0, eos0, nullptr, D.mfx, D.mfy,
-                            D.mfz));
+                            D.mfz, vertical, &closed));
         AcousticDevice E = D;
         E.u = alt.u; E.v = alt.v; E.w = alt.w;
-        launch_boundaries(ctx, st, B, E, alt.rho, wave);
+        launch_boundaries(ctx, st, B, E, alt.rho, wave, closed);
         std::swap(cur, alt);
     }
     if (cur.u != user.u)
@@ -758,7 +776,7 @@ nimbus_status nimbus_cuda_acoustic_boundaries(nimbus_cuda_context* ctx, const ni
     D.u = a->u; D.v = a->v; D.w = a->w; D.rho = a->rho; D.p = a->p;
     // Without radiation the history is never read; any valid pointer will do.
     float* wave = a->wave_history ? a->wave_history : a->u;
-    launch_boundaries(ctx, st, B, D, a->rho, wave);
+    launch_boundaries(ctx, st, B, D, a->rho, wave, false);
     NB_CUDA(ctx, cudaGetLastError());
     return NIMBUS_OK;
 }

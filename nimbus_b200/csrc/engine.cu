@@ -783,12 +783,10 @@ int nimbus_engine_detail::launch_microphysics(nimbus_engine* e, cudaStream_t st,
     LaunchTimer t(ctx, st, NIMBUS_KERNEL_MICROPHYSICS);
     if (ctx->precision == NIMBUS_PRECISION_FP32)
         engine_microphysics_eos_kernel<true>
-            <<<engine_grid(e, reinterpret_cast<const void*>(engine_microphysics_eos_kernel<true>), tiles),
-               kEngineBlock, 0, st>>>(table, prefix, tiles);
+            <<<tile_grid(tiles), kEngineBlock, 0, st>>>(table, prefix, tiles);
     else
         engine_microphysics_eos_kernel<false>
-            <<<engine_grid(e, reinterpret_cast<const void*>(engine_microphysics_eos_kernel<false>), tiles),
-               kEngineBlock, 0, st>>>(table, prefix, tiles);
+            <<<tile_grid(tiles), kEngineBlock, 0, st>>>(table, prefix, tiles);
     return 1;
 }
 

@@ -143,6 +143,14 @@ unsigned engine_grid(nimbus_engine* e, const void* kernel, long long tiles, int 
     return static_cast<unsigned>(g < 1 ? 1 : g);
 }
 
+// One CTA a tile: for the passes whose cells differ in cost (face values near
+// walls, cloud and rain), where the block scheduler evens out what a fixed
+// round of tiles per CTA does not.  Reference precision, 3.0M cells: Kessler
+// and EOS 1.01 -> 0.76 ms; FP32, 5.2M cells: faces 2.37 -> 2.12, Kessler and
+// EOS 1.76 -> 1.57 (the streaming passes lose 5 to 15 % by it: each CTA finds
+// its member anew).
+unsigned tile_grid(long long tiles) { return static_cast<unsigned>(tiles < 0x7fffffffll ? tiles : 0x7fffffffll); }
+
 // The bulk-staged acoustic forms: dynamic shared memory of kBulkStages
 // stages plus their barriers, at most kBulkSmemLimit (a lane whose members
 // need more takes the constant-bank form).
@@ -205,6 +213,16 @@ long long tiles_of(const nimbus_engine* e, const nimbus_engine_detail::Lane& L, 
             LaunchTimer t_(ctx, st, family);                                                             \
             kernel<<<engine_grid_smem(e, reinterpret_cast<const void*>(kernel), tiles_, (smem)),         \
                      kEngineBlock, (smem), st>>>(__VA_ARGS__);                                           \
+            ++count;                                                                                     \
+        }                                                                                                \
+    } while (0)
+#define ENGINE_LAUNCH_TILES(family, kernel, tiles, ...)                                                  \
+    do {                                                                                                 \
+        const long long tiles_ = (tiles);                                                                \
+        if (tiles_ > 0)                                                                                  \
+        {                                                                                                \
+            LaunchTimer t_(ctx, st, family);                                                             \
+            kernel<<<tile_grid(tiles_), kEngineBlock, 0, st>>>(__VA_ARGS__);                             \
             ++count;                                                                                     \
         }                                                                                                \
     } while (0)
@@ -480,8 +498,8 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
             A.qc = H.qc;
             A.status = H.status;
         }
-        ENGINE_LAUNCH(NIMBUS_KERNEL_TRANSPORT_FACES, engine_transport_faces_const_kernel<kFp32>, cells, 1, *tl, T,
-                      cells);
+        ENGINE_LAUNCH_TILES(NIMBUS_KERNEL_TRANSPORT_FACES, engine_transport_faces_const_kernel<kFp32>, cells, *tl, T,
+                            cells);
         ENGINE_LAUNCH(NIMBUS_KERNEL_TRANSPORT_LIMITER, engine_transport_limiter_const_kernel<kFp32>, cells, 1, *tl, T,
                       cells);
         ENGINE_LAUNCH(NIMBUS_KERNEL_TRANSPORT_UPDATE, engine_transport_update_const_kernel<kFp32>, cells, 1, *tl, T,

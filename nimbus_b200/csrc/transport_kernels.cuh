@@ -109,6 +109,15 @@ __device__ __forceinline__ double mc_slope(double qm, double q0, double qp)
 template <class V>
 struct Lanes;
 
+// Approximate reciprocal (at most 1 ulp off) of a normal number: the form
+// without the scaling that subnormal operands need.
+__device__ __forceinline__ float rcp_normal(float a)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+
 template <>
 struct Lanes<float>
 {
@@ -118,8 +127,7 @@ struct Lanes<float>
     static __device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
     static __device__ __forceinline__ float maxf(float a, float b) { return fmaxf(a, b); }
     static __device__ __forceinline__ float absf(float a) { return fabsf(a); }
-    static __device__ __forceinline__ float rcp(float a) { return __fdividef(1.0f, a); }
-    static __device__ __forceinline__ float div(float a, float b) { return __fdividef(a, b); }
+    static __device__ __forceinline__ float rcp(float a) { return rcp_normal(a); }
     static __device__ __forceinline__ float finite_or_zero(float a) { return isfinite(a) ? a : 0.0f; }
 };
 
@@ -135,14 +143,7 @@ struct Lanes<float2>
         return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y));
     }
     static __device__ __forceinline__ float2 absf(float2 a) { return make_float2(fabsf(a.x), fabsf(a.y)); }
-    static __device__ __forceinline__ float2 rcp(float2 a)
-    {
-        return make_float2(__fdividef(1.0f, a.x), __fdividef(1.0f, a.y));
-    }
-    static __device__ __forceinline__ float2 div(float2 a, float2 b)
-    {
-        return make_float2(__fdividef(a.x, b.x), __fdividef(a.y, b.y));
-    }
+    static __device__ __forceinline__ float2 rcp(float2 a) { return make_float2(rcp_normal(a.x), rcp_normal(a.y)); }
     static __device__ __forceinline__ float2 finite_or_zero(float2 a)
     {
         return make_float2(isfinite(a.x) ? a.x : 0.0f, isfinite(a.y) ? a.y : 0.0f);
@@ -155,11 +156,14 @@ struct Lanes<float2>
 // include/numerics/advection/weno5_face.hpp:88-120: differences from the
 // donor, eps = 1e-6 * relative^2 + (1e-20 / scale)^2, ideal weights 1/10,
 // 6/10, 3/10, p = 2), so moisture-scale fields keep their nonlinear weights.
-// After normalisation every eps + beta_k is at least 1e-6, so the weights
-// d_k / (eps + beta_k)^2 are formed directly from approximate reciprocals
-// instead of the reference's min-normalised ratios: the same weights to FP32
-// rounding in about half the instructions.  A non-finite result falls back to
-// the donor value (offset 0).  V = float2 evaluates two stencils at once.
+// After normalisation every e_k = eps + beta_k lies between 1e-6 and 64, so
+// the weights d_k / e_k^2 are formed as d_k times the square of the other two
+// e's product, all three scaled alike (between 1e-24 and 2e7): the same
+// weights to FP32 rounding with one reciprocal, of their sum, where three
+// reciprocals and a quotient took a third of the face pass' issue slots
+// (FP32 reciprocals and quotients cost several instructions for the subnormal
+// operands that cannot occur here).  A non-finite result falls back to the
+// donor value (offset 0).  V = float2 evaluates two stencils at once.
 template <class V>
 __device__ __forceinline__ V weno5_offset_lanes(V a, V b, V c, V d, V e)
 {
@@ -184,13 +188,14 @@ __device__ __forceinline__ V weno5_offset_lanes(V a, V b, V c, V d, V e)
     const V relative = L::mul(magnitude, inv);
     const V flo = L::mul(L::splat(1e-20f), inv);
     const V epsilon = L::fma(L::mul(relative, L::splat(1e-6f)), relative, L::mul(flo, flo));
-    const V r0 = L::rcp(L::add(epsilon, b0)), r1 = L::rcp(L::add(epsilon, b1)), r2 = L::rcp(L::add(epsilon, b2));
+    const V e0 = L::add(epsilon, b0), e1 = L::add(epsilon, b1), e2 = L::add(epsilon, b2);
+    const V r0 = L::mul(e1, e2), r1 = L::mul(e0, e2), r2 = L::mul(e0, e1);
     const V a0 = L::mul(L::mul(r0, L::splat(0.1f)), r0);
     const V a1 = L::mul(L::mul(r1, L::splat(0.6f)), r1);
     const V a2 = L::mul(L::mul(r2, L::splat(0.3f)), r2);
     const V num = L::fma(a2, p2, L::fma(a1, p1, L::mul(a0, p0)));
     const V den = L::add(L::add(a0, a1), a2);
-    return L::finite_or_zero(L::mul(scale, L::div(num, den)));
+    return L::finite_or_zero(L::mul(scale, L::mul(num, L::rcp(den))));
 }
 
 __device__ __forceinline__ float weno5_offset_f32(float a, float b, float c, float d, float e)
@@ -245,6 +250,16 @@ __device__ __forceinline__ FaceStencil face_stencil(int base, int stride, int l,
     return f;
 }
 
+// Whether every value of a five-point stencil is +0: its face value is then
+// the donor's, +0, in either precision, and its flux mflux * 0 (as the
+// weights would give it).  Cloud and rain are zero over most of a domain, and
+// a warp whose stencils all are skips their weights.
+__device__ __forceinline__ bool zero_stencil(const float (&v)[5])
+{
+    return (__float_as_uint(v[0]) | __float_as_uint(v[1]) | __float_as_uint(v[2]) | __float_as_uint(v[3]) |
+            __float_as_uint(v[4])) == 0u;
+}
+
 // The face flux of one scalar on a prepared stencil
 // (advection_cartesian.cpp:1943-2172).  FP32 form: M * donor + M * offset
 // with the normalised WENO5 offset; reference precision: M times the FP64
@@ -259,7 +274,11 @@ __device__ __forceinline__ float stencil_flux_values(const float (&v)[5], const 
     {
         const float q0 = v[2];
         float offset;
-        if (f.weno) offset = weno5_offset_f32(v[0], v[1], q0, v[3], v[4]);
+        if (f.weno)
+        {
+            if (zero_stencil(v)) return mflux * q0;
+            offset = weno5_offset_f32(v[0], v[1], q0, v[3], v[4]);
+        }
         else
         {
             const float sl = f.slope ? mc_slope_f32(v[0], q0, v[3]) : 0.0f;
@@ -271,7 +290,11 @@ __device__ __forceinline__ float stencil_flux_values(const float (&v)[5], const 
     {
         const double q0 = (double)v[2];
         double face;
-        if (f.weno) face = weno5_face((double)v[0], (double)v[1], q0, (double)v[3], (double)v[4]);
+        if (f.weno)
+        {
+            if (zero_stencil(v)) return (float)((double)mflux * q0);
+            face = weno5_face((double)v[0], (double)v[1], q0, (double)v[3], (double)v[4]);
+        }
         else
         {
             const double sl = f.slope ? mc_slope((double)v[0], q0, (double)v[3]) : 0.0;
@@ -295,7 +318,12 @@ __device__ __forceinline__ float2 stencil_flux_pair_values(const float2 (&v)[5],
 {
     const float2 q0 = v[2];
     float2 offset;
-    if (f.weno) offset = weno5_offset_lanes<float2>(v[0], v[1], q0, v[3], v[4]);
+    if (f.weno)
+    {
+        const float a[5] = {v[0].x, v[1].x, v[2].x, v[3].x, v[4].x}, b[5] = {v[0].y, v[1].y, v[2].y, v[3].y, v[4].y};
+        if (zero_stencil(a) && zero_stencil(b)) return make_float2(mflux * q0.x, mflux * q0.y);
+        offset = weno5_offset_lanes<float2>(v[0], v[1], q0, v[3], v[4]);
+    }
     else
     {
         const float h = f.pos ? 0.5f : -0.5f;

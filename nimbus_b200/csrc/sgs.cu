@@ -44,26 +44,48 @@ const char* check_closure(const nimbus_smagorinsky_args* a, std::vector<double>&
     return nullptr;
 }
 
-// Device copies of dz and the filter widths, back to back.
+// The per-level tables on the device, one block: dz, the filter widths, the
+// FP64 reciprocals of dz, of the centres' distances and of the sums of two
+// layers, then the FP32 reciprocals of dz and of the distances.
 nimbus_status stage_tables(nimbus_cuda_context* ctx, cudaStream_t st, const double* dz,
                            const std::vector<double>& delta, SgsParams& P)
 {
     const size_t nz = delta.size();
     double* dev = nullptr;
-    NB_TRY(ensure(ctx, kSgsTables, 3 * nz, &dev));  // dz, delta, then the FP32 reciprocals of dz and dzc
+    NB_TRY(ensure(ctx, kSgsTables, 6 * nz, &dev));
+    std::vector<double> tab(6 * nz, 0.0);
     std::vector<float> inv(2 * nz, 0.0f);
-    for (size_t k = 0; k < nz; ++k) inv[k] = static_cast<float>(1.0 / dz[k]);
-    for (size_t k = 0; k + 1 < nz; ++k) inv[nz + k] = static_cast<float>(1.0 / (0.5 * (dz[k] + dz[k + 1])));
+    auto in_range = [](double d) { return d >= 0x1p-60 && d <= 0x1p60; };
+    bool fast = in_range(P.dx) && in_range(P.dy) && in_range(P.Pr_t) && in_range(P.Sc_t);
+    for (size_t k = 0; k < nz; ++k)
+    {
+        tab[k] = dz[k];
+        tab[nz + k] = delta[k];
+        tab[2 * nz + k] = 1.0 / dz[k];
+        inv[k] = static_cast<float>(1.0 / dz[k]);
+        fast = fast && in_range(dz[k]);
+    }
+    for (size_t k = 0; k + 1 < nz; ++k)
+    {
+        const double centres = 0.5 * (dz[k] + dz[k + 1]), sum = dz[k] + dz[k + 1];
+        tab[3 * nz + k] = 1.0 / centres;
+        tab[4 * nz + k] = 1.0 / sum;
+        inv[nz + k] = static_cast<float>(1.0 / centres);
+        fast = fast && in_range(centres) && in_range(sum);
+    }
     // No centre above the top level: a use of DZC(nz - 1) shows up as NaN.
+    tab[4 * nz - 1] = tab[5 * nz - 1] = std::numeric_limits<double>::quiet_NaN();
     inv[2 * nz - 1] = std::numeric_limits<float>::quiet_NaN();
-    NB_CUDA(ctx, cudaMemcpyAsync(dev, dz, nz * sizeof(double), cudaMemcpyHostToDevice, st));
-    NB_CUDA(ctx, cudaMemcpyAsync(dev + nz, delta.data(), nz * sizeof(double), cudaMemcpyHostToDevice, st));
-    float* inv_dev = reinterpret_cast<float*>(dev + 2 * nz);
-    NB_CUDA(ctx, cudaMemcpyAsync(inv_dev, inv.data(), 2 * nz * sizeof(float), cudaMemcpyHostToDevice, st));
+    std::memcpy(tab.data() + 5 * nz, inv.data(), 2 * nz * sizeof(float));
+    NB_CUDA(ctx, cudaMemcpyAsync(dev, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     P.dz = dev;
     P.delta = dev + nz;
-    P.inv_dz_f = inv_dev;
-    P.inv_dzc_f = inv_dev + nz;
+    P.y_dz = dev + 2 * nz;
+    P.y_dzc = dev + 3 * nz;
+    P.y_dzs = dev + 4 * nz;
+    P.inv_dz_f = reinterpret_cast<float*>(dev + 5 * nz);
+    P.inv_dzc_f = P.inv_dz_f + nz;
+    P.fast = fast ? 1 : 0;
     return NIMBUS_OK;
 }
 
@@ -83,6 +105,10 @@ SgsParams params_of(const nimbus_smagorinsky_args* a)
     P.Sc_t = a->Sc_t;
     P.nu_max = a->nu_t_max;
     P.K_max = a->K_max;
+    P.y_dx = 1.0 / a->dx;
+    P.y_dy = 1.0 / a->dy;
+    P.y_pr = 1.0 / a->Pr_t;
+    P.y_sc = 1.0 / a->Sc_t;
     P.inv_dx_f = static_cast<float>(1.0 / a->dx);
     P.inv_dy_f = static_cast<float>(1.0 / a->dy);
     return P;
@@ -101,20 +127,15 @@ nimbus_status launch_closure(nimbus_cuda_context* ctx, cudaStream_t st, const Sg
 {
     const int grid = grid_for(ctx, P.d.cells());
     LaunchTimer t(ctx, st, NIMBUS_KERNEL_SGS);
+    auto both = [&](auto coefficients, auto tendencies) {
+        coefficients<<<grid, kThreads, 0, st>>>(P, D.u, D.v, D.w, D.theta, D.qv, D.rho, D.nu, D.kt, D.kq, status);
+        tendencies<<<grid, kThreads, 0, st>>>(P, D.u, D.v, D.w, D.theta, D.qv, D.rho, D.nu, D.kt, D.kq, D.du, D.dv,
+                                              D.dw, D.dth, D.dqv);
+    };
     if (ctx->precision == NIMBUS_PRECISION_FP32)
-    {
-        sgs_coefficients_kernel<float><<<grid, kThreads, 0, st>>>(P, D.u, D.v, D.w, D.theta, D.qv, D.rho, D.nu,
-                                                                  D.kt, D.kq, status);
-        sgs_tendencies_kernel<float><<<grid, kThreads, 0, st>>>(P, D.u, D.v, D.w, D.theta, D.qv, D.rho, D.nu, D.kt,
-                                                                D.kq, D.du, D.dv, D.dw, D.dth, D.dqv);
-    }
-    else
-    {
-        sgs_coefficients_kernel<double><<<grid, kThreads, 0, st>>>(P, D.u, D.v, D.w, D.theta, D.qv, D.rho, D.nu,
-                                                                   D.kt, D.kq, status);
-        sgs_tendencies_kernel<double><<<grid, kThreads, 0, st>>>(P, D.u, D.v, D.w, D.theta, D.qv, D.rho, D.nu, D.kt,
-                                                                 D.kq, D.du, D.dv, D.dw, D.dth, D.dqv);
-    }
+        both(sgs_coefficients_kernel<float, false>, sgs_tendencies_kernel<float, false>);
+    else if (P.fast) both(sgs_coefficients_kernel<double, true>, sgs_tendencies_kernel<double, true>);
+    else both(sgs_coefficients_kernel<double, false>, sgs_tendencies_kernel<double, false>);
     ctx->launches += 2;
     NB_CUDA(ctx, cudaGetLastError());
     return NIMBUS_OK;

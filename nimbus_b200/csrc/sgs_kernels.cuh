@@ -34,29 +34,45 @@ struct SgsParams
     int px, py;           // periodic x / y
     int open[4];          // W, E, S, N lateral faces open (scalar fluxes pass)
     double Cs, Pr_t, Sc_t, nu_max, K_max;
-    // FP32 form: reciprocals of the spacings (it multiplies where the
-    // reference form divides).
+    // Reciprocals of the divisors (Recip): FP64 of dx, dy, the Prandtl and
+    // Schmidt numbers and, per level (device), of dz, of the distance between
+    // centres k and k+1 and of dz_k + dz_k+1; FP32 of the spacings.
+    double y_dx, y_dy, y_pr, y_sc;
+    const double *y_dz, *y_dzc, *y_dzs;
     float inv_dx_f, inv_dy_f;
     const float* inv_dz_f;   // [nz] (device)
-    const float* inv_dzc_f;  // [nz] (device): 1 / distance between centres k and k+1
+    const float* inv_dzc_f;  // [nz] (device)
+    int fast;                // every divisor lies where Recip's three operations give the quotient
 };
 
-// A divisor: the reference form divides by d; the FP32 form multiplies by the
-// FP32 reciprocal (one rounding more, no division sequence).
-template <class R>
+// A divisor d that many cells divide by: a spacing or a sum of spacings, or a
+// Prandtl number.  The FP32 form multiplies by its FP32 reciprocal (one
+// rounding more, no division sequence).  The reference form divides, and its
+// quotients must round as a division does: with F, from y = RN(1 / d) formed
+// on the host, q = RN(x y) is within an ulp of x / d, its residual d q - x is
+// exact in one FMA, and q - residual * y rounds to RN(x / d) (Markstein, IBM
+// J. Res. Dev. 34, 1990): three operations where the general division takes
+// about ten and a branch, and the closure divides some ninety times a cell.
+// (The residual with this sign also keeps a zero's sign.)  Without F (a
+// divisor outside [2^-60, 2^60], where a residual could leave the normal
+// range) the form divides.
+template <class R, bool F>
 struct Recip
 {
-    double d;
+    double d, y;
     float inv;
 };
 
-template <class R>
-__device__ __forceinline__ R operator/(R x, Recip<R> r)
+template <class R, bool F>
+__device__ __forceinline__ R operator/(R x, Recip<R, F> r)
 {
-    if constexpr (sizeof(R) == sizeof(float))
-        return x * r.inv;
-    else
-        return x / R(r.d);
+    if constexpr (sizeof(R) == sizeof(float)) return x * r.inv;
+    else if constexpr (F)
+    {
+        const double q = x * r.y;
+        return __fma_rn(-__fma_rn(r.d, q, -x), r.y, q);
+    }
+    else return x / R(r.d);
 }
 
 // Neighbour rows (eddy_viscosity.cpp:69-105): clamped to the allocated
@@ -73,7 +89,7 @@ __device__ __forceinline__ int sgs_next(int i, int n, int periodic)
     return i >= n - 2 ? 1 : (i + 1 > 1 ? i + 1 : 1);
 }
 
-template <class R>
+template <class R, bool F>
 struct SgsAt
 {
     const SgsParams& P;
@@ -87,14 +103,35 @@ struct SgsAt
     {
         return k < 0 ? R(0.0) : f(w, i, j, k);
     }
-    __device__ __forceinline__ Recip<R> DX() const { return {P.dx, P.inv_dx_f}; }
-    __device__ __forceinline__ Recip<R> DY() const { return {P.dy, P.inv_dy_f}; }
-    __device__ __forceinline__ Recip<R> DZ(int k) const { return {P.dz[k], P.inv_dz_f[k]}; }
+    __device__ __forceinline__ Recip<R, F> DX() const { return {P.dx, P.y_dx, P.inv_dx_f}; }
+    __device__ __forceinline__ Recip<R, F> DY() const { return {P.dy, P.y_dy, P.inv_dy_f}; }
+    __device__ __forceinline__ Recip<R, F> DZ(int k) const { return level(P.dz, P.y_dz, P.inv_dz_f, k); }
     // Distance between centres k and k+1 as a divisor (the reference form
     // divides by 0.5 (dz_k + dz_k+1)).  Defined for k < nz - 1 only: every
     // caller guards that; the FP32 table holds NaN at nz - 1 and dz has no
     // element nz.
-    __device__ __forceinline__ Recip<R> DZC(int k) const { return {0.5 * (P.dz[k] + P.dz[k + 1]), P.inv_dzc_f[k]}; }
+    __device__ __forceinline__ Recip<R, F> DZC(int k) const
+    {
+        Recip<R, F> r{};
+        if constexpr (sizeof(R) == sizeof(float)) r.inv = P.inv_dzc_f[k];
+        else
+        {
+            r.d = 0.5 * (P.dz[k] + P.dz[k + 1]);
+            r.y = P.y_dzc[k];
+        }
+        return r;
+    }
+    __device__ __forceinline__ Recip<R, F> level(const double* d, const double* y, const float* inv, int k) const
+    {
+        Recip<R, F> r{};
+        if constexpr (sizeof(R) == sizeof(float)) r.inv = inv[k];
+        else
+        {
+            r.d = d[k];
+            r.y = y[k];
+        }
+        return r;
+    }
     __device__ __forceinline__ R dzc(int k) const { return R(0.5) * (R(P.dz[k]) + R(P.dz[k + 1])); }
     // mu = rho nu at a centre; on an xy edge (four-point mean); on an xz or yz
     // edge (pair means of the two levels, weighted by the other level's
@@ -113,16 +150,18 @@ struct SgsAt
     {
         const R lo = R(0.5) * (mu(rho, nu, i, j, k) + mu(rho, nu, i1, j1, k));
         const R up = R(0.5) * (mu(rho, nu, i, j, k + 1) + mu(rho, nu, i1, j1, k + 1));
-        return (R(P.dz[k + 1]) * lo + R(P.dz[k]) * up) / (R(P.dz[k]) + R(P.dz[k + 1]));
+        const R sum = R(P.dz[k + 1]) * lo + R(P.dz[k]) * up;
+        if constexpr (sizeof(R) == sizeof(float)) return sum / (R(P.dz[k]) + R(P.dz[k + 1]));
+        else return sum / Recip<R, F>{P.dz[k] + P.dz[k + 1], P.y_dzs[k], 0.0f};
     }
 };
 
 // Strain-rate square at a scalar centre (compute_directional_strain_sq_centered).
-template <class R>
+template <class R, bool F>
 __device__ R sgs_strain_sq(const SgsParams& P, const float* u, const float* v, const float* w, int i, int j,
                                 int k)
 {
-    const SgsAt<R> A{P};
+    const SgsAt<R, F> A{P};
     const int nx = P.d.nx, ny = P.d.ny, nz = P.d.nz;
     const int jm = sgs_prev(j, ny, P.py), im = sgs_prev(i, nx, P.px);
     const R s11 = (A.f(u, i, j, k) - A.f(u, im, j, k)) / A.DX();
@@ -153,7 +192,7 @@ __device__ R sgs_strain_sq(const SgsParams& P, const float* u, const float* v, c
                 xz0[e] = xz1[e] = yz0[e] = yz1[e] = R(0.0);
                 continue;
             }
-            const Recip<R> dzc = A.DZC(kk);
+            const Recip<R, F> dzc = A.DZC(kk);
             const int ii = xi[e], ii1 = sgs_next(ii, nx, P.px);
             xz0[e] = (A.f(u, ii, j, kk + 1) - A.f(u, ii, j, kk)) / dzc;
             xz1[e] = (A.wf(w, ii1, j, kk) - A.wf(w, ii, j, kk)) / A.DX();
@@ -186,7 +225,7 @@ __device__ __forceinline__ R sgs_min(R a, R b) { return b < a ? b : a; }  // std
 // Eddy coefficients of every cell; a cell whose inputs break the reference's
 // field contract (validate_scheme_inputs, eddy_viscosity.cpp:1088-1175) or
 // whose coefficient is not finite raises kStatusSgsInvalid.
-template <class R>
+template <class R, bool F>
 __global__ void __launch_bounds__(256, 3) sgs_coefficients_kernel(SgsParams P, const float* __restrict__ u,
                                                                const float* __restrict__ v,
                                                                const float* __restrict__ w,
@@ -204,11 +243,21 @@ __global__ void __launch_bounds__(256, 3) sgs_coefficients_kernel(SgsParams P, c
         const float th = theta[c], r = rho[c];
         bool bad = !isfinite(u[c]) || !isfinite(v[c]) || !isfinite(w[c]) || !isfinite(th) || !(th > 0.0f) ||
                    !isfinite(r) || !(r > 0.0f) || (qv && (!isfinite(qv[c]) || qv[c] < 0.0f));
-        const R strain = sqrt(sgs_strain_sq<R>(P, u, v, w, i, j, k));
+        const R strain = sqrt(sgs_strain_sq<R, F>(P, u, v, w, i, j, k));
         R nu = R(P.Cs) * R(P.Cs) * R(P.delta[k]) * R(P.delta[k]) * strain * R(1.0);
         bad |= !isfinite(strain) || !isfinite(nu);
         nu = sgs_min(nu, R(P.nu_max));
-        const R kt = nu / R(P.Pr_t), kq = nu / R(P.Sc_t);
+        R kt, kq;
+        if constexpr (sizeof(R) == sizeof(float))
+        {
+            kt = nu / R(P.Pr_t);
+            kq = nu / R(P.Sc_t);
+        }
+        else
+        {
+            kt = nu / Recip<R, F>{P.Pr_t, P.y_pr, 0.0f};
+            kq = nu / Recip<R, F>{P.Sc_t, P.y_sc, 0.0f};
+        }
         bad |= !isfinite(kt) || !isfinite(kq);
         if (bad) atomicOr(status, kStatusSgsInvalid);
         nu_t[c] = (float)nu;
@@ -218,11 +267,11 @@ __global__ void __launch_bounds__(256, 3) sgs_coefficients_kernel(SgsParams P, c
 }
 
 // Scalar diffusion tendency at one cell (compute_scalar_diffusion_tendencies).
-template <class R>
+template <class R, bool F>
 __device__ R sgs_scalar_rate(const SgsParams& P, const float* rho, const float* K, const float* phi, int i,
                                   int j, int k)
 {
-    const SgsAt<R> A{P};
+    const SgsAt<R, F> A{P};
     const int nx = P.d.nx, ny = P.d.ny, nz = P.d.nz;
     const int jmm = !P.py && !P.open[2] && j == 1 ? j : sgs_prev(j, ny, P.py);
     const int jpp = !P.py && !P.open[3] && j == ny - 2 ? j : sgs_next(j, ny, P.py);
@@ -259,22 +308,22 @@ __device__ R sgs_scalar_rate(const SgsParams& P, const float* rho, const float* 
 // shared by du (its upper edge) and dw (its east edge); T23 likewise on the
 // yz edge.  In each stress mode the reference's du / dw (dv / dw) forms of
 // T13 (T23) reduce to the same expression.
-template <class R>
+template <class R, bool F>
 __device__ __forceinline__ R sgs_t12(const SgsParams& P, const float* u, const float* v, const float* rho,
                                           const float* nu, int i, int j, int k)
 {
-    const SgsAt<R> A{P};
+    const SgsAt<R, F> A{P};
     const int i1 = sgs_next(i, P.d.nx, P.px), j1 = sgs_next(j, P.d.ny, P.py);
     const R s12 =
         R(0.5) * ((A.f(u, i, j1, k) - A.f(u, i, j, k)) / A.DY() + (A.f(v, i1, j, k) - A.f(v, i, j, k)) / A.DX());
     return R(2.0) * A.mu_xy(rho, nu, i, j, k) * s12;
 }
 
-template <class R>
+template <class R, bool F>
 __device__ __forceinline__ R sgs_t13(const SgsParams& P, const float* u, const float* w, const float* rho,
                                           const float* nu, int i, int j, int k)
 {
-    const SgsAt<R> A{P};
+    const SgsAt<R, F> A{P};
     const int i1 = sgs_next(i, P.d.nx, P.px);
     const R dwdx = (A.wf(w, i1, j, k) - A.wf(w, i, j, k)) / A.DX();
     R grad = dwdx;
@@ -286,11 +335,11 @@ __device__ __forceinline__ R sgs_t13(const SgsParams& P, const float* u, const f
     return A.mu_z(rho, nu, i, j, i1, j, k) * grad;
 }
 
-template <class R>
+template <class R, bool F>
 __device__ __forceinline__ R sgs_t23(const SgsParams& P, const float* v, const float* w, const float* rho,
                                           const float* nu, int i, int j, int k)
 {
-    const SgsAt<R> A{P};
+    const SgsAt<R, F> A{P};
     const int j1 = sgs_next(j, P.d.ny, P.py);
     const R dwdy = (A.wf(w, i, j1, k) - A.wf(w, i, j, k)) / A.DY();
     R grad = dwdy;
@@ -304,11 +353,11 @@ __device__ __forceinline__ R sgs_t23(const SgsParams& P, const float* v, const f
 
 // du/dt at x-face (i, j, k) (compute_momentum_diffusion_tendencies, first
 // loop); t12 / t13: the shared corner stresses above.
-template <class R>
+template <class R, bool F>
 __device__ R sgs_du(const SgsParams& P, const float* u, const float* v, const float* w, const float* rho,
                          const float* nu, int i, int j, int k, R t12, R t13)
 {
-    const SgsAt<R> A{P};
+    const SgsAt<R, F> A{P};
     const int nx = P.d.nx, ny = P.d.ny;
     const int jmm = sgs_prev(j, ny, P.py), imm = sgs_prev(i, nx, P.px), ipp = sgs_next(i, nx, P.px);
     R div = R(0.0);
@@ -317,23 +366,23 @@ __device__ R sgs_du(const SgsParams& P, const float* u, const float* v, const fl
         const R s_r = (A.f(u, ipp, j, k) - A.f(u, i, j, k)) / A.DX();
         const R s_l = (A.f(u, i, j, k) - A.f(u, imm, j, k)) / A.DX();
         div += (R(2.0) * A.mu(rho, nu, ipp, j, k) * s_r - R(2.0) * A.mu(rho, nu, i, j, k) * s_l) / A.DX();
-        div += (t12 - sgs_t12<R>(P, u, v, rho, nu, i, jmm, k)) / A.DY();
+        div += (t12 - sgs_t12<R, F>(P, u, v, rho, nu, i, jmm, k)) / A.DY();
     }
     if (P.use_v)
     {
         // T13 on the z-faces k (upper) and k-1 (lower; zero at the ground).
-        const R lower = k > 0 ? sgs_t13<R>(P, u, w, rho, nu, i, j, k - 1) : R(0.0);
+        const R lower = k > 0 ? sgs_t13<R, F>(P, u, w, rho, nu, i, j, k - 1) : R(0.0);
         div += (t13 - lower) / A.DZ(k);
     }
     return div / (R(0.5) * (A.f(rho, i, j, k) + A.f(rho, ipp, j, k)));
 }
 
 // dv/dt at y-face (i, j, k) (second loop).
-template <class R>
+template <class R, bool F>
 __device__ R sgs_dv(const SgsParams& P, const float* u, const float* v, const float* w, const float* rho,
                          const float* nu, int i, int j, int k, R t12, R t23)
 {
-    const SgsAt<R> A{P};
+    const SgsAt<R, F> A{P};
     const int nx = P.d.nx, ny = P.d.ny;
     const int jmm = sgs_prev(j, ny, P.py), jpp = sgs_next(j, ny, P.py), imm = sgs_prev(i, nx, P.px);
     R div = R(0.0);
@@ -342,11 +391,11 @@ __device__ R sgs_dv(const SgsParams& P, const float* u, const float* v, const fl
         const R s_n = (A.f(v, i, jpp, k) - A.f(v, i, j, k)) / A.DY();
         const R s_s = (A.f(v, i, j, k) - A.f(v, i, jmm, k)) / A.DY();
         div += (R(2.0) * A.mu(rho, nu, i, jpp, k) * s_n - R(2.0) * A.mu(rho, nu, i, j, k) * s_s) / A.DY();
-        div += (t12 - sgs_t12<R>(P, u, v, rho, nu, imm, j, k)) / A.DX();
+        div += (t12 - sgs_t12<R, F>(P, u, v, rho, nu, imm, j, k)) / A.DX();
     }
     if (P.use_v)
     {
-        const R lower = k > 0 ? sgs_t23<R>(P, v, w, rho, nu, i, j, k - 1) : R(0.0);
+        const R lower = k > 0 ? sgs_t23<R, F>(P, v, w, rho, nu, i, j, k - 1) : R(0.0);
         div += (t23 - lower) / A.DZ(k);
     }
     return div / (R(0.5) * (A.f(rho, i, j, k) + A.f(rho, i, jpp, k)));
@@ -354,11 +403,11 @@ __device__ R sgs_dv(const SgsParams& P, const float* u, const float* v, const fl
 
 // dw/dt at z-face (i, j, k) (third loop): stress divergence over the dual
 // column mass.
-template <class R>
+template <class R, bool F>
 __device__ R sgs_dw(const SgsParams& P, const float* u, const float* v, const float* w, const float* rho,
                          const float* nu, int i, int j, int k, R t13, R t23)
 {
-    const SgsAt<R> A{P};
+    const SgsAt<R, F> A{P};
     const int imm = sgs_prev(i, P.d.nx, P.px), jmm = sgs_prev(j, P.d.ny, P.py);
     const R dzb = R(P.dz[k]), dzt = R(P.dz[k + 1]), dzd = A.dzc(k);
     const R mass = R(0.5) * (A.f(rho, i, j, k) * dzb + A.f(rho, i, j, k + 1) * dzt);
@@ -371,15 +420,15 @@ __device__ R sgs_dw(const SgsParams& P, const float* u, const float* v, const fl
     }
     if (P.use_h)
     {
-        force += dzd * (t13 - sgs_t13<R>(P, u, w, rho, nu, imm, j, k)) / A.DX();
-        force += dzd * (t23 - sgs_t23<R>(P, v, w, rho, nu, i, jmm, k)) / A.DY();
+        force += dzd * (t13 - sgs_t13<R, F>(P, u, w, rho, nu, imm, j, k)) / A.DX();
+        force += dzd * (t23 - sgs_t23<R, F>(P, v, w, rho, nu, i, jmm, k)) / A.DY();
     }
     return force / mass;
 }
 
 // The five tendencies of every cell; zero where the reference leaves its
 // pre-cleared outputs untouched.
-template <class R>
+template <class R, bool F>
 __global__ void __launch_bounds__(256, 4) sgs_tendencies_kernel(
     SgsParams P, const float* __restrict__ u, const float* __restrict__ v, const float* __restrict__ w,
     const float* __restrict__ theta, const float* __restrict__ qv, const float* __restrict__ rho,
@@ -400,17 +449,17 @@ __global__ void __launch_bounds__(256, 4) sgs_tendencies_kernel(
         {
             const bool du_on = i <= (P.px ? nx - 2 : nx - 3);
             const bool dv_on = j <= (P.py ? ny - 2 : ny - 3);
-            const R t12 = P.use_h && (du_on || dv_on) ? sgs_t12<R>(P, u, v, rho, nu_t, i, j, k) : R(0.0);
-            const R t13 = (du_on && P.use_v) || P.use_h ? sgs_t13<R>(P, u, w, rho, nu_t, i, j, k) : R(0.0);
-            const R t23 = (dv_on && P.use_v) || P.use_h ? sgs_t23<R>(P, v, w, rho, nu_t, i, j, k) : R(0.0);
-            if (du_on) ru = (float)sgs_du<R>(P, u, v, w, rho, nu_t, i, j, k, t12, t13);
-            if (dv_on) rv = (float)sgs_dv<R>(P, u, v, w, rho, nu_t, i, j, k, t12, t23);
-            rw = (float)sgs_dw<R>(P, u, v, w, rho, nu_t, i, j, k, t13, t23);
+            const R t12 = P.use_h && (du_on || dv_on) ? sgs_t12<R, F>(P, u, v, rho, nu_t, i, j, k) : R(0.0);
+            const R t13 = (du_on && P.use_v) || P.use_h ? sgs_t13<R, F>(P, u, w, rho, nu_t, i, j, k) : R(0.0);
+            const R t23 = (dv_on && P.use_v) || P.use_h ? sgs_t23<R, F>(P, v, w, rho, nu_t, i, j, k) : R(0.0);
+            if (du_on) ru = (float)sgs_du<R, F>(P, u, v, w, rho, nu_t, i, j, k, t12, t13);
+            if (dv_on) rv = (float)sgs_dv<R, F>(P, u, v, w, rho, nu_t, i, j, k, t12, t23);
+            rw = (float)sgs_dw<R, F>(P, u, v, w, rho, nu_t, i, j, k, t13, t23);
         }
         if (column)
         {
-            rt = (float)sgs_scalar_rate<R>(P, rho, K_theta, theta, i, j, k);
-            if (qv) rq = (float)sgs_scalar_rate<R>(P, rho, K_q, qv, i, j, k);
+            rt = (float)sgs_scalar_rate<R, F>(P, rho, K_theta, theta, i, j, k);
+            if (qv) rq = (float)sgs_scalar_rate<R, F>(P, rho, K_q, qv, i, j, k);
         }
         dudt[c] = ru;
         dvdt[c] = rv;

@@ -204,69 +204,69 @@ struct BoundaryAxis
     float inv, frame_n, frame_c;
 };
 
-// The low then the high face of one row along an axis, for V levels from
-// `base` (the row's cell 0): boundary_conditions_cartesian_cgrid.cpp:927-1121.
-// normal and cross are the velocities along and across the axis; hist_lo and
-// hist_hi the rows' KW78 memory.  The faces share no cell (n >= 4; the low one
-// writes cell 0, the high one reads cells 1 and up), so every value is loaded
-// before any is stored.
+// The low (high = false) or high face of one row along an axis, for V levels
+// from `base` (the row's cell 0): boundary_conditions_cartesian_cgrid.cpp:927-1121.
+// normal and cross are the velocities along and across the axis; hist the
+// row's KW78 memory on that face.  The two faces of a row share no cell (n >= 4:
+// the low one reads cell 1, or n-2 when periodic, and writes cell 0; the high
+// one reads cells 1 and n-3 up and writes n-2 and n-1), except that a periodic
+// low face takes the normal velocity of n-2 before the high face writes it:
+// bc_axis_face then closes the two in that order in one thread.
 template <int V>
-__device__ __forceinline__ void bc_axis_row(const BoundaryAxis& A, float dt_rad, float* normal, float* cross, float* w,
-                                            float* rho, float* p, float* hist_lo, float* hist_hi, int base)
+__device__ __forceinline__ void bc_low_face(const BoundaryAxis& A, float dt_rad, float* normal, float* cross, float* w,
+                                            float* rho, float* p, float* hist, int base)
 {
-    const bool radiate = dt_rad > 0.0f;
-    const bool rad_lo = A.lo == kBcRadiative && radiate, rad_hi = A.hi == kBcRadiative && radiate;
-    const int in = base + A.stride, a = base + (A.n - 2) * A.stride;
-    const int g0 = base, g1 = base + (A.n - 1) * A.stride, am = base + (A.n - 3) * A.stride;
-    const int sl = A.lo == kBcPeriodic ? a : in, sh = A.hi == kBcPeriodic ? in : a;
-    Levels<V> nl = load_levels<V>(normal + sl), cl = load_levels<V>(cross + sl), wl = load_levels<V>(w + sl);
-    const Levels<V> rl = load_levels<V>(rho + sl), pl = load_levels<V>(p + sl);
-    Levels<V> nh = load_levels<V>(normal + sh), ch = load_levels<V>(cross + sh), wh = load_levels<V>(w + sh);
-    const Levels<V> rh = load_levels<V>(rho + sh), ph = load_levels<V>(p + sh);
-    const Levels<V> nm = load_levels<V>(normal + am);
-    Levels<V> fl = nl, fh = nh;  // the faces' memory
-    if (rad_lo) fl = load_levels<V>(hist_lo);
-    if (rad_hi) fh = load_levels<V>(hist_hi);
-    // ---- low: ghost 0, wall face normal[0] ----
+    const bool radiate = A.lo == kBcRadiative && dt_rad > 0.0f;
+    const int src = base + (A.lo == kBcPeriodic ? A.n - 2 : 1) * A.stride;
+    Levels<V> nl = load_levels<V>(normal + src), cl = load_levels<V>(cross + src), wl = load_levels<V>(w + src);
+    const Levels<V> rl = load_levels<V>(rho + src), pl = load_levels<V>(p + src);
     bool store_n = true;
-    if (A.lo != kBcPeriodic)
+    if (A.lo == kBcRadiative)
     {
-        if (A.lo == kBcRadiative)
+        store_n = radiate;
+        if (radiate)
         {
-            store_n = rad_lo;
-            if (rad_lo)
-            {
-#pragma unroll
-                for (int q = 0; q < V; ++q)
-                {
-                    const float up = fl.v[q];
-                    const float phase = __fsub_rn(__fsub_rn(up, A.frame_n), kCStar);
-                    nl.v[q] = kw78_updated_face(up, phase, __fsub_rn(nl.v[q], up), dt_rad, A.inv, true);
-                }
-                store_levels<V>(hist_lo, nl);
-            }
-        }
-        else if (A.lo != kBcZeroGradient)
-        {
-#pragma unroll
-            for (int q = 0; q < V; ++q) nl.v[q] = A.frame_n;
-        }
-        if (A.lo == kBcRigid)
-        {
+            const Levels<V> f = load_levels<V>(hist);
 #pragma unroll
             for (int q = 0; q < V; ++q)
             {
-                cl.v[q] = A.frame_c;
-                wl.v[q] = 0.0f;
+                const float up = f.v[q];
+                const float phase = __fsub_rn(__fsub_rn(up, A.frame_n), kCStar);
+                nl.v[q] = kw78_updated_face(up, phase, __fsub_rn(nl.v[q], up), dt_rad, A.inv, true);
             }
+            store_levels<V>(hist, nl);
         }
     }
-    if (store_n) store_levels<V>(normal + g0, nl);
-    store_levels<V>(cross + g0, cl);
-    store_levels<V>(w + g0, wl);
-    store_levels<V>(rho + g0, rl);
-    store_levels<V>(p + g0, pl);
-    // ---- high: ghost n-1, wall face normal[n-2] ----
+    else if (A.lo == kBcRigid || A.lo == kBcRigidSlip)
+    {
+#pragma unroll
+        for (int q = 0; q < V; ++q) nl.v[q] = A.frame_n;
+    }
+    if (A.lo == kBcRigid)
+    {
+#pragma unroll
+        for (int q = 0; q < V; ++q)
+        {
+            cl.v[q] = A.frame_c;
+            wl.v[q] = 0.0f;
+        }
+    }
+    if (store_n) store_levels<V>(normal + base, nl);
+    store_levels<V>(cross + base, cl);
+    store_levels<V>(w + base, wl);
+    store_levels<V>(rho + base, rl);
+    store_levels<V>(p + base, pl);
+}
+
+template <int V>
+__device__ __forceinline__ void bc_high_face(const BoundaryAxis& A, float dt_rad, float* normal, float* cross,
+                                             float* w, float* rho, float* p, float* hist, int base)
+{
+    const bool radiate = A.hi == kBcRadiative && dt_rad > 0.0f;
+    const int a = base + (A.n - 2) * A.stride, g = base + (A.n - 1) * A.stride;
+    const int src = A.hi == kBcPeriodic ? base + A.stride : a;
+    Levels<V> nh = load_levels<V>(normal + src), ch = load_levels<V>(cross + src), wh = load_levels<V>(w + src);
+    const Levels<V> rh = load_levels<V>(rho + src), ph = load_levels<V>(p + src);
     if (A.hi != kBcPeriodic)
     {
         bool store_a = true;
@@ -275,18 +275,19 @@ __device__ __forceinline__ void bc_axis_row(const BoundaryAxis& A, float dt_rad,
 #pragma unroll
             for (int q = 0; q < V; ++q) nh.v[q] = A.frame_n;
         }
-        else if (rad_hi)
+        else if (radiate)
         {
+            const Levels<V> inner = load_levels<V>(normal + base + (A.n - 3) * A.stride), f = load_levels<V>(hist);
 #pragma unroll
             for (int q = 0; q < V; ++q)
             {
-                const float up = fh.v[q];
+                const float up = f.v[q];
                 const float phase = __fadd_rn(__fsub_rn(up, A.frame_n), kCStar);
-                nh.v[q] = kw78_updated_face(up, phase, __fsub_rn(up, nm.v[q]), dt_rad, A.inv, false);
+                nh.v[q] = kw78_updated_face(up, phase, __fsub_rn(up, inner.v[q]), dt_rad, A.inv, false);
             }
-            store_levels<V>(hist_hi, nh);
+            store_levels<V>(hist, nh);
         }
-        else if (A.hi == kBcZeroGradient) nh = nm;
+        else if (A.hi == kBcZeroGradient) nh = load_levels<V>(normal + base + (A.n - 3) * A.stride);
         else store_a = false;  // radiative without radiation keeps its face
         if (store_a) store_levels<V>(normal + a, nh);
         if (A.hi == kBcRigid)
@@ -299,11 +300,23 @@ __device__ __forceinline__ void bc_axis_row(const BoundaryAxis& A, float dt_rad,
             }
         }
     }
-    store_levels<V>(normal + g1, nh);
-    store_levels<V>(cross + g1, ch);
-    store_levels<V>(w + g1, wh);
-    store_levels<V>(rho + g1, rh);
-    store_levels<V>(p + g1, ph);
+    store_levels<V>(normal + g, nh);
+    store_levels<V>(cross + g, ch);
+    store_levels<V>(w + g, wh);
+    store_levels<V>(rho + g, rh);
+    store_levels<V>(p + g, ph);
+}
+
+// The low (side = 0) or high (side = 1) face of a row; with a periodic low
+// face, side 0 closes both in order and side 1 nothing.
+template <int V>
+__device__ __forceinline__ void bc_axis_face(const BoundaryAxis& A, int side, float dt_rad, float* normal,
+                                             float* cross, float* w, float* rho, float* p, float* hist_lo,
+                                             float* hist_hi, int base)
+{
+    const bool ordered = A.lo == kBcPeriodic;
+    if (side == 0) bc_low_face<V>(A, dt_rad, normal, cross, w, rho, p, hist_lo, base);
+    if (ordered ? side == 0 : side == 1) bc_high_face<V>(A, dt_rad, normal, cross, w, rho, p, hist_hi, base);
 }
 
 // Vertical closure for one (i,j) column: boundary_conditions_cartesian_cgrid.cpp:1124-1175.
@@ -341,14 +354,43 @@ __device__ __forceinline__ bool bc_inner_column(const Dims& d, int i, int j)
 }
 
 // The closure is independent from level to level except for the top level,
-// which takes the one below: a CTA closes a band of four levels (the last one
-// up to seven) all around the member, with a block barrier between the
-// reference's steps W,E -> S,N -> vertical instead of a launch.  A ring is a
-// few thousand values, so its time is the latency of its chain of loads and
-// stores: three launches took 19 us between events at every size up to
-// 160x160x56, one takes a third of that.
+// which takes the one below: a cluster of one to four CTAs closes a band of
+// four levels (the last one up to seven) all around the member, with a cluster
+// barrier between the reference's steps W,E -> S,N -> vertical instead of a
+// launch.  A ring is a few thousand values, so its time is the latency of its
+// chain of loads and stores; the cluster spreads a long ring over more SMs.
+// One CTA a band -> the cluster: ten closures of 512x512x128 0.47 -> 0.21 ms,
+// ten steps of a 256x256x80 member 1.89 -> 1.45 ms.
 constexpr int kRingLevels = 4;
-constexpr int kRingBlock = 512;
+constexpr int kRingBlock = 256;
+
+// CTAs a band of `rows` rows takes: one face of a row a thread, up to four CTAs.
+__host__ __device__ __forceinline__ int ring_cluster(int rows)
+{
+    return 2 * rows <= kRingBlock ? 1 : rows <= kRingBlock ? 2 : 4;
+}
+
+// The CTA's place in its cluster and the cluster's size (0 and 1 without one).
+__device__ __forceinline__ int cluster_rank()
+{
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return (int)r;
+}
+__device__ __forceinline__ int cluster_size()
+{
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return (int)r;
+}
+// Barrier of all threads of the cluster; global writes before it are visible
+// after it.
+__device__ __forceinline__ void cluster_barrier(int size)
+{
+    if (size == 1) __syncthreads();
+    else
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 __host__ __device__ __forceinline__ int ring_bands(int nz)
 {
@@ -358,90 +400,134 @@ __host__ __device__ __forceinline__ int ring_bands(int nz)
 
 // One band.  vertical: also close the perimeter's columns (their bottom and
 // top levels, in the bands that hold them); seed: then fill the KW78 memory
-// from the closed faces (seed_radiative_state).  Every thread of the block
+// from the closed faces (seed_radiative_state).  Every thread of the cluster
 // calls it.
 template <int V>
 __device__ __forceinline__ void bc_ring_levels(const BoundaryParams& B, float* u, float* v, float* w, float* rho,
                                                float* p, float* wave, int band, bool vertical, bool seed)
 {
     const Dims d = B.d;
+    const int size = cluster_size();
+    const int first = cluster_rank() * (int)blockDim.x + (int)threadIdx.x, step = size * (int)blockDim.x;
     const int last = ring_bands(d.nz) - 1;
     const int k0 = band * kRingLevels, k1 = band == last ? d.nz : k0 + kRingLevels;
     const int runs = (k1 - k0 + V - 1) / V;
     const int yz = d.ny * d.pz, xz = d.nx * d.pz;
     {
         const BoundaryAxis A{d.nx, d.sx(), B.west, B.east, B.inv_dx, B.frame_u, B.frame_v};
-        for (int t = threadIdx.x; t < d.ny * runs; t += blockDim.x)
+        const int count = d.ny * runs;
+        for (int t = first; t < 2 * count; t += step)
         {
-            const int j = t / runs, k = k0 + V * (t - j * runs), r = j * d.pz + k;
-            bc_axis_row<V>(A, B.dt_rad, u, v, w, rho, p, wave + r, wave + yz + r, d.at(0, j, k));
+            const int side = t >= count, q = t - side * count;
+            const int j = q / runs, k = k0 + V * (q - j * runs), r = j * d.pz + k;
+            bc_axis_face<V>(A, side, B.dt_rad, u, v, w, rho, p, wave + r, wave + yz + r, d.at(0, j, k));
         }
     }
-    __syncthreads();
+    cluster_barrier(size);
     {
         const BoundaryAxis A{d.ny, d.sy(), B.south, B.north, B.inv_dy, B.frame_v, B.frame_u};
         float* south = wave + 2 * yz;
-        for (int t = threadIdx.x; t < d.nx * runs; t += blockDim.x)
+        const int count = d.nx * runs;
+        for (int t = first; t < 2 * count; t += step)
         {
-            const int i = t / runs, k = k0 + V * (t - i * runs), r = i * d.pz + k;
-            bc_axis_row<V>(A, B.dt_rad, v, u, w, rho, p, south + r, south + xz + r, d.at(i, 0, k));
+            const int side = t >= count, q = t - side * count;
+            const int i = q / runs, k = k0 + V * (q - i * runs), r = i * d.pz + k;
+            bc_axis_face<V>(A, side, B.dt_rad, v, u, w, rho, p, south + r, south + xz + r, d.at(i, 0, k));
         }
     }
     if (vertical && (k0 == 0 || k1 == d.nz))
     {
-        __syncthreads();
-        // Rows j < lo and j > ny-4 for every i, then i < lo and i > nx-4 between them.
+        cluster_barrier(size);
+        // Rows j < loj and j > ny-4 for every i, then i < loi and i > nx-4 between them.
         const int loj = min(2, d.ny - 3), loi = min(2, d.nx - 3);
         const int rows = (loj + 3) * d.nx, sides = loi + 3, mid = d.ny - 3 - loj;
-        for (int q = threadIdx.x; q < rows + sides * mid; q += blockDim.x)
+        const int columns = rows + sides * mid;
+        const bool bottom = k0 == 0 && B.bottom == kBottomNoSlip, top = k1 == d.nz, open = B.top == kTopOpen;
+        // A few columns at a time, their loads together.
+        constexpr int kBatch = 4;
+        for (int q0 = first; q0 < columns; q0 += kBatch * step)
         {
-            int i, j;
-            if (q < rows)
+            int c[kBatch];
+            float um[kBatch], vm[kBatch], wm[kBatch];
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b)
             {
-                j = q / d.nx;
-                i = q - j * d.nx;
-                if (j >= loj) j += mid;
+                const int q = min(q0 + b * step, columns - 1);
+                int i, j;
+                if (q < rows)
+                {
+                    j = q / d.nx;
+                    i = q - j * d.nx;
+                    if (j >= loj) j += mid;
+                }
+                else
+                {
+                    const int r = q - rows;
+                    j = r / sides;
+                    i = r - j * sides;
+                    j += loj;
+                    if (i >= loi) i += d.nx - 3 - loi;
+                }
+                c[b] = d.at(i, j, 0);
+                const int km = c[b] + d.nz - 2;
+                um[b] = top ? u[km] : 0.0f;
+                vm[b] = top ? v[km] : 0.0f;
+                wm[b] = top && open ? w[km] : 0.0f;
             }
-            else
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b)
             {
-                const int r = q - rows;
-                j = r / sides;
-                i = r - j * sides;
-                j += loj;
-                if (i >= loi) i += d.nx - 3 - loi;
-            }
-            const int c = d.at(i, j, 0);
-            if (k0 == 0 && B.bottom == kBottomNoSlip)
-            {
-                u[c] = 0.0f;
-                v[c] = 0.0f;
-            }
-            if (k1 == d.nz)
-            {
-                const int kt = c + d.nz - 1, km = kt - 1;
-                // With two levels the level below is the zeroed bottom.
-                w[kt] = (B.top == kTopOpen) ? w[km] : 0.0f;
-                u[kt] = u[km];
-                v[kt] = v[km];
+                if (q0 + b * step >= columns) break;
+                if (bottom)
+                {
+                    u[c[b]] = 0.0f;
+                    v[c[b]] = 0.0f;
+                    if (d.nz == 2) um[b] = vm[b] = 0.0f;  // the level below the top is the bottom
+                }
+                if (top)
+                {
+                    const int kt = c[b] + d.nz - 1;
+                    w[kt] = wm[b];
+                    u[kt] = um[b];
+                    v[kt] = vm[b];
+                }
             }
         }
     }
     if (seed)
     {
-        __syncthreads();
-        for (int t = threadIdx.x; t < d.ny * (k1 - k0); t += blockDim.x)
+        cluster_barrier(size);
+        const int levels = k1 - k0;
+        for (int t = first; t < d.ny * levels; t += step)
         {
-            const int j = t / (k1 - k0), k = k0 + (t - j * (k1 - k0)), r = j * d.pz + k;
+            const int j = t / levels, k = k0 + (t - j * levels), r = j * d.pz + k;
             wave[r] = u[d.at(0, j, k)];
             wave[yz + r] = u[d.at(d.nx - 2, j, k)];
         }
-        for (int t = threadIdx.x; t < d.nx * (k1 - k0); t += blockDim.x)
+        for (int t = first; t < d.nx * levels; t += step)
         {
-            const int i = t / (k1 - k0), k = k0 + (t - i * (k1 - k0)), r = i * d.pz + k;
+            const int i = t / levels, k = k0 + (t - i * levels), r = i * d.pz + k;
             wave[2 * yz + r] = v[d.at(i, 0, k)];
             wave[2 * yz + xz + r] = v[d.at(i, d.ny - 2, k)];
         }
     }
+}
+
+// A launch of `bands` clusters of `cluster` CTAs.
+template <class Kernel, class... Args>
+inline cudaError_t launch_ring(Kernel kernel, int bands, int cluster, cudaStream_t st, Args... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(bands * cluster));
+    cfg.blockDim = dim3(kRingBlock);
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 template <int V>
@@ -449,7 +535,7 @@ static __global__ void __launch_bounds__(kRingBlock) acoustic_bc_ring_kernel(Bou
                                                                              float* w, float* rho, float* p,
                                                                              float* wave, int vertical)
 {
-    bc_ring_levels<V>(B, u, v, w, rho, p, wave, (int)blockIdx.x, vertical != 0, false);
+    bc_ring_levels<V>(B, u, v, w, rho, p, wave, (int)blockIdx.x / cluster_size(), vertical != 0, false);
 }
 
 // seed_radiative_state (boundary_conditions_cartesian_cgrid.cpp:798-822) for

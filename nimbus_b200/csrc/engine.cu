@@ -306,7 +306,8 @@ void destroy_graphs(nimbus_engine* e)
 constexpr size_t kExecCache = 8;  // instantiated topologies kept per part
 
 // Topology key of a captured graph: its node and edge counts and, in node
-// order, each node's type and, for kernel nodes, the kernel.  Graphs with
+// order, each node's type and, for kernel nodes, the kernel and its cluster
+// size.  Graphs with
 // equal keys are captured by the same launch sequence; an update that the
 // runtime refuses all the same only costs the instantiation it would have
 // taken anyway.
@@ -337,6 +338,11 @@ uint64_t graph_topology_key(cudaGraph_t g)
             cudaKernelNodeParams kp{};
             if (cudaGraphKernelNodeGetParams(node, &kp) != cudaSuccess) return 0;
             mix(reinterpret_cast<uint64_t>(kp.func));
+            cudaLaunchAttributeValue cluster{};
+            if (cudaGraphKernelNodeGetAttribute(node, cudaLaunchAttributeClusterDimension, &cluster) == cudaSuccess)
+                mix(cluster.clusterDim.x);
+            else
+                (void)cudaGetLastError();  // a node without the attribute
         }
     }
     return h == 0 ? 1 : h;

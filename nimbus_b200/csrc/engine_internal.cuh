@@ -244,9 +244,23 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
     int count = 0;
     EngineMember* T = e->d_table + L.first;
     const long long* pc = prefix_of(e, L, kItemCells);
-    const long long* pring = prefix_of(e, L, kItemRing);
     const long long* pcol = prefix_of(e, L, kItemColumns);
     const long long cells = tiles_of(e, L, kItemCells, n);
+    // The lateral closures of the lane's first `members` members.
+    int rows = 0;
+    for (int r = 0; r < n; ++r)
+    {
+        const Dims& d = e->slots[static_cast<size_t>(e->order[static_cast<size_t>(L.first + r)])].m.F.d;
+        rows = std::max({rows, d.nx, d.ny});
+    }
+    auto ring = [&](int members, int s, int refresh) {
+        const int bands = static_cast<int>(tiles_of(e, L, kItemRing, members));
+        if (bands <= 0) return;
+        LaunchTimer t(ctx, st, NIMBUS_KERNEL_ACOUSTIC_BOUNDARY);
+        launch_ring(engine_bc_ring_kernel, bands, ring_cluster(rows), st, static_cast<const EngineMember*>(T),
+                    prefix_of(e, L, kItemRing), s, refresh);
+        ++count;
+    };
 
     if (part == 0)
     {
@@ -296,8 +310,7 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
     }
     // seed_acoustic_radiation: apply_acoustic(0) then the KW78 seed (its rows
     // lie in perimeter columns, which the ring closes before it seeds).
-    ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_ring_kernel, tiles_of(e, L, kItemRing, n),
-                        kRingBlock, T, pring, tiles_of(e, L, kItemRing, n), 0, 1);
+    ring(n, 0, 1);
     ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_vertical_kernel, tiles_of(e, L, kItemColumns, n), 1, T,
                   pcol, tiles_of(e, L, kItemColumns, n), 1);
     return count;
@@ -454,8 +467,7 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
             ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, engine_momentum_kernel<Policy>, tiles, 1, T, pc, tiles,
                           si);
         }
-        ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_ring_kernel, tiles_of(e, L, kItemRing, a),
-                            kRingBlock, T, pring, tiles_of(e, L, kItemRing, a), si, 0);
+        ring(a, si, 0);
     }
     engine_swap_kernel<<<(n + 127) / 128, 128, 0, st>>>(T, n, 0);
     ++count;
@@ -521,8 +533,7 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
     // for the members that ask for it, on the published density and pressure.
     if (L.closing)
     {
-        ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_ring_kernel, tiles_of(e, L, kItemRing, n),
-                            kRingBlock, T, pring, tiles_of(e, L, kItemRing, n), 0, 2);
+        ring(n, 0, 2);
         ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_vertical_kernel, tiles_of(e, L, kItemColumns, n), 1,
                       T, pcol, tiles_of(e, L, kItemColumns, n), 2);
     }

@@ -287,26 +287,24 @@ __device__ __forceinline__ float* engine_density(const EngineMember& M, int s, b
     return written ? (even ? M.rho_alt : M.rho) : (even ? M.rho : M.rho_alt);
 }
 
-// The closure of a band of levels per CTA (bc_ring_levels).  refresh 0: inside
-// the acoustic loop, after substep s, with the perimeter's vertical closure
-// (the momentum pass closes the inner columns itself, fuse_vertical); 1 before
-// the loop, seeding the KW78 memory as well; 2 the closing refresh, of the
-// members that ask for it.
+// The closure of a band of levels per cluster (bc_ring_levels), one band a
+// tile.  refresh 0: inside the acoustic loop, after substep s, with the
+// perimeter's vertical closure (the momentum pass closes the inner columns
+// itself, fuse_vertical); 1 before the loop, seeding the KW78 memory as well;
+// 2 the closing refresh, of the members that ask for it.
 static __global__ void __launch_bounds__(kRingBlock) engine_bc_ring_kernel(const EngineMember* __restrict__ table,
-                                                                           const long long* __restrict__ prefix,
-                                                                           long long tiles, int s, int refresh)
+                                                                           const long long* __restrict__ prefix, int s,
+                                                                           int refresh)
 {
+    const int t = (int)blockIdx.x / cluster_size();
     int m = 0;
-    for (long long t = blockIdx.x; t < tiles; t += gridDim.x)
-    {
-        while (t >= prefix[m + 1]) ++m;
-        const EngineMember& M = table[m];
-        if (refresh == 2 && !M.close_step) continue;
-        BoundaryParams B = M.B;
-        if (refresh) B.dt_rad = 0.0f;
-        bc_ring_levels<4>(B, M.u, M.v, M.w, refresh ? M.rho : engine_density(M, s, true), M.p, M.wave,
-                          (int)(t - prefix[m]), true, refresh == 1);
-    }
+    while (t >= prefix[m + 1]) ++m;
+    const EngineMember& M = table[m];
+    if (refresh == 2 && !M.close_step) return;
+    BoundaryParams B = M.B;
+    if (refresh) B.dt_rad = 0.0f;
+    bc_ring_levels<4>(B, M.u, M.v, M.w, refresh ? M.rho : engine_density(M, s, true), M.p, M.wave,
+                      t - (int)prefix[m], true, refresh == 1);
 }
 
 // refresh: 1 before the acoustic loop, 2 the closing refresh at the end of the

@@ -16,6 +16,7 @@
 #include "relaxation_kernels.cuh"
 #include "transport_kernels.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdint>
@@ -194,12 +195,15 @@ void launch_boundaries(nimbus_cuda_context* ctx, cudaStream_t st, const Boundary
 {
     const Dims d = B.d;
     LaunchTimer t(ctx, st, NIMBUS_KERNEL_ACOUSTIC_BOUNDARY);
-    const int bands = ring_bands(d.nz);
+    const int bands = ring_bands(d.nz), rows = std::max(d.nx, d.ny);
+    const int closed = inner_closed ? 1 : 0;
     if (d.nz % 4 == 0 && aligned16(D.u) && aligned16(D.v) && aligned16(D.w) && aligned16(rho) && aligned16(D.p) &&
         aligned16(wave))
-        acoustic_bc_ring_kernel<4><<<bands, kRingBlock, 0, st>>>(B, D.u, D.v, D.w, rho, D.p, wave, inner_closed);
+        launch_ring(acoustic_bc_ring_kernel<4>, bands, ring_cluster(rows), st, B, D.u, D.v, D.w, rho, D.p, wave,
+                    closed);
     else
-        acoustic_bc_ring_kernel<1><<<bands, kRingBlock, 0, st>>>(B, D.u, D.v, D.w, rho, D.p, wave, inner_closed);
+        launch_ring(acoustic_bc_ring_kernel<1>, bands, ring_cluster(kRingLevels * rows), st, B, D.u, D.v, D.w, rho,
+                    D.p, wave, closed);
     ctx->launches += 1;
     if (inner_closed) return;
     acoustic_bc_vertical_kernel<<<grid_for(ctx, d.nx * d.ny), kThreads, 0, st>>>(B, D.u, D.v, D.w);

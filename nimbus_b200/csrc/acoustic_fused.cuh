@@ -479,9 +479,9 @@ static __global__ void __launch_bounds__(BLOCK, 3) acoustic_substep_fused_kernel
                         const float sxr = (isfinite(rho_x) && rho_x > 1.0e-6f) ? rho_x : 1.0f;
                         const float syr = (isfinite(rho_y) && rho_y > 1.0e-6f) ? rho_y : 1.0f;
                         const float szr = (isfinite(rho_z) && rho_z > 1.0e-6f) ? rho_z : 1.0f;
-                        const float a = __fdividef(-(pnx[t] - pc) * P.inv_dx_f, sxr);
-                        const float b = __fdividef(-(pn[t + nz] - pc) * P.inv_dy_f, syr);
-                        const float c = __fdividef(-dpz * P.inv_dz_f, szr);
+                        const float a = -(pnx[t] - pc) * P.inv_dx_f * rcp_normal(sxr);
+                        const float b = -(pn[t + nz] - pc) * P.inv_dy_f * rcp_normal(syr);
+                        const float c = -dpz * P.inv_dz_f * rcp_normal(szr);
                         du = isfinite(a) ? a : 0.0f;
                         dv = isfinite(b) ? b : 0.0f;
                         dw = isfinite(c) ? c : 0.0f;

@@ -407,9 +407,9 @@ __device__ __forceinline__ float3 momentum_point(const FusedParams& P, const Mom
             const float sxr = (isfinite(rho_x) && rho_x > 1.0e-6f) ? rho_x : 1.0f;
             const float syr = (isfinite(rho_y) && rho_y > 1.0e-6f) ? rho_y : 1.0f;
             const float szr = (isfinite(rho_z) && rho_z > 1.0e-6f) ? rho_z : 1.0f;
-            const float a = __fdividef(-(s.px - s.pc) * P.inv_dx_f, sxr);
-            const float b = __fdividef(-(s.py - s.pc) * P.inv_dy_f, syr);
-            const float cz = __fdividef(-dpz * P.inv_dz_f, szr);
+            const float a = -(s.px - s.pc) * P.inv_dx_f * rcp_normal(sxr);  // the densities exceed 1e-6
+            const float b = -(s.py - s.pc) * P.inv_dy_f * rcp_normal(syr);
+            const float cz = -dpz * P.inv_dz_f * rcp_normal(szr);
             du = isfinite(a) ? a : 0.0f;
             dv = isfinite(b) ? b : 0.0f;
             dw = isfinite(cz) ? cz : 0.0f;

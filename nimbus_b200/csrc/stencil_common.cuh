@@ -119,11 +119,21 @@ __device__ __forceinline__ void decompose(const Dims& d, int c, int& i, int& j, 
 __device__ __forceinline__ double finite_or_zero(double v) { return isfinite(v) ? v : 0.0; }
 __device__ __forceinline__ double safe_rho(double v) { return (isfinite(v) && v > 1.0e-6) ? v : 1.0; }
 
+// Approximate reciprocal (at most 1 ulp off) of a normal number: the form
+// without the scaling that subnormal operands need, one instruction where the
+// other takes about five.
+__device__ __forceinline__ float rcp_normal(float a)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+
 // std::clamp after a non-finite fallback (acoustic_cgrid_fast.cpp:38-43).
 __device__ __forceinline__ float clamp_value(float v, float fallback, float lo, float hi)
 {
     if (!isfinite(v)) v = fallback;
-    return v < lo ? lo : (hi < v ? hi : v);
+    return fminf(fmaxf(v, lo), hi);
 }
 
 // ---- Acoustic speed scan ------------------------------------------------

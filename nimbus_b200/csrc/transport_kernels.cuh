@@ -109,15 +109,6 @@ __device__ __forceinline__ double mc_slope(double qm, double q0, double qp)
 template <class V>
 struct Lanes;
 
-// Approximate reciprocal (at most 1 ulp off) of a normal number: the form
-// without the scaling that subnormal operands need.
-__device__ __forceinline__ float rcp_normal(float a)
-{
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
-    return r;
-}
-
 template <>
 struct Lanes<float>
 {

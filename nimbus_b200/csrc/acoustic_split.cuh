@@ -689,6 +689,13 @@ __device__ __forceinline__ void momentum_quad(const FusedParams& P, const float*
 
 constexpr int kQuadBlock = 128;  // threads of a quad kernel
 
+// Cells from which the quad kernels are launched: below, a cell per thread
+// fills the SMs better than the quad saves instructions (four CTAs of quads an
+// SM on 148 SMs).  A launch of 164 thousand cells, continuity, us between
+// events: FP32 8.4 against 8.6 with quads, reference precision 10.7 / 12.6;
+// of 1.4 million, 19.5 / 18.6 and 33.2 / 30.9.
+constexpr long long kQuadCells = 4LL * kQuadBlock * 4 * 148;
+
 template <class Policy>
 static __global__ void __launch_bounds__(kQuadBlock, 8) split_continuity_quad_kernel(
     FusedParams P, const float* __restrict__ rho, const float* __restrict__ u, const float* __restrict__ v,

@@ -10,6 +10,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <type_traits>
 #include <vector>
 
 namespace nimbus_engine_detail
@@ -216,6 +217,9 @@ long long tiles_of(const nimbus_engine* e, const nimbus_engine_detail::Lane& L, 
             ++count;                                                                                     \
         }                                                                                                \
     } while (0)
+// A launch whose tiles are cut further: units of work for the grid.
+#define ENGINE_LAUNCH_UNITS(family, kernel, units, block, ...) \
+    ENGINE_LAUNCH_GRID(family, kernel, units, 1, block, __VA_ARGS__)
 #define ENGINE_LAUNCH_TILES(family, kernel, tiles, ...)                                                  \
     do {                                                                                                 \
         const long long tiles_ = (tiles);                                                                \
@@ -394,6 +398,18 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
             A.march_blocks = H.march_blocks;
         }
     }
+    // The constant-bank continuity with C cells per thread.
+    auto continuity_const = [&](auto C, long long quad_tiles, int si) {
+        constexpr int kCells = decltype(C)::value;
+        auto launch = [&](auto kernel) {
+            ENGINE_LAUNCH_UNITS(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, kernel, (4 / kCells) * quad_tiles, kQuadTile, *al, T,
+                                quad_tiles, si);
+        };
+        if (si == 0 && shared) launch(engine_continuity_const_kernel<Policy, true, true, kCells>);
+        else if (si == 0) launch(engine_continuity_const_kernel<Policy, true, false, kCells>);
+        else if (shared) launch(engine_continuity_const_kernel<Policy, false, true, kCells>);
+        else launch(engine_continuity_const_kernel<Policy, false, false, kCells>);
+    };
     for (size_t s = 0; s < L.active.size(); ++s)
     {
         const int a = L.active[s];
@@ -401,25 +417,12 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
         const long long tiles = tiles_of(e, L, kItemCells, a);
         const long long march_tiles = tiles_of(e, L, kItemMarch, a);
         const long long quad_tiles = tiles_of(e, L, kItemQuads, a);
+        const bool small = 4 * kQuadTile * quad_tiles < kQuadCells;
         switch (cform)
         {
         case NIMBUS_ACOUSTIC_CONST:
-            if (s == 0 && shared)
-                ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP,
-                                    (engine_continuity_const_kernel<Policy, true, true>), quad_tiles, kQuadTile, *al,
-                                    T, quad_tiles, si);
-            else if (s == 0)
-                ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP,
-                                    (engine_continuity_const_kernel<Policy, true, false>), quad_tiles, kQuadTile, *al,
-                                    T, quad_tiles, si);
-            else if (shared)
-                ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP,
-                                    (engine_continuity_const_kernel<Policy, false, true>), quad_tiles, kQuadTile, *al,
-                                    T, quad_tiles, si);
-            else
-                ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP,
-                                    (engine_continuity_const_kernel<Policy, false, false>), quad_tiles, kQuadTile, *al,
-                                    T, quad_tiles, si);
+            if (small) continuity_const(std::integral_constant<int, 1>{}, quad_tiles, si);
+            else continuity_const(std::integral_constant<int, 4>{}, quad_tiles, si);
             break;
         case NIMBUS_ACOUSTIC_MARCH:
             ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, engine_continuity_march_kernel<Policy>, march_tiles, 1, T,
@@ -448,8 +451,12 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
         switch (mform)
         {
         case NIMBUS_ACOUSTIC_CONST:
-            ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, engine_momentum_const_kernel<Policy>, quad_tiles,
-                                kQuadTile, *al, T, quad_tiles, si);
+            if (small)
+                ENGINE_LAUNCH_UNITS(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, (engine_momentum_const_kernel<Policy, 1>),
+                                    4 * quad_tiles, kQuadTile, *al, T, quad_tiles, si);
+            else
+                ENGINE_LAUNCH_UNITS(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, (engine_momentum_const_kernel<Policy, 4>),
+                                    quad_tiles, kQuadTile, *al, T, quad_tiles, si);
             break;
         case NIMBUS_ACOUSTIC_MARCH:
             ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, engine_momentum_march_kernel<Policy>, march_tiles, 1, T,

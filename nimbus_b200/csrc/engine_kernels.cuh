@@ -142,10 +142,10 @@ __device__ __forceinline__ void for_member_rows(const EngineMember* __restrict__
 
 // ---- Heun slow step -------------------------------------------------------
 
-// Resident CTAs per SM of the slow Heun pair: the FP32 form at 5 (48
-// registers; measured 3.14 -> 2.88 ms per ensemble step against 4), the
-// reference-precision form at 4 (64 registers; its FP64 arithmetic spills
-// heavily at 48).
+// Resident CTAs per SM of the slow Heun pair: the reference-precision form at
+// 4 of 256 threads (64 registers), the FP32 form at 5 of kQuadTile threads (96
+// registers; 4, 6 and 8 CTAs: 1.11, 1.05 and 1.20 ms a step against 1.00 on 24
+// members of 16.5 million cells).
 #ifndef NIMBUS_SLOW_MINB
 #define NIMBUS_SLOW_MINB 4
 #endif
@@ -153,7 +153,7 @@ __device__ __forceinline__ void for_member_rows(const EngineMember* __restrict__
 #define NIMBUS_SLOW_MINB_F32 5
 #endif
 template <class Policy>
-static __global__ void __launch_bounds__(256, NIMBUS_SLOW_MINB) engine_slow_predict_kernel(const EngineMember* __restrict__ table,
+static __global__ void __launch_bounds__(256, 4) engine_slow_predict_kernel(const EngineMember* __restrict__ table,
                                                                   const long long* __restrict__ prefix,
                                                                   long long tiles)
 {
@@ -167,7 +167,7 @@ static __global__ void __launch_bounds__(256, NIMBUS_SLOW_MINB) engine_slow_pred
 }
 
 template <class Policy>
-static __global__ void __launch_bounds__(256, NIMBUS_SLOW_MINB) engine_slow_correct_kernel(const EngineMember* __restrict__ table,
+static __global__ void __launch_bounds__(256, 4) engine_slow_correct_kernel(const EngineMember* __restrict__ table,
                                                                   const long long* __restrict__ prefix,
                                                                   long long tiles)
 {
@@ -480,52 +480,63 @@ struct AcousticLaunch
 };
 static_assert(sizeof(AcousticLaunch) <= 32000, "a kernel parameter block holds at most 32764 bytes");
 
-// Four cells per thread (continuity_eos_quad, momentum_quad).
+// Calls fn(A, M, c) for the first tiles' cells: kCells = 4, one group of four
+// cells per thread of a kItemQuads tile; kCells = 1, one cell per thread, a CTA
+// taking a quarter of a tile (small lanes, kQuadCells).
+template <int kCells, class Fn>
+__device__ __forceinline__ void for_const_cells(const AcousticLaunch& L, const EngineMember* __restrict__ table,
+                                                int tiles, Fn&& fn)
+{
+    constexpr int kParts = 4 / kCells;
+    int m = 0;
+    for (int t = blockIdx.x; t < kParts * tiles; t += gridDim.x)
+    {
+        while (t >= kParts * L.quad_prefix[m + 1]) ++m;
+        const AcousticConst& A = L.m[m];
+        const int c = kCells * ((t - kParts * L.quad_prefix[m]) * kQuadTile + (int)threadIdx.x);
+        if (c >= A.F.d.cells()) continue;
+        fn(A, table[m], c);
+    }
+}
+
 // kFirst: the first substep of the step (the retained fluxes are written, not
 // accumulated, and the beginning density is kept).
 // kShared: every member's shared values equal L.shared (acoustic_shared_of).
-template <class Policy, bool kFirst, bool kShared>
+template <class Policy, bool kFirst, bool kShared, int kCells>
 static __global__ void __launch_bounds__(kQuadTile, NIMBUS_CONST_MINB) engine_continuity_const_kernel(const __grid_constant__ AcousticLaunch L,
                                                                       const EngineMember* __restrict__ table,
                                                                       long long tiles, int s)
 {
     const bool even = (s & 1) == 0;
-    int m = 0;
-    const int ntiles = (int)tiles;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
-    {
-        while (t >= L.quad_prefix[m + 1]) ++m;
-        const AcousticConst& A = L.m[m];
-        const int c = 4 * ((t - L.quad_prefix[m]) * kQuadTile + (int)threadIdx.x);
-        if (c >= A.F.d.cells()) continue;
-        const EngineMember& M = table[m];
+    for_const_cells<kCells>(L, table, (int)tiles, [&](const AcousticConst& A, const EngineMember& M, int c) {
         unsigned flags = 0;
         const FusedParams F = kShared ? with_shared(A.F, L.shared) : A.F;
-        continuity_eos_quad<Policy>(F, even ? M.rho : M.rho_alt, A.u, A.v, A.w, A.theta, A.rho0, A.eos0,
-                                    even ? M.rho_alt : M.rho, M.p, A.mfx, A.mfy, A.mfz, c, flags, kFirst,
-                                    kFirst ? A.rho_begin : nullptr);
+        float* const before = even ? M.rho : M.rho_alt;
+        float* const after = even ? M.rho_alt : M.rho;
+        float* const begin = kFirst ? A.rho_begin : nullptr;
+        if constexpr (kCells == 4)
+            continuity_eos_quad<Policy>(F, before, A.u, A.v, A.w, A.theta, A.rho0, A.eos0, after, M.p, A.mfx, A.mfy,
+                                        A.mfz, c, flags, kFirst, begin);
+        else
+            continuity_eos_cell<Policy>(F, before, A.u, A.v, A.w, A.theta, A.rho0, A.eos0, after, M.p, nullptr, A.mfx,
+                                        A.mfy, A.mfz, c, flags, kFirst, begin);
         if (flags) atomicOr(A.status, flags);
-    }
+    });
 }
 
-template <class Policy>
+template <class Policy, int kCells>
 static __global__ void __launch_bounds__(kQuadTile, NIMBUS_CONST_MINB_MOM) engine_momentum_const_kernel(const __grid_constant__ AcousticLaunch L,
                                                                     const EngineMember* __restrict__ table,
                                                                     long long tiles, int s)
 {
     const bool even = (s & 1) == 0;
-    int m = 0;
-    const int ntiles = (int)tiles;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
-    {
-        while (t >= L.quad_prefix[m + 1]) ++m;
-        const AcousticConst& A = L.m[m];
-        const int c = 4 * ((t - L.quad_prefix[m]) * kQuadTile + (int)threadIdx.x);
-        if (c >= A.F.d.cells()) continue;
-        const EngineMember& M = table[m];
-        momentum_quad<Policy>(A.F, even ? M.rho_alt : M.rho, M.p, A.p0, A.dp0, A.u, A.v, A.w, A.u, A.v, A.w, c,
-                              A.vertical);
-    }
+    for_const_cells<kCells>(L, table, (int)tiles, [&](const AcousticConst& A, const EngineMember& M, int c) {
+        const float* rho = even ? M.rho_alt : M.rho;
+        if constexpr (kCells == 4)
+            momentum_quad<Policy>(A.F, rho, M.p, A.p0, A.dp0, A.u, A.v, A.w, A.u, A.v, A.w, c, A.vertical);
+        else
+            momentum_cell<Policy>(A.F, rho, M.p, A.p0, A.dp0, A.u, A.v, A.w, A.u, A.v, A.w, c, A.vertical);
+    });
 }
 
 // The marching passes with the members' constants in the constant bank.

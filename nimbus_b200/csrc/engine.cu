@@ -781,18 +781,34 @@ const char* check_state(const nimbus_member_state* s)
 
 }  // namespace
 
-int nimbus_engine_detail::launch_microphysics(nimbus_engine* e, cudaStream_t st, const nimbus::EngineMember* table,
-                                              const long long* prefix, long long tiles)
+int nimbus_engine_detail::launch_microphysics(nimbus_engine* e, int lane, cudaStream_t st)
 {
+    const Lane& L = e->lanes[static_cast<size_t>(lane)];
+    const int n = L.members;
+    const long long tiles = tiles_of(e, L, kItemCells, n);
     if (tiles <= 0) return 0;
     nimbus_cuda_context* ctx = e->ctx;
+    const bool fp32 = ctx->precision == NIMBUS_PRECISION_FP32;
+    const EngineMember* table = e->d_table + L.first;
     LaunchTimer t(ctx, st, NIMBUS_KERNEL_MICROPHYSICS);
-    if (ctx->precision == NIMBUS_PRECISION_FP32)
-        engine_microphysics_eos_kernel<true>
-            <<<tile_grid(tiles), kEngineBlock, 0, st>>>(table, prefix, tiles);
+    if (n <= kMicroConstMembers)
+    {
+        std::unique_ptr<MicroLaunch> ml(new MicroLaunch());
+        const long long* p = e->prefix.data() + L.prefix_first + static_cast<size_t>(kItemCells) * (n + 1);
+        for (int r = 0; r <= n; ++r) ml->prefix[r] = p[r];
+        for (int r = 0; r < n; ++r)
+            ml->m[r] = micro_const_of(e->slots[static_cast<size_t>(e->order[static_cast<size_t>(L.first + r)])].m);
+        if (fp32)
+            engine_microphysics_eos_const_kernel<true><<<tile_grid(tiles), kEngineBlock, 0, st>>>(*ml, table, tiles);
+        else
+            engine_microphysics_eos_const_kernel<false><<<tile_grid(tiles), kEngineBlock, 0, st>>>(*ml, table, tiles);
+        return 1;
+    }
+    const long long* prefix = prefix_of(e, L, kItemCells);
+    if (fp32)
+        engine_microphysics_eos_kernel<true><<<tile_grid(tiles), kEngineBlock, 0, st>>>(table, prefix, tiles);
     else
-        engine_microphysics_eos_kernel<false>
-            <<<tile_grid(tiles), kEngineBlock, 0, st>>>(table, prefix, tiles);
+        engine_microphysics_eos_kernel<false><<<tile_grid(tiles), kEngineBlock, 0, st>>>(table, prefix, tiles);
     return 1;
 }
 

@@ -41,8 +41,7 @@ struct Lane
 // The Kessler + EOS pass (FP64 in the reference-precision form, FP32 in the
 // FP32 form) is launched from the uncontracted unit (engine.cu), so the engine
 // and the per-operation path share its rounding.  Returns the launch count.
-int launch_microphysics(nimbus_engine* e, cudaStream_t st, const nimbus::EngineMember* table,
-                        const long long* prefix, long long tiles);
+int launch_microphysics(nimbus_engine* e, int lane, cudaStream_t st);
 }  // namespace nimbus_engine_detail
 
 struct nimbus_engine
@@ -533,7 +532,7 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
     }
     // Kessler step and the EOS pressure re-projection (one pass), then the
     // pointer rotation that publishes the new qr and pressure.
-    count += nimbus_engine_detail::launch_microphysics(e, st, T, pc, cells);
+    count += nimbus_engine_detail::launch_microphysics(e, lane, st);
     engine_swap_kernel<<<(n + 127) / 128, 128, 0, st>>>(T, n, 1);
     ++count;
     // The closing boundary refresh (apply_full_attributed, after the sponge)

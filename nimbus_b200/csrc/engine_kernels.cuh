@@ -1185,57 +1185,133 @@ static __global__ void __launch_bounds__(kQuadTile) engine_sound_speed_kernel(co
 // pressure is formed from the applied state while it is still in registers
 // and written to the member's candidate buffer; engine_swap_kernel publishes
 // it by exchanging p and the candidate unless the projection was refused.
-// Resident CTAs per SM of the Kessler + EOS pass: the FP32 form at 5 (48
-// registers; 1.03 -> 0.99 ms per ensemble step), the reference-precision
-// form at 4.
+// Resident CTAs per SM of the Kessler + EOS pass: the FP32 form at 6, the
+// reference-precision form at 4.
 #ifndef NIMBUS_MICRO_MINB_F32
-#define NIMBUS_MICRO_MINB_F32 5
+#define NIMBUS_MICRO_MINB_F32 6
 #endif
+
+// A member's constants of the pass, and its buffers that do not rotate.
+struct MicroConst
+{
+    KesslerParams K;
+    float *u, *v, *w, *theta, *qv, *qc;
+    unsigned* status;
+    const float4* eos0;
+    EosSeries eos_series;
+    double gamma;
+    RelaxTables R;
+    int microphysics;
+};
+
+// The buffers that rotate: density, pressure, rain and its new values, and
+// the candidate pressure.
+struct MicroRotating
+{
+    const float *rho, *p, *qr;
+    float *qr_alt, *eos;
+};
+
+__host__ __device__ __forceinline__ MicroConst micro_const_of(const EngineMember& M)
+{
+    MicroConst A;
+    A.K = M.K;
+    A.u = M.u;
+    A.v = M.v;
+    A.w = M.w;
+    A.theta = M.theta;
+    A.qv = M.qv;
+    A.qc = M.qc;
+    A.status = M.status;
+    A.eos0 = M.eos0;
+    A.eos_series = M.eos_series;
+    A.gamma = M.gamma;
+    A.R = M.R;
+    A.microphysics = M.microphysics;
+    return A;
+}
+
+template <bool kFp32>
+__device__ __forceinline__ void microphysics_eos_cell(const MicroConst& A, const MicroRotating& M, int c)
+{
+    unsigned flags = 0;
+    int i, j, k;
+    decompose(A.K.d, c, i, j, k);
+    if (k >= A.K.d.nz) return;
+    float4 s;
+    const float po = M.p[c];
+    if (A.microphysics)
+    {
+        if constexpr (kFp32)
+            kessler_cell_f32<true>(A.K, A.theta, A.qv, A.qc, M.qr, M.p, M.rho, M.qr_alt, nullptr, nullptr, nullptr,
+                                   nullptr, c, &s);
+        else
+            kessler_cell<true>(A.K, A.theta, A.qv, A.qc, M.qr, M.p, M.rho, M.qr_alt, nullptr, nullptr, nullptr,
+                               nullptr, c, &s);
+    }
+    else
+        s = make_float4(A.theta[c], A.qv[c], A.qc[c], M.qr[c]);
+    float p_new;
+    bool ok;
+    if constexpr (kFp32)
+        ok = eos_candidate_value_f32(A.K.d, c, k, M.rho[c], s.x, A.eos0, A.eos_series, A.gamma, true, po, s.y, s.z,
+                                     s.w, p_new, flags);
+    else
+        ok = eos_candidate_value(A.K.d, c, M.rho[c], s.x, A.gamma, true, po, s.y, s.z, s.w, p_new, flags);
+    if (ok) M.eos[c] = p_new;
+    if (flags) atomicOr(A.status, flags);
+    // The end-of-step sponge after the EOS projection (dynamics.cpp:7323-7340).
+    if (A.R.do_upper | A.R.do_w_only | A.R.do_lateral)
+    {
+        float uu = A.u[c], vv = A.v[c], ww = A.w[c], th = s.x;
+        if (relax_cell(A.R, A.K.d.nx, A.K.d.ny, i, j, k, uu, vv, ww, th))
+        {
+            A.u[c] = uu;
+            A.v[c] = vv;
+            A.w[c] = ww;
+            A.theta[c] = th;
+        }
+    }
+}
+
 template <bool kFp32>
 static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_MICRO_MINB_F32 : 4) engine_microphysics_eos_kernel(const EngineMember* __restrict__ table,
                                                                              const long long* __restrict__ prefix,
                                                                              long long tiles)
 {
     for_member_items(table, prefix, tiles, kItemCells, [&](const EngineMember& M, int c) {
-        unsigned flags = 0;
-        int i, j, k;
-        decompose(M.K.d, c, i, j, k);
-        if (k >= M.K.d.nz) return;
-        float4 s;
-        const float po = M.p[c];
-        if (M.microphysics)
-        {
-            if constexpr (kFp32)
-                kessler_cell_f32<true>(M.K, M.theta, M.qv, M.qc, M.qr, M.p, M.rho, M.qr_alt, nullptr, nullptr,
-                                       nullptr, nullptr, c, &s);
-            else
-                kessler_cell<true>(M.K, M.theta, M.qv, M.qc, M.qr, M.p, M.rho, M.qr_alt, nullptr, nullptr, nullptr,
-                                   nullptr, c, &s);
-        }
-        else
-            s = make_float4(M.theta[c], M.qv[c], M.qc[c], M.qr[c]);
-        float p_new;
-        bool ok;
-        if constexpr (kFp32)
-            ok = eos_candidate_value_f32(M.K.d, c, k, M.rho[c], s.x, M.eos0, M.eos_series, M.gamma, true,
-                                         po, s.y, s.z, s.w, p_new, flags);
-        else
-            ok = eos_candidate_value(M.K.d, c, M.rho[c], s.x, M.gamma, true, po, s.y, s.z, s.w, p_new, flags);
-        if (ok) M.eos[c] = p_new;
-        if (flags) atomicOr(M.status, flags);
-        // The end-of-step sponge after the EOS projection (dynamics.cpp:7323-7340).
-        if (M.R.do_upper | M.R.do_w_only | M.R.do_lateral)
-        {
-            float uu = M.u[c], vv = M.v[c], ww = M.w[c], th = s.x;
-            if (relax_cell(M.R, M.K.d.nx, M.K.d.ny, i, j, k, uu, vv, ww, th))
-            {
-                M.u[c] = uu;
-                M.v[c] = vv;
-                M.w[c] = ww;
-                M.theta[c] = th;
-            }
-        }
+        microphysics_eos_cell<kFp32>(micro_const_of(M), MicroRotating{M.rho, M.p, M.qr, M.qr_alt, M.eos}, c);
     });
+}
+
+// The same with the members' constants in the constant bank, for lanes whose
+// constants fit a parameter block: the member table's loads and the registers
+// that held them go.  24 members of 16.5 million cells, ten steps 5.45 -> 4.93
+// ms; 256x256x80 1.54 -> 1.42; reference precision, 3.0 million cells 0.76 ->
+// 0.73.
+constexpr int kMicroConstMembers = 64;
+
+struct MicroLaunch
+{
+    long long prefix[kMicroConstMembers + 1];
+    MicroConst m[kMicroConstMembers];
+};
+static_assert(sizeof(MicroLaunch) <= 32000, "a kernel parameter block holds at most 32764 bytes");
+
+template <bool kFp32>
+static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_MICRO_MINB_F32 : 4) engine_microphysics_eos_const_kernel(
+    const __grid_constant__ MicroLaunch L, const EngineMember* __restrict__ table, long long tiles)
+{
+    int m = 0;
+    for (long long t = blockIdx.x; t < tiles; t += gridDim.x)
+    {
+        while (t >= L.prefix[m + 1]) ++m;
+        const MicroConst& A = L.m[m];
+        const int c = (int)((t - L.prefix[m]) * blockDim.x) + (int)threadIdx.x;
+        if (c >= A.K.d.cells()) continue;
+        const EngineMember& M = table[m];
+        microphysics_eos_cell<kFp32>(A, MicroRotating{M.rho, M.p, M.qr, M.qr_alt, M.eos}, c);
+    }
 }
 
 }  // namespace nimbus

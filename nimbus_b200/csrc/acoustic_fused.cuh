@@ -188,7 +188,7 @@ __device__ __forceinline__ float substep_pressure(const FusedParams& P, const fl
         const double thv = (double)th;
         if (thv > 0.0)
         {
-            const double x = (double)rho_stored * kRd * thv / kP00;
+            const double x = divided_by((double)rho_stored * kRd * thv, kP00);
             p_new = kP00 * pow(x, P.gamma);
         }
         if (!isfinite(p_new) || p_new <= 0.0) p_new = (double)P.p_ref_fallback;

@@ -51,7 +51,7 @@ __device__ __forceinline__ double k_theta_to_temperature(double theta, double p)
 {
     if (!isfinite(theta) || !isfinite(p)) return kKT0;
     const double th = kclamp(theta, 150.0, 700.0), ps = kclamp(p, 100.0, 200000.0);
-    const double T = th * pow(ps / kKP0, kKRd / kKCp);
+    const double T = th * pow(divided_by(ps, kKP0), kKRd / kKCp);
     return isfinite(T) ? T : kKT0;
 }
 
@@ -61,7 +61,7 @@ __device__ __forceinline__ double k_qvs_water(double T, double p)
     if (isfinite(T))
     {
         const double tc = kclamp(T, 150.0, 400.0) - kKT0;
-        const double value = 611.21 * exp((18.678 - tc / 234.5) * tc / (257.14 + tc));
+        const double value = 611.21 * exp((18.678 - divided_by(tc, 234.5)) * tc / (257.14 + tc));
         e = isfinite(value) ? kmax(0.0, value) : 0.0;
     }
     if (!isfinite(e) || !isfinite(p)) return 0.0;
@@ -76,8 +76,8 @@ __device__ __forceinline__ double k_sat_slope(double temperature, double saturat
     const double vapor = saturation * pressure / (0.62198 + saturation);
     const double tc = temperature - kKT0;
     const double den = 257.14 + tc;
-    const double num = (18.678 - tc / 234.5) * tc;
-    const double num_slope = 18.678 - 2.0 * tc / 234.5;
+    const double num = (18.678 - divided_by(tc, 234.5)) * tc;
+    const double num_slope = 18.678 - divided_by(2.0 * tc, 234.5);
     const double lps = (num_slope * den - num) / (den * den);
     return saturation * pressure / kmax(pressure - vapor, 1.0) * lps;
 }
@@ -579,7 +579,7 @@ __device__ __forceinline__ bool eos_candidate_value(const Dims& d, int c, float 
                                                     float po, float q, float qc, float qr, float& p_new,
                                                     unsigned& flags)
 {
-    const double diagnosed = kP00 * pow((double)r * kRd * (double)th / kP00, gamma);
+    const double diagnosed = kP00 * pow(divided_by((double)r * kRd * (double)th, kP00), gamma);
     if (!isfinite(r) || !(r > 0.0f) || !isfinite(th) || !(th > 0.0f) || !isfinite(diagnosed) || diagnosed <= 0.0 ||
         !isfinite((float)diagnosed))
     {

@@ -116,6 +116,18 @@ __device__ __forceinline__ void decompose(const Dims& d, int c, int& i, int& j, 
     i = t / d.ny;
 }
 
+// x / d rounded as the division rounds it, for a literal d well inside the
+// normal range and a finite x whose quotient is far from its ends: with
+// y = RN(1 / d), a constant, RN(x y) is within an ulp of the quotient, its
+// residual is exact in one FMA and one correction rounds to RN(x / d)
+// (Markstein, IBM J. Res. Dev. 34, 1990); three operations for the general
+// division's ten and a branch.  A non-finite x gives a non-finite result.
+__device__ __forceinline__ double divided_by(double x, double d)
+{
+    const double y = 1.0 / d, q = x * y;
+    return __fma_rn(-__fma_rn(d, q, -x), y, q);
+}
+
 __device__ __forceinline__ double finite_or_zero(double v) { return isfinite(v) ? v : 0.0; }
 __device__ __forceinline__ double safe_rho(double v) { return (isfinite(v) && v > 1.0e-6) ? v : 1.0; }
 

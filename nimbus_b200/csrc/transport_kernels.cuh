@@ -479,6 +479,19 @@ __device__ __forceinline__ float limiter_factor(const TP& T, float fxp, float fx
     }
 }
 
+// Whether a scalar has no flux through any of a cell's six faces (+-0 each), as
+// cloud and rain have over most of a domain.  In reference precision warps
+// whose cells are all calm skip that scalar's FP64 arithmetic, whose result is
+// then known exactly (member engine, 3.0M cells: update 0.477 -> 0.350 ms,
+// limiter 0.247 -> 0.226); the FP32 sums cost less than the test (update
+// 3.63 -> 4.17 ms on 16.5M cells).
+__device__ __forceinline__ bool calm(float a, float b, float c, float d, float e, float f)
+{
+    return ((__float_as_uint(a) | __float_as_uint(b) | __float_as_uint(c) | __float_as_uint(d) | __float_as_uint(e) |
+             __float_as_uint(f)) &
+            0x7fffffffu) == 0u;
+}
+
 // The limiter factor of every positive-definite scalar at cell c; sf is
 // [scalars][3][cells], rl [scalars][cells].
 template <bool kFp32, class QIn>
@@ -500,8 +513,11 @@ __device__ __forceinline__ void transport_limiter_cell(const TransportParams& T,
         const float* __restrict__ sfx = sf + (size_t)s * 3 * n;
         const float* __restrict__ sfy = sfx + n;
         const float* __restrict__ sfz = sfy + n;
-        rl[(size_t)s * n + c] = limiter_factor<kFp32>(T, sfx[c], sfx[cxm], sfy[c], sfy[cym], sfz[c], sfz[czm], xp,
-                                                      xm, yp, ym, zp, zm, rb, q_of(s)[c]);
+        const float fxp = sfx[c], fxm = sfx[cxm], fyp = sfy[c], fym = sfy[cym], fzp = sfz[c], fzm = sfz[czm];
+        rl[(size_t)s * n + c] =
+            !kFp32 && calm(fxp, fxm, fyp, fym, fzp, fzm)
+                ? 1.0f  // nothing leaves the cell
+                : limiter_factor<kFp32>(T, fxp, fxm, fyp, fym, fzp, fzm, xp, xm, yp, ym, zp, zm, rb, q_of(s)[c]);
     }
 }
 
@@ -624,6 +640,11 @@ __device__ __forceinline__ void transport_update_cell(const TransportParams& T, 
         const float fxp = sfx[c], fxm = sfx[cxm], fyp = sfy[c], fym = sfy[cym];
         const float fzp = sfz[c], fzm = sfz[czm];
         const float qraw = q_of(s)[c];
+        if (!kFp32 && pd && __float_as_uint(qraw) == 0u && isfinite(rb) && calm(fxp, fxm, fyp, fym, fzp, fzm))
+        {
+            qo_of(s)[c] = 0.0f;  // (rho_b 0 - dt 0 + dt 0) / rho_e
+            continue;
+        }
         float rc = 1.0f, rxp = 1.0f, rxm = 1.0f, ryp = 1.0f, rym = 1.0f, rzp = 1.0f, rzm = 1.0f;
         if (pd)
         {
@@ -695,20 +716,6 @@ __device__ __forceinline__ float4 stencil_flux4(const float4* __restrict__ q4, c
     }
 }
 
-// Whether scalar s has no flux through any of a cell's six faces (+-0 each), as
-// cloud and rain have over most of a domain.  In reference precision warps
-// whose cells are all calm skip that scalar's FP64 arithmetic, whose result is
-// then known exactly (3.0M cells: update 0.477 -> 0.350 ms, limiter
-// 0.247 -> 0.226); the FP32 sums cost less than the test (update
-// 3.63 -> 4.17 ms).
-__device__ __forceinline__ bool calm(const float4& a, const float4& b, const float4& c, const float4& d,
-                                     const float4& e, const float4& f, int s)
-{
-    return ((__float_as_uint(lane4(a, s)) | __float_as_uint(lane4(b, s)) | __float_as_uint(lane4(c, s)) |
-             __float_as_uint(lane4(d, s)) | __float_as_uint(lane4(e, s)) | __float_as_uint(lane4(f, s))) &
-            0x7fffffffu) == 0u;
-}
-
 // The cell functions below take the transport parameters as any type with
 // TransportParams' geometry and flag fields (the member engine passes a
 // compact copy through the constant bank).
@@ -772,7 +779,8 @@ __device__ __forceinline__ void transport_limiter_cell4(const TP& T, const float
     float r[4];  // without any flux nothing leaves the cell: factor 1
 #pragma unroll
     for (int s = 0; s < 4; ++s)
-        r[s] = T.positive_definite[s] && (kFp32 || !calm(fxp, fxm, fyp, fym, fzp, fzm, s))
+        r[s] = T.positive_definite[s] && (kFp32 || !calm(lane4(fxp, s), lane4(fxm, s), lane4(fyp, s), lane4(fym, s),
+                                                         lane4(fzp, s), lane4(fzm, s)))
                    ? limiter_factor<kFp32>(T, lane4(fxp, s), lane4(fxm, s), lane4(fyp, s), lane4(fym, s),
                                            lane4(fzp, s), lane4(fzm, s), xp, xm, yp, ym, zp, zm, rb, lane4(q, s))
                    : 1.0f;
@@ -817,7 +825,8 @@ __device__ __forceinline__ void transport_update_cell4(const TP& T, const float4
     for (int s = 0; s < 4; ++s)
     {
         const bool pd = T.positive_definite[s] != 0;
-        if (!kFp32 && pd && __float_as_uint(qraw[s]) == 0u && isfinite(rb) && calm(fxp, fxm, fyp, fym, fzp, fzm, s))
+        if (!kFp32 && pd && __float_as_uint(qraw[s]) == 0u && isfinite(rb) &&
+            calm(lane4(fxp, s), lane4(fxm, s), lane4(fyp, s), lane4(fym, s), lane4(fzp, s), lane4(fzm, s)))
         {
             qo_of(s)[c] = 0.0f;  // (rho_b 0 - dt 0 + dt 0) / rho_e
             continue;

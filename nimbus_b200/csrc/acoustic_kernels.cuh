@@ -341,6 +341,7 @@ __device__ __forceinline__ void bc_vertical_column(const BoundaryParams& B, floa
 static __global__ void acoustic_bc_vertical_kernel(BoundaryParams B, float* __restrict__ u, float* __restrict__ v,
                                             float* __restrict__ w)
 {
+    grid_dependency();
     const int cols = B.d.nx * B.d.ny;
     for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < cols; col += gridDim.x * blockDim.x)
         bc_vertical_column(B, u, v, w, col);
@@ -513,28 +514,12 @@ __device__ __forceinline__ void bc_ring_levels(const BoundaryParams& B, float* u
     }
 }
 
-// A launch of `bands` clusters of `cluster` CTAs.
-template <class Kernel, class... Args>
-inline cudaError_t launch_ring(Kernel kernel, int bands, int cluster, cudaStream_t st, Args... args)
-{
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(bands * cluster));
-    cfg.blockDim = dim3(kRingBlock);
-    cfg.stream = st;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = static_cast<unsigned>(cluster);
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 template <int V>
 static __global__ void __launch_bounds__(kRingBlock) acoustic_bc_ring_kernel(BoundaryParams B, float* u, float* v,
                                                                              float* w, float* rho, float* p,
                                                                              float* wave, int vertical)
 {
+    grid_dependency();
     bc_ring_levels<V>(B, u, v, w, rho, p, wave, (int)blockIdx.x / cluster_size(), vertical != 0, false);
 }
 

@@ -309,6 +309,7 @@ static __global__ void __launch_bounds__(256) split_continuity_eos_kernel(
     float* __restrict__ drho_out, float* __restrict__ mfx, float* __restrict__ mfy, float* __restrict__ mfz,
     unsigned* __restrict__ status)
 {
+    grid_dependency();
     const int n = P.d.cells();
     unsigned flags = 0;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
@@ -703,6 +704,7 @@ static __global__ void __launch_bounds__(kQuadBlock, 8) split_continuity_quad_ke
     const float4* __restrict__ eos0, float* __restrict__ rho_out, float* __restrict__ p_out,
     float* __restrict__ mfx, float* __restrict__ mfy, float* __restrict__ mfz, unsigned* __restrict__ status)
 {
+    grid_dependency();
     const int n = P.d.cells();
     unsigned flags = 0;
     for (int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x); c < n; c += 4 * gridDim.x * blockDim.x)
@@ -718,6 +720,7 @@ static __global__ void __launch_bounds__(kQuadBlock, 8) split_momentum_quad_kern
     const float* __restrict__ w, float* __restrict__ u_out, float* __restrict__ v_out, float* __restrict__ w_out,
     int fuse_vertical)
 {
+    grid_dependency();
     const int n = P.d.cells();
     for (int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x); c < n; c += 4 * gridDim.x * blockDim.x)
         momentum_quad<Policy>(P, rho, p, p0, dp0_split, u, v, w, u_out, v_out, w_out, c, fuse_vertical);
@@ -730,6 +733,7 @@ static __global__ void __launch_bounds__(256) split_momentum_kernel(
     const float* __restrict__ w, float* __restrict__ u_out, float* __restrict__ v_out, float* __restrict__ w_out,
     int fuse_vertical)
 {
+    grid_dependency();
     const int n = P.d.cells();
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
         momentum_cell<Policy>(P, rho, p, p0, dp0_split, u, v, w, u_out, v_out, w_out, c, fuse_vertical);

@@ -305,10 +305,9 @@ void destroy_graphs(nimbus_engine* e)
 
 constexpr size_t kExecCache = 8;  // instantiated topologies kept per part
 
-// Topology key of a captured graph: its node and edge counts and, in node
-// order, each node's type and, for kernel nodes, the kernel and its cluster
-// size.  Graphs with
-// equal keys are captured by the same launch sequence; an update that the
+// Topology key of a captured graph: its nodes' number, its edges' number and
+// kinds and, in node order, each node's type and, for kernel nodes, the kernel
+// and its cluster size.  Graphs with equal keys are captured by the same launch sequence; an update that the
 // runtime refuses all the same only costs the instantiation it would have
 // taken anyway.
 uint64_t graph_topology_key(cudaGraph_t g)
@@ -323,9 +322,16 @@ uint64_t graph_topology_key(cudaGraph_t g)
     };
     size_t n = 0, edges = 0;
     if (cudaGraphGetNodes(g, nullptr, &n) != cudaSuccess) return 0;
-    if (cudaGraphGetEdges(g, nullptr, nullptr, &edges) != cudaSuccess) return 0;
+    if (cudaGraphGetEdges_v2(g, nullptr, nullptr, nullptr, &edges) != cudaSuccess) return 0;
     mix(n);
     mix(edges);
+    if (edges)
+    {
+        std::vector<cudaGraphNode_t> from(edges), to(edges);
+        std::vector<cudaGraphEdgeData> kind(edges);
+        if (cudaGraphGetEdges_v2(g, from.data(), to.data(), kind.data(), &edges) != cudaSuccess) return 0;
+        for (const cudaGraphEdgeData& k : kind) mix(k.type);
+    }
     std::vector<cudaGraphNode_t> nodes(n);
     if (n && cudaGraphGetNodes(g, nodes.data(), &n) != cudaSuccess) return 0;
     for (cudaGraphNode_t node : nodes)
@@ -788,7 +794,7 @@ int nimbus_engine_detail::launch_microphysics(nimbus_engine* e, int lane, cudaSt
     const long long tiles = tiles_of(e, L, kItemCells, n);
     if (tiles <= 0) return 0;
     nimbus_cuda_context* ctx = e->ctx;
-    const bool fp32 = ctx->precision == NIMBUS_PRECISION_FP32;
+    const bool fp32 = ctx->precision == NIMBUS_PRECISION_FP32, early = starts_early(e, L);
     const EngineMember* table = e->d_table + L.first;
     LaunchTimer t(ctx, st, NIMBUS_KERNEL_MICROPHYSICS);
     if (n <= kMicroConstMembers)
@@ -799,9 +805,11 @@ int nimbus_engine_detail::launch_microphysics(nimbus_engine* e, int lane, cudaSt
         for (int r = 0; r < n; ++r)
             ml->m[r] = micro_const_of(e->slots[static_cast<size_t>(e->order[static_cast<size_t>(L.first + r)])].m);
         if (fp32)
-            engine_microphysics_eos_const_kernel<true><<<tile_grid(tiles), kEngineBlock, 0, st>>>(*ml, table, tiles);
+            launch_after(early, engine_microphysics_eos_const_kernel<true>, tile_grid(tiles), kEngineBlock, 1u, st, *ml,
+                         table, tiles);
         else
-            engine_microphysics_eos_const_kernel<false><<<tile_grid(tiles), kEngineBlock, 0, st>>>(*ml, table, tiles);
+            launch_after(early, engine_microphysics_eos_const_kernel<false>, tile_grid(tiles), kEngineBlock, 1u, st, *ml,
+                         table, tiles);
         return 1;
     }
     const long long* prefix = prefix_of(e, L, kItemCells);

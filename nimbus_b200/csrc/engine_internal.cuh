@@ -194,14 +194,24 @@ long long tiles_of(const nimbus_engine* e, const nimbus_engine_detail::Lane& L, 
     return e->prefix[L.prefix_first + static_cast<size_t>(kind) * (L.members + 1) + members];
 }
 
-#define ENGINE_LAUNCH_GRID(family, kernel, tiles, gy, block, ...)                                       \
+// Whether a lane's kernels start early (launch_after): a small lane alone on
+// the GPU, whose step is a chain of launches of a few microseconds (32x32x40
+// member 0.137 -> 0.128 ms a step).  Long kernels gain nothing from it (5.2
+// million cells 1.424 -> 1.428 ms), and beside other lanes the waiting CTAs
+// would hold the room that those lanes' kernels fill.
+inline bool starts_early(const nimbus_engine* e, const nimbus_engine_detail::Lane& L)
+{
+    return e->lanes.size() == 1 && tiles_of(e, L, kItemCells, L.members) * kEngineBlock < kQuadCells;
+}
+
+#define ENGINE_LAUNCH_BLOCK(family, kernel, tiles, block, ...)                                           \
     do {                                                                                                 \
         const long long tiles_ = (tiles);                                                                \
         if (tiles_ > 0)                                                                                  \
         {                                                                                                \
             LaunchTimer t_(ctx, st, family);                                                             \
-            kernel<<<dim3(engine_grid(e, reinterpret_cast<const void*>(kernel), tiles_, (block)), gy),   \
-                     (block), 0, st>>>(__VA_ARGS__);                                                     \
+            launch_after(early, kernel, engine_grid(e, reinterpret_cast<const void*>(kernel), tiles_, (block)), \
+                         (block), 1u, st, __VA_ARGS__);                                                  \
             ++count;                                                                                     \
         }                                                                                                \
     } while (0)
@@ -216,23 +226,18 @@ long long tiles_of(const nimbus_engine* e, const nimbus_engine_detail::Lane& L, 
             ++count;                                                                                     \
         }                                                                                                \
     } while (0)
-// A launch whose tiles are cut further: units of work for the grid.
-#define ENGINE_LAUNCH_UNITS(family, kernel, units, block, ...) \
-    ENGINE_LAUNCH_GRID(family, kernel, units, 1, block, __VA_ARGS__)
 #define ENGINE_LAUNCH_TILES(family, kernel, tiles, ...)                                                  \
     do {                                                                                                 \
         const long long tiles_ = (tiles);                                                                \
         if (tiles_ > 0)                                                                                  \
         {                                                                                                \
             LaunchTimer t_(ctx, st, family);                                                             \
-            kernel<<<tile_grid(tiles_), kEngineBlock, 0, st>>>(__VA_ARGS__);                             \
+            launch_after(early, kernel, tile_grid(tiles_), kEngineBlock, 1u, st, __VA_ARGS__);           \
             ++count;                                                                                     \
         }                                                                                                \
     } while (0)
-#define ENGINE_LAUNCH(family, kernel, tiles, gy, ...) \
-    ENGINE_LAUNCH_GRID(family, kernel, tiles, gy, kEngineBlock, __VA_ARGS__)
-#define ENGINE_LAUNCH_BLOCK(family, kernel, tiles, block, ...) \
-    ENGINE_LAUNCH_GRID(family, kernel, tiles, 1, block, __VA_ARGS__)
+#define ENGINE_LAUNCH(family, kernel, tiles, ...) \
+    ENGINE_LAUNCH_BLOCK(family, kernel, tiles, kEngineBlock, __VA_ARGS__)
 
 // Enqueues part `part` of one large step of the members of one lane on `st`
 // (0: Heun slow step, boundary refresh and KW78 seed; 1: the acoustic loop,
@@ -245,6 +250,7 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
     const nimbus_engine_detail::Lane& L = e->lanes[static_cast<size_t>(lane)];
     const int n = L.members;
     int count = 0;
+    const bool early = starts_early(e, L);
     EngineMember* T = e->d_table + L.first;
     const long long* pc = prefix_of(e, L, kItemCells);
     const long long* pcol = prefix_of(e, L, kItemColumns);
@@ -260,8 +266,9 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
         const int bands = static_cast<int>(tiles_of(e, L, kItemRing, members));
         if (bands <= 0) return;
         LaunchTimer t(ctx, st, NIMBUS_KERNEL_ACOUSTIC_BOUNDARY);
-        launch_ring(engine_bc_ring_kernel, bands, ring_cluster(rows), st, static_cast<const EngineMember*>(T),
-                    prefix_of(e, L, kItemRing), s, refresh);
+        launch_after(early, engine_bc_ring_kernel, static_cast<unsigned>(bands * ring_cluster(rows)), kRingBlock,
+                     static_cast<unsigned>(ring_cluster(rows)), st, static_cast<const EngineMember*>(T),
+                     prefix_of(e, L, kItemRing), s, refresh);
         ++count;
     };
 
@@ -302,19 +309,19 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
         }
         else
         {
-            ENGINE_LAUNCH(NIMBUS_KERNEL_SLOW, engine_slow_predict_const_kernel<Policy>, cells, 1, *sl, T, cells);
-            ENGINE_LAUNCH(NIMBUS_KERNEL_SLOW, engine_slow_correct_const_kernel<Policy>, cells, 1, *sl, T, cells);
+            ENGINE_LAUNCH(NIMBUS_KERNEL_SLOW, engine_slow_predict_const_kernel<Policy>, cells, *sl, T, cells);
+            ENGINE_LAUNCH(NIMBUS_KERNEL_SLOW, engine_slow_correct_const_kernel<Policy>, cells, *sl, T, cells);
         }
     }
     else
     {
-        ENGINE_LAUNCH(NIMBUS_KERNEL_SLOW, engine_slow_predict_kernel<Policy>, cells, 1, T, pc, cells);
-        ENGINE_LAUNCH(NIMBUS_KERNEL_SLOW, engine_slow_correct_kernel<Policy>, cells, 1, T, pc, cells);
+        ENGINE_LAUNCH(NIMBUS_KERNEL_SLOW, engine_slow_predict_kernel<Policy>, cells, T, pc, cells);
+        ENGINE_LAUNCH(NIMBUS_KERNEL_SLOW, engine_slow_correct_kernel<Policy>, cells, T, pc, cells);
     }
     // seed_acoustic_radiation: apply_acoustic(0) then the KW78 seed (its rows
     // lie in perimeter columns, which the ring closes before it seeds).
     ring(n, 0, 1);
-    ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_vertical_kernel, tiles_of(e, L, kItemColumns, n), 1, T,
+    ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_vertical_kernel, tiles_of(e, L, kItemColumns, n), T,
                   pcol, tiles_of(e, L, kItemColumns, n), 1);
     return count;
     }
@@ -401,7 +408,7 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
     auto continuity_const = [&](auto C, long long quad_tiles, int si) {
         constexpr int kCells = decltype(C)::value;
         auto launch = [&](auto kernel) {
-            ENGINE_LAUNCH_UNITS(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, kernel, (4 / kCells) * quad_tiles, kQuadTile, *al, T,
+            ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, kernel, (4 / kCells) * quad_tiles, kQuadTile, *al, T,
                                 quad_tiles, si);
         };
         if (si == 0 && shared) launch(engine_continuity_const_kernel<Policy, true, true, kCells>);
@@ -424,16 +431,16 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
             else continuity_const(std::integral_constant<int, 4>{}, quad_tiles, si);
             break;
         case NIMBUS_ACOUSTIC_MARCH:
-            ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, engine_continuity_march_kernel<Policy>, march_tiles, 1, T,
+            ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, engine_continuity_march_kernel<Policy>, march_tiles, T,
                           pm, march_tiles, si);
             break;
         case NIMBUS_ACOUSTIC_CMARCH:
             if (s == 0)
                 ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, (engine_continuity_cmarch_kernel<Policy, true>),
-                              march_tiles, 1, *al, T, march_tiles, si);
+                              march_tiles, *al, T, march_tiles, si);
             else
                 ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, (engine_continuity_cmarch_kernel<Policy, false>),
-                              march_tiles, 1, *al, T, march_tiles, si);
+                              march_tiles, *al, T, march_tiles, si);
             break;
         case NIMBUS_ACOUSTIC_BULK:
             if (s == 0)
@@ -444,21 +451,21 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
                                    tiles, smem_cont, *al, T, tiles, si);
             break;
         default:
-            ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, engine_continuity_kernel<Policy>, tiles, 1, T, pc, tiles,
+            ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_SUBSTEP, engine_continuity_kernel<Policy>, tiles, T, pc, tiles,
                           si);
         }
         switch (mform)
         {
         case NIMBUS_ACOUSTIC_CONST:
             if (small)
-                ENGINE_LAUNCH_UNITS(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, (engine_momentum_const_kernel<Policy, 1>),
+                ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, (engine_momentum_const_kernel<Policy, 1>),
                                     4 * quad_tiles, kQuadTile, *al, T, quad_tiles, si);
             else
-                ENGINE_LAUNCH_UNITS(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, (engine_momentum_const_kernel<Policy, 4>),
+                ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, (engine_momentum_const_kernel<Policy, 4>),
                                     quad_tiles, kQuadTile, *al, T, quad_tiles, si);
             break;
         case NIMBUS_ACOUSTIC_MARCH:
-            ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, engine_momentum_march_kernel<Policy>, march_tiles, 1, T,
+            ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, engine_momentum_march_kernel<Policy>, march_tiles, T,
                           pm, march_tiles, si);
             break;
         case NIMBUS_ACOUSTIC_BULK:
@@ -466,11 +473,11 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
                                *al, T, tiles, si);
             break;
         case NIMBUS_ACOUSTIC_CMARCH:
-            ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, engine_momentum_cmarch_kernel<Policy>, march_tiles, 1, *al,
+            ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, engine_momentum_cmarch_kernel<Policy>, march_tiles, *al,
                           T, march_tiles, si);
             break;
         default:
-            ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, engine_momentum_kernel<Policy>, tiles, 1, T, pc, tiles,
+            ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_MOMENTUM, engine_momentum_kernel<Policy>, tiles, T, pc, tiles,
                           si);
         }
         ring(a, si, 0);
@@ -518,17 +525,17 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
         }
         ENGINE_LAUNCH_TILES(NIMBUS_KERNEL_TRANSPORT_FACES, engine_transport_faces_const_kernel<kFp32>, cells, *tl, T,
                             cells);
-        ENGINE_LAUNCH(NIMBUS_KERNEL_TRANSPORT_LIMITER, engine_transport_limiter_const_kernel<kFp32>, cells, 1, *tl, T,
+        ENGINE_LAUNCH(NIMBUS_KERNEL_TRANSPORT_LIMITER, engine_transport_limiter_const_kernel<kFp32>, cells, *tl, T,
                       cells);
-        ENGINE_LAUNCH(NIMBUS_KERNEL_TRANSPORT_UPDATE, engine_transport_update_const_kernel<kFp32>, cells, 1, *tl, T,
+        ENGINE_LAUNCH(NIMBUS_KERNEL_TRANSPORT_UPDATE, engine_transport_update_const_kernel<kFp32>, cells, *tl, T,
                       cells);
     }
     else
     {
-        ENGINE_LAUNCH(NIMBUS_KERNEL_TRANSPORT_FACES, engine_transport_faces_kernel<kFp32>, cells, 1, T, pc, cells);
-        ENGINE_LAUNCH(NIMBUS_KERNEL_TRANSPORT_LIMITER, engine_transport_limiter_kernel<kFp32>, cells, 1, T, pc,
+        ENGINE_LAUNCH(NIMBUS_KERNEL_TRANSPORT_FACES, engine_transport_faces_kernel<kFp32>, cells, T, pc, cells);
+        ENGINE_LAUNCH(NIMBUS_KERNEL_TRANSPORT_LIMITER, engine_transport_limiter_kernel<kFp32>, cells, T, pc,
                       cells);
-        ENGINE_LAUNCH(NIMBUS_KERNEL_TRANSPORT_UPDATE, engine_transport_update_kernel<kFp32>, cells, 1, T, pc, cells);
+        ENGINE_LAUNCH(NIMBUS_KERNEL_TRANSPORT_UPDATE, engine_transport_update_kernel<kFp32>, cells, T, pc, cells);
     }
     // Kessler step and the EOS pressure re-projection (one pass), then the
     // pointer rotation that publishes the new qr and pressure.
@@ -540,7 +547,7 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
     if (L.closing)
     {
         ring(n, 0, 2);
-        ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_vertical_kernel, tiles_of(e, L, kItemColumns, n), 1,
+        ENGINE_LAUNCH(NIMBUS_KERNEL_ACOUSTIC_BOUNDARY, engine_bc_vertical_kernel, tiles_of(e, L, kItemColumns, n),
                       T, pcol, tiles_of(e, L, kItemColumns, n), 2);
     }
     // The acoustic speed scan of the state the next step starts from.

@@ -157,6 +157,7 @@ static __global__ void __launch_bounds__(256, 4) engine_slow_predict_kernel(cons
                                                                   const long long* __restrict__ prefix,
                                                                   long long tiles)
 {
+    grid_dependency();
     for_member_items(table, prefix, tiles, kItemCells, [&](const EngineMember& M, int c) {
         slow_predict_packed<Policy>(M.S, M.u, M.v, M.w, M.rho, M.p, M.qv, M.qc, M.qr, M.rho0, M.qv0, M.u0, M.v0,
                                     reinterpret_cast<float4*>(M.k1), reinterpret_cast<float4*>(M.xs), c);
@@ -171,6 +172,7 @@ static __global__ void __launch_bounds__(256, 4) engine_slow_correct_kernel(cons
                                                                   const long long* __restrict__ prefix,
                                                                   long long tiles)
 {
+    grid_dependency();
     for_member_items(table, prefix, tiles, kItemCells, [&](const EngineMember& M, int c) {
         slow_correct_packed<Policy>(M.S, reinterpret_cast<const float4*>(M.xs), M.rho, M.qv, M.qc, M.qr, M.rho0,
                                     M.qv0, M.u0, M.v0, reinterpret_cast<const float4*>(M.k1), M.u, M.v, M.w, M.p, c);
@@ -204,6 +206,7 @@ template <class Policy>
 static __global__ void __launch_bounds__(256, NIMBUS_SLOW_MINB) engine_slow_predict_const_kernel(
     const __grid_constant__ SlowLaunch L, const EngineMember* __restrict__ table, long long tiles)
 {
+    grid_dependency();
     int m = 0;
     for (long long t = blockIdx.x; t < tiles; t += gridDim.x)
     {
@@ -222,6 +225,7 @@ template <class Policy>
 static __global__ void __launch_bounds__(256, NIMBUS_SLOW_MINB) engine_slow_correct_const_kernel(
     const __grid_constant__ SlowLaunch L, const EngineMember* __restrict__ table, long long tiles)
 {
+    grid_dependency();
     int m = 0;
     for (long long t = blockIdx.x; t < tiles; t += gridDim.x)
     {
@@ -241,6 +245,7 @@ template <class Policy>
 static __global__ void __launch_bounds__(kQuadTile, NIMBUS_SLOW_MINB_F32) engine_slow_predict_quad_kernel(
     const __grid_constant__ SlowLaunch L, const EngineMember* __restrict__ table, long long tiles)
 {
+    grid_dependency();
     int m = 0;
     for (long long t = blockIdx.x; t < tiles; t += gridDim.x)
     {
@@ -261,6 +266,7 @@ template <class Policy>
 static __global__ void __launch_bounds__(kQuadTile, NIMBUS_SLOW_MINB_F32) engine_slow_correct_quad_kernel(
     const __grid_constant__ SlowLaunch L, const EngineMember* __restrict__ table, long long tiles)
 {
+    grid_dependency();
     int m = 0;
     for (long long t = blockIdx.x; t < tiles; t += gridDim.x)
     {
@@ -296,6 +302,7 @@ static __global__ void __launch_bounds__(kRingBlock) engine_bc_ring_kernel(const
                                                                            const long long* __restrict__ prefix, int s,
                                                                            int refresh)
 {
+    grid_dependency();
     const int t = (int)blockIdx.x / cluster_size();
     int m = 0;
     while (t >= prefix[m + 1]) ++m;
@@ -313,6 +320,7 @@ static __global__ void __launch_bounds__(256) engine_bc_vertical_kernel(const En
                                                                  const long long* __restrict__ prefix,
                                                                  long long tiles, int refresh)
 {
+    grid_dependency();
     for_member_items(table, prefix, tiles, kItemColumns, [&](const EngineMember& M, int col) {
         if (refresh == 2 && !M.close_step) return;
         bc_vertical_column(M.B, M.u, M.v, M.w, col);
@@ -326,6 +334,7 @@ static __global__ void __launch_bounds__(256, 5) engine_continuity_kernel(const 
                                                                 const long long* __restrict__ prefix,
                                                                 long long tiles, int s)
 {
+    grid_dependency();
     const bool first = s == 0;
     for_member_items(table, prefix, tiles, kItemCells, [&](const EngineMember& M, int c) {
         unsigned flags = 0;
@@ -341,6 +350,7 @@ static __global__ void __launch_bounds__(256) engine_momentum_kernel(const Engin
                                                               const long long* __restrict__ prefix, long long tiles,
                                                               int s)
 {
+    grid_dependency();
     for_member_items(table, prefix, tiles, kItemCells, [&](const EngineMember& M, int c) {
         const int vertical = kFuseVertical | (M.B.bottom == kBottomNoSlip ? kFuseNoSlipBottom : 0) |
                              (M.B.top == kTopOpen ? kFuseOpenTop : 0);
@@ -359,6 +369,7 @@ static __global__ void __launch_bounds__(256, NIMBUS_MARCH_MINB) engine_continui
                                                                       const long long* __restrict__ prefix,
                                                                       long long tiles, int s)
 {
+    grid_dependency();
     const bool first = s == 0;
     for_member_rows(table, prefix, tiles, [&](const EngineMember& M, int i0, int i1, int j, int k, int q) {
         unsigned flags = 0;
@@ -374,6 +385,7 @@ static __global__ void __launch_bounds__(256) engine_momentum_march_kernel(const
                                                                     const long long* __restrict__ prefix,
                                                                     long long tiles, int s)
 {
+    grid_dependency();
     for_member_rows(table, prefix, tiles, [&](const EngineMember& M, int i0, int i1, int j, int k, int q) {
         const int vertical = kFuseVertical | (M.B.bottom == kBottomNoSlip ? kFuseNoSlipBottom : 0) |
                              (M.B.top == kTopOpen ? kFuseOpenTop : 0);
@@ -507,6 +519,7 @@ static __global__ void __launch_bounds__(kQuadTile, NIMBUS_CONST_MINB) engine_co
                                                                       const EngineMember* __restrict__ table,
                                                                       long long tiles, int s)
 {
+    grid_dependency();
     const bool even = (s & 1) == 0;
     for_const_cells<kCells>(L, table, (int)tiles, [&](const AcousticConst& A, const EngineMember& M, int c) {
         unsigned flags = 0;
@@ -529,6 +542,7 @@ static __global__ void __launch_bounds__(kQuadTile, NIMBUS_CONST_MINB_MOM) engin
                                                                     const EngineMember* __restrict__ table,
                                                                     long long tiles, int s)
 {
+    grid_dependency();
     const bool even = (s & 1) == 0;
     for_const_cells<kCells>(L, table, (int)tiles, [&](const AcousticConst& A, const EngineMember& M, int c) {
         const float* rho = even ? M.rho_alt : M.rho;
@@ -569,6 +583,7 @@ template <class Policy, bool kFirst>
 static __global__ void __launch_bounds__(256, NIMBUS_CMARCH_MINB) engine_continuity_cmarch_kernel(
     const __grid_constant__ AcousticLaunch L, const EngineMember* __restrict__ table, long long tiles, int s)
 {
+    grid_dependency();
     const bool even = (s & 1) == 0;
     for_const_rows(L, table, tiles, [&](const AcousticConst& A, const EngineMember& M, int i0, int i1, int j, int k,
                                         int q) {
@@ -584,6 +599,7 @@ template <class Policy>
 static __global__ void __launch_bounds__(256, NIMBUS_CMARCH_MINB) engine_momentum_cmarch_kernel(
     const __grid_constant__ AcousticLaunch L, const EngineMember* __restrict__ table, long long tiles, int s)
 {
+    grid_dependency();
     const bool even = (s & 1) == 0;
     for_const_rows(L, table, tiles, [&](const AcousticConst& A, const EngineMember& M, int i0, int i1, int j, int k,
                                         int q) {
@@ -687,6 +703,7 @@ static __global__ void __launch_bounds__(256, NIMBUS_BULK_MINB) engine_continuit
                                                                      const EngineMember* __restrict__ table,
                                                                      long long tiles, int s)
 {
+    grid_dependency();
     extern __shared__ __align__(16) unsigned char bulk_smem[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(bulk_smem);
     float* stages = reinterpret_cast<float*>(bulk_smem + kBulkBarrierBytes);
@@ -821,6 +838,7 @@ static __global__ void __launch_bounds__(256, NIMBUS_BULK_MINB) engine_momentum_
                                                                    const EngineMember* __restrict__ table,
                                                                    long long tiles, int s)
 {
+    grid_dependency();
     extern __shared__ __align__(16) unsigned char bulk_smem[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(bulk_smem);
     float* stages = reinterpret_cast<float*>(bulk_smem + kBulkBarrierBytes);
@@ -1022,6 +1040,7 @@ static __global__ void __launch_bounds__(256, NIMBUS_FACES_MINB) engine_transpor
                                                                             const long long* __restrict__ prefix,
                                                                             long long tiles)
 {
+    grid_dependency();
     for_member_items(table, prefix, tiles, kItemCells, [&](const EngineMember& M, int c) {
         transport_faces_cell4<kFp32>(M.T, reinterpret_cast<const float4*>(M.q4), M.mfx, M.mfy, M.mfz,
                                      reinterpret_cast<float4*>(M.sf), c);
@@ -1033,6 +1052,7 @@ static __global__ void __launch_bounds__(256) engine_transport_limiter_kernel(co
                                                                               const long long* __restrict__ prefix,
                                                                               long long tiles)
 {
+    grid_dependency();
     for_member_items(table, prefix, tiles, kItemCells, [&](const EngineMember& M, int c) {
         transport_limiter_cell4<kFp32>(M.T, reinterpret_cast<const float4*>(M.q4), M.rho_begin,
                                        reinterpret_cast<const float4*>(M.sf), reinterpret_cast<float4*>(M.rl), c);
@@ -1044,6 +1064,7 @@ static __global__ void __launch_bounds__(256) engine_transport_update_kernel(con
                                                                              const long long* __restrict__ prefix,
                                                                              long long tiles)
 {
+    grid_dependency();
     for_member_items(table, prefix, tiles, kItemCells, [&](const EngineMember& M, int c) {
         unsigned flags = 0;
         transport_update_cell4<kFp32>(M.T, reinterpret_cast<const float4*>(M.q4), [&](int s) { return engine_scalar(M, s); },
@@ -1097,6 +1118,7 @@ template <bool kFp32>
 static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_FACES_MINB_F32 : NIMBUS_FACES_MINB) engine_transport_faces_const_kernel(
     const __grid_constant__ TransportLaunch L, const EngineMember* __restrict__ table, long long tiles)
 {
+    grid_dependency();
     for_transport_cells(L, table, tiles, [&](const TransportConst& A, const EngineMember&, int c) {
         transport_faces_cell4<kFp32>(A.T, A.q4, A.mfx, A.mfy, A.mfz, A.sf, c);
     });
@@ -1109,6 +1131,7 @@ template <bool kFp32>
 static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_LIMITER_MINB_F32 : 3) engine_transport_limiter_const_kernel(
     const __grid_constant__ TransportLaunch L, const EngineMember* __restrict__ table, long long tiles)
 {
+    grid_dependency();
     for_transport_cells(L, table, tiles, [&](const TransportConst& A, const EngineMember&, int c) {
         transport_limiter_cell4<kFp32>(A.T, A.q4, A.rho_begin, A.sf, A.rl, c);
     });
@@ -1124,6 +1147,7 @@ template <bool kFp32>
 static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_UPDATE_MINB_F32 : 3) engine_transport_update_const_kernel(
     const __grid_constant__ TransportLaunch L, const EngineMember* __restrict__ table, long long tiles)
 {
+    grid_dependency();
     for_transport_cells(L, table, tiles, [&](const TransportConst& A, const EngineMember& M, int c) {
         unsigned flags = 0;
         float* const in_place[4] = {A.theta, A.qv, A.qc, M.qr};
@@ -1145,6 +1169,7 @@ static __global__ void __launch_bounds__(kQuadTile) engine_sound_speed_kernel(co
                                                                               const long long* __restrict__ prefix,
                                                                               long long tiles, unsigned long long* c2)
 {
+    grid_dependency();
     int m = 0, held = -1;
     unsigned long long best = 0;
     for (long long t = blockIdx.x; t < tiles; t += gridDim.x)
@@ -1279,6 +1304,7 @@ static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_MICRO_MINB_F32 : 4)
                                                                              const long long* __restrict__ prefix,
                                                                              long long tiles)
 {
+    grid_dependency();
     for_member_items(table, prefix, tiles, kItemCells, [&](const EngineMember& M, int c) {
         microphysics_eos_cell<kFp32>(micro_const_of(M), MicroRotating{M.rho, M.p, M.qr, M.qr_alt, M.eos}, c);
     });
@@ -1302,6 +1328,7 @@ template <bool kFp32>
 static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_MICRO_MINB_F32 : 4) engine_microphysics_eos_const_kernel(
     const __grid_constant__ MicroLaunch L, const EngineMember* __restrict__ table, long long tiles)
 {
+    grid_dependency();
     int m = 0;
     for (long long t = blockIdx.x; t < tiles; t += gridDim.x)
     {

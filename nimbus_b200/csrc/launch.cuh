@@ -96,21 +96,22 @@ nimbus_status launch_split_impl(nimbus_cuda_context* ctx, cudaStream_t st, Fused
                                 float* mfy, float* mfz, int vertical)
 {
     const long long n = F.d.cells();
-    if (n >= kQuadCells && F.d.nz % 4 == 0 && drho == nullptr && aligned16(in.rho) && aligned16(in.u) && aligned16(in.v) &&
-        aligned16(in.w) && aligned16(out.rho) && aligned16(out.u) && aligned16(out.v) && aligned16(out.w) &&
+    const bool early = not_captured(st);
+    if (n >= kQuadCells && F.d.nz % 4 == 0 && drho == nullptr && aligned16(in.rho) && aligned16(in.u) &&
+        aligned16(in.v) && aligned16(in.w) && aligned16(out.rho) && aligned16(out.u) && aligned16(out.v) && aligned16(out.w) &&
         aligned16(p) && aligned16(theta) && aligned16(mfx) && aligned16(mfy) && aligned16(mfz))
     {
         const long long quads = n / 4;
         long long qblocks = (quads + kQuadBlock - 1) / kQuadBlock;
         {
             LaunchTimer t(ctx, st, NIMBUS_KERNEL_ACOUSTIC_SUBSTEP);
-            split_continuity_quad_kernel<Policy><<<static_cast<int>(qblocks), kQuadBlock, 0, st>>>(
-                F, in.rho, in.u, in.v, in.w, theta, rho0, eos0, out.rho, p, mfx, mfy, mfz, ctx->status);
+            launch_after(early, split_continuity_quad_kernel<Policy>, static_cast<unsigned>(qblocks), kQuadBlock, 1u,
+                         st, F, in.rho, in.u, in.v, in.w, theta, rho0, eos0, out.rho, p, mfx, mfy, mfz, ctx->status);
         }
         {
             LaunchTimer t(ctx, st, NIMBUS_KERNEL_ACOUSTIC_MOMENTUM);
-            split_momentum_quad_kernel<Policy><<<static_cast<int>(qblocks), kQuadBlock, 0, st>>>(
-                F, out.rho, p, p0, dp0, in.u, in.v, in.w, out.u, out.v, out.w, vertical);
+            launch_after(early, split_momentum_quad_kernel<Policy>, static_cast<unsigned>(qblocks), kQuadBlock, 1u, st,
+                         F, out.rho, p, p0, dp0, in.u, in.v, in.w, out.u, out.v, out.w, vertical);
         }
         ctx->launches += 2;
         return NIMBUS_OK;
@@ -120,13 +121,13 @@ nimbus_status launch_split_impl(nimbus_cuda_context* ctx, cudaStream_t st, Fused
     if (blocks > cap) blocks = cap;
     {
         LaunchTimer t(ctx, st, NIMBUS_KERNEL_ACOUSTIC_SUBSTEP);
-        split_continuity_eos_kernel<Policy><<<static_cast<int>(blocks), kThreads, 0, st>>>(
-            F, in.rho, in.u, in.v, in.w, theta, rho0, eos0, out.rho, p, drho, mfx, mfy, mfz, ctx->status);
+        launch_after(early, split_continuity_eos_kernel<Policy>, static_cast<unsigned>(blocks), kThreads, 1u, st, F,
+                     in.rho, in.u, in.v, in.w, theta, rho0, eos0, out.rho, p, drho, mfx, mfy, mfz, ctx->status);
     }
     {
         LaunchTimer t(ctx, st, NIMBUS_KERNEL_ACOUSTIC_MOMENTUM);
-        split_momentum_kernel<Policy><<<static_cast<int>(blocks), kThreads, 0, st>>>(F, out.rho, p, p0, dp0, in.u,
-                                                                                      in.v, in.w, out.u, out.v, out.w, vertical);
+        launch_after(early, split_momentum_kernel<Policy>, static_cast<unsigned>(blocks), kThreads, 1u, st, F, out.rho,
+                     p, p0, dp0, in.u, in.v, in.w, out.u, out.v, out.w, vertical);
     }
     ctx->launches += 2;
     return NIMBUS_OK;

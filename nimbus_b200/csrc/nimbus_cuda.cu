@@ -197,13 +197,15 @@ void launch_boundaries(nimbus_cuda_context* ctx, cudaStream_t st, const Boundary
     LaunchTimer t(ctx, st, NIMBUS_KERNEL_ACOUSTIC_BOUNDARY);
     const int bands = ring_bands(d.nz), rows = std::max(d.nx, d.ny);
     const int closed = inner_closed ? 1 : 0;
+    const bool early = not_captured(st);
     if (d.nz % 4 == 0 && aligned16(D.u) && aligned16(D.v) && aligned16(D.w) && aligned16(rho) && aligned16(D.p) &&
         aligned16(wave))
-        launch_ring(acoustic_bc_ring_kernel<4>, bands, ring_cluster(rows), st, B, D.u, D.v, D.w, rho, D.p, wave,
-                    closed);
+        launch_after(early, acoustic_bc_ring_kernel<4>, static_cast<unsigned>(bands * ring_cluster(rows)), kRingBlock,
+                     static_cast<unsigned>(ring_cluster(rows)), st, B, D.u, D.v, D.w, rho, D.p, wave, closed);
     else
-        launch_ring(acoustic_bc_ring_kernel<1>, bands, ring_cluster(kRingLevels * rows), st, B, D.u, D.v, D.w, rho,
-                    D.p, wave, closed);
+        launch_after(early, acoustic_bc_ring_kernel<1>, static_cast<unsigned>(bands * ring_cluster(kRingLevels * rows)),
+                     kRingBlock, static_cast<unsigned>(ring_cluster(kRingLevels * rows)), st, B, D.u, D.v, D.w, rho,
+                     D.p, wave, closed);
     ctx->launches += 1;
     if (inner_closed) return;
     acoustic_bc_vertical_kernel<<<grid_for(ctx, d.nx * d.ny), kThreads, 0, st>>>(B, D.u, D.v, D.w);

@@ -116,6 +116,16 @@ __device__ __forceinline__ void decompose(const Dims& d, int c, int& i, int& j, 
     i = t / d.ny;
 }
 
+// The first statement of a kernel that launch_after may start before the
+// kernels it follows in its stream have ended: waits until they have and their
+// writes are visible, then lets the next such kernel start its CTAs, which
+// wait here in turn.  A kernel launched the ordinary way passes through.
+__device__ __forceinline__ void grid_dependency()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // x / d rounded as the division rounds it, for a literal d well inside the
 // normal range and a finite x whose quotient is far from its ends: with
 // y = RN(1 / d), a constant, RN(x y) is within an ulp of the quotient, its
@@ -209,6 +219,45 @@ static __global__ void __launch_bounds__(256) max_sound_speed_kernel(const float
 
 namespace nimbus_host
 {
+// False while the caller captures the stream (whose last node may be a copy).
+inline bool not_captured(cudaStream_t st)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusActive;
+    return cudaStreamIsCapturing(st, &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
+}
+
+// Launches a kernel that begins with grid_dependency(), in clusters of
+// `cluster` CTAs.  early: its CTAs may be resident before the kernel before it
+// in the stream ends, which takes the launch latency and the ramp off a chain
+// of short dependent kernels.
+template <class Kernel, class... Args>
+inline cudaError_t launch_after(bool early, Kernel kernel, unsigned grid, unsigned block, unsigned cluster,
+                                cudaStream_t st, Args&&... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2]{};
+    unsigned n = 0;
+    if (cluster > 1)
+    {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    if (early)
+    {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...);
+}
+
 // SplitExplicitScheme::resolve_substep_count
 // (src/numerics/time_stepping/schemes/split_explicit/split_explicit.cpp:67-170)
 // with a positive minimum spacing: N = max(requested, max(ceil(dt c_max /

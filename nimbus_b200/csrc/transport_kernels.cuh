@@ -448,14 +448,15 @@ __device__ __forceinline__ float limiter_factor(const TP& T, float fxp, float fx
     const real idy = kFp32 ? (real)T.inv_dy_f : (real)T.inv_dy;
     const real idz = kFp32 ? (real)T.inv_dz_f : (real)T.inv_dz;
     real out = 0;
-    if (xp && fxp > 0.0f) out += (real)fxp * idx;
-    if (xm && fxm < 0.0f) out -= (real)fxm * idx;
-    if (yp && fyp > 0.0f) out += (real)fyp * idy;
-    if (ym && fym < 0.0f) out -= (real)fym * idy;
-    if (zp && fzp > 0.0f) out += (real)fzp * idz;
-    if (zm && fzm < 0.0f) out -= (real)fzm * idz;
     if constexpr (kFp32)
     {
+        // Axis by axis without branches (a NaN flux counts as none), every
+        // operation fixed so that the engine's and the per-operation kernels
+        // round alike.
+        const float ox = (xp ? fmaxf(fxp, 0.0f) : 0.0f) - (xm ? fminf(fxm, 0.0f) : 0.0f);
+        const float oy = (yp ? fmaxf(fyp, 0.0f) : 0.0f) - (ym ? fminf(fym, 0.0f) : 0.0f);
+        const float oz = (zp ? fmaxf(fzp, 0.0f) : 0.0f) - (zm ? fminf(fzm, 0.0f) : 0.0f);
+        out = __fmaf_rn(oz, idz, __fmaf_rn(oy, idy, __fmul_rn(ox, idx)));
         float r = 1.0f;
         if (out > 0.0f)
         {
@@ -465,7 +466,13 @@ __device__ __forceinline__ float limiter_factor(const TP& T, float fxp, float fx
         }
         return (r > 0.0f && r < 1.0f) ? nextafterf(__fmul_rn(r, 1.0f - 32.0f * 1.1920928955078125e-7f), 0.0f) : r;
     }
-    else
+    if (xp && fxp > 0.0f) out += (real)fxp * idx;
+    if (xm && fxm < 0.0f) out -= (real)fxm * idx;
+    if (yp && fyp > 0.0f) out += (real)fyp * idy;
+    if (ym && fym < 0.0f) out -= (real)fym * idy;
+    if (zp && fzp > 0.0f) out += (real)fzp * idz;
+    if (zm && fzm < 0.0f) out -= (real)fzm * idz;
+    if constexpr (!kFp32)
     {
         double r = 1.0;
         if (out > 0.0)
@@ -563,6 +570,35 @@ __device__ __forceinline__ float update_value(const TP& T, bool pd, float fxp, f
     const real idy = kFp32 ? (real)T.inv_dy_f : (real)T.inv_dy;
     const real idz = kFp32 ? (real)T.inv_dz_f : (real)T.inv_dz;
     const real dt = kFp32 ? (real)T.dt_f : (real)T.dt;
+    if constexpr (kFp32)
+    {
+        if (pd)
+        {
+            // What leaves through the faces carries this cell's factor, what
+            // comes in the neighbour's: the flux's positive part and the
+            // exact rest (a non-finite flux leaves a non-finite rest).  No
+            // branch and no selection: 24 members of 16.5 million cells, ten
+            // steps 3.63 -> 3.48 ms.
+            const float zt = has_top ? fzp : 0.0f, zb = has_bottom ? fzm : 0.0f;
+            const float xa = fmaxf(fxp, 0.0f), xb = fmaxf(fxm, 0.0f);
+            const float ya = fmaxf(fyp, 0.0f), yb = fmaxf(fym, 0.0f);
+            const float za = fmaxf(zt, 0.0f), zc = fmaxf(zb, 0.0f);
+            const float xin = fxp - xa, xout = fxm - xb, yin = fyp - ya, yout = fym - yb, zin = zt - za,
+                        zout = zb - zc;
+            auto through = [&](float x, float y, float z) {
+                return __fmaf_rn(z, idz, __fmaf_rn(y, idy, __fmul_rn(x, idx)));
+            };
+            auto into = [](float lo, float r_lo, float hi, float r_hi) {
+                return __fmaf_rn(lo, r_lo, -__fmul_rn(hi, r_hi));
+            };
+            const float outgoing = __fmul_rn(rc, through(xa - xout, ya - yout, za - zout));
+            const float incoming = through(into(xb, rxm, xin, rxp), into(yb, rym, yin, ryp), into(zc, rzm, zin, rzp));
+            const float rho_phi = __fmaf_rn(dt, incoming, __fmaf_rn(-dt, outgoing, __fmul_rn(rb, qraw)));
+            const float out = __fdividef(rho_phi, denom);
+            if (!isfinite(out)) flags |= kStatusNonfiniteTransport;
+            return out;
+        }
+    }
     const real sxp = limited_face<kFp32>(fxp, pd, rc, rxp);
     const real sxm = limited_face<kFp32>(fxm, pd, rxm, rc);
     const real syp = limited_face<kFp32>(fyp, pd, rc, ryp);

@@ -62,6 +62,45 @@ __host__ __device__ inline void finish_fp32(SlowParams& S)
     }
 }
 
+// The FP32 form.  fd5 as its centred part plus, by the sign of the wind, its
+// dissipative part: the differences and sums of the mirrored points once each
+// and no selection (17 operations of the paired form for two cells, where the
+// selected one-sided stencil took 14 a cell).
+template <class V>
+__device__ __forceinline__ V fd5_lanes(V m3, V m2, V m1, V c, V p1, V p2, V p3, V a, float inv_d60)
+{
+    using L = Lanes<V>;
+    const V minus = L::splat(-1.0f);
+    const V d1 = L::fma(m1, minus, p1), d2 = L::fma(m2, minus, p2), d3 = L::fma(m3, minus, p3);
+    const V s1 = L::add(p1, m1), s2 = L::add(p2, m2), s3 = L::add(p3, m3);
+    const V centred = L::fma(d1, L::splat(45.0f), L::fma(d2, L::splat(-9.0f), d3));
+    const V biased = L::fma(c, L::splat(20.0f),
+                            L::fma(s1, L::splat(-15.0f), L::fma(s3, minus, L::mul(s2, L::splat(6.0f)))));
+    return L::mul(L::add(centred, L::signed_by(biased, a)), L::splat(inv_d60));
+}
+
+// fd3 (half 2) and fd1 (half 1) on the points mirrored by the wind's sign: x
+// upwind, y downwind of the centre.
+__device__ __forceinline__ float fd3_f32(float cc, float x1, float x2, float y1, float inv_d6)
+{
+    return __fmul_rn(__fmaf_rn(2.0f, y1, __fmaf_rn(3.0f, cc, __fmaf_rn(-6.0f, x1, x2))), inv_d6);
+}
+__device__ __forceinline__ float fd1_f32(float cc, float x1, float inv_d)
+{
+    return __fmul_rn(__fadd_rn(cc, -x1), inv_d);
+}
+
+__device__ __forceinline__ float upwind_f32(int half, float cc, float m1, float p1, float m2, float p2, float m3,
+                                            float p3, float a, float inv_d, float inv_d6, float inv_d60)
+{
+    if (half <= 0) return 0.0f;
+    if (half >= 3) return fd5_lanes<float>(m3, m2, m1, cc, p1, p2, p3, a, inv_d60);
+    const bool pos = a >= 0.0f;
+    const float x1 = pos ? m1 : p1;
+    const float v = half == 1 ? fd1_f32(cc, x1, inv_d) : fd3_f32(cc, x1, pos ? m2 : p2, pos ? p1 : m1, inv_d6);
+    return pos ? v : -v;
+}
+
 // upwind_dx/dy/dz (derivative_operators.hpp:324-395): fd5 upwind-biased in
 // the interior, fd3 two points from a boundary, fd1 next to it, 0 on it.
 // Away from the boundary the side is selected, not branched on: the a < 0
@@ -72,6 +111,7 @@ template <class real>
 __device__ __forceinline__ real upwind_from(int half, real cc, real m1, real p1, real m2, real p2, real m3, real p3,
                                             real a, real inv_d, real inv_d6, real inv_d60)
 {
+    if constexpr (sizeof(real) == 4) return upwind_f32(half, cc, m1, p1, m2, p2, m3, p3, a, inv_d, inv_d6, inv_d60);
     if (half <= 0) return (real)0;
     const bool pos = a >= (real)0;
     if (half == 1)
@@ -507,10 +547,15 @@ __device__ __forceinline__ Quad upwind_quad(const QuadStencil& t, int half, cons
     Quad o;
     if (half >= 3)
     {
+        auto two = [](const Quad& f, int q) { return make_float2(f.v[q], f.v[q + 1]); };
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            o.v[q] = upwind_from<float>(3, t.c.v[q], t.m1.v[q], t.p1.v[q], t.m2.v[q], t.p2.v[q], t.m3.v[q], t.p3.v[q],
-                                        a.v[q], inv_d, d6, d60);
+        for (int q = 0; q < 4; q += 2)
+        {
+            const float2 r = fd5_lanes<float2>(two(t.m3, q), two(t.m2, q), two(t.m1, q), two(t.c, q), two(t.p1, q),
+                                               two(t.p2, q), two(t.p3, q), two(a, q), d60);
+            o.v[q] = r.x;
+            o.v[q + 1] = r.y;
+        }
     }
     else
     {
@@ -537,16 +582,20 @@ __device__ __forceinline__ Quad upwind_quad_z(const Quad& lo, const Quad& cc, co
                                     d6, d60);
     if (k < 3 || k + 3 > nz - 4)
     {
+        // Every warp holds a column's end, so the three cases are formed
+        // together rather than branched on.
 #pragma unroll
         for (int q = 0; q < 4; ++q)
         {
             const int kq = k + q, half = min(kq, nz - 1 - kq);
-            if (kq == 0)
-                o.v[q] = (a.v[q] >= 0.0f) ? (vertical_w ? (t[q + 3] - 0.0f) * inv_d : 0.0f)
-                                          : (t[q + 4] - t[q + 3]) * inv_d;
-            else if (half < 3)
-                o.v[q] = upwind_from<float>(half, t[q + 3], t[q + 2], t[q + 4], t[q + 1], t[q + 5], 0.0f, 0.0f, a.v[q],
-                                            inv_d, d6, d60);
+            const bool pos = a.v[q] >= 0.0f;
+            const float cc_q = t[q + 3];
+            float x1 = pos ? t[q + 2] : t[q + 4];
+            const float x2 = pos ? t[q + 1] : t[q + 5], y1 = pos ? t[q + 4] : t[q + 2];
+            const float three = fd3_f32(cc_q, x1, x2, y1, d6);
+            if (kq == 0 && pos) x1 = vertical_w ? 0.0f : cc_q;  // the ground: w 0 below it, no gradient of u and v
+            const float v = half == 2 ? three : fd1_f32(cc_q, x1, inv_d);
+            if (half < 3) o.v[q] = pos ? v : -v;
         }
     }
     return o;

@@ -151,6 +151,56 @@ __device__ __forceinline__ float rcp_normal(float a)
     return r;
 }
 
+// Lane arithmetic of the FP32 stencils: one stencil (float) or two independent
+// ones at once (float2, Blackwell's paired f32x2 FMA / MUL / ADD: two IEEE
+// round-to-nearest operations per instruction).  Every operation
+// is an explicit round-to-nearest intrinsic, so the scalar and paired forms
+// run the same operation sequence and give the same bits; only the
+// reciprocals, the final quotient and the finiteness test act per lane.
+template <class V>
+struct Lanes;
+
+template <>
+struct Lanes<float>
+{
+    static __device__ __forceinline__ float splat(float x) { return x; }
+    static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
+    static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+    static __device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+    static __device__ __forceinline__ float maxf(float a, float b) { return fmaxf(a, b); }
+    static __device__ __forceinline__ float absf(float a) { return fabsf(a); }
+    static __device__ __forceinline__ float rcp(float a) { return rcp_normal(a); }
+    static __device__ __forceinline__ float finite_or_zero(float a) { return isfinite(a) ? a : 0.0f; }
+    // x, negated where a is negative.
+    static __device__ __forceinline__ float signed_by(float x, float a)
+    {
+        return __uint_as_float(__float_as_uint(x) ^ (__float_as_uint(a) & 0x80000000u));
+    }
+};
+
+template <>
+struct Lanes<float2>
+{
+    static __device__ __forceinline__ float2 splat(float x) { return make_float2(x, x); }
+    static __device__ __forceinline__ float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+    static __device__ __forceinline__ float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+    static __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+    static __device__ __forceinline__ float2 maxf(float2 a, float2 b)
+    {
+        return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y));
+    }
+    static __device__ __forceinline__ float2 absf(float2 a) { return make_float2(fabsf(a.x), fabsf(a.y)); }
+    static __device__ __forceinline__ float2 rcp(float2 a) { return make_float2(rcp_normal(a.x), rcp_normal(a.y)); }
+    static __device__ __forceinline__ float2 finite_or_zero(float2 a)
+    {
+        return make_float2(isfinite(a.x) ? a.x : 0.0f, isfinite(a.y) ? a.y : 0.0f);
+    }
+    static __device__ __forceinline__ float2 signed_by(float2 x, float2 a)
+    {
+        return make_float2(Lanes<float>::signed_by(x.x, a.x), Lanes<float>::signed_by(x.y, a.y));
+    }
+};
+
 // std::clamp after a non-finite fallback (acoustic_cgrid_fast.cpp:38-43).
 __device__ __forceinline__ float clamp_value(float v, float fallback, float lo, float hi)
 {

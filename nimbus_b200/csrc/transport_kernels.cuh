@@ -100,47 +100,6 @@ __device__ __forceinline__ double mc_slope(double qm, double q0, double qp)
     return 0.0;
 }
 
-// Lane arithmetic for the FP32 face offset: one scalar stencil (float) or two
-// independent stencils at once (float2, Blackwell's paired f32x2 FMA / MUL /
-// ADD: two IEEE round-to-nearest operations per instruction).  Every operation
-// is an explicit round-to-nearest intrinsic, so the scalar and paired forms
-// run the same operation sequence and give the same bits; only the
-// reciprocals, the final quotient and the finiteness test act per lane.
-template <class V>
-struct Lanes;
-
-template <>
-struct Lanes<float>
-{
-    static __device__ __forceinline__ float splat(float x) { return x; }
-    static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
-    static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
-    static __device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-    static __device__ __forceinline__ float maxf(float a, float b) { return fmaxf(a, b); }
-    static __device__ __forceinline__ float absf(float a) { return fabsf(a); }
-    static __device__ __forceinline__ float rcp(float a) { return rcp_normal(a); }
-    static __device__ __forceinline__ float finite_or_zero(float a) { return isfinite(a) ? a : 0.0f; }
-};
-
-template <>
-struct Lanes<float2>
-{
-    static __device__ __forceinline__ float2 splat(float x) { return make_float2(x, x); }
-    static __device__ __forceinline__ float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
-    static __device__ __forceinline__ float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-    static __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-    static __device__ __forceinline__ float2 maxf(float2 a, float2 b)
-    {
-        return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y));
-    }
-    static __device__ __forceinline__ float2 absf(float2 a) { return make_float2(fabsf(a.x), fabsf(a.y)); }
-    static __device__ __forceinline__ float2 rcp(float2 a) { return make_float2(rcp_normal(a.x), rcp_normal(a.y)); }
-    static __device__ __forceinline__ float2 finite_or_zero(float2 a)
-    {
-        return make_float2(isfinite(a.x) ? a.x : 0.0f, isfinite(a.y) ? a.y : 0.0f);
-    }
-};
-
 // FP32 face offset from the donor value c (face = c + offset): WENO5-JS on
 // the stencil normalised by its largest magnitude, as the reference's FP32
 // GPU form normalises it (weno5_face_offset_fp32,

@@ -24,6 +24,7 @@
 //               sums and the density update are single-rounding FMAs.
 #pragma once
 
+#include "power_table.cuh"
 #include "stencil_common.cuh"
 
 namespace nimbus
@@ -189,7 +190,7 @@ __device__ __forceinline__ float substep_pressure(const FusedParams& P, const fl
         if (thv > 0.0)
         {
             const double x = divided_by((double)rho_stored * kRd * thv, kP00);
-            p_new = kP00 * pow(x, P.gamma);
+            p_new = kP00 * eos_power(x, P.gamma);
         }
         if (!isfinite(p_new) || p_new <= 0.0) p_new = (double)P.p_ref_fallback;
         return clamp_value((float)p_new, 101325.0f, P.p_min, P.p_max);

@@ -15,6 +15,7 @@
 //                    W,E -> S,N -> vertical, one launch (bc_ring_levels).
 #pragma once
 
+#include "power_table.cuh"
 #include "stencil_common.cuh"
 
 namespace nimbus
@@ -106,7 +107,7 @@ static __global__ void __launch_bounds__(256) acoustic_continuity_eos_kernel(
 
         double p_new = (double)P.p_ref_fallback;
         const double th = (double)theta[c];
-        if (th > 0.0) p_new = kP00 * pow((double)rho_stored * kRd * th / kP00, P.gamma);
+        if (th > 0.0) p_new = kP00 * eos_power((double)rho_stored * kRd * th / kP00, P.gamma);
         if (!isfinite(p_new) || p_new <= 0.0) p_new = (double)P.p_ref_fallback;
         p_out[c] = clamp_value((float)p_new, 101325.0f, P.p_min, P.p_max);
     }

@@ -11,6 +11,7 @@
 // original qr of this cell).
 #pragma once
 
+#include "power_table.cuh"
 #include "stencil_common.cuh"
 
 namespace nimbus
@@ -51,7 +52,7 @@ __device__ __forceinline__ double k_theta_to_temperature(double theta, double p)
 {
     if (!isfinite(theta) || !isfinite(p)) return kKT0;
     const double th = kclamp(theta, 150.0, 700.0), ps = kclamp(p, 100.0, 200000.0);
-    const double T = th * pow(divided_by(ps, kKP0), kKRd / kKCp);
+    const double T = th * exner_power(divided_by(ps, kKP0));
     return isfinite(T) ? T : kKT0;
 }
 
@@ -258,7 +259,7 @@ __device__ __forceinline__ void kessler_cell(const KesslerParams& K, float* __re
                     else
                     {
                         const double ps = kclamp(pv, 100.0, 200000.0);
-                        r = dT * pow(kKP0 / ps, kKRd / kKCp);
+                        r = dT * exner_power(kKP0 / ps);
                         if (!isfinite(r)) r = 0.0;
                     }
                 }
@@ -624,7 +625,7 @@ __device__ __forceinline__ bool eos_candidate_value(const Dims& d, int c, float 
                                                     float po, float q, float qc, float qr, float& p_new,
                                                     unsigned& flags)
 {
-    const double diagnosed = kP00 * pow(divided_by((double)r * kRd * (double)th, kP00), gamma);
+    const double diagnosed = kP00 * eos_power(divided_by((double)r * kRd * (double)th, kP00), gamma);
     if (!isfinite(r) || !(r > 0.0f) || !isfinite(th) || !(th > 0.0f) || !isfinite(diagnosed) || diagnosed <= 0.0 ||
         !isfinite((float)diagnosed))
     {

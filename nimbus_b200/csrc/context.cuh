@@ -4,12 +4,14 @@
 #pragma once
 
 #include "../../include/nimbus_cuda.h"
+#include "host_copy.cuh"
 #include "transport_kernels.cuh"
 
 #include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <limits>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -66,6 +68,8 @@ struct nimbus_cuda_context
     std::atomic<uint64_t> launches{0};  // engines of this context may step from their own host threads
     std::string error;
     nimbus_host::DeviceBuffer ws[nimbus_host::kSlotCount];
+    std::shared_ptr<nimbus_host::HostCopier> copier;  // of large pageable copies
+    size_t pageable = 0;                              // bytes of them so far
 };
 
 namespace nimbus_host
@@ -179,15 +183,47 @@ inline bool cells_fit(int nx, int ny, int nz)
     return static_cast<long long>(nx) * ny * nz < static_cast<long long>(std::numeric_limits<int>::max()) / 4;
 }
 
+// Copies by the device's copier where it helps: false, with nothing done,
+// where the ordinary copy is as good (small, pinned, the context's first ones),
+// the stream is being captured, no thread is to be had or another context is
+// copying.
+inline bool copied(nimbus_cuda_context* ctx, bool up, void* device, void* host, size_t bytes, cudaError_t* result)
+{
+    if (bytes < HostCopier::kSmallest || !not_captured(ctx->stream)) return false;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, host) != cudaSuccess)
+    {
+        (void)cudaGetLastError();
+        return false;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return false;
+    try
+    {
+        if (!ctx->copier) ctx->copier = HostCopier::of_device(ctx->device, ctx->pageable >= HostCopier::kSetUpAfter);
+    }
+    catch (...)
+    {
+        return false;
+    }
+    ctx->pageable += bytes;
+    return ctx->copier && ctx->copier->ready() && ctx->copier->copy(up, device, host, bytes, ctx->stream, result);
+}
+
 inline nimbus_status upload(nimbus_cuda_context* ctx, void* dst, const void* src, size_t bytes)
 {
-    NB_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    cudaError_t result = cudaSuccess;
+    if (!copied(ctx, true, dst, const_cast<void*>(src), bytes, &result))
+        result = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
+    if (result != cudaSuccess) return cuda_fail(ctx, result, "cudaMemcpyAsync");
     return NIMBUS_OK;
 }
 
 inline nimbus_status download(nimbus_cuda_context* ctx, void* dst, const void* src, size_t bytes)
 {
-    NB_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    cudaError_t result = cudaSuccess;
+    if (!copied(ctx, false, const_cast<void*>(src), dst, bytes, &result))
+        result = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+    if (result != cudaSuccess) return cuda_fail(ctx, result, "cudaMemcpyAsync");
     return NIMBUS_OK;
 }
 

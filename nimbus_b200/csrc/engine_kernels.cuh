@@ -1313,8 +1313,8 @@ static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_MICRO_MINB_F32 : 4)
 // The same with the members' constants in the constant bank, for lanes whose
 // constants fit a parameter block: the member table's loads and the registers
 // that held them go.  24 members of 16.5 million cells, ten steps 5.45 -> 4.93
-// ms; 256x256x80 1.54 -> 1.42; reference precision, 3.0 million cells 0.76 ->
-// 0.73.
+// ms; 256x256x80 1.54 -> 1.42; four steps of 3.0 million cells in reference
+// precision 0.76 -> 0.73.
 constexpr int kMicroConstMembers = 64;
 
 struct MicroLaunch

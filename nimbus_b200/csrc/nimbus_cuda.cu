@@ -714,6 +714,7 @@ void nimbus_cuda_destroy(nimbus_cuda_context* ctx)
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    ctx->copier.reset();
     drain_timing(ctx);
     for (cudaEvent_t e : ctx->event_pool) cudaEventDestroy(e);
     for (auto& b : ctx->ws)

@@ -8,7 +8,7 @@
 // terms of the binomial series (table-driven evaluation after Tang, ACM TOMS 16,
 // 1990).  14 FP64 operations for the general power's hundred, and an error of
 // at most 0.51 ulp against 60 digits over 2^-12 .. 2^12 (the general power: up
-// to 2 ulp by its specification).  Continuity and EOS of 3.0 million cells, ten
+// to 2 ulp by its specification).  Continuity and EOS of 3.0 million cells, four
 // steps 1.93 -> 1.50 ms, Kessler and EOS 0.68 -> 0.57.  Outside that range, zeros, negative and
 // non-finite values among them, and for another gamma, the general power.
 #pragma once

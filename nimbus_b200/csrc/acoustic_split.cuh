@@ -690,6 +690,14 @@ __device__ __forceinline__ void momentum_quad(const FusedParams& P, const float*
 
 constexpr int kQuadBlock = 128;  // threads of a quad kernel
 
+// CTAs per SM that a quad kernel's launch bounds ask for.  FP32 at 8 (64
+// registers without spills; 512x512x128, ps per cell, continuity / momentum at
+// 8, 7, 6: 8.98 / 4.70, 9.72 / 4.81, 10.27; one cell per thread 11.1 / 6.8),
+// reference precision at 7 (72; four steps of 3.0 million cells at 8 / 7 / 6:
+// 1.51 / 1.48 / 1.53 and 1.13 / 1.09 / 1.12 ms).
+template <class Policy>
+constexpr int kQuadCtas = sizeof(typename Policy::real) == 4 ? 8 : 7;
+
 // Cells from which the quad kernels are launched: below, a cell per thread
 // fills the SMs better than the quad saves instructions (four CTAs of quads an
 // SM on 148 SMs).  A launch of 164 thousand cells, continuity, us between
@@ -698,7 +706,7 @@ constexpr int kQuadBlock = 128;  // threads of a quad kernel
 constexpr long long kQuadCells = 4LL * kQuadBlock * 4 * 148;
 
 template <class Policy>
-static __global__ void __launch_bounds__(kQuadBlock, 8) split_continuity_quad_kernel(
+static __global__ void __launch_bounds__(kQuadBlock, kQuadCtas<Policy>) split_continuity_quad_kernel(
     FusedParams P, const float* __restrict__ rho, const float* __restrict__ u, const float* __restrict__ v,
     const float* __restrict__ w, const float* __restrict__ theta, const double* __restrict__ rho0,
     const float4* __restrict__ eos0, float* __restrict__ rho_out, float* __restrict__ p_out,
@@ -714,7 +722,7 @@ static __global__ void __launch_bounds__(kQuadBlock, 8) split_continuity_quad_ke
 }
 
 template <class Policy>
-static __global__ void __launch_bounds__(kQuadBlock, 8) split_momentum_quad_kernel(
+static __global__ void __launch_bounds__(kQuadBlock, kQuadCtas<Policy>) split_momentum_quad_kernel(
     FusedParams P, const float* __restrict__ rho, const float* __restrict__ p, const double* __restrict__ p0,
     const float2* __restrict__ dp0_split, const float* __restrict__ u, const float* __restrict__ v,
     const float* __restrict__ w, float* __restrict__ u_out, float* __restrict__ v_out, float* __restrict__ w_out,

@@ -171,7 +171,10 @@ inline void drain_timing(nimbus_cuda_context* ctx)
 inline int grid_for(const nimbus_cuda_context* ctx, long long work)
 {
     long long blocks = (work + kThreads - 1) / kThreads;
-    const long long cap = static_cast<long long>(ctx->sm_count) * 16;
+    // Many small grid-stride shares, so that cells that cost more (cloud, steep
+    // stencils) even out: 16, 64 and 128 CTAs an SM, transport of 256x256x80 in
+    // reference precision 0.72, 0.65 and 0.63 ms.
+    const long long cap = static_cast<long long>(ctx->sm_count) * 128;
     if (blocks > cap) blocks = cap;
     return blocks < 1 ? 1 : static_cast<int>(blocks);
 }

@@ -143,14 +143,14 @@ __device__ __forceinline__ void for_member_rows(const EngineMember* __restrict__
 // ---- Heun slow step -------------------------------------------------------
 
 // Resident CTAs per SM of the slow Heun pair: the reference-precision form at
-// 4 of 256 threads (64 registers), the FP32 form at 5 of kQuadTile threads (96
-// registers; 4, 6 and 8 CTAs: 1.11, 1.05 and 1.20 ms a step against 1.00 on 24
-// members of 16.5 million cells).
+// 4 of 256 threads (64 registers; four steps of 3.0 million cells at 3 / 4 / 5:
+// 1.60 / 1.41 / 1.72 ms), the FP32 form at 6 of kQuadTile threads (80; ten steps
+// of 24 members, 16.5 million cells, at 4 / 5 / 6: 10.4 / 9.44 / 9.27 ms).
 #ifndef NIMBUS_SLOW_MINB
 #define NIMBUS_SLOW_MINB 4
 #endif
 #ifndef NIMBUS_SLOW_MINB_F32
-#define NIMBUS_SLOW_MINB_F32 5
+#define NIMBUS_SLOW_MINB_F32 6
 #endif
 template <class Policy>
 static __global__ void __launch_bounds__(256, 4) engine_slow_predict_kernel(const EngineMember* __restrict__ table,
@@ -469,18 +469,6 @@ __device__ __forceinline__ FusedParams with_shared(const FusedParams& F, const A
     return P;
 }
 
-// Resident CTAs (of kQuadTile threads) per SM the launch bounds ask for
-// (continuity, momentum): at 8 the FP32 form keeps to 64 registers without
-// spills.  FP32, 512x512x128, ps per cell: 8 / 8 8.98 / 4.70, 7 / 7
-// 9.72 / 4.81, 6 / 8 10.27 / 4.71 (one cell per thread 11.1 / 6.8); reference
-// precision, 256x256x80: 17.1 / 9.5 (one cell 19.3 / 10.2).
-#ifndef NIMBUS_CONST_MINB
-#define NIMBUS_CONST_MINB 8
-#endif
-#ifndef NIMBUS_CONST_MINB_MOM
-#define NIMBUS_CONST_MINB_MOM 8
-#endif
-
 struct AcousticLaunch
 {
     long long prefix[kConstMembers + 1];        // first cell tile of each member
@@ -515,7 +503,7 @@ __device__ __forceinline__ void for_const_cells(const AcousticLaunch& L, const E
 // accumulated, and the beginning density is kept).
 // kShared: every member's shared values equal L.shared (acoustic_shared_of).
 template <class Policy, bool kFirst, bool kShared, int kCells>
-static __global__ void __launch_bounds__(kQuadTile, NIMBUS_CONST_MINB) engine_continuity_const_kernel(const __grid_constant__ AcousticLaunch L,
+static __global__ void __launch_bounds__(kQuadTile, kQuadCtas<Policy>) engine_continuity_const_kernel(const __grid_constant__ AcousticLaunch L,
                                                                       const EngineMember* __restrict__ table,
                                                                       long long tiles, int s)
 {
@@ -538,7 +526,7 @@ static __global__ void __launch_bounds__(kQuadTile, NIMBUS_CONST_MINB) engine_co
 }
 
 template <class Policy, int kCells>
-static __global__ void __launch_bounds__(kQuadTile, NIMBUS_CONST_MINB_MOM) engine_momentum_const_kernel(const __grid_constant__ AcousticLaunch L,
+static __global__ void __launch_bounds__(kQuadTile, kQuadCtas<Policy>) engine_momentum_const_kernel(const __grid_constant__ AcousticLaunch L,
                                                                     const EngineMember* __restrict__ table,
                                                                     long long tiles, int s)
 {
@@ -1027,14 +1015,15 @@ static __global__ void engine_swap_kernel(EngineMember* table, int members, int 
 // ---- Transport (every scalar of a cell in one thread) -----------------------
 
 template <bool kFp32>
-// Resident CTAs per SM of the face-flux pass: the FP32 form at 4 (64
-// registers; 1.85 -> 1.81 ms per ensemble step), the reference-precision
-// form at 2 (its natural 90 registers).
+// Resident CTAs per SM of the face-flux pass: the FP32 form at 5 (48
+// registers; ten steps of 24 members, 16.5 million cells, at 3 / 4 / 5 / 6:
+// 6.09 / 5.27 / 4.97 / 5.22 ms), the reference-precision form at 4 (64; four
+// steps of 3.0 million cells at 2 / 3 / 4 / 5: 1.14 / 0.94 / 0.88 / 0.93 ms).
 #ifndef NIMBUS_FACES_MINB
-#define NIMBUS_FACES_MINB 2
+#define NIMBUS_FACES_MINB 4
 #endif
 #ifndef NIMBUS_FACES_MINB_F32
-#define NIMBUS_FACES_MINB_F32 4
+#define NIMBUS_FACES_MINB_F32 5
 #endif
 static __global__ void __launch_bounds__(256, NIMBUS_FACES_MINB) engine_transport_faces_kernel(const EngineMember* __restrict__ table,
                                                                             const long long* __restrict__ prefix,
@@ -1124,8 +1113,10 @@ static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_FACES_MINB_F32 : NI
     });
 }
 
+// Of the limiter: the FP32 form at 5 (4 / 5 / 6 / 8: 2.31 / 2.31 / 2.39 / 3.10
+// ms), the reference-precision form at 3 (3 / 6 / 8: 0.23 / 0.26 / 0.30).
 #ifndef NIMBUS_LIMITER_MINB_F32
-#define NIMBUS_LIMITER_MINB_F32 6
+#define NIMBUS_LIMITER_MINB_F32 5
 #endif
 template <bool kFp32>
 static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_LIMITER_MINB_F32 : 3) engine_transport_limiter_const_kernel(
@@ -1137,11 +1128,11 @@ static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_LIMITER_MINB_F32 : 
     });
 }
 
-// Resident CTAs per SM of the update pass: the FP32 form at 4 (64
-// registers; 0.88 -> 0.83 ms per ensemble step), the reference-precision
-// form at 3 (at most 85 registers).
+// Of the update: both at 3, since the loads of a cell's six faces for four
+// scalars are in flight together (FP32 2 / 3 / 4 / 5: 3.55 / 2.91 / 3.49 / 5.41
+// ms; reference precision 2 / 3 / 4: 0.42 / 0.35 / 0.41).
 #ifndef NIMBUS_UPDATE_MINB_F32
-#define NIMBUS_UPDATE_MINB_F32 4
+#define NIMBUS_UPDATE_MINB_F32 3
 #endif
 template <bool kFp32>
 static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_UPDATE_MINB_F32 : 3) engine_transport_update_const_kernel(
@@ -1210,8 +1201,9 @@ static __global__ void __launch_bounds__(kQuadTile) engine_sound_speed_kernel(co
 // pressure is formed from the applied state while it is still in registers
 // and written to the member's candidate buffer; engine_swap_kernel publishes
 // it by exchanging p and the candidate unless the projection was refused.
-// Resident CTAs per SM of the Kessler + EOS pass: the FP32 form at 6, the
-// reference-precision form at 4.
+// Resident CTAs per SM of the Kessler + EOS pass: the FP32 form at 6 (5 / 6 / 7:
+// 4.55 / 4.47 / 4.62 ms), the reference-precision form at 5 (3 / 4 / 5 / 6:
+// 0.64 / 0.57 / 0.55 / 0.58).
 #ifndef NIMBUS_MICRO_MINB_F32
 #define NIMBUS_MICRO_MINB_F32 6
 #endif
@@ -1300,7 +1292,7 @@ __device__ __forceinline__ void microphysics_eos_cell(const MicroConst& A, const
 }
 
 template <bool kFp32>
-static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_MICRO_MINB_F32 : 4) engine_microphysics_eos_kernel(const EngineMember* __restrict__ table,
+static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_MICRO_MINB_F32 : 5) engine_microphysics_eos_kernel(const EngineMember* __restrict__ table,
                                                                              const long long* __restrict__ prefix,
                                                                              long long tiles)
 {
@@ -1325,7 +1317,7 @@ struct MicroLaunch
 static_assert(sizeof(MicroLaunch) <= 32000, "a kernel parameter block holds at most 32764 bytes");
 
 template <bool kFp32>
-static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_MICRO_MINB_F32 : 4) engine_microphysics_eos_const_kernel(
+static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_MICRO_MINB_F32 : 5) engine_microphysics_eos_const_kernel(
     const __grid_constant__ MicroLaunch L, const EngineMember* __restrict__ table, long long tiles)
 {
     grid_dependency();

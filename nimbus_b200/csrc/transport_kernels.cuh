@@ -371,8 +371,12 @@ __device__ __forceinline__ void transport_faces_cell(const TransportParams& T, i
     }
 }
 
+// CTAs per SM of the three passes: faces 5 in FP32 and 4 in reference precision
+// (4 / 5 / 6: 0.216 / 0.206 / 0.213 ms and 3 / 4 / 5: 0.47 / 0.41 / 0.41 on
+// 256x256x80), limiter and update 8, whose loads wait (6 / 8: 0.099 / 0.084 and
+// 0.127 / 0.115, reference precision 0.103 / 0.092 and 0.148 / 0.136).
 template <bool kFp32>
-static __global__ void __launch_bounds__(256) transport_faces_kernel(TransportParams T, const float* __restrict__ mfx,
+static __global__ void __launch_bounds__(256, kFp32 ? 5 : 4) transport_faces_kernel(TransportParams T, const float* __restrict__ mfx,
                                                                      const float* __restrict__ mfy,
                                                                      const float* __restrict__ mfz,
                                                                      float* __restrict__ sf)
@@ -488,7 +492,7 @@ __device__ __forceinline__ void transport_limiter_cell(const TransportParams& T,
 }
 
 template <bool kFp32>
-static __global__ void __launch_bounds__(256) transport_limiter_kernel(TransportParams T,
+static __global__ void __launch_bounds__(256, 8) transport_limiter_kernel(TransportParams T,
                                                                        const float* __restrict__ rho_begin,
                                                                        const float* __restrict__ sf,
                                                                        float* __restrict__ rl)
@@ -651,7 +655,7 @@ __device__ __forceinline__ void transport_update_cell(const TransportParams& T, 
 }
 
 template <bool kFp32>
-static __global__ void __launch_bounds__(256) transport_update_kernel(TransportParams T,
+static __global__ void __launch_bounds__(256, 8) transport_update_kernel(TransportParams T,
                                                                       const float* __restrict__ rho_end,
                                                                       const float* __restrict__ rho_begin,
                                                                       const float* __restrict__ sf,

@@ -356,7 +356,7 @@ __device__ __forceinline__ bool bc_inner_column(const Dims& d, int i, int j)
 }
 
 // The closure is independent from level to level except for the top level,
-// which takes the one below: a cluster of one to four CTAs closes a band of
+// which takes the one below: a cluster of one to eight CTAs closes a band of
 // four levels (the last one up to seven) all around the member, with a cluster
 // barrier between the reference's steps W,E -> S,N -> vertical instead of a
 // launch.  A ring is a few thousand values, so its time is the latency of its
@@ -366,10 +366,10 @@ __device__ __forceinline__ bool bc_inner_column(const Dims& d, int i, int j)
 constexpr int kRingLevels = 4;
 constexpr int kRingBlock = 256;
 
-// CTAs a band of `rows` rows takes: one face of a row a thread, up to four CTAs.
+// CTAs a band of `rows` rows takes: one face of a row a thread, up to eight CTAs.
 __host__ __device__ __forceinline__ int ring_cluster(int rows)
 {
-    return 2 * rows <= kRingBlock ? 1 : rows <= kRingBlock ? 2 : 4;
+    return 2 * rows <= kRingBlock ? 1 : rows <= kRingBlock ? 2 : rows <= 2 * kRingBlock ? 4 : 8;
 }
 
 // The CTA's place in its cluster and the cluster's size (0 and 1 without one).

@@ -168,13 +168,15 @@ inline void drain_timing(nimbus_cuda_context* ctx)
     ctx->pending.clear();
 }
 
-inline int grid_for(const nimbus_cuda_context* ctx, long long work)
+// The grid of a grid-stride kernel.  uneven: cells that cost more (steep
+// stencils, the closure's edges) even out over many small shares; 16, 64 and 128
+// CTAs an SM, transport of 256x256x80 in reference precision 0.72, 0.65 and
+// 0.63 ms.  Streaming passes and reductions gain nothing (193x161x61 Kessler and
+// EOS 60 us at 16, 66 at 128; the largest sound speed 41 and 63).
+inline int grid_for(const nimbus_cuda_context* ctx, long long work, bool uneven = false)
 {
     long long blocks = (work + kThreads - 1) / kThreads;
-    // Many small grid-stride shares, so that cells that cost more (cloud, steep
-    // stencils) even out: 16, 64 and 128 CTAs an SM, transport of 256x256x80 in
-    // reference precision 0.72, 0.65 and 0.63 ms.
-    const long long cap = static_cast<long long>(ctx->sm_count) * 128;
+    const long long cap = static_cast<long long>(ctx->sm_count) * (uneven ? 128 : 16);
     if (blocks > cap) blocks = cap;
     return blocks < 1 ? 1 : static_cast<int>(blocks);
 }

@@ -171,7 +171,7 @@ nimbus_status launch_transport_impl(nimbus_cuda_context* ctx, cudaStream_t st, c
                                     const float* rho_end, const float* rho_begin, const float* mfx, const float* mfy,
                                     const float* mfz, float* sf, float* rl)
 {
-    const dim3 grid(grid_for(ctx, T.d.cells()));
+    const dim3 grid(grid_for(ctx, T.d.cells(), true));
     {
         LaunchTimer t(ctx, st, NIMBUS_KERNEL_TRANSPORT_FACES);
         transport_faces_kernel<kFp32><<<grid, kThreads, 0, st>>>(T, mfx, mfy, mfz, sf);

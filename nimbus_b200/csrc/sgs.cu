@@ -125,7 +125,7 @@ struct ClosureDevice
 nimbus_status launch_closure(nimbus_cuda_context* ctx, cudaStream_t st, const SgsParams& P, const ClosureDevice& D,
                              unsigned* status)
 {
-    const int grid = grid_for(ctx, P.d.cells());
+    const int grid = grid_for(ctx, P.d.cells(), true);
     LaunchTimer t(ctx, st, NIMBUS_KERNEL_SGS);
     auto both = [&](auto coefficients, auto tendencies) {
         coefficients<<<grid, kThreads, 0, st>>>(P, D.u, D.v, D.w, D.theta, D.qv, D.rho, D.nu, D.kt, D.kq, status);

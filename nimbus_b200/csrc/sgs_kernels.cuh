@@ -226,12 +226,12 @@ __device__ __forceinline__ R sgs_min(R a, R b) { return b < a ? b : a; }  // std
 // field contract (validate_scheme_inputs, eddy_viscosity.cpp:1088-1175) or
 // whose coefficient is not finite raises kStatusSgsInvalid.
 //
-// The FP64 form at 5 CTAs per SM (48 registers, some spilled) and its
-// tendencies at 6: both wait for loads more than they issue.  320x320x64, the
-// pair: 3 and 4 CTAs 0.94 ms, 4 and 4 0.87, 5 and 5 0.82, 5 and 6 0.82, 6 and 6
-// 0.83.
+// At 5 CTAs per SM (48 registers, some spilled in FP64) and the tendencies at 6:
+// both wait for loads more than they issue.  320x320x64 in FP64, the pair: 3 and
+// 4 CTAs 0.94 ms, 4 and 4 0.87, 5 and 5 0.82, 5 and 6 0.82, 6 and 6 0.83;
+// 160x160x64 in FP32: 3 and 4 0.188, 4 and 5 0.171, 5 and 6 0.161, 6 and 8 0.162.
 template <class R, bool F>
-__global__ void __launch_bounds__(256, sizeof(R) == 8 ? 5 : 3) sgs_coefficients_kernel(SgsParams P, const float* __restrict__ u,
+__global__ void __launch_bounds__(256, 5) sgs_coefficients_kernel(SgsParams P, const float* __restrict__ u,
                                                                const float* __restrict__ v,
                                                                const float* __restrict__ w,
                                                                const float* __restrict__ theta,
@@ -434,7 +434,7 @@ __device__ R sgs_dw(const SgsParams& P, const float* u, const float* v, const fl
 // The five tendencies of every cell; zero where the reference leaves its
 // pre-cleared outputs untouched.
 template <class R, bool F>
-__global__ void __launch_bounds__(256, sizeof(R) == 8 ? 6 : 4) sgs_tendencies_kernel(
+__global__ void __launch_bounds__(256, 6) sgs_tendencies_kernel(
     SgsParams P, const float* __restrict__ u, const float* __restrict__ v, const float* __restrict__ w,
     const float* __restrict__ theta, const float* __restrict__ qv, const float* __restrict__ rho,
     const float* __restrict__ nu_t, const float* __restrict__ K_theta, const float* __restrict__ K_q,

@@ -407,8 +407,11 @@ __device__ __forceinline__ void slow_predict_cell(
     }
 }
 
+// The pair at 4 CTAs per SM: 160x160x64 in reference precision, two steps, at 2
+// (97 registers) / 3 / 4 / 5: 0.54 / 0.46 / 0.37 / 0.46 ms; 256x256x80 in FP32,
+// at 3 / 4 / 5: 1.11 / 0.82 / 0.88.
 template <class Policy>
-static __global__ void __launch_bounds__(256) slow_predict_kernel(
+static __global__ void __launch_bounds__(256, 4) slow_predict_kernel(
     SlowParams S, const float* __restrict__ u, const float* __restrict__ v, const float* __restrict__ w,
     const float* __restrict__ rho, const float* __restrict__ p, const float* __restrict__ qv,
     const float* __restrict__ qc, const float* __restrict__ qr, const double* __restrict__ rho0,
@@ -832,7 +835,7 @@ __device__ __forceinline__ void slow_correct_quad(
 }
 
 template <class Policy>
-static __global__ void __launch_bounds__(256) slow_correct_kernel(
+static __global__ void __launch_bounds__(256, 4) slow_correct_kernel(
     SlowParams S, const float* __restrict__ su, const float* __restrict__ sv, const float* __restrict__ sw,
     const float* __restrict__ rho, const float* __restrict__ sp, const float* __restrict__ qv,
     const float* __restrict__ qc, const float* __restrict__ qr, const double* __restrict__ rho0,

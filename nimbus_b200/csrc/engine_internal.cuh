@@ -304,8 +304,10 @@ int enqueue_step(nimbus_engine* e, int lane, cudaStream_t st, int part)
         if constexpr (kFp32)
         {
             const long long quads = tiles_of(e, L, kItemQuads, n);
-            ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_SLOW, engine_slow_predict_quad_kernel<Policy>, quads, kQuadTile, *sl, T, quads);
-            ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_SLOW, engine_slow_correct_quad_kernel<Policy>, quads, kQuadTile, *sl, T, quads);
+            ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_SLOW, engine_slow_predict_quad_kernel<Policy>, quads, kQuadTile, *sl, T,
+                                quads);
+            ENGINE_LAUNCH_BLOCK(NIMBUS_KERNEL_SLOW, engine_slow_correct_quad_kernel<Policy>, quads, kQuadTile, *sl, T,
+                                quads);
         }
         else
         {

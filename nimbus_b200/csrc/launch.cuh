@@ -98,8 +98,8 @@ nimbus_status launch_split_impl(nimbus_cuda_context* ctx, cudaStream_t st, Fused
     const long long n = F.d.cells();
     const bool early = not_captured(st);
     if (n >= kQuadCells && F.d.nz % 4 == 0 && drho == nullptr && aligned16(in.rho) && aligned16(in.u) &&
-        aligned16(in.v) && aligned16(in.w) && aligned16(out.rho) && aligned16(out.u) && aligned16(out.v) && aligned16(out.w) &&
-        aligned16(p) && aligned16(theta) && aligned16(mfx) && aligned16(mfy) && aligned16(mfz))
+        aligned16(in.v) && aligned16(in.w) && aligned16(out.rho) && aligned16(out.u) && aligned16(out.v) &&
+        aligned16(out.w) && aligned16(p) && aligned16(theta) && aligned16(mfx) && aligned16(mfy) && aligned16(mfz))
     {
         const long long quads = n / 4;
         long long qblocks = (quads + kQuadBlock - 1) / kQuadBlock;

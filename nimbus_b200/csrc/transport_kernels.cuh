@@ -556,7 +556,10 @@ __device__ __forceinline__ float update_value(const TP& T, bool pd, float fxp, f
             };
             const float outgoing = __fmul_rn(rc, through(xa - xout, ya - yout, za - zout));
             const float incoming = through(into(xb, rxm, xin, rxp), into(yb, rym, yin, ryp), into(zc, rzm, zin, rzp));
-            const float rho_phi = __fmaf_rn(dt, incoming, __fmaf_rn(-dt, outgoing, __fmul_rn(rb, qraw)));
+            // rho_b q is not rounded on its own: it is the largest term, and where
+            // nearly all of it leaves its rounding would be the result's error
+            // (rounded first, the update is a tenth farther from 64 bits).
+            const float rho_phi = __fmaf_rn(dt, incoming, __fmaf_rn(rb, qraw, -__fmul_rn(dt, outgoing)));
             const float out = __fdividef(rho_phi, denom);
             if (!isfinite(out)) flags |= kStatusNonfiniteTransport;
             return out;

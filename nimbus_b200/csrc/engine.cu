@@ -768,10 +768,15 @@ struct StateStage
         }
         return NIMBUS_OK;
     }
-    void move(const EngineMember& M, int gather)
+    // The launch's own error (the stream's device has to be current).
+    cudaError_t move(const EngineMember& M, int gather)
     {
-        member_image_kernel<<<grid_for(e->ctx, M.items[kItemCells]), kThreads, 0, e->stream>>>(M, block, gather);
-        e->ctx->launches += 1;
+        const cudaError_t err = launch_after(false, member_image_kernel,
+                                             static_cast<unsigned>(grid_for(e->ctx, M.items[kItemCells])), kThreads,
+                                             1u, e->stream, M, block, gather);
+        if (err != cudaSuccess) (void)cudaGetLastError();  // reported here, not by a later call
+        else e->ctx->launches += 1;
+        return err;
     }
 };
 
@@ -995,7 +1000,7 @@ nimbus_status nimbus_cuda_engine_admit(nimbus_engine* e, const nimbus_member_des
     // arrays and the local vectors may go); pinned ones are read by the copy.
     for (int f = 0; f < 9 && err == cudaSuccess; ++f)
         err = cudaMemcpyAsync(dst[f], src[f], bytes, cudaMemcpyHostToDevice, e->stream);
-    if (err == cudaSuccess && padded(M)) stage.move(M, 0);
+    if (err == cudaSuccess && padded(M)) err = stage.move(M, 0);
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(prof, hp.data(), hp.size() * sizeof(double), cudaMemcpyHostToDevice, e->stream);
     M.R = RelaxTables{};
@@ -1057,6 +1062,7 @@ nimbus_status nimbus_cuda_engine_read_async(nimbus_engine* e, int member_id, con
     if (const char* why = check_state(out)) return fail(ctx, NIMBUS_ERR_INVALID_ARGUMENT, why);
     MemberSlot* s = find_slot(e, member_id);
     if (!s) return fail(ctx, NIMBUS_ERR_INVALID_ARGUMENT, "unknown member id");
+    NB_CUDA(ctx, cudaSetDevice(ctx->device));
     if (!e->mirror_exact) NB_TRY(sync_table_to_host(e));
     const EngineMember& M = s->m;
     const size_t cells = state_cells(*s), bytes = cells * sizeof(float);
@@ -1066,7 +1072,7 @@ nimbus_status nimbus_cuda_engine_read_async(nimbus_engine* e, int member_id, con
     if (padded(M))
     {
         NB_TRY(stage.open(cells));
-        stage.move(M, 1);
+        NB_CUDA(ctx, stage.move(M, 1));
         for (int f = 0; f < 9; ++f) src[f] = stage.block + static_cast<size_t>(f) * cells;
     }
     for (int f = 0; f < 9; ++f)
@@ -1082,6 +1088,7 @@ nimbus_status nimbus_cuda_engine_write_async(nimbus_engine* e, int member_id, co
     if (const char* why = check_state(in)) return fail(ctx, NIMBUS_ERR_INVALID_ARGUMENT, why);
     MemberSlot* s = find_slot(e, member_id);
     if (!s) return fail(ctx, NIMBUS_ERR_INVALID_ARGUMENT, "unknown member id");
+    NB_CUDA(ctx, cudaSetDevice(ctx->device));
     if (!e->mirror_exact) NB_TRY(sync_table_to_host(e));
     const EngineMember& M = s->m;
     const size_t cells = state_cells(*s), bytes = cells * sizeof(float);
@@ -1095,8 +1102,7 @@ nimbus_status nimbus_cuda_engine_write_async(nimbus_engine* e, int member_id, co
     }
     for (int f = 0; f < 9; ++f)
         NB_CUDA(ctx, cudaMemcpyAsync(dst[f], src[f], bytes, cudaMemcpyHostToDevice, e->stream));
-    if (padded(M)) stage.move(M, 0);
-    NB_CUDA(ctx, cudaGetLastError());
+    if (padded(M)) NB_CUDA(ctx, stage.move(M, 0));
     return NIMBUS_OK;
 }
 
@@ -1129,7 +1135,7 @@ nimbus_status nimbus_cuda_engine_history_async(nimbus_engine* e, int member_id, 
     if (padded(M))
     {
         NB_TRY(stage.open(cells));
-        stage.move(M, 1);
+        NB_CUDA(ctx, stage.move(M, 1));
         for (int f = 0; f < kHistoryFields; ++f) src[f] = stage.block + static_cast<size_t>(f) * cells;
     }
     return enqueue_history(ctx, e->stream, src, fields, nullptr, s->desc.nx, s->desc.ny, s->desc.nz, e->d_centre,

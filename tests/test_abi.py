@@ -137,3 +137,24 @@ def test_argument_blocks_keep_their_arrays_alive():
             assert addr in kept, name
     for i in range(2):
         assert ctypes.cast(a.q_in[i], ctypes.c_void_p).value in kept_addresses(a)
+
+
+def test_engine_calls_make_their_device_current_before_they_enqueue():
+    """CUDA refuses a launch or an allocation on a stream of another device
+    than the calling thread's: every engine entry point that enqueues any makes
+    the engine's device current first (itself or in prepare_image)."""
+    text = (ROOT / "nimbus_b200" / "csrc" / "engine.cu").read_text()
+    text = re.sub(r"//[^\n]*", "", text[text.index('extern "C" {'):])
+    starts = [m for m in re.finditer(r"^[\w ]+\*? ?(nimbus_cuda_engine_\w+)\([^;{]*\)\s*\{", text, re.M)]
+    enqueues = re.compile(r"<<<|\bmove\(|\blaunch_\w+\(|\benqueue\w*\(|cudaMalloc\w*\(|cudaGraphLaunch\(")
+    current = re.compile(r"cudaSetDevice\(|\bprepare_image\(")
+    checked = []
+    for m, following in zip(starts, starts[1:] + [None]):
+        body = text[m.end():following.start() if following else len(text)]
+        first = enqueues.search(body)
+        if first:
+            device = current.search(body)
+            assert device and device.start() < first.start(), m.group(1)
+            checked.append(m.group(1))
+    assert {"nimbus_cuda_engine_read_async", "nimbus_cuda_engine_write_async", "nimbus_cuda_engine_admit",
+            "nimbus_cuda_engine_step"} <= set(checked)

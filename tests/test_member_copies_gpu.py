@@ -1,0 +1,78 @@
+"""Single members read, written and recorded from threads that have made no
+CUDA call yet, or have another device current, with padded columns (every nz
+modulo four) and without."""
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+from nimbus_b200 import cuda
+from nimbus_b200.initial import Case, perturbed_state
+from nimbus_b200.run import EngineRun
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("u", "v", "w", "rho", "p", "theta", "qv", "qc", "qr")
+
+
+def _members(run, levels=(8, 9, 10, 11)):
+    out = []
+    for m, nz in enumerate(levels):
+        case = Case(9, 8, nz, 900.0, 850.0, 600.0, 2.0, seed=2, member=m)
+        st, base = perturbed_state(case, seed=60 + m)
+        out.append((run.admit(case, st, base, n_substeps=2), st))
+    return out
+
+
+def _in_thread(work):
+    failed = []
+
+    def body():
+        try:
+            work()
+        except BaseException as error:  # handed to the test's own thread
+            failed.append(error)
+
+    t = threading.Thread(target=body)
+    t.start()
+    t.join(120)
+    assert not t.is_alive()
+    if failed:
+        raise failed[0]
+
+
+def _read_and_write(run, members):
+    for mid, st in members:
+        got = run.read(mid)
+        for k in FIELDS:
+            assert np.array_equal(got[k].view(np.uint32), st[k].view(np.uint32)), k
+        st["theta"] = st["theta"] + np.float32(1.0)
+        run.engine.write(mid, st)
+        got = run.read(mid)
+        assert np.array_equal(got["theta"], st["theta"])
+
+
+def test_members_move_in_a_new_thread():
+    ctx = cuda.Context(0)
+    run = EngineRun(ctx)
+    members = _members(run)
+    _in_thread(lambda: _read_and_write(run, members))
+    run.close()
+    ctx.close()
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs a second device")
+def test_members_move_with_another_device_current():
+    ctx = cuda.Context(1)
+    run = EngineRun(ctx)
+    members = _members(run)
+
+    def work():
+        torch.cuda.set_device(0)
+        torch.zeros(1, device="cuda:0")
+        _read_and_write(run, members)
+
+    _in_thread(work)
+    run.close()
+    ctx.close()

@@ -745,42 +745,26 @@ void launch_image(nimbus_engine* e, int gather, float* image = nullptr)
     }
 }
 
-// A stream-ordered device block holding one member's unpadded state, for
-// members whose columns are padded (nz not a multiple of four): the host's
-// nine fields move to and from it in plain copies and member_image_kernel
-// spreads it into the member's buffers or collects it from them.
-struct StateStage
-{
-    nimbus_engine* e;
-    float* block = nullptr;
-    ~StateStage()
-    {
-        if (block) cudaFreeAsync(block, e->stream);  // after what is enqueued on it
-    }
-    nimbus_status open(size_t cells)
-    {
-        const cudaError_t err =
-            cudaMallocAsync(reinterpret_cast<void**>(&block), 9 * cells * sizeof(float), e->stream);
-        if (err != cudaSuccess)
-        {
-            block = nullptr;
-            return cuda_fail(e->ctx, err, "member staging");
-        }
-        return NIMBUS_OK;
-    }
-    // The launch's own error (the stream's device has to be current).
-    cudaError_t move(const EngineMember& M, int gather)
-    {
-        const cudaError_t err = launch_after(false, member_image_kernel,
-                                             static_cast<unsigned>(grid_for(e->ctx, M.items[kItemCells])), kThreads,
-                                             1u, e->stream, M, block, gather);
-        if (err != cudaSuccess) (void)cudaGetLastError();  // reported here, not by a later call
-        else e->ctx->launches += 1;
-        return err;
-    }
-};
-
 bool padded(const EngineMember& M) { return M.F.d.pz != M.F.d.nz; }
+
+// The unpadded state of a member whose columns are padded (nz not a multiple of
+// four), nine fields of `cells` cells: the host's arrays move to and from it in
+// plain copies, and move_state spreads it into the member's buffers (gather 0)
+// or collects it from them (1).  It lies in the member's face fluxes, 12 values
+// a cell that hold nothing between steps, so that a copy needs no memory that
+// admission has not counted.
+float* staged_field(const EngineMember& M, size_t cells, int f) { return M.sf + static_cast<size_t>(f) * cells; }
+
+// The launch's own error (the stream's device has to be current).
+cudaError_t move_state(nimbus_engine* e, const EngineMember& M, int gather)
+{
+    const cudaError_t err = launch_after(false, member_image_kernel,
+                                         static_cast<unsigned>(grid_for(e->ctx, M.items[kItemCells])), kThreads, 1u,
+                                         e->stream, M, M.sf, gather);
+    if (err != cudaSuccess) (void)cudaGetLastError();  // reported here, not by a later call
+    else e->ctx->launches += 1;
+    return err;
+}
 
 const char* check_state(const nimbus_member_state* s)
 {
@@ -986,21 +970,13 @@ nimbus_status nimbus_cuda_engine_admit(nimbus_engine* e, const nimbus_member_des
     const float* src[9] = {initial->u, initial->v, initial->w, initial->rho, initial->p, initial->theta,
                            initial->qv, initial->qc, initial->qr};
     float* dst[9] = {M.u, M.v, M.w, M.rho, M.p, M.theta, M.qv, M.qc, M.qr};
-    StateStage stage{e};
     if (padded(M))
-    {
-        if (const nimbus_status rc = stage.open(cells); rc != NIMBUS_OK)
-        {
-            cudaFreeAsync(slot.arena, e->stream);
-            return rc;
-        }
-        for (int f = 0; f < 9; ++f) dst[f] = stage.block + static_cast<size_t>(f) * cells;
-    }
+        for (int f = 0; f < 9; ++f) dst[f] = staged_field(M, cells, f);
     // Pageable sources are staged before each call returns (the caller's
     // arrays and the local vectors may go); pinned ones are read by the copy.
     for (int f = 0; f < 9 && err == cudaSuccess; ++f)
         err = cudaMemcpyAsync(dst[f], src[f], bytes, cudaMemcpyHostToDevice, e->stream);
-    if (err == cudaSuccess && padded(M)) err = stage.move(M, 0);
+    if (err == cudaSuccess && padded(M)) err = move_state(e, M, 0);
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(prof, hp.data(), hp.size() * sizeof(double), cudaMemcpyHostToDevice, e->stream);
     M.R = RelaxTables{};
@@ -1068,12 +1044,10 @@ nimbus_status nimbus_cuda_engine_read_async(nimbus_engine* e, int member_id, con
     const size_t cells = state_cells(*s), bytes = cells * sizeof(float);
     const float* src[9] = {M.u, M.v, M.w, M.rho, M.p, M.theta, M.qv, M.qc, M.qr};
     float* dst[9] = {out->u, out->v, out->w, out->rho, out->p, out->theta, out->qv, out->qc, out->qr};
-    StateStage stage{e};
     if (padded(M))
     {
-        NB_TRY(stage.open(cells));
-        NB_CUDA(ctx, stage.move(M, 1));
-        for (int f = 0; f < 9; ++f) src[f] = stage.block + static_cast<size_t>(f) * cells;
+        NB_CUDA(ctx, move_state(e, M, 1));
+        for (int f = 0; f < 9; ++f) src[f] = staged_field(M, cells, f);
     }
     for (int f = 0; f < 9; ++f)
         NB_CUDA(ctx, cudaMemcpyAsync(dst[f], src[f], bytes, cudaMemcpyDeviceToHost, e->stream));
@@ -1094,15 +1068,11 @@ nimbus_status nimbus_cuda_engine_write_async(nimbus_engine* e, int member_id, co
     const size_t cells = state_cells(*s), bytes = cells * sizeof(float);
     const float* src[9] = {in->u, in->v, in->w, in->rho, in->p, in->theta, in->qv, in->qc, in->qr};
     float* dst[9] = {M.u, M.v, M.w, M.rho, M.p, M.theta, M.qv, M.qc, M.qr};
-    StateStage stage{e};
     if (padded(M))
-    {
-        NB_TRY(stage.open(cells));
-        for (int f = 0; f < 9; ++f) dst[f] = stage.block + static_cast<size_t>(f) * cells;
-    }
+        for (int f = 0; f < 9; ++f) dst[f] = staged_field(M, cells, f);
     for (int f = 0; f < 9; ++f)
         NB_CUDA(ctx, cudaMemcpyAsync(dst[f], src[f], bytes, cudaMemcpyHostToDevice, e->stream));
-    if (padded(M)) NB_CUDA(ctx, stage.move(M, 0));
+    if (padded(M)) NB_CUDA(ctx, move_state(e, M, 0));
     return NIMBUS_OK;
 }
 
@@ -1131,12 +1101,10 @@ nimbus_status nimbus_cuda_engine_history_async(nimbus_engine* e, int member_id, 
         e->centre_cap = need;
     }
     const float* src[kHistoryFields] = {M.u, M.v, M.w, M.rho, M.p, M.theta, M.qv, M.qc, M.qr};
-    StateStage stage{e};
     if (padded(M))
     {
-        NB_TRY(stage.open(cells));
-        NB_CUDA(ctx, stage.move(M, 1));
-        for (int f = 0; f < kHistoryFields; ++f) src[f] = stage.block + static_cast<size_t>(f) * cells;
+        NB_CUDA(ctx, move_state(e, M, 1));
+        for (int f = 0; f < kHistoryFields; ++f) src[f] = staged_field(M, cells, f);
     }
     return enqueue_history(ctx, e->stream, src, fields, nullptr, s->desc.nx, s->desc.ny, s->desc.nz, e->d_centre,
                            static_cast<float*>(host_image));

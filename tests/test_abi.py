@@ -146,7 +146,7 @@ def test_engine_calls_make_their_device_current_before_they_enqueue():
     text = (ROOT / "nimbus_b200" / "csrc" / "engine.cu").read_text()
     text = re.sub(r"//[^\n]*", "", text[text.index('extern "C" {'):])
     starts = [m for m in re.finditer(r"^[\w ]+\*? ?(nimbus_cuda_engine_\w+)\([^;{]*\)\s*\{", text, re.M)]
-    enqueues = re.compile(r"<<<|\bmove\(|\blaunch_\w+\(|\benqueue\w*\(|cudaMalloc\w*\(|cudaGraphLaunch\(")
+    enqueues = re.compile(r"<<<|\bmove_state\(|\blaunch_\w+\(|\benqueue\w*\(|cudaMalloc\w*\(|cudaGraphLaunch\(")
     current = re.compile(r"cudaSetDevice\(|\bprepare_image\(")
     checked = []
     for m, following in zip(starts, starts[1:] + [None]):

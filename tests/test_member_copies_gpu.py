@@ -1,6 +1,7 @@
 """Single members read, written and recorded from threads that have made no
 CUDA call yet, or have another device current, with padded columns (every nz
 modulo four) and without."""
+import ctypes
 import threading
 
 import numpy as np
@@ -74,5 +75,42 @@ def test_members_move_with_another_device_current():
         _read_and_write(run, members)
 
     _in_thread(work)
+    run.close()
+    ctx.close()
+
+
+def _pool_high_water(reset=False):
+    """Most bytes in use at once of the device's default memory pool since the
+    last reset."""
+    driver = ctypes.CDLL("libcuda.so.1")
+    pool, value = ctypes.c_void_p(), ctypes.c_uint64(0)
+    assert driver.cuDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    used_high = 8  # CU_MEMPOOL_ATTR_USED_MEM_HIGH
+    if reset:
+        assert driver.cuMemPoolSetAttribute(pool, used_high, ctypes.byref(value)) == 0
+    assert driver.cuMemPoolGetAttribute(pool, used_high, ctypes.byref(value)) == 0
+    return value.value
+
+
+def test_a_member_moves_within_its_own_memory():
+    """Admission, read, write and history of a padded member take no device
+    memory beyond member_bytes: what fits at admission keeps fitting."""
+    ctx = cuda.Context(0)
+    run = EngineRun(ctx)
+    first = _members(run, levels=(9,))
+    _read_and_write(run, first)
+    case = Case(41, 40, 13, 900.0, 850.0, 600.0, 2.0, seed=2)
+    st, base = perturbed_state(case, seed=70)
+    desc = cuda.member_desc(case.shape, (case.dx, case.dy, case.dz), case.dt, 2, case.bc, base)
+    before = _pool_high_water(reset=True)
+    mid = run.engine.admit(desc, st)
+    run.engine.synchronize()
+    assert _pool_high_water() - before <= run.engine.member_bytes(desc) + 4096  # the pool's granularity
+    held = _pool_high_water(reset=True)
+    _read_and_write(run, [(mid, st)])
+    frame = np.empty(9 * st["u"].size, np.float32)
+    run.engine.history_async(mid, cuda.HISTORY_CORE, frame)
+    run.engine.synchronize()
+    assert _pool_high_water() == held
     run.close()
     ctx.close()

@@ -752,15 +752,15 @@ bool padded(const EngineMember& M) { return M.F.d.pz != M.F.d.nz; }
 // plain copies, and move_state spreads it into the member's buffers (gather 0)
 // or collects it from them (1).  It lies in the member's face fluxes, 12 values
 // a cell that hold nothing between steps, so that a copy needs no memory that
-// admission has not counted.
+// admission has not counted.  fields: the bits of the fields to move.
 float* staged_field(const EngineMember& M, size_t cells, int f) { return M.sf + static_cast<size_t>(f) * cells; }
 
 // The launch's own error (the stream's device has to be current).
-cudaError_t move_state(nimbus_engine* e, const EngineMember& M, int gather)
+cudaError_t move_state(nimbus_engine* e, const EngineMember& M, int gather, unsigned fields = ~0u)
 {
     const cudaError_t err = launch_after(false, member_image_kernel,
                                          static_cast<unsigned>(grid_for(e->ctx, M.items[kItemCells])), kThreads, 1u,
-                                         e->stream, M, M.sf, gather);
+                                         e->stream, M, M.sf, gather, fields);
     if (err != cudaSuccess) (void)cudaGetLastError();  // reported here, not by a later call
     else e->ctx->launches += 1;
     return err;
@@ -1103,7 +1103,7 @@ nimbus_status nimbus_cuda_engine_history_async(nimbus_engine* e, int member_id, 
     const float* src[kHistoryFields] = {M.u, M.v, M.w, M.rho, M.p, M.theta, M.qv, M.qc, M.qr};
     if (padded(M))
     {
-        NB_CUDA(ctx, move_state(e, M, 1));
+        NB_CUDA(ctx, move_state(e, M, 1, fields));
         for (int f = 0; f < kHistoryFields; ++f) src[f] = staged_field(M, cells, f);
     }
     return enqueue_history(ctx, e->stream, src, fields, nullptr, s->desc.nx, s->desc.ny, s->desc.nz, e->d_centre,

@@ -932,8 +932,9 @@ static __global__ void __launch_bounds__(256, NIMBUS_BULK_MINB) engine_momentum_
 // A member's nine prognostic fields back to back (u, v, w, rho, p, theta, qv,
 // qc, qr, each nx ny nz floats without padding), the host's form of a state.
 // gather = 0 scatters an image into the member's current buffers, gather = 1
-// collects them into it.
-__device__ __forceinline__ void image_cell(const EngineMember& M, float* __restrict__ image, int c, int gather)
+// collects them into it; only the fields whose bits are set.
+__device__ __forceinline__ void image_cell(const EngineMember& M, float* __restrict__ image, int c, int gather,
+                                           unsigned fields)
 {
     int i, j, k;
     const Dims d = M.F.d;
@@ -946,16 +947,20 @@ __device__ __forceinline__ void image_cell(const EngineMember& M, float* __restr
     if (gather)
     {
 #pragma unroll
-        for (int f = 0; f < 9; ++f) x[f] = field[f][c];
+        for (int f = 0; f < 9; ++f)
+            if (fields >> f & 1u) x[f] = field[f][c];
 #pragma unroll
-        for (int f = 0; f < 9; ++f) blk[f * n] = x[f];
+        for (int f = 0; f < 9; ++f)
+            if (fields >> f & 1u) blk[f * n] = x[f];
     }
     else
     {
 #pragma unroll
-        for (int f = 0; f < 9; ++f) x[f] = blk[f * n];
+        for (int f = 0; f < 9; ++f)
+            if (fields >> f & 1u) x[f] = blk[f * n];
 #pragma unroll
-        for (int f = 0; f < 9; ++f) field[f][c] = x[f];
+        for (int f = 0; f < 9; ++f)
+            if (fields >> f & 1u) field[f][c] = x[f];
     }
 }
 
@@ -967,15 +972,16 @@ static __global__ void __launch_bounds__(256) engine_image_kernel(const EngineMe
                                                                   int gather)
 {
     for_member_items(table, prefix, tiles, kItemCells,
-                     [&](const EngineMember& M, int c) { image_cell(M, image + M.image_offset, c, gather); });
+                     [&](const EngineMember& M, int c) { image_cell(M, image + M.image_offset, c, gather, ~0u); });
 }
 
 // One member's image (its table entry by value, before or beside the table).
 static __global__ void __launch_bounds__(256) member_image_kernel(const __grid_constant__ EngineMember M,
-                                                                  float* __restrict__ image, int gather)
+                                                                  float* __restrict__ image, int gather,
+                                                                  unsigned fields)
 {
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < M.items[kItemCells]; c += gridDim.x * blockDim.x)
-        image_cell(M, image, c, gather);
+        image_cell(M, image, c, gather, fields);
 }
 
 // Pointer rotation after the acoustic loop (rho: with an odd substep count

@@ -114,3 +114,20 @@ def test_a_member_moves_within_its_own_memory():
     assert _pool_high_water() == held
     run.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("names", [("rho",), ("u",), ("w", "qr"), ("v", "theta", "qc")], ids="-".join)
+def test_history_of_some_fields_of_a_padded_member(names):
+    ctx = cuda.Context(0)
+    run = EngineRun(ctx)
+    for mid, st in _members(run, levels=(9, 10, 11)):
+        want = np.empty(9 * st["u"].size, np.float32)
+        run.engine.history_async(mid, cuda.HISTORY_CORE, want)
+        got = np.full(len(names) * st["u"].size, np.nan, np.float32)
+        run.engine.history_async(mid, cuda.history_mask(names), got)
+        run.engine.synchronize()
+        want, got = (x.reshape(-1, *st["u"].shape) for x in (want, got))
+        for k, frame in zip(names, got):
+            assert np.array_equal(frame.view(np.uint32), want[FIELDS.index(k)].view(np.uint32)), k
+    run.close()
+    ctx.close()

@@ -65,8 +65,11 @@ ArenaLayout arena_layout(const nimbus_member_desc* d)
     L.off_sf = off;     off += align_up(3 * kEngineScalars * L.cells * sizeof(float));
     L.off_rl = off;     off += align_up(kEngineScalars * L.cells * sizeof(float));
     L.off_q4 = off;     off += align_up(kEngineScalars * L.cells * sizeof(float));
-    L.off_k1 = off;     off += align_up(4 * L.cells * sizeof(float));
-    L.off_xs = off;     off += align_up(4 * L.cells * sizeof(float));
+    // The Heun pair's k1 and predictor are done with before transport forms its
+    // face fluxes, and lie in them: 36 values a cell instead of 44, which is
+    // more than the padding of columns of 14 levels and up adds.
+    L.off_k1 = L.off_sf;
+    L.off_xs = L.off_k1 + align_up(4 * L.cells * sizeof(float));
     L.off_eos = off;    off += field;
     L.off_status = off; off += kAlign;
     // Per-level tables, one entry a stored level.

@@ -52,7 +52,7 @@ struct __align__(16) EngineMember
     float *sf;        // [3][cells] float4 face fluxes (one lane per scalar)
     float *rl;        // [cells] float4 limiter factors
     float *q4;        // [cells] float4 theta, qv, qc, qr before transport (written by the slow predictor)
-    float *k1, *xs;   // [cells] float4 {u, v, w, p}: Heun k1 and predictor state
+    float *k1, *xs;   // [cells] float4 {u, v, w, p}: Heun k1 and predictor state (within sf)
     float *eos;       // EOS candidate pressure
     unsigned* status; // this member's status word (kStatus* bits)
     const double *rho0, *p0, *qv0, *u0, *v0;

@@ -7,6 +7,7 @@ import re
 import subprocess
 from pathlib import Path
 
+import numpy as np
 import pytest
 
 from nimbus_b200 import cuda
@@ -158,3 +159,16 @@ def test_engine_calls_make_their_device_current_before_they_enqueue():
             checked.append(m.group(1))
     assert {"nimbus_cuda_engine_read_async", "nimbus_cuda_engine_write_async", "nimbus_cuda_engine_admit",
             "nimbus_cuda_engine_step"} <= set(checked)
+
+
+def test_a_member_takes_no_more_memory_than_its_unpadded_cells():
+    """Columns are padded to a multiple of four levels; a member's footprint
+    stays within the 44 values a cell (and the tables and alignment) that one
+    without padding takes when no buffer serves twice."""
+    lib = cuda.load_library()
+    for nz in range(14, 81):
+        base = {k: np.ones(nz) for k in ("rho0", "p0", "qv0", "u0", "v0")}
+        desc = cuda.member_desc((23, 19, nz), (500.0, 500.0, 300.0), 3.0, 4, (1, 1, 1, 1, 1, 0), base)
+        cells, faces = 23 * 19 * nz, 2 * (23 + 19) * nz
+        bound = 4 * (44 * cells + faces) + 64 * nz + 26 * 256
+        assert 0 < lib.nimbus_cuda_engine_member_bytes(ctypes.byref(desc)) <= bound, nz

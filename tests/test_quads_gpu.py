@@ -140,3 +140,30 @@ def test_acoustic_loop_and_its_ring(ctx, shape, bc):
     for a, k in enumerate(("mfx", "mfy", "mfz")):
         _same(mf[a].cpu().numpy(), loop[k], k)
     _same(wave.cpu().numpy(), loop["wave"].astype(np.float32), "wave")
+
+
+@pytest.mark.parametrize("precision", [cuda.PRECISION_FP32, cuda.PRECISION_REFERENCE], ids=["fp32", "reference"])
+def test_members_of_a_crowded_lane_keep_their_bits(ctx, precision):
+    """A lane of more than 64 members takes the member-table forms of every
+    pass (one cell per thread), a smaller one the constant-bank forms (four
+    cells per thread in the FP32 slow pair, and in the acoustic passes of the
+    large member's lane): a member's result does not depend on which."""
+    shapes = [GRIDS[m % len(GRIDS)] for m in range(65)] + [(70, 67, 65)]
+    members = []
+    for m, shape in enumerate(shapes):
+        case = _case(shape, (OPEN, CHANNEL, WALLS)[m % 3], m)
+        members.append((case, *cloudy_state(case, seed=70 + m)))
+
+    def stepped(chosen):
+        run = EngineRun(ctx, precision=precision, lanes=1)
+        ids = [run.admit(*members[m], coriolis_f=1e-4, n_substeps=3 + m % 3) for m in chosen]
+        run.step(2)
+        out = {m: run.read(mid) for m, mid in zip(chosen, ids)}
+        run.close()
+        return out
+
+    together = stepped(range(len(members)))
+    apart = {**stepped(range(40)), **stepped(range(40, 65)), **stepped([65])}
+    for m, (case, _, _) in enumerate(members):
+        for k in FIELDS:
+            _same(together[m][k], apart[m][k], f"member {m} {case.shape} {k}")

@@ -20,6 +20,7 @@ pytestmark = [pytest.mark.gpu,
 
 OPEN, CHANNEL, WALLS = (1, 1, 1, 1, 1, 0), (0, 0, 0, 0, 0, 2), (2, 3, 4, 3, 0, 1)
 FIELDS = ("u", "v", "w", "rho", "p", "theta", "qv", "qc", "qr")
+QUAD_CELLS = 4 * 128 * 4 * 148  # stored cells from which the acoustic passes take groups of four
 # (nx, ny, nz): every nz mod 4 (2 and 3 are the shortest columns), the
 # narrowest members, 128-cell tiles that end inside a column.
 GRIDS = [(4, 4, 2), (5, 4, 3), (4, 7, 5), (9, 8, 6), (8, 11, 9), (13, 6, 12), (17, 19, 23), (12, 31, 41)]
@@ -42,15 +43,23 @@ def _case(shape, bc, m):
     return Case(nx, ny, nz, 900.0, 850.0, 20000.0 / max(nz, 20), 2.0, bc=bc, seed=11, member=m)
 
 
+@pytest.mark.parametrize("large", [None, (88, 87, 41)], ids=["one-cell", "quads"])
 @pytest.mark.parametrize("bc", [OPEN, CHANNEL, WALLS], ids=["open", "channel", "walls"])
-def test_engine_step_on_every_column_length(ctx, bc):
-    run = EngineRun(ctx, precision=cuda.PRECISION_REFERENCE)
+def test_engine_step_on_every_column_length(ctx, bc, large):
+    """Lanes below the size from which the acoustic passes take four cells a
+    thread, and one lane that a large member takes above it: the lane's total
+    decides, so the small members' columns go through the groups too, in every
+    substep (the large member has the most)."""
+    run = EngineRun(ctx, precision=cuda.PRECISION_REFERENCE, lanes=1 if large else None)
     cpu = oracle.Restatement("f32")
     members = []
-    for m, shape in enumerate(GRIDS):
+    for m, shape in enumerate(GRIDS + ([large] if large else [])):
         case = _case(shape, bc, m)
         st, base = cloudy_state(case, seed=20 + m)
-        members.append((run.admit(case, st, base, coriolis_f=1e-4, n_substeps=3 + m % 3), case, st, base, 3 + m % 3))
+        n = 6 if shape == large else 3 + m % 3
+        members.append((run.admit(case, st, base, coriolis_f=1e-4, n_substeps=n), case, st, base, n))
+    stored = sum(c.nx * c.ny * (-(-c.nz // 4) * 4) for _, c, _, _, _ in members)
+    assert (stored >= QUAD_CELLS) == bool(large)
     run.step(2)
     for mid, case, st, base, n in members:
         want = {k: v.copy() for k, v in st.items()}
@@ -94,10 +103,12 @@ def test_padded_state_moves_unchanged(ctx):
     run.close()
 
 
-@pytest.mark.parametrize("shape", [(66, 70, 64), (70, 67, 65), (37, 29, 45)], ids=["quads", "odd", "small"])
+@pytest.mark.parametrize("shape", [(68, 72, 64), (66, 70, 64), (70, 67, 65), (37, 29, 45)],
+                         ids=["quads", "just-below", "odd", "small"])
 def test_fp32_engine_equals_the_per_operation_path(ctx, shape):
-    """Both sides of the size from which groups are launched (303,104 cells),
-    and columns the per-operation path cannot group: the same FP32 bits."""
+    """Both sides of the size from which groups are launched (303,104 cells:
+    313,344 and 295,680), and columns the per-operation path cannot group
+    (318,920 stored cells in the engine): the same FP32 bits."""
     case = _case(shape, OPEN, 0)
     st, base = cloudy_state(case, seed=3)
     plain = ResidentRun(ctx, case, {k: v.copy() for k, v in st.items()}, base, precision=cuda.PRECISION_FP32,

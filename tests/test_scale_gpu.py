@@ -279,19 +279,22 @@ T, C, M, P2, B, CM = (cuda.ACOUSTIC_TABLE, cuda.ACOUSTIC_CONST, cuda.ACOUSTIC_MA
 FORM_MEMBERS = (0, 1, 5, 6)
 
 
-@pytest.mark.parametrize("forms,march", [((T, T), 16), ((M, M), 5), ((M, M), 1000), ((P2, P2), 16),
-                                         ((C, M), 16), ((P2, T), 7), ((T, P2), 16), ((B, B), 16), ((B, M), 16),
-                                         ((C, B), 16), ((CM, CM), 16), ((CM, M), 3), ((T, CM), 1000)],
-                         ids=["table", "march5", "whole-rows", "pair", "const-march", "pair-table", "table-pair",
-                              "bulk", "bulk-march", "const-bulk", "cmarch", "cmarch-march3", "table-cmarch-rows"])
-def test_engine_acoustic_kernel_form_does_not_change_results(ctx, multi_tile, forms, march):
+@pytest.mark.parametrize("forms,march,lanes", [((T, T), 16, 4), ((M, M), 5, 4), ((M, M), 1000, 4), ((P2, P2), 16, 4),
+                                               ((C, C), 16, 1), ((C, M), 16, 4), ((C, T), 7, 1), ((T, C), 16, 1),
+                                               ((B, B), 16, 4), ((B, M), 16, 4), ((C, B), 16, 4), ((CM, CM), 16, 4),
+                                               ((CM, M), 3, 4), ((T, CM), 1000, 4)],
+                         ids=["table", "march5", "whole-rows", "pair", "const-one-lane", "const-march", "const-table",
+                              "table-const", "bulk", "bulk-march", "const-bulk", "cmarch", "cmarch-march3",
+                              "table-cmarch-rows"])
+def test_engine_acoustic_kernel_form_does_not_change_results(ctx, multi_tile, forms, march, lanes):
     """The continuity and momentum passes in each kernel form (member table,
-    constant-bank parameters -- the default, covered above -- marching along x
-    over chunks of `march` planes, two cells per thread, or tiles staged in
-    shared memory by bulk copies), alone and mixed between the passes, give
-    the oracle's bits."""
+    constant-bank parameters, marching along x over chunks of `march` planes,
+    or tiles staged in shared memory by bulk copies), alone and mixed between
+    the passes, give the oracle's bits.  The constant-bank form takes four
+    cells per thread in the one lane of all members, and one or four in the
+    lane of each; PAIR is accepted and runs as it."""
     members, want = multi_tile
-    run = EngineRun(ctx, precision=cuda.PRECISION_REFERENCE)
+    run = EngineRun(ctx, precision=cuda.PRECISION_REFERENCE, lanes=lanes)
     if forms[0] == forms[1]:
         run.engine.set_acoustic_form(forms[0])
     else:
@@ -322,15 +325,19 @@ def fp32_const(ctx, multi_tile):
     return out
 
 
-@pytest.mark.parametrize("forms", [(T, T), (P2, P2), (P2, M), (C, P2), (M, M), (CM, CM), (B, B)],
-                         ids=["table", "pair", "pair-march", "const-pair", "march", "cmarch", "bulk"])
-def test_fp32_kernel_forms_give_the_same_bits(ctx, multi_tile, fp32_const, forms):
+@pytest.mark.parametrize("forms,lanes", [((T, T), 4), ((P2, P2), 4), ((C, C), 1), ((C, M), 4), ((C, T), 1),
+                                         ((M, M), 4), ((CM, CM), 4), ((B, B), 4)],
+                         ids=["table", "pair", "const-one-lane", "const-march", "const-table", "march", "cmarch",
+                              "bulk"])
+def test_fp32_kernel_forms_give_the_same_bits(ctx, multi_tile, fp32_const, forms, lanes):
     """In the FP32 form too, every acoustic kernel form gives the bits of the
     constant-bank default (the arithmetic is one sequence; the FP32 unit's FMA
     contraction must not differ between the forms), for members with odd and
-    even nz (the two-cell form's paired loads)."""
+    even nz.  The default run has one member a lane, the smallest of them
+    below the size from which the form takes four cells per thread; one lane
+    of all members is above it."""
     members, _ = multi_tile
-    run = EngineRun(ctx, precision=cuda.PRECISION_FP32)
+    run = EngineRun(ctx, precision=cuda.PRECISION_FP32, lanes=lanes)
     run.engine.set_pass_forms(*forms)
     ids = [run.admit(*members[i][:3], coriolis_f=1e-4) for i in FORM_MEMBERS]
     run.step(2)

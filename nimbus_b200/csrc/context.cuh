@@ -204,14 +204,19 @@ inline bool copied(nimbus_cuda_context* ctx, bool up, void* device, void* host, 
     if (at.type != cudaMemoryTypeUnregistered) return false;
     try
     {
-        if (!ctx->copier) ctx->copier = HostCopier::of_device(ctx->device, ctx->pageable >= HostCopier::kSetUpAfter);
+        if (!ctx->copier)
+        {
+            const bool make = ctx->pageable >= HostCopier::kSetUpAfter;
+            ctx->copier = HostCopier::of_device(ctx->device, make);
+            if (make && !ctx->copier) ctx->pageable = 0;  // tried again after as much more
+        }
     }
     catch (...)
     {
         return false;
     }
     ctx->pageable += bytes;
-    return ctx->copier && ctx->copier->ready() && ctx->copier->copy(up, device, host, bytes, ctx->stream, result);
+    return ctx->copier && ctx->copier->copy(up, device, host, bytes, ctx->stream, result);
 }
 
 inline nimbus_status upload(nimbus_cuda_context* ctx, void* dst, const void* src, size_t bytes)

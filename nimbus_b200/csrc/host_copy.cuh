@@ -85,7 +85,8 @@ public:
 
     bool ready() const { return ready_; }
 
-    // The device's copier; where no context holds one, a new one or null.
+    // The device's copier; where no context holds one, a new one or null (not
+    // asked for, or its set-up failed: then a later call may try again).
     static std::shared_ptr<HostCopier> of_device(int device, bool make)
     {
         static std::mutex mutex;
@@ -94,7 +95,12 @@ public:
         if (all.size() <= static_cast<size_t>(device)) all.resize(static_cast<size_t>(device) + 1);
         std::weak_ptr<HostCopier>& slot = all[static_cast<size_t>(device)];
         std::shared_ptr<HostCopier> c = slot.lock();
-        if (!c && make) slot = c = std::make_shared<HostCopier>(device);
+        if (!c && make)
+        {
+            c = std::make_shared<HostCopier>(device);
+            if (!c->ready()) return nullptr;
+            slot = c;
+        }
         return c;
     }
 

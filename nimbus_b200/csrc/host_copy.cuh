@@ -142,6 +142,10 @@ private:
     void serve(unsigned lane)
     {
         cudaSetDevice(device_);
+        // These threads capture nothing: whether a copy may run beside another
+        // thread's capture is for the calling thread's mode to say.
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
         unsigned long long seen = 0;
         for (;;)
         {

@@ -1,8 +1,8 @@
 """The host copier (csrc/host_copy.cuh) against a stand-in for the CUDA
-runtime, on the CPU: what its copies do around its piece size, and after a
-set-up that the runtime refused.  In the stand-in a transfer runs only when an
-event recorded behind it is waited for, or at the end, so a buffer that is
-written too early shows in the data."""
+runtime, on the CPU: what its copies do around its piece size, after a set-up
+that the runtime refused, and in which capture mode its threads wait.  In the
+stand-in a transfer runs only when an event recorded behind it is waited for,
+or at the end, so a buffer that is written too early shows in the data."""
 import shutil
 import subprocess
 from pathlib import Path
@@ -25,6 +25,8 @@ static std::mutex lock;
 static std::deque<std::pair<int, std::function<void()>>> queue;  // transfers, by their number
 static std::map<cudaEvent_t, int> recorded;
 static int enqueued = 0, refuse_pinned = 0;
+static thread_local cudaStreamCaptureMode mode = cudaStreamCaptureModeGlobal;
+static std::atomic<int> strict_waits{0};
 
 static void run_to(int number)
 {
@@ -58,6 +60,7 @@ cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t)
 cudaError_t cudaEventSynchronize(cudaEvent_t e)
 {
     std::lock_guard<std::mutex> g(lock);
+    if (mode != cudaStreamCaptureModeRelaxed) ++strict_waits;
     run_to(recorded[e]);
     return cudaSuccess;
 }
@@ -69,6 +72,7 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cu
 }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode* m) { std::swap(*m, mode); return cudaSuccess; }
 }
 
 using nimbus_host::HostCopier;
@@ -110,6 +114,13 @@ int main(int, char** argv)
     HostCopier c(0);
     EXPECT(c.ready());
     if (what == "sizes") sizes(c);
+    if (what == "mode")
+    {
+        cudaStreamCaptureMode relaxed = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&relaxed);  // as the caller chose for its own thread
+        sizes(c);
+        EXPECT(strict_waits == 0);
+    }
     return failures;
 }
 """
@@ -126,7 +137,7 @@ def program(tmp_path_factory):
     return folder / "copier"
 
 
-@pytest.mark.parametrize("what", ["sizes", "setup"])
+@pytest.mark.parametrize("what", ["sizes", "setup", "mode"])
 def test_copier(program, what):
     done = subprocess.run([program, what], capture_output=True, text=True, timeout=60)
     assert done.returncode == 0, done.stdout

@@ -1,7 +1,9 @@
 """Host-memory entry points around the size from which their copies are staged
-by several threads: arrays below it, of whole pieces, with a last piece of a
-few bytes, with more pieces than buffers, and two contexts copying at once,
-each against the same call on device memory, bit for bit."""
+by several threads, once a context has copied enough for them: arrays below
+it, of whole pieces, with a short last piece, with more pieces than buffers,
+and two contexts copying at once, each against the same call on device memory,
+bit for bit."""
+import os
 import threading
 from contextlib import closing
 
@@ -33,14 +35,32 @@ def _on_device(ctx, st):
     return {k: dev[k].cpu().numpy() for k in FIELDS}
 
 
-# 2^18 floats are four pieces, the smallest array that is staged so.
+def _threads():
+    return len(os.listdir("/proc/self/task"))
+
+
+def _warmed(ctx):
+    """Copies host arrays until the device's copier is set up: 64 MiB the
+    ordinary way, then a call that starts its threads.  No copier is held when
+    this is first called (every context of this file is closed), so the threads
+    are new."""
+    before = _threads()
+    st = _cloudy((96, 95, 61), 1)
+    for _ in range(5):  # ten copies of 2.1 MiB a call
+        ctx.check(ctx.kessler_step(cuda.kessler_args({k: v.copy() for k, v in st.items()}, 300.0, 4.0)))
+    return _threads() - before
+
+
+# 2^18 floats are four pieces, the smallest array that is staged so; the next
+# has a last piece of 8,880 bytes, the last more pieces than there are buffers.
 @pytest.mark.parametrize("shape", [(64, 64, 63), (64, 64, 64), (43, 53, 116), (96, 95, 61)],
                          ids=["below", "pieces", "tail", "more"])
 def test_host_arrays_give_the_device_result(shape):
     with closing(cuda.Context(0)) as ctx:
+        assert _warmed(ctx) == min(4, os.cpu_count()) - 1
         st = _cloudy(shape, 5)
         want = _on_device(ctx, st)
-        for _ in range(5):  # the first ones go the ordinary way while the copier is set up
+        for _ in range(3):
             got = {k: v.copy() for k, v in st.items()}
             ctx.check(ctx.kessler_step(cuda.kessler_args(got, 300.0, 4.0)))
             for k in FIELDS:
@@ -48,24 +68,30 @@ def test_host_arrays_give_the_device_result(shape):
 
 
 def test_two_contexts_copy_at_once():
+    """Both hold the device's copier, and the one that finds it busy copies the
+    ordinary way."""
     shape = (96, 95, 61)
     states = [_cloudy(shape, 7 + t) for t in range(2)]
     with closing(cuda.Context(0)) as ctx:
         want = [_on_device(ctx, st) for st in states]
     got = [None, None]
+    together = threading.Barrier(2)
+    with closing(cuda.Context(0)) as holder:
+        assert _warmed(holder) == min(4, os.cpu_count()) - 1
 
-    def work(t):
-        with closing(cuda.Context(0)) as ctx:
-            for _ in range(4):
-                mine = {k: v.copy() for k, v in states[t].items()}
-                ctx.check(ctx.kessler_step(cuda.kessler_args(mine, 300.0, 4.0)))
-            got[t] = mine
+        def work(t):
+            with closing(cuda.Context(0)) as ctx:
+                together.wait(60)
+                for _ in range(8):
+                    mine = {k: v.copy() for k, v in states[t].items()}
+                    ctx.check(ctx.kessler_step(cuda.kessler_args(mine, 300.0, 4.0)))
+                got[t] = mine
 
-    threads = [threading.Thread(target=work, args=(t,)) for t in range(2)]
-    for t in threads:
-        t.start()
-    for t in threads:
-        t.join(60)
+        threads = [threading.Thread(target=work, args=(t,)) for t in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join(60)
     for t in range(2):
         for k in FIELDS:
             _same(got[t][k], want[t][k], f"{t} {k}")

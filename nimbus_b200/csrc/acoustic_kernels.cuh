@@ -357,7 +357,7 @@ __device__ __forceinline__ bool bc_inner_column(const Dims& d, int i, int j)
 
 // The closure is independent from level to level except for the top level,
 // which takes the one below: a cluster of one to eight CTAs closes a band of
-// four levels (the last one up to seven) all around the member, with a cluster
+// four levels (the last one up to five) all around the member, with a cluster
 // barrier between the reference's steps W,E -> S,N -> vertical instead of a
 // launch.  A ring is a few thousand values, so its time is the latency of its
 // chain of loads and stores; the cluster spreads a long ring over more SMs.

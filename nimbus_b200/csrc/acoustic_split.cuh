@@ -1,5 +1,6 @@
-// Two-launch acoustic substep (one thread per cell, grid-stride), templated on
-// the precision policy of acoustic_fused.cuh:
+// Two-launch acoustic substep, templated on the precision policy of
+// acoustic_fused.cuh; one thread per cell (grid-stride), marching along x, or
+// four vertically adjacent cells per thread (from kQuadCells on):
 //   split_continuity_eos : retained mass flux from the old state, continuity,
 //                          rho forward Euler, EOS; new rho to a ping-pong
 //                          buffer, p in place.
@@ -700,9 +701,11 @@ constexpr int kQuadCtas = sizeof(typename Policy::real) == 4 ? 8 : 7;
 
 // Cells from which the quad kernels are launched: below, a cell per thread
 // fills the SMs better than the quad saves instructions (four CTAs of quads an
-// SM on 148 SMs).  A launch of 164 thousand cells, continuity, us between
-// events: FP32 8.4 against 8.6 with quads, reference precision 10.7 / 12.6;
-// of 1.4 million, 19.5 / 18.6 and 33.2 / 30.9.
+// SM on the B200's 148 SMs).  The line lies between those of the two precisions;
+// a substep of the per-operation loop, us with quads / one cell per thread:
+// FP32 164 thousand cells 14.0 / 13.5, 207 15.1 / 15.5, 310 17.1 / 17.4, 1024
+// 25.4 / 30.2; reference precision 207 18.1 / 17.3, 310 21.0 / 20.5, 369
+// 20.9 / 20.8, 433 22.8 / 23.6, 1024 32.9 / 38.2.
 constexpr long long kQuadCells = 4LL * kQuadBlock * 4 * 148;
 
 template <class Policy>

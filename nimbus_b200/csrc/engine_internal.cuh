@@ -194,11 +194,13 @@ long long tiles_of(const nimbus_engine* e, const nimbus_engine_detail::Lane& L, 
     return e->prefix[L.prefix_first + static_cast<size_t>(kind) * (L.members + 1) + members];
 }
 
-// Whether a lane's kernels start early (launch_after): a small lane alone on
-// the GPU, whose step is a chain of launches of a few microseconds (32x32x40
-// member 0.137 -> 0.128 ms a step).  Long kernels gain nothing from it (5.2
-// million cells 1.424 -> 1.428 ms), and beside other lanes the waiting CTAs
-// would hold the room that those lanes' kernels fill.
+// Whether a lane's kernels start early (launch_after): a small lane, alone in
+// its engine, whose step is a chain of launches of a few microseconds (32x32x40
+// member 0.137 -> 0.133 ms a step).  Long kernels gain nothing from it (5.2
+// million cells 1.424 -> 1.428 ms).  Other engines on the device do not speak
+// against it: engines of one 64x64x40 member each, stepping at once, two 0.212
+// -> 0.218 ms, four 0.355 -> 0.321, eight 0.634 -> 0.556; eight of 32x32x40
+// 0.250 -> 0.261, of four such members each 0.657 -> 0.580.
 inline bool starts_early(const nimbus_engine* e, const nimbus_engine_detail::Lane& L)
 {
     return e->lanes.size() == 1 && tiles_of(e, L, kItemCells, L.members) * kEngineBlock < kQuadCells;

@@ -1,9 +1,9 @@
 // Batched kernels of the member engine: one launch per phase advances that
 // phase for every resident member.
 //
-// Work layout.  Each phase has an item kind (cells, west/east boundary rows,
-// south/north rows, columns, KW78 history slots).  A member's items are cut
-// into tiles of one block (blockDim.x items) and the members' tiles are laid
+// Work layout.  Each phase has an item kind (ItemKind: cells, groups of four
+// cells, columns, rows along x, bands of levels of the boundary ring).  A
+// member's items are cut into tiles of one block and the members' tiles are laid
 // end to end; prefix[kind][m] is the first tile of member m.  A persistent
 // grid (a few CTAs per SM) strides over the tiles, so the member of a tile is
 // uniform across its block and the per-member parameters are warp-broadcast

@@ -808,8 +808,7 @@ __device__ __forceinline__ void slow_predict_quad(
     }
 }
 
-// k2 at the predictor, the Heun average and its application; the averaged
-// tendencies to `out` (four planes) when given.
+// k2 at the predictor, the Heun average and its application.
 __device__ __forceinline__ void slow_correct_quad(
     const SlowParams& S, const float* __restrict__ xs, const float* __restrict__ rho, const float* __restrict__ qv,
     const float* __restrict__ qc, const float* __restrict__ qr, const double* __restrict__ rho0,

@@ -71,6 +71,36 @@ def test_slow_tendencies_around_an_infinite_wind(ctx, field, sign):
         assert off.max() <= 1e-5, (k, off.max(), np.argwhere(off > 1e-5)[:4].tolist())
 
 
+@pytest.mark.parametrize("sign", [1.0, -1.0], ids=["ahead", "behind"])
+@pytest.mark.parametrize("axis,field", [(0, "u"), (1, "v"), (2, "w")])
+def test_slow_tendencies_behind_a_huge_wind(ctx, axis, field, sign):
+    """One wind of 1e38 m/s, two and three cells downwind: the first enters the
+    derivative three times, the second not at all, and no sum on the way
+    overflows that the tendency does not.  The tendencies (up to 1e36) agree
+    with reference precision to a few roundings (1e-6 of the value; 1e-5 is
+    allowed, and 1e-5 as beside an infinite wind)."""
+    shape, at = (17, 16, 18), np.array((8, 8, 9))
+    case = Case(*shape, 500.0, 450.0, 300.0, 2.0, seed=4)
+    st, base = perturbed_state(case, seed=4)
+    rng = np.random.default_rng(9)
+    for k, mean in (("u", 10.0), ("v", 8.0), ("w", 4.0)):
+        st[k] = (sign * mean + rng.uniform(-2, 2, shape)).astype(np.float32)
+    st[field][tuple(at)] = 1e38
+    got = []
+    for precision in (cuda.PRECISION_FP32, cuda.PRECISION_REFERENCE):
+        ctx.set_precision(precision)
+        outs = [np.zeros(shape, np.float32) for _ in range(4)]
+        ctx.check(ctx.slow_tendencies(cuda.slow_args(st, base, (case.dx, case.dy, case.dz), outputs=outs)))
+        got.append(outs[axis])
+    ctx.set_precision(cuda.PRECISION_FP32)
+    for away in (2, 3):
+        cell = at.copy()
+        cell[axis] -= int(sign) * away
+        mine, want = (float(g[tuple(cell)]) for g in got)
+        assert (abs(want) > 1e34) == (away == 2)
+        assert abs(mine - want) <= 1e-5 * abs(want) + 1e-5, (away, mine, want)
+
+
 def _weno_offsets(v, real, fma):
     """The normalised WENO5-JS offset from the donor v[2], every weight by its
     own reciprocal, in `real` arithmetic with a fused multiply-add."""

@@ -546,8 +546,9 @@ __device__ __forceinline__ float update_value(const TP& T, bool pd, float fxp, f
             // What leaves through the faces carries this cell's factor, what
             // comes in the neighbour's: the flux's positive part and the
             // exact rest (a non-finite flux leaves a non-finite rest).  No
-            // branch and no selection: 24 members of 16.5 million cells, ten
-            // steps 3.63 -> 3.48 ms.
+            // branch: 24 members of 16.5 million cells, ten steps 3.63 -> 3.48
+            // ms.  A neighbour that gives nothing does not count, whatever its
+            // factor (a density of -infinity makes it infinite).
             const float zt = has_top ? fzp : 0.0f, zb = has_bottom ? fzm : 0.0f;
             const float xa = fmaxf(fxp, 0.0f), xb = fmaxf(fxm, 0.0f);
             const float ya = fmaxf(fyp, 0.0f), yb = fmaxf(fym, 0.0f);
@@ -561,7 +562,9 @@ __device__ __forceinline__ float update_value(const TP& T, bool pd, float fxp, f
                 return __fmaf_rn(lo, r_lo, -__fmul_rn(hi, r_hi));
             };
             const float outgoing = __fmul_rn(rc, through(xa - xout, ya - yout, za - zout));
-            const float incoming = through(into(xb, rxm, xin, rxp), into(yb, rym, yin, ryp), into(zc, rzm, zin, rzp));
+            const float incoming = through(into(xb, xb > 0.0f ? rxm : 0.0f, xin, xin < 0.0f ? rxp : 0.0f),
+                                           into(yb, yb > 0.0f ? rym : 0.0f, yin, yin < 0.0f ? ryp : 0.0f),
+                                           into(zc, zc > 0.0f ? rzm : 0.0f, zin, zin < 0.0f ? rzp : 0.0f));
             // rho_b q is not rounded on its own: it is the largest term, and where
             // nearly all of it leaves its rounding would be the result's error
             // (rounded first, the update is a tenth farther from 64 bits).

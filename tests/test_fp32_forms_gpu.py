@@ -41,6 +41,37 @@ def test_update_of_a_nearly_emptied_cell(ctx, left):
     assert off.max() <= 4 * 2.0 ** -23, off.max()
 
 
+@pytest.mark.parametrize("way", [1.0, -1.0], ids=["west-outflow", "west-inflow"])
+def test_update_beside_a_density_that_is_not_finite(ctx, way):
+    """A boundary cell whose old density is -infinity and that gives to another
+    boundary cell has a limiter factor that is not finite.  The cell beside it loses its value if it takes from there,
+    and keeps it if it gives: to a few roundings of reference precision
+    (1e-5 is allowed)."""
+    shape, edge = (9, 8, 10), (0, 4, 5)
+    rng = np.random.default_rng(6)
+    q = rng.uniform(1e-3, 1e-2, shape).astype(np.float32)
+    rho = rng.uniform(0.8, 1.0, shape).astype(np.float32)
+    begin = rho.copy()
+    begin[edge] = -np.inf
+    zero = np.zeros(shape, np.float32)
+    mfx, mfy = np.full(shape, -5.0 * way, np.float32), zero.copy()
+    mfy[edge] = 2.0
+    got, codes = [], []
+    for precision in (cuda.PRECISION_FP32, cuda.PRECISION_REFERENCE):
+        ctx.set_precision(precision)
+        out = np.zeros(shape, np.float32)
+        codes.append(ctx.scalar_transport(cuda.transport_args([q], [out], [1], rho, begin, mfx, mfy, zero, 2.0,
+                                                              (500.0, 500.0, 300.0))))
+        got.append(out)
+    ctx.set_precision(cuda.PRECISION_FP32)
+    assert codes[0] == codes[1]
+    if way > 0:
+        assert codes[0] == 0
+        np.testing.assert_allclose(got[0][1:-1, 1:-1], got[1][1:-1, 1:-1], rtol=1e-5)
+    else:
+        assert codes[0] != 0
+
+
 @pytest.mark.parametrize("sign", [1.0, -1.0], ids=["ahead", "behind"])
 @pytest.mark.parametrize("field", ["u", "v", "w"])
 def test_slow_tendencies_around_an_infinite_wind(ctx, field, sign):

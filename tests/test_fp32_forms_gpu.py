@@ -2,6 +2,7 @@
 one rounding or one stencil point each."""
 import numpy as np
 import pytest
+import torch
 
 from nimbus_b200 import cuda
 from nimbus_b200.initial import Case, perturbed_state
@@ -70,6 +71,27 @@ def test_update_beside_a_density_that_is_not_finite(ctx, way):
         np.testing.assert_allclose(got[0][1:-1, 1:-1], got[1][1:-1, 1:-1], rtol=1e-5)
     else:
         assert codes[0] != 0
+
+
+def test_update_takes_in_an_infinite_scalar(ctx):
+    """What flows in from an infinite value on the boundary is infinite, not
+    undefined, as in reference precision (the step's rain evaporates by it)."""
+    shape, edge = (9, 8, 10), (0, 4, 5)
+    rng = np.random.default_rng(6)
+    q = rng.uniform(1e-3, 1e-2, shape).astype(np.float32)
+    q[edge] = np.inf
+    rho = rng.uniform(0.8, 1.0, shape).astype(np.float32)
+    q, rho, mfx, zero = (torch.from_numpy(x).cuda() for x in (q, rho, np.full(shape, 5.0, np.float32),
+                                                             np.zeros(shape, np.float32)))
+    for precision in (cuda.PRECISION_REFERENCE, cuda.PRECISION_FP32):
+        ctx.set_precision(precision)
+        out = torch.zeros(shape, device="cuda")
+        torch.cuda.synchronize()
+        ctx.check(ctx.scalar_transport(cuda.transport_args([q], [out], [1], rho, rho, mfx, zero, zero, 2.0,
+                                                           (500.0, 500.0, 300.0), memory=cuda.MEMORY_DEVICE)))
+        with pytest.raises(RuntimeError, match="NONFINITE"):
+            ctx.synchronize()
+        assert out[1, 4, 5] == np.inf, precision
 
 
 @pytest.mark.parametrize("sign", [1.0, -1.0], ids=["ahead", "behind"])

@@ -144,13 +144,13 @@ __device__ __forceinline__ void for_member_rows(const EngineMember* __restrict__
 
 // Resident CTAs per SM of the slow Heun pair: the reference-precision form at
 // 4 of 256 threads (64 registers; four steps of 3.0 million cells at 3 / 4 / 5:
-// 1.60 / 1.41 / 1.72 ms), the FP32 form at 6 of kQuadTile threads (80; ten steps
-// of 24 members, 16.5 million cells, at 4 / 5 / 6: 10.4 / 9.44 / 9.27 ms).
+// 1.60 / 1.41 / 1.72 ms), the FP32 form at 5 of kQuadTile threads (96; ten steps of
+// 24 members, 17.4 million cells, at 5 / 6 / 7: 9.77 / 9.86 / 9.81 ms).
 #ifndef NIMBUS_SLOW_MINB
 #define NIMBUS_SLOW_MINB 4
 #endif
 #ifndef NIMBUS_SLOW_MINB_F32
-#define NIMBUS_SLOW_MINB_F32 6
+#define NIMBUS_SLOW_MINB_F32 5
 #endif
 template <class Policy>
 static __global__ void __launch_bounds__(256, 4) engine_slow_predict_kernel(const EngineMember* __restrict__ table,
@@ -1022,8 +1022,8 @@ static __global__ void engine_swap_kernel(EngineMember* table, int members, int 
 
 template <bool kFp32>
 // Resident CTAs per SM of the face-flux pass: the FP32 form at 5 (48
-// registers; ten steps of 24 members, 16.5 million cells, at 3 / 4 / 5 / 6:
-// 6.09 / 5.27 / 4.97 / 5.22 ms), the reference-precision form at 4 (64; four
+// registers; ten steps of 24 members, 17.4 million cells, at 4 / 5 / 6: 5.68 /
+// 5.38 / 5.59 ms), the reference-precision form at 4 (64; four
 // steps of 3.0 million cells at 2 / 3 / 4 / 5: 1.14 / 0.94 / 0.88 / 0.93 ms).
 #ifndef NIMBUS_FACES_MINB
 #define NIMBUS_FACES_MINB 4
@@ -1135,8 +1135,8 @@ static __global__ void __launch_bounds__(256, kFp32 ? NIMBUS_LIMITER_MINB_F32 : 
 }
 
 // Of the update: both at 3, since the loads of a cell's six faces for four
-// scalars are in flight together (FP32 2 / 3 / 4 / 5: 3.55 / 2.91 / 3.49 / 5.41
-// ms; reference precision 2 / 3 / 4: 0.42 / 0.35 / 0.41).
+// scalars are in flight together (FP32 2 / 3 / 4: 3.83 / 3.12 / 3.63 ms;
+// reference precision 2 / 3 / 4: 0.42 / 0.35 / 0.41).
 #ifndef NIMBUS_UPDATE_MINB_F32
 #define NIMBUS_UPDATE_MINB_F32 3
 #endif

@@ -20,6 +20,7 @@
 #include <vector>
 
 #include <cuda_runtime.h>
+#include <pthread.h>
 
 namespace nimbus_host
 {
@@ -141,6 +142,7 @@ private:
 
     void serve(unsigned lane)
     {
+        pthread_setname_np(pthread_self(), "nimbus-copy");
         cudaSetDevice(device_);
         // These threads capture nothing: whether a copy may run beside another
         // thread's capture is for the calling thread's mode to say.
